@@ -122,10 +122,10 @@ int pc_setup_layout(pc_handle* h, int fs, int buffer_size, int n_in, int n_out, 
 int pc_set_relaxed(pc_handle* h, int relaxed);
 
 /*
- * Offline throughput option, no reference counterpart: compute k base blocks
- * per step (k a power of two, 1..8; call before setup; up to 4 are used).  Each step's
- * level-0 work for all PCs is one launch that transforms and convolves k
- * consecutive blocks at once, and every larger level runs beside the steps.
+ * Throughput option for calls of a few blocks, no reference counterpart:
+ * compute k base blocks per step (k a power of two, 1..8; call before setup;
+ * up to 4 are used).  Each step's level-0 work for all PCs is one launch that
+ * transforms and convolves k consecutive blocks at once.
  * The output equals that of k times as many one-block steps to float32
  * rounding (the same partitions and products, summed in another order).
  * Setup lowers k to the largest value the layouts allow (k buffer_size <=
@@ -159,7 +159,9 @@ int pc_run(pc_handle* h, float* output, const float* input, int frame_count);
  * Batched form of run(): frames (a multiple of buffer_size) are processed as
  * frames/buffer_size consecutive callbacks with results identical to that
  * many pc_run calls.  Host buffers in the given layout (PC_INTERLEAVED or
- * PC_PLANAR with row length frames).  Steps run as CUDA-graph replays.
+ * PC_PLANAR with row length frames).  Calls of more than a few blocks run
+ * block-parallel: whole chunks of callbacks per launch, bit for bit the
+ * results of pc_run.
  * No reference counterpart (the reference has only run()).
  */
 int pc_process(pc_handle* h, float* output, const float* input, long long frames, int layout);

@@ -33,6 +33,7 @@
 #include "engine_types.h"
 #include "fft_smem.cuh"
 #include "kernels.h"
+#include "wide.h"
 
 namespace cg = cooperative_groups;
 
@@ -169,8 +170,7 @@ __device__ __forceinline__ void setup_geo(Geo& g, int N, const float2* W, int wl
 
 // One fire per cluster: task blockIdx.x / 8 of this launch.
 __global__ void __cluster_dims__(kC, 1, 1) __launch_bounds__(kNT)
-    cluster_fire_kernel(Bank bank, const Task* __restrict__ tasks, RunState rs_val, const RunState* rs_dev,
-                        int step_in_batch) {
+    cluster_fire_kernel(Bank bank, const Task* __restrict__ tasks, RunState rs_val) {
     extern __shared__ float4 dyn_smem[];
     __shared__ __align__(16) Task tk;
     __shared__ __align__(16) RunState rs;
@@ -178,13 +178,8 @@ __global__ void __cluster_dims__(kC, 1, 1) __launch_bounds__(kNT)
     cudaTriggerProgrammaticLaunchCompletion();
     const int tid = threadIdx.x;
     const int ti = blockIdx.x / kC;
-    if (tid < 12) {
-        reinterpret_cast<int4*>(&tk)[tid] = __ldg(reinterpret_cast<const int4*>(tasks + ti) + tid);
-    } else if (tid >= 32 && tid < 37) {
-        const int j = tid - 32;
-        if (rs_dev) reinterpret_cast<int4*>(&rs)[j] = __ldcg(reinterpret_cast<const int4*>(rs_dev) + j);
-    }
-    if (!rs_dev && tid == 64) rs = rs_val;
+    if (tid < kTaskVec) reinterpret_cast<int4*>(&tk)[tid] = __ldg(reinterpret_cast<const int4*>(tasks + ti) + tid);
+    if (tid == 64) rs = rs_val;
     float2* S = reinterpret_cast<float2*>(dyn_smem);
     float2* twt = S + kMaxM;
     __syncthreads();
@@ -194,7 +189,7 @@ __global__ void __cluster_dims__(kC, 1, 1) __launch_bounds__(kNT)
 #pragma unroll
     for (int r = 0; r < 8; ++r) rem[r] = cl.map_shared_rank(S, r);
 
-    long long c = rs.step_base + step_in_batch;
+    long long c = rs.step_base;
     const long long io_step = c - rs.io.step0;
     c -= tk.origin;
     const int N = tk.N, P = tk.P, cs = tk.cs, N0 = bank.N0;
@@ -234,9 +229,10 @@ __global__ void __cluster_dims__(kC, 1, 1) __launch_bounds__(kNT)
     const bool two = dfer;
     const bool use_x1 = two && P >= 2;
     const bool use_yp = (two && P >= 3) || (!two && P >= 2);
-    const int slot = (int)(((b % P) + P) % P);
+    const int R = tk.slots;
+    const int slot = (int)(((b % R) + R) % R);
     float2* Xs = tk.X + (size_t)slot * cs;
-    const float2* X1 = tk.X + (size_t)((((b - 1) % P) + P) % P) * cs;
+    const float2* X1 = tk.X + (size_t)((((b - 1) % R) + R) % R) * cs;
     const float2* Ypb = tk.Yp + (two ? (size_t)(b & 1) * cs : 0);
     const int npart = tk.k0 > 0 ? tk.k0 : 1;
     const size_t rstride = 2 * (size_t)cs;
@@ -285,6 +281,86 @@ __global__ void __cluster_dims__(kC, 1, 1) __launch_bounds__(kNT)
         const long long t0 = b * (long long)N + 2LL * g.rank * g.m;
         for (int j2 = tid; j2 < g.m; j2 += kNT)
             *reinterpret_cast<float2*>(tk.yring + ((t0 + 2 * j2) & tk.rmask)) = S[sidx<true>(j2)];
+    }
+}
+
+// Block-parallel processing (wide.cu): the forward half of a fire -- window,
+// transform, spectrum row -- or its inverse half -- summed spectrum, inverse
+// transform, output ring -- of one block per cluster, with the operations of
+// cluster_fire_kernel in the same order.
+template <bool INV>
+__global__ void __cluster_dims__(kC, 1, 1) __launch_bounds__(kNT)
+    wide_cluster_kernel(const int2* __restrict__ map, WArgs a) {
+    extern __shared__ float4 dyn_smem[];
+    cg::cluster_group cl = cg::this_cluster();
+    const int tid = threadIdx.x;
+    const int2 e = map[blockIdx.x / kC];
+    const WLevel& l = a.lv[e.x];
+    const long long b0 = (a.c0 + l.s_blocks) >> l.logT;
+    const int nb = (int)(((a.c0 + a.nsteps + l.s_blocks) >> l.logT) - b0);
+    if (e.y >= nb) return;   // the whole cluster
+    const long long b = b0 + e.y;
+    const int N = l.N;
+    float2* S = reinterpret_cast<float2*>(dyn_smem);
+    float2* twt = S + kMaxM;
+    Geo g;
+    setup_geo(g, N, a.W, a.wlog, twt);
+    float2* rem[8];
+#pragma unroll
+    for (int r = 0; r < 8; ++r) rem[r] = cl.map_shared_rank(S, r);
+    const Twiddles tw{twt, g.logm};
+    const int np = pair_count(g);
+    if constexpr (!INV) {
+        const long long t_end = (b + 1) * (long long)N - (long long)l.s_blocks * a.N0;
+        const long long w0 = t_end - 2LL * N, t_in0 = a.io.step0 * (long long)a.N0;
+        const float* in = a.io.in + (long long)l.in_ch * a.io.in_ch;
+        const long long isamp = a.io.in_sample;
+        for (int j2 = tid; j2 < g.m; j2 += kNT) {
+            const long long ta = w0 + 2LL * (g.rank * (long long)g.m + j2);
+            float2 v;
+            if (ta >= t_in0) {
+                const float* p = in + (ta - t_in0) * isamp;
+                v = make_float2(p[0] * l.scale, p[isamp] * l.scale);
+            } else {
+                v = __ldcg(reinterpret_cast<const float2*>(l.xring + (ta & l.rin_mask)));
+            }
+            S[sidx<true>(j2)] = v;
+        }
+        cl.sync();
+        column_pass_fwd(g, rem, cl);
+        fft_smem<kNT, kMaxB, true>(S, g.m, g.logm, tw, false);
+        cl.sync();
+        float2* Xs = l.X + (size_t)(((b % l.slots) + l.slots) % l.slots) * l.cs;
+        for (int pi = tid; pi < np; pi += kNT) {
+            const Pair pq = pair_at(g, pi);
+            const float2 zk = S[sidx<true>(pq.k2)];
+            const bool self = (pq.nk == pq.k);
+            const float2 znk = (pq.k == 0 || self) ? zk : rem[pq.pr][sidx<true>(pq.pk2)];
+            float2 xk, xnk;
+            split_pair(g, zk, znk, pq.k, xk, xnk);
+            Xs[bin_pos(g, pq.k)] = xk;
+            if (!self) Xs[bin_pos(g, pq.nk)] = xnk;
+        }
+        cl.sync();   // no CTA leaves while others may still read its shared memory
+    } else {
+        const float2* Y = l.Yw + (size_t)e.y * l.cs;
+        cl.sync();   // every CTA of the cluster runs before its shared memory is written
+        for (int pi = tid; pi < np; pi += kNT) {
+            const Pair pq = pair_at(g, pi);
+            float2 zk, znk;
+            merge_pair(g, __ldcg(&Y[bin_pos(g, pq.k)]), __ldcg(&Y[bin_pos(g, pq.nk)]), pq.k, zk, znk);
+            S[sidx<true>(pq.k2)] = zk;
+            if (pq.k != 0 && pq.nk != pq.k) rem[pq.pr][sidx<true>(pq.pk2)] = znk;
+        }
+        cl.sync();
+        fft_smem<kNT, kMaxB, true>(S, g.m, g.logm, tw, true);
+        cl.sync();
+        column_pass_inv(g, rem, cl);
+        if (g.rank < kC / 2) {
+            const long long t0 = b * (long long)N + 2LL * g.rank * g.m;
+            for (int j2 = tid; j2 < g.m; j2 += kNT)
+                *reinterpret_cast<float2*>(l.yring + ((t0 + 2 * j2) & l.rmask)) = S[sidx<true>(j2)];
+        }
     }
 }
 
@@ -425,8 +501,19 @@ cudaError_t prepare_cluster_kernels() {
     e = cudaFuncSetAttribute(cluster_filter_level_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)cluster_smem_bytes());
     if (e != cudaSuccess) return e;
+    for (auto fn : {wide_cluster_kernel<false>, wide_cluster_kernel<true>}) {
+        e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cluster_smem_bytes());
+        if (e != cudaSuccess) return e;
+    }
     return cudaFuncSetAttribute(cluster_spectra_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)cluster_smem_bytes());
+}
+
+cudaError_t launch_wide_cluster(bool inverse, int grid, const int2* map, const WArgs& a, cudaStream_t st) {
+    if (grid <= 0) return cudaSuccess;
+    if (inverse) wide_cluster_kernel<true><<<grid * kC, kNT, cluster_smem_bytes(), st>>>(map, a);
+    else wide_cluster_kernel<false><<<grid * kC, kNT, cluster_smem_bytes(), st>>>(map, a);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_cluster_filter_level(int N, int P, int cs, unsigned bcurr, const float2* H, float2* X,
@@ -437,31 +524,20 @@ cudaError_t launch_cluster_filter_level(int N, int P, int cs, unsigned bcurr, co
     return cudaGetLastError();
 }
 
-cudaError_t launch_cluster_fire(int ntasks, const Bank& bank, const Task* tasks, const RunState& rs,
-                                const RunState* rs_dev, int step_in_batch, cudaStream_t st, bool pdl, int prio) {
+cudaError_t launch_cluster_fire(int ntasks, const Bank& bank, const Task* tasks, const RunState& rs, cudaStream_t st,
+                                bool pdl) {
     if (ntasks <= 0) return cudaSuccess;
-    static int least = 0, greatest = 0;
-    static const bool have_range = cudaDeviceGetStreamPriorityRange(&least, &greatest) == cudaSuccess;
-    cudaLaunchAttribute attr[2];
-    int na = 0;
-    if (pdl) {
-        attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[na].val.programmaticStreamSerializationAllowed = 1;
-        ++na;
-    }
-    if (prio != 0 && have_range) {
-        attr[na].id = cudaLaunchAttributePriority;
-        attr[na].val.priority = prio > 0 ? greatest : least;
-        ++na;
-    }
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(ntasks * kC);
     cfg.blockDim = dim3(kNT);
     cfg.dynamicSmemBytes = cluster_smem_bytes();
     cfg.stream = st;
     cfg.attrs = attr;
-    cfg.numAttrs = na;
-    return cudaLaunchKernelEx(&cfg, cluster_fire_kernel, bank, tasks, rs, rs_dev, step_in_batch);
+    cfg.numAttrs = pdl ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, cluster_fire_kernel, bank, tasks, rs);
 }
 
 cudaError_t launch_cluster_spectra(int njobs, const SpectraJob* jobs, const float2* W, int wlog, cudaStream_t st) {

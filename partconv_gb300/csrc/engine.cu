@@ -8,15 +8,14 @@
 // workers become a static per-phase task table: the level schedule repeats
 // every H = max_L N_L / N0 base steps, so for each phase and kernel class the
 // host lists the level blocks that fire and the MAC slices spread over the
-// steps between a level's blocks.  A base step is one launch per kernel
-// class that has work in that phase (level 0 fires every step, so its class
-// always runs); batches of steps replay a captured CUDA graph whose nodes
-// have their phase baked in.
+// steps between a level's blocks.  A base step (one callback) is one launch
+// per kernel class that has work in that phase (level 0 fires every step, so
+// its class always runs).  A call of many steps runs block-parallel instead
+// (wide.cu): whole chunks of steps per launch, with the same results.
 #include <cuda_runtime.h>
 
 #include <algorithm>
 #include <map>
-#include <tuple>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -27,15 +26,24 @@
 
 #include "../../include/partconv_gb300.h"
 #include "engine_types.h"
+#include "fft_reg.cuh"
 #include "io.h"
 #include "kernels.h"
+#include "wide.h"
 
 using namespace pcg;
 
 namespace {
 
 constexpr int kWlog = 17;          // twiddle table 2^17 entries: real FFTs up to 2 * 65536
-constexpr int kMinGraphSteps = 128;   // base steps per captured graph (a multiple of the hyperperiod)
+// Calls of at least this many base steps run block-parallel (wide.cu).
+constexpr int kWideMinSteps = 8;
+// Base steps per block-parallel chunk: as many as keep the chunk's spectra
+// (one ring row per block of every level) within kWideBytes, so that they and
+// the summed spectra, as many again, are still in the 129 MB L2 when the next
+// kernel reads them.
+constexpr size_t kWideBytes = (size_t)32 << 20;
+constexpr int kWideMinChunk = 32, kWideMaxChunk = 4096;
 constexpr int kMinN0 = 16;
 constexpr int kClasses = kNumClasses;
 
@@ -136,8 +144,6 @@ struct pc_handle {
     bool ready = false;
     int device = -1;
     cudaStream_t stream = nullptr;
-    cudaStream_t side[kClasses] = {};    // graph-capture branches
-    cudaStream_t aside[kClasses] = {};   // deferred fires (graph capture)
     cudaStream_t cin = nullptr, cout = nullptr;   // pc_process copy pipeline
 
     int fs = 0, N0 = 0, n_in = 0, n_out = 0;
@@ -151,10 +157,11 @@ struct pc_handle {
 
     std::vector<DevPC> h_pcs;
     std::vector<DevLevel> h_lv;
+    std::vector<int> dfl;      // per level: runs in the deferred form
     std::vector<int> lv_cls;   // kernel class of each level's fires (spectra layout follows it)
     Bank bank{};
     int H = 1;        // hyperperiod (base steps)
-    int G = 64;       // base steps per captured graph (multiple of H and KB)
+    int C = 32;       // base steps per block-parallel chunk (a multiple of KB)
     int req_kb = 1;   // base blocks per step requested (pc_set_step_blocks)
     int req_tile_bins = 0, req_tile_parts = 0;   // spread tile shape requested (pc_set_tiles; 0: default)
     int TB = 0, TP = 0;                          // spread tile shape in use: bins and parts per task
@@ -169,22 +176,41 @@ struct pc_handle {
     std::vector<double> alg_bytes[kClasses];
     // Deferred fires (levels >= 1 whose output is due more than one step
     // after their block completes; with several base blocks per step, every
-    // level >= 1): launched after the step that completed the block, on a
-    // low-priority stream, and joined `due` steps later.
+    // level >= 1): launched after the step that completed the block, in
+    // stream order.
     struct DGroup {
-        int cls, phase, due, off, cnt;
+        int cls, phase, off, cnt;
         double bytes;
     };
     std::vector<DGroup> dgroups;
     std::vector<std::vector<int>> dg_of_phase;   // phase -> indices into dgroups
     // spread tasks of levels >= 1 with several base blocks per step: their own
-    // launch per step on `sside`, beside the step chain; only the levels'
-    // deferred fires wait for them
-    cudaStream_t sside = nullptr;
+    // launch per step
     std::vector<int> sp_off, sp_cnt;
     std::vector<double> sp_bytes;
     int class_maxN[kClasses] = {};
-    RunState* d_rs = nullptr;
+
+    // block-parallel processing (wide.cu)
+    struct WGroup {         // levels of one block size: CTAs in order of their first block's step
+        int N;
+        bool l0, cluster;
+        const int2* map;
+        std::vector<int> upto;   // upto[n]: CTAs whose first block can complete within n + 1 steps
+    };
+    std::vector<WGroup> wgroups;
+    struct WMac {           // one launch of the sum over parts
+        int G;
+        const int2* map;
+        std::vector<int> upto;
+    };
+    std::vector<WMac> wmacs;
+    int w_part_nt = 0, w_part_lanes = 0, w_part_n = 0;   // partial sums at the end of a call
+    const int4* w_part_map = nullptr;
+    const WLevel* d_wlv = nullptr;
+    const float2* d_wtab = nullptr;
+    const int* d_lv0 = nullptr;    // level-0 index of every PC
+    int n_zero = 0, max_ring = 0;
+    bool mixed = false;
 
     // run() staging and Relaxed carry (planar [n_out][N0])
     float* d_in1 = nullptr;
@@ -199,9 +225,6 @@ struct pc_handle {
     size_t big_in_cap = 0, big_out_cap = 0;
     float* d_rtmp = nullptr;
     size_t rtmp_cap = 0;
-
-    cudaGraphExec_t gexec = nullptr;
-    long long graph_kernels = 0;   // kernel nodes per replay
 
     long long frame_num = 0;
     long long launches = 0;
@@ -226,8 +249,6 @@ int cuda_fail(pc_handle* h, cudaError_t e, const char* where) {
 
 void free_device(pc_handle* h) {
     if (h->device >= 0) cudaSetDevice(h->device);
-    if (h->gexec) cudaGraphExecDestroy(h->gexec);
-    h->gexec = nullptr;
     if (h->arena) cudaFree(h->arena);
     if (h->h_in1) cudaFreeHost(h->h_in1);
     if (h->h_out1) cudaFreeHost(h->h_out1);
@@ -238,16 +259,6 @@ void free_device(pc_handle* h) {
     if (h->d_rtmp) cudaFree(h->d_rtmp);
     h->d_big_in = h->d_big_out = h->d_rtmp = nullptr;
     h->big_in_cap = h->big_out_cap = h->rtmp_cap = 0;
-    for (auto& s : h->side) {
-        if (s) cudaStreamDestroy(s);
-        s = nullptr;
-    }
-    for (auto& s : h->aside) {
-        if (s) cudaStreamDestroy(s);
-        s = nullptr;
-    }
-    if (h->sside) cudaStreamDestroy(h->sside);
-    h->sside = nullptr;
     if (h->cin) cudaStreamDestroy(h->cin);
     if (h->cout) cudaStreamDestroy(h->cout);
     h->cin = h->cout = nullptr;
@@ -264,20 +275,37 @@ long long floordiv(long long a, long long b) {
     return (a % b != 0 && ((a < 0) != (b < 0))) ? q - 1 : q;
 }
 
+WArgs wide_args(const pc_handle* h, const IOView& view, int n) {
+    WArgs a{};
+    a.lv = h->d_wlv;
+    a.tab = h->d_wtab;
+    a.W = h->bank.W;
+    a.wlog = kWlog;
+    a.N0 = h->N0;
+    a.c0 = h->frame_num;
+    a.nsteps = n;
+    a.kb = h->KB;
+    a.io = view;
+    // float2 accesses: unit stride and 8-byte aligned channel rows
+    a.vec_in = view.in_sample == 1 && (h->n_in == 1 || view.in_ch % 2 == 0) && (reinterpret_cast<uintptr_t>(view.in) & 7) == 0;
+    a.vec_out = view.out_sample == 1 && (h->n_out == 1 || view.out_ch % 2 == 0) && (reinterpret_cast<uintptr_t>(view.out) & 7) == 0;
+    return a;
+}
+
 // One base step by direct launches (classes with work in this phase).
 // first: the preceding work in the stream is not one of this handle's step
 // kernels, so the launch must not overlap it.
 int launch_step_direct(pc_handle* h, const RunState& rs, cudaStream_t st, bool first) {
     const int ph = phase_of(h, rs.step_base);
     if (h->sp_cnt[ph] > 0) {   // levels' spread tasks first, in stream order
-        CK(launch_side_spreads(h->sp_cnt[ph], h->d_tasks + h->sp_off[ph], rs, nullptr, 0, st), "spread launch");
+        CK(launch_side_spreads(h->sp_cnt[ph], h->d_tasks + h->sp_off[ph], rs.step_base, st), "spread launch");
         h->launches += 1;
     }
     for (int k = 0; k < kClasses; ++k) {
         const int cls = (h->l0_class + k) % kClasses;   // level-0 class first
         const int n = h->cnt[cls][ph];
         if (n <= 0) continue;
-        CK(launch_step_class(cls, n, h->class_maxN[cls], h->bank, h->d_tasks + h->off[cls][ph], rs, nullptr, 0, st,
+        CK(launch_step_class(cls, n, h->class_maxN[cls], h->bank, h->d_tasks + h->off[cls][ph], rs, st,
                              !first),
            "step launch");
         first = false;
@@ -287,7 +315,7 @@ int launch_step_direct(pc_handle* h, const RunState& rs, cudaStream_t st, bool f
     // direct step does not overlap them with later steps)
     for (int gi : h->dg_of_phase[ph]) {
         const pc_handle::DGroup& gr = h->dgroups[gi];
-        CK(launch_step_class(gr.cls, gr.cnt, h->class_maxN[gr.cls], h->bank, h->d_tasks + gr.off, rs, nullptr, 0, st,
+        CK(launch_step_class(gr.cls, gr.cnt, h->class_maxN[gr.cls], h->bank, h->d_tasks + gr.off, rs, st,
                              !first),
            "deferred fire launch");
         first = false;
@@ -296,110 +324,114 @@ int launch_step_direct(pc_handle* h, const RunState& rs, cudaStream_t st, bool f
     return PC_OK;
 }
 
-// Capture G steps starting at a step with phase 0.  Classes other than the
-// level-0 class run on side branches joined at the end of their step.
-int build_graph(pc_handle* h) {
-    cudaGraph_t g = nullptr;
-    std::vector<cudaEvent_t> evs;
-    auto mk = [&]() {
-        cudaEvent_t e;
-        cudaEventCreateWithFlags(&e, cudaEventDisableTiming);
-        evs.push_back(e);
-        return e;
+// CTA maps of the block-parallel kernels, built on the host in the order in
+// which their first blocks complete, so a short call launches a prefix.
+struct WideMaps {
+    struct G {
+        int N;
+        bool l0, cluster;
+        std::vector<std::pair<int, int2>> e;   // (first relative step at which the entry may have work, entry)
     };
-    cudaError_t e = cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal);
-    if (e != cudaSuccess) return cuda_fail(h, e, "begin capture");
-    RunState dummy{};
-    long long kernels = 0;
-    struct Pending {
-        int due_step;
-        cudaEvent_t done;
+    std::vector<G> groups;
+    struct Mc {
+        int G;
+        std::vector<std::pair<int, int2>> e;
     };
-    std::vector<Pending> pending;   // deferred fires in flight
-    cudaEvent_t sp_last = nullptr;  // completion of the newest side spread launch
-    for (int s = 0; s < h->G && e == cudaSuccess; s += h->KB) {   // s: first base step of the step
-        const int ph = phase_of(h, s);
-        // deferred fires whose output this step emits join the chain here
-        for (size_t i = 0; i < pending.size() && e == cudaSuccess;) {
-            if (pending[i].due_step <= s) {
-                e = cudaStreamWaitEvent(h->stream, pending[i].done, 0);
-                pending.erase(pending.begin() + i);
-            } else {
-                ++i;
-            }
-        }
-        // levels' spread tasks (several base blocks per step): their own branch,
-        // waited for only by the levels' deferred fires and the graph's end
-        if (h->sp_cnt[ph] > 0 && e == cudaSuccess) {
-            cudaEvent_t fork = mk();
-            e = cudaEventRecord(fork, h->stream);
-            if (e == cudaSuccess) e = cudaStreamWaitEvent(h->sside, fork, 0);
-            if (e == cudaSuccess)
-                e = launch_side_spreads(h->sp_cnt[ph], h->d_tasks + h->sp_off[ph], dummy, h->d_rs, s, h->sside);
-            cudaEvent_t done = mk();
-            if (e == cudaSuccess) e = cudaEventRecord(done, h->sside);
-            sp_last = done;
-            ++kernels;
-        }
-        std::vector<cudaEvent_t> joins;
-        for (int cls = 0; cls < kClasses && e == cudaSuccess; ++cls) {
-            if (cls == h->l0_class || h->cnt[cls][ph] <= 0) continue;
-            cudaEvent_t fork = mk();
-            e = cudaEventRecord(fork, h->stream);
-            if (e == cudaSuccess) e = cudaStreamWaitEvent(h->side[cls], fork, 0);
-            if (e == cudaSuccess)
-                e = launch_step_class(cls, h->cnt[cls][ph], h->class_maxN[cls], h->bank,
-                                      h->d_tasks + h->off[cls][ph], dummy, h->d_rs, s, h->side[cls], false);
-            cudaEvent_t join = mk();
-            if (e == cudaSuccess) e = cudaEventRecord(join, h->side[cls]);
-            joins.push_back(join);
-            ++kernels;
-        }
-        const int c0 = h->l0_class;
-        if (e == cudaSuccess)
-            e = launch_step_class(c0, h->cnt[c0][ph], h->class_maxN[c0], h->bank, h->d_tasks + h->off[c0][ph], dummy,
-                                  h->d_rs, s, h->stream, s > 0, 1);
-        ++kernels;
-        for (auto j : joins)
-            if (e == cudaSuccess) e = cudaStreamWaitEvent(h->stream, j, 0);
-        // fires of blocks this step completed: forked after the step, low
-        // priority, joined before the step that first emits their output
-        for (int gi : h->dg_of_phase[ph]) {
-            if (e != cudaSuccess) break;
-            const pc_handle::DGroup& gr = h->dgroups[gi];
-            cudaEvent_t fork = mk();
-            e = cudaEventRecord(fork, h->stream);
-            if (e == cudaSuccess) e = cudaStreamWaitEvent(h->aside[gr.cls], fork, 0);
-            if (e == cudaSuccess && sp_last) e = cudaStreamWaitEvent(h->aside[gr.cls], sp_last, 0);
-            // a large deferred fire takes a whole SM (shared memory), so it
-            // never shares one with the step chain's kernels
-            if (e == cudaSuccess)
-                e = launch_step_class(gr.cls, gr.cnt, h->class_maxN[gr.cls], h->bank, h->d_tasks + gr.off, dummy,
-                                      h->d_rs, s, h->aside[gr.cls], false, -1, gr.cls != h->l0_class);
-            cudaEvent_t done = mk();
-            if (e == cudaSuccess) e = cudaEventRecord(done, h->aside[gr.cls]);
-            pending.push_back({s + gr.due * h->KB, done});
-            ++kernels;
-        }
+    std::vector<Mc> macs;
+    std::vector<int4> part;
+
+    size_t bytes() const {
+        size_t n = sizeof(int4) * part.size() + 256;
+        for (auto& g : groups) n += sizeof(int2) * g.e.size() + 256;
+        for (auto& m : macs) n += sizeof(int2) * m.e.size() + 256;
+        return n;
     }
-    // the graph ends with every deferred fire joined (a replay must not
-    // overlap the next one's state update)
-    for (auto& pd : pending)
-        if (e == cudaSuccess) e = cudaStreamWaitEvent(h->stream, pd.done, 0);
-    if (sp_last && e == cudaSuccess) e = cudaStreamWaitEvent(h->stream, sp_last, 0);
-    cudaError_t e2 = cudaStreamEndCapture(h->stream, &g);
-    for (auto ev : evs) cudaEventDestroy(ev);
-    if (e == cudaSuccess) e = e2;
-    // with several base blocks per step the graph runs its nodes at their own
-    // priorities (chain high, deferred fires low): 61.3k against 60.3k
-    // audio-s/s on 32 streams; with one block per step that slowed the chain
-    // (58.0k against 59.6k), so it keeps the stream's priority
-    if (e == cudaSuccess)
-        e = cudaGraphInstantiate(&h->gexec, g, h->KB > 1 ? cudaGraphInstantiateFlagUseNodePriority : 0);
-    if (g) cudaGraphDestroy(g);
-    if (e != cudaSuccess) return cuda_fail(h, e, "graph capture");
-    h->graph_kernels = kernels;
-    return PC_OK;
+    static std::vector<int> prefix(const std::vector<std::pair<int, int2>>& e, int C) {
+        std::vector<int> u(C, 0);
+        size_t j = 0;
+        for (int n = 0; n < C; ++n) {   // a call of n + 1 steps: entries that start at step n or before
+            while (j < e.size() && e[j].first <= n) ++j;
+            u[n] = (int)j;
+        }
+        return u;
+    }
+    cudaError_t place(pc_handle* h, char* base) {
+        size_t off = 0;
+        cudaError_t err = cudaSuccess;
+        auto put = [&](const void* src, size_t n) {
+            char* dst = base + off;
+            if (n && err == cudaSuccess) err = cudaMemcpyAsync(dst, src, n, cudaMemcpyHostToDevice, h->stream);
+            off += (n + 255) & ~(size_t)255;
+            return dst;
+        };
+        auto entries = [&](std::vector<std::pair<int, int2>>& e) {
+            std::stable_sort(e.begin(), e.end(), [](auto& a, auto& b) { return a.first < b.first; });
+            std::vector<int2> v;
+            v.reserve(e.size());
+            for (auto& x : e) v.push_back(x.second);
+            const int2* d = reinterpret_cast<const int2*>(put(v.data(), sizeof(int2) * v.size()));
+            if (err == cudaSuccess) err = cudaStreamSynchronize(h->stream);
+            return d;
+        };
+        h->wgroups.clear();
+        for (auto& g : groups) {
+            const int2* d = entries(g.e);
+            h->wgroups.push_back({g.N, g.l0, g.cluster, d, prefix(g.e, h->C)});
+        }
+        h->wmacs.clear();
+        for (auto& m : macs) {
+            const int2* d = entries(m.e);
+            h->wmacs.push_back({m.G, d, prefix(m.e, h->C)});
+        }
+        h->w_part_map = reinterpret_cast<const int4*>(put(part.data(), sizeof(int4) * part.size()));
+        h->w_part_n = (int)part.size();
+        return err;
+    }
+};
+
+void build_wide_maps(pc_handle* h, WideMaps& m) {
+    // thread groups of the handle's spread tasks (they fix the order of the
+    // partial sums): step_kernel runs them with the level-0 class's threads
+    // over the tile width's lanes; with several base blocks per step the
+    // levels' run in spread_kernel, level 0's with the default width
+    const int nt = h->KB > 1 ? 256 : class_threads(h->l0_class);
+    const int lanes = h->l0_class == 0 ? h->TB / 2 : spread_task_bins() / 2;
+    const int nlv = (int)h->h_lv.size();
+    h->w_part_nt = nt;
+    h->w_part_lanes = lanes;
+    auto group = [&](int N, bool l0, bool cluster) -> WideMaps::G& {
+        for (auto& g : m.groups)
+            if (g.N == N && g.l0 == l0 && g.cluster == cluster) return g;
+        m.groups.push_back({N, l0, cluster, {}});
+        return m.groups.back();
+    };
+    auto mac = [&](int G) -> WideMaps::Mc& {
+        for (auto& x : m.macs)
+            if (x.G == G) return x;
+        m.macs.push_back({G, {}});
+        return m.macs.back();
+    };
+    for (int li = 0; li < nlv; ++li) {
+        const DevLevel& l = h->h_lv[li];
+        const bool l0 = l.T == 1, cluster = h->lv_cls[li] == 3;
+        const int nb = (h->C + l.T - 1) / l.T;   // most blocks of the level in a chunk
+        const int per = cluster ? 1 : wide_transforms_per_cta(l.N);
+        auto& g = group(l.N, l0, cluster);
+        for (int i = 0; i < nb; i += per) g.e.push_back({i * l.T, make_int2(li, i)});
+        const int G = l0 && h->KB > 1 ? 4 : nt / lanes, run = wide_run(G);
+        const int items = (nb + run - 1) / run * l.cs;
+        auto& mc = mac(G);
+        for (int i = 0; i < items; i += kWideMacNT) mc.e.push_back({i / l.cs * run * l.T, make_int2(li, i)});
+        // partial sums: one CTA per tile of bins and row
+        const int QC = h->KB > 1 ? multi_fire_parts(h->N0, h->KB) : 2;
+        const int p_lo = l0 ? (h->KB > 1 ? std::min(l.P, QC) : 2) : (h->dfl[li] ? 2 : 1);
+        const int tile = l0 && h->KB > 1 ? spread_task_bins() : 2 * lanes;
+        if (l.P > p_lo)
+            for (int k = 0; k < l.cs; k += tile)
+                for (int r = 0; r < l.npart; ++r) m.part.push_back(make_int4(li, k, r, std::min(l.cs, k + tile)));
+    }
+    // larger blocks first (their inverse transforms feed level 0's output)
+    std::stable_sort(m.groups.begin(), m.groups.end(), [](auto& a, auto& b) { return a.N > b.N; });
 }
 
 int do_setup(pc_handle* h, int fs, int buffer_size, int n_in, int n_out, std::vector<PCSpec>&& specs) {
@@ -424,10 +456,8 @@ int do_setup(pc_handle* h, int fs, int buffer_size, int n_in, int n_out, std::ve
     int prio_least = 0, prio_greatest = 0;
     CK(cudaDeviceGetStreamPriorityRange(&prio_least, &prio_greatest), "priority range");
     CK(cudaStreamCreateWithPriority(&h->stream, cudaStreamNonBlocking, prio_greatest), "stream create");
-    for (auto& s : h->side) CK(cudaStreamCreateWithPriority(&s, cudaStreamNonBlocking, prio_greatest), "stream create");
-    for (auto& s : h->aside) CK(cudaStreamCreateWithPriority(&s, cudaStreamNonBlocking, prio_least), "stream create");
-    CK(cudaStreamCreateWithPriority(&h->sside, cudaStreamNonBlocking, prio_least), "stream create");
     CK(prepare_kernels(), "kernel attributes");
+    CK(prepare_wide_kernels(), "kernel attributes");
 
     h->fs = fs;
     h->N0 = buffer_size;
@@ -444,7 +474,6 @@ int do_setup(pc_handle* h, int fs, int buffer_size, int n_in, int n_out, std::ve
         Hh = std::max(Hh, p.N.back() / N0);
     }
     h->H = Hh;
-    h->G = std::max(Hh, kMinGraphSteps);
     h->maxN = maxN;
     h->l0_class = fire_class_of(N0);
     // base blocks per step: at most what the level-0 kernel supports, and
@@ -456,17 +485,27 @@ int do_setup(pc_handle* h, int fs, int buffer_size, int n_in, int n_out, std::ve
     h->KB = KB;
     h->Hs = std::max(1, Hh / KB);
     // spread tile shape: bins and parts per spread task
-    const int TB = h->req_tile_bins > 0 ? h->req_tile_bins : spread_task_bins();
+    // (the step kernels of larger base blocks have the default width only)
+    const int TB = h->req_tile_bins > 0 && h->l0_class == 0 ? h->req_tile_bins : spread_task_bins();
     const int TP = h->req_tile_parts > 0 ? h->req_tile_parts : spread_task_parts();
     h->TB = TB;
     h->TP = TP;
     // parts a K-block level-0 fire sums itself; spread rows take the rest
     const int QC = KB > 1 ? multi_fire_parts(N0, KB) : 2;
-    h->G = std::max(h->G, KB);
+    {
+        // a block of N samples adds a row of N + 2 bins per N / N0 steps
+        const double row = sizeof(float2) * (double)N0 * nlv;   // bytes of spectra per base step
+        int C = kWideMaxChunk;
+        while (C > kWideMinChunk && C * row > (double)kWideBytes) C >>= 1;
+        h->C = C;
+    }
 
     // ---- arena layout --------------------------------------------------------------
     Carve cv;
     const size_t off_W = cv.take(sizeof(float2) << kWlog);
+    const size_t off_wtab = cv.take(sizeof(float2) * kFftTabEntries);
+    const size_t off_wlv = cv.take(sizeof(WLevel) * nlv);
+    const size_t off_lv0 = cv.take(sizeof(int) * npc);
     const size_t off_pcs = cv.take(sizeof(DevPC) * npc);
     const size_t off_lv = cv.take(sizeof(DevLevel) * nlv);
     std::vector<size_t> off_H(nlv);
@@ -488,7 +527,6 @@ int do_setup(pc_handle* h, int fs, int buffer_size, int n_in, int n_out, std::ve
     const size_t off_out_off = cv.take(sizeof(int) * (n_out + 1));
     const size_t off_out_pcs = cv.take(sizeof(int) * std::max<size_t>(1, out_pcs.size()));
     const size_t off_zero = cv.take(sizeof(int) * std::max<size_t>(1, zero_list.size()));
-    const size_t off_rs = cv.take(sizeof(RunState));
     const size_t off_in1 = cv.take(sizeof(float) * (size_t)N0 * n_in);
     const size_t off_out1 = cv.take(sizeof(float) * (size_t)N0 * n_out);
     // task table size is known only after enumeration; it goes last in the static part
@@ -503,19 +541,21 @@ int do_setup(pc_handle* h, int fs, int buffer_size, int n_in, int n_out, std::ve
     // Deferral window of each level (0: fires within its step).  Level L's
     // first output sample of a block is due slack = (s_L - N_L)/N0 steps
     // after the step that completes the block; the fire is deferred by
-    // w = min(slack, T - 2) steps so that it is joined before the level's
-    // next block completes (the spreads of the block after next read its
-    // spectrum).  Its window stays in the input ring meanwhile.
+    // w = min(slack, T - 2) steps at most, so that it has run before the
+    // level's next block completes (the spreads of the block after next read
+    // its spectrum).  Its window stays in the input ring meanwhile.
     //
     // With KB > 1 base blocks per step every level >= 1 is deferred: its
     // block completes inside some step S, its fire is launched after S and
-    // joined w' + 1 steps later, w' = min(floor(slack / KB), N_L / (KB N0) - 1).
+    // has w' + 1 steps to run, w' = min(floor(slack / KB), N_L / (KB N0) - 1).
     // The first output sample is due at the start of step S + floor(slack /
     // KB) + 1 (outputs of a level block start on a multiple of N_L, a
     // multiple of KB N0), and the cap keeps the fire ahead of the spreads of
     // the block after next.
     // dfl: the level runs in the deferred form (parts >= 2 from double-buffered rows).
-    std::vector<int> rin(npc), rl(nlv), dwin(nlv, 0), dfl(nlv, 0);
+    std::vector<int> rin(npc), rl(nlv), dwin(nlv, 0);
+    std::vector<int>& dfl = h->dfl;
+    dfl.assign(nlv, 0);
     {
         int li = 0;
         for (int i = 0; i < npc; ++i) {
@@ -550,7 +590,8 @@ int do_setup(pc_handle* h, int fs, int buffer_size, int n_in, int n_out, std::ve
             long s = 0;
             for (size_t L = 0; L < p.N.size(); ++L, ++li) {
                 long r = p.N[L];
-                while (r < s + (long)KB * N0) r <<= 1;
+                // samples in flight: due later (up to s + KB N0), or a whole chunk's
+                while (r < s + (long)std::max(KB, h->C) * N0) r <<= 1;
                 rl[li] = (int)r;
                 s += (long)p.N[L] * p.P[L];
             }
@@ -559,8 +600,8 @@ int do_setup(pc_handle* h, int fs, int buffer_size, int n_in, int n_out, std::ve
     // Kernel class per level.  A fire within its step sits on the step chain,
     // where its latency counts: levels of 8192 and 16384 samples then run on
     // a cluster (class 3) when few of them share a handle, so that all their
-    // clusters fit the GPU at once; otherwise (and for deferred fires, which
-    // overlap later steps) one CTA per fire.
+    // clusters fit the GPU at once; otherwise (and for deferred fires) one CTA
+    // per fire.
     h->lv_cls.assign(nlv, 0);
     {
         int li = 0, instep_big = 0;
@@ -606,6 +647,7 @@ int do_setup(pc_handle* h, int fs, int buffer_size, int n_in, int n_out, std::ve
                 l.cs = p.N[L] + 2;
                 l.rmask = rl[li] - 1;
                 l.pc = i;
+                l.slots = l.P + std::max((h->C + l.T - 1) / l.T, wide_run());
                 {   // spread tasks sum parts >= 2 KB (level 0), >= 2 (deferred levels) or >= 1
                     const int p_lo = L == 0 ? (KB > 1 ? std::min(p.P[L], QC) : 2) : (dfl[li] ? 2 : 1);
                     const int np = p.P[L] - p_lo;
@@ -621,8 +663,8 @@ int do_setup(pc_handle* h, int fs, int buffer_size, int n_in, int n_out, std::ve
     // are known; first count them to size the table.
     const int NP = h->Hs;   // phases
     std::vector<std::vector<std::vector<Task>>> lists(kClasses, std::vector<std::vector<Task>>(NP));
-    std::map<std::tuple<int, int, int>, std::vector<Task>> dlists;   // (phase, due, class) -> deferred fires
-    std::map<std::tuple<int, int, int>, double> dbytes;
+    std::map<std::pair<int, int>, std::vector<Task>> dlists;   // (phase, class) -> deferred fires
+    std::map<std::pair<int, int>, double> dbytes;
     std::vector<std::vector<Task>> sp_lists(NP);   // side spread tasks per phase (KB > 1)
     h->sp_bytes.assign(NP, 0.0);
     for (int cls = 0; cls < kClasses; ++cls) h->alg_bytes[cls].assign(NP, 0.0);
@@ -643,6 +685,7 @@ int do_setup(pc_handle* h, int fs, int buffer_size, int n_in, int n_out, std::ve
             t.N = l.N;
             t.logN = l.logN;
             t.P = l.P;
+            t.slots = l.slots;
             t.T = l.T;
             t.s_blocks = l.s_blocks;
             t.cs = l.cs;
@@ -673,8 +716,8 @@ int do_setup(pc_handle* h, int fs, int buffer_size, int n_in, int n_out, std::ve
             t.k0 = l.npart;   // partial-sum rows the fire adds
             if (dwin[li] > 0) {
                 t.dfer = 1;
-                dlists[std::make_tuple(g, dwin[li] + 1, cls)].push_back(t);
-                dbytes[std::make_tuple(g, dwin[li] + 1, cls)] += b;
+                dlists[{g, cls}].push_back(t);
+                dbytes[{g, cls}] += b;
                 continue;
             }
             lists[cls][g].push_back(t);
@@ -713,6 +756,7 @@ int do_setup(pc_handle* h, int fs, int buffer_size, int n_in, int n_out, std::ve
                     t.kind = 1;
                     t.N = l.N;
                     t.P = l.P;
+            t.slots = l.slots;
                     t.T = l.T;
                     t.s_blocks = l.s_blocks;
                     t.cs = l.cs;
@@ -743,6 +787,7 @@ int do_setup(pc_handle* h, int fs, int buffer_size, int n_in, int n_out, std::ve
             t.N = l.N;
             t.logN = l.logN;
             t.P = l.P;
+            t.slots = l.slots;
             t.T = l.T;
             t.s_blocks = l.s_blocks;
             t.cs = l.cs;
@@ -787,8 +832,8 @@ int do_setup(pc_handle* h, int fs, int buffer_size, int n_in, int n_out, std::ve
             t.origin = -(cb - c0);
             const double b =
                 16.0 * C + 12.0 * l.N + 8.0 * C * (l.P >= 2 ? 2.0 : 0.0) + (l.P >= 3 ? 8.0 * C * l.npart : 0.0);
-            dlists[std::make_tuple(g, dwin[li] + 1, cls)].push_back(t);
-            dbytes[std::make_tuple(g, dwin[li] + 1, cls)] += b;
+            dlists[{g, cls}].push_back(t);
+            dbytes[{g, cls}] += b;
         }
         const int sc = h->l0_class;
         for (int li = 0; li < nlv; ++li) {
@@ -803,6 +848,7 @@ int do_setup(pc_handle* h, int fs, int buffer_size, int n_in, int n_out, std::ve
                         t.kind = 1;
                         t.N = l.N;
                         t.P = l.P;
+            t.slots = l.slots;
                         t.T = l.T;
                         t.s_blocks = l.s_blocks;
                         t.cs = l.cs;
@@ -856,9 +902,8 @@ int do_setup(pc_handle* h, int fs, int buffer_size, int n_in, int n_out, std::ve
     h->dg_of_phase.assign(NP, {});
     for (auto& kv : dlists) {
         pc_handle::DGroup gr;
-        gr.phase = std::get<0>(kv.first);
-        gr.due = std::get<1>(kv.first);
-        gr.cls = std::get<2>(kv.first);
+        gr.phase = kv.first.first;
+        gr.cls = kv.first.second;
         gr.off = (int)ntasks;
         gr.cnt = (int)kv.second.size();
         gr.bytes = dbytes[kv.first];
@@ -888,13 +933,24 @@ int do_setup(pc_handle* h, int fs, int buffer_size, int n_in, int n_out, std::ve
     so.yr.resize(nlv);
     for (int li = 0; li < nlv; ++li) {
         const DevLevel& l = h->h_lv[li];
-        so.X[li] = cv.take(sizeof(float2) * (size_t)l.P * l.cs);
+        so.X[li] = cv.take(sizeof(float2) * (size_t)l.slots * l.cs);
         so.Yp[li] = cv.take(sizeof(float2) * 2 * (l.T == 1 ? KB : 1) * (size_t)l.npart * l.cs);
         so.yr[li] = cv.take(sizeof(float) * (size_t)(l.rmask + 1));
     }
     so.mix = cv.take(sizeof(int) * n_out);
     so.carry = cv.take(sizeof(float) * (size_t)N0 * n_out);
     const size_t state_end = cv.take(0);
+
+    // block-parallel workspace: summed spectra of a chunk's blocks, mixed
+    // outputs' samples, and the CTA maps
+    std::vector<size_t> off_Yw(nlv), off_pcw(npc, 0);
+    for (int li = 0; li < nlv; ++li)
+        off_Yw[li] = cv.take(sizeof(float2) * (size_t)((h->C + h->h_lv[li].T - 1) / h->h_lv[li].T) * h->h_lv[li].cs);
+    for (int i = 0; i < npc; ++i)
+        if (h->h_pcs[i].mix_mode == 2) off_pcw[i] = cv.take(sizeof(float) * (size_t)h->C * N0);
+    WideMaps wm;
+    build_wide_maps(h, wm);
+    const size_t off_wmap = cv.take(wm.bytes());
 
     h->arena_bytes = cv.off;
     cudaError_t e = cudaMalloc(&h->arena, h->arena_bytes);
@@ -954,6 +1010,56 @@ int do_setup(pc_handle* h, int fs, int buffer_size, int n_in, int n_out, std::ve
         const int cls = h->lv_cls[li];
         h->class_maxN[cls] = std::max(h->class_maxN[cls], h->h_lv[li].N);
     }
+    {
+        std::vector<WLevel> wl(nlv);
+        std::vector<int> lv0(npc);
+        for (int i = 0; i < npc; ++i) {
+            const DevPC& d = h->h_pcs[i];
+            lv0[i] = d.lv0;
+            for (int L = 0; L < d.M; ++L) {
+                const int li = d.lv0 + L;
+                const DevLevel& l = h->h_lv[li];
+                WLevel& w = wl[li];
+                w = WLevel{};
+                w.N = l.N;
+                w.logN = l.logN;
+                w.P = l.P;
+                w.logT = ilog2(l.T);
+                w.s_blocks = l.s_blocks;
+                w.cs = l.cs;
+                w.slots = l.slots;
+                w.rmask = l.rmask;
+                w.two = L == 0 || dfl[li];
+                w.p_lo = L == 0 && KB > 1 ? std::min(l.P, QC) : (w.two ? 2 : 1);
+                w.nrows = l.npart;
+                w.form = L == 0 && KB > 1 ? kFormMulti : (h->lv_cls[li] == 3 ? kFormCluster : kFormFire);
+                w.in_ch = d.in_ch;
+                w.out_ch = d.out_ch;
+                w.mix_mode = d.mix_mode;
+                w.M = d.M;
+                w.rin_mask = d.rin_mask;
+                w.lv0 = d.lv0;
+                w.dfer = dfl[li];
+                w.scale = d.scale;
+                w.H = l.H;
+                w.X = l.X;
+                w.Yw = reinterpret_cast<float2*>(A + off_Yw[li]);
+                w.Yp = l.Yp;
+                w.yring = l.yring;
+                w.xring = d.xring;
+                w.pcw = d.mix_mode == 2 ? reinterpret_cast<float*>(A + off_pcw[i]) : nullptr;
+                h->max_ring = std::max(h->max_ring, d.rin_mask + 1);
+            }
+        }
+        CK(cudaMemcpyAsync(A + off_wlv, wl.data(), sizeof(WLevel) * nlv, cudaMemcpyHostToDevice, h->stream),
+           "upload levels");
+        CK(cudaMemcpyAsync(A + off_lv0, lv0.data(), sizeof(int) * npc, cudaMemcpyHostToDevice, h->stream),
+           "upload levels");
+        h->d_wlv = reinterpret_cast<const WLevel*>(A + off_wlv);
+        h->d_lv0 = reinterpret_cast<const int*>(A + off_lv0);
+        h->d_wtab = reinterpret_cast<const float2*>(A + off_wtab);
+        CK(wm.place(h, A + off_wmap), "upload maps");
+    }
     // the level-0 class also runs spread tasks; its smem must fit its fires
     if (h->class_maxN[h->l0_class] == 0) h->class_maxN[h->l0_class] = N0;
 
@@ -965,6 +1071,9 @@ int do_setup(pc_handle* h, int fs, int buffer_size, int n_in, int n_out, std::ve
             W[m] = make_float2((float)std::cos(a), (float)std::sin(a));
         }
         CK(cudaMemcpyAsync(A + off_W, W.data(), sizeof(float2) * W.size(), cudaMemcpyHostToDevice, h->stream),
+           "upload twiddles");
+        const std::vector<float2> tab = build_fft_tables(W, kWlog);
+        CK(cudaMemcpyAsync(A + off_wtab, tab.data(), sizeof(float2) * tab.size(), cudaMemcpyHostToDevice, h->stream),
            "upload twiddles");
         CK(cudaStreamSynchronize(h->stream), "sync");
     }
@@ -983,7 +1092,6 @@ int do_setup(pc_handle* h, int fs, int buffer_size, int n_in, int n_out, std::ve
         CK(cudaMemcpyAsync(A + off_zero, zero_list.data(), sizeof(int) * zero_list.size(), cudaMemcpyHostToDevice,
                            h->stream),
            "upload zero list");
-    h->d_rs = reinterpret_cast<RunState*>(A + off_rs);
     h->d_in1 = reinterpret_cast<float*>(A + off_in1);
     h->d_out1 = reinterpret_cast<float*>(A + off_out1);
     // pinned staging: a callback's block crosses PCIe/C2C as a true async
@@ -1068,13 +1176,9 @@ int do_setup(pc_handle* h, int fs, int buffer_size, int n_in, int n_out, std::ve
         }
     }
 
-    int r = build_graph(h);
-    if (r) {
-        std::string m = h->err;
-        free_device(h);
-        h->err = m;
-        return r;
-    }
+    h->n_zero = (int)zero_list.size();
+    h->mixed = false;
+    for (auto& o : out_list) h->mixed = h->mixed || o.size() > 1;
     h->frame_num = 0;
     h->ready = true;
     if (h->verbosity > 0) {
@@ -1089,10 +1193,7 @@ int do_setup(pc_handle* h, int fs, int buffer_size, int n_in, int n_out, std::ve
     return PC_OK;
 }
 
-// ch_stride: frames between channel rows of a planar buffer (0: frames)
-IOView make_view(const pc_handle* h, const float* in, float* out, long long frames, int layout, long long step0,
-                 long long ch_stride = 0) {
-    if (ch_stride <= 0) ch_stride = frames;
+IOView make_view(const pc_handle* h, const float* in, float* out, long long frames, int layout, long long step0) {
     IOView v;
     v.in = in;
     v.out = out;
@@ -1100,10 +1201,10 @@ IOView make_view(const pc_handle* h, const float* in, float* out, long long fram
     if (layout == PC_PLANAR) {
         v.in_step = h->N0;
         v.in_sample = 1;
-        v.in_ch = ch_stride;
+        v.in_ch = frames;
         v.out_step = h->N0;
         v.out_sample = 1;
-        v.out_ch = ch_stride;
+        v.out_ch = frames;
     } else {
         v.in_step = (long long)h->N0 * h->n_in;
         v.in_sample = h->n_in;
@@ -1115,38 +1216,76 @@ IOView make_view(const pc_handle* h, const float* in, float* out, long long fram
     return v;
 }
 
+// One chunk of n <= h->C base steps from h->frame_num, block-parallel.
+int run_chunk(pc_handle* h, const IOView& view, int n, cudaStream_t st) {
+    WArgs a = wide_args(h, view, n);
+    for (auto& g : h->wgroups) {
+        const int grid = g.upto[n - 1];
+        CK(g.cluster ? launch_wide_cluster(false, grid, g.map, a, st) : launch_wide_fft(g.N, grid, g.map, a, st),
+           "window transforms");
+        h->launches += grid > 0;
+    }
+    for (auto& m : h->wmacs) {
+        CK(launch_wide_mac(m.G, h->TP, m.upto[n - 1], m.map, a, st), "sum over parts");
+        h->launches += 1;
+    }
+    for (auto& g : h->wgroups) {
+        const int grid = g.upto[n - 1];
+        CK(g.cluster ? launch_wide_cluster(true, grid, g.map, a, st)
+                     : launch_wide_ifft(g.N, g.l0, grid, g.map, a, st),
+           "inverse transforms");
+        h->launches += grid > 0;
+    }
+    if (h->mixed || h->n_zero) {
+        CK(launch_wide_mix(h->bank, h->n_zero, h->mixed, a, st), "mix");
+        h->launches += 1;
+    }
+    h->frame_num += n;
+    return PC_OK;
+}
+
+// After a call's last chunk: the state one-block steps would have left.
+int finish_wide(pc_handle* h, const IOView& view, cudaStream_t st) {
+    WArgs a = wide_args(h, view, 0);
+    const long long t_end = h->frame_num * (long long)h->N0;
+    CK(launch_wide_ring(h->d_wlv, h->d_lv0, (int)h->h_pcs.size(), a, t_end, t_end - view.step0 * (long long)h->N0,
+                        h->max_ring, st),
+       "input rings");
+    h->launches += 1;
+    if (h->w_part_n > 0) {
+        CK(launch_wide_partials(h->w_part_nt, h->w_part_lanes, h->w_part_n, h->w_part_map, h->d_wlv, h->TP,
+                                h->frame_num, h->KB, st),
+           "partial sums");
+        h->launches += 1;
+    }
+    return PC_OK;
+}
+
 // Run nsteps base steps starting at h->frame_num through the view: direct
-// launches up to the next graph boundary, graph replays, direct remainder.
-int run_steps(pc_handle* h, const IOView& view, long long nsteps, cudaStream_t st) {
-    long long done = 0;
-    RunState rs;
-    rs.io = view;
-    bool first = true;   // the stream's preceding work is not a step kernel
-    auto direct = [&](long long upto) -> int {
-        for (; done < upto; done += h->KB) {
-            rs.step_base = h->frame_num + done;
-            int r = launch_step_direct(h, rs, st, first);
+// launches for a few steps, block-parallel chunks for more.  A call in several
+// pieces (pc_process's pipeline, one view for all of them) passes more = true
+// for all but the last and again = true for all but the first.
+int run_steps(pc_handle* h, const IOView& view, long long nsteps, cudaStream_t st, bool again = false,
+              bool more = false) {
+    if (nsteps < kWideMinSteps && !again && !more) {
+        RunState rs;
+        rs.io = view;
+        for (long long done = 0; done < nsteps; done += h->KB) {
+            rs.step_base = h->frame_num;
+            // the stream's work before the first step is not a step kernel
+            int r = launch_step_direct(h, rs, st, done == 0);
             if (r) return r;
-            first = false;
+            h->frame_num += h->KB;
         }
         return PC_OK;
-    };
-    const long long G = h->G;
-    const long long misalign = (G - (h->frame_num % G)) % G;
-    int r = direct(std::min(nsteps, misalign));
-    if (r) return r;
-    while (nsteps - done >= G && h->gexec) {
-        rs.step_base = h->frame_num + done;
-        CK(launch_set_state(h->d_rs, rs, st), "state launch");
-        CK(cudaGraphLaunch(h->gexec, st), "graph launch");
-        h->launches += 1 + h->graph_kernels;
-        done += G;
-        first = true;
     }
-    r = direct(nsteps);
-    if (r) return r;
-    h->frame_num += nsteps;
-    return PC_OK;
+    while (nsteps > 0) {
+        const int n = (int)std::min<long long>(nsteps, h->C);
+        int r = run_chunk(h, view, n, st);
+        if (r) return r;
+        nsteps -= n;
+    }
+    return more ? PC_OK : finish_wide(h, view, st);
 }
 
 __global__ void relaxed_shift_kernel(float* out, const float* res, const float* carry, long long frames, int N0,
@@ -1373,11 +1512,12 @@ int pc_process(pc_handle* h, float* output, const float* input, long long frames
     // Long calls run as a pipeline of chunks: the input copy of chunk i + 1
     // and the output copy of chunk i - 1 (own streams) overlap the steps of
     // chunk i (the handle's stream); the steps of one call stay in order.
-    const long long chunk = (long long)std::max(h->G, 128) * h->N0;   // a multiple of KB N0
+    const long long chunk = (long long)std::max(h->C, 128) * h->N0;   // a multiple of KB N0
     if (!h->relaxed && frames >= 2 * chunk) {
         if (!h->cin) CK(cudaStreamCreateWithFlags(&h->cin, cudaStreamNonBlocking), "stream create");
         if (!h->cout) CK(cudaStreamCreateWithFlags(&h->cout, cudaStreamNonBlocking), "stream create");
         const bool planar = layout == PC_PLANAR;
+        const IOView v = make_view(h, h->d_big_in, h->d_big_out, frames, layout, h->frame_num);
         const long long nch = (frames + chunk - 1) / chunk;
         std::vector<cudaEvent_t> evs;
         auto mkev = [&](cudaEvent_t* e) {
@@ -1402,10 +1542,7 @@ int pc_process(pc_handle* h, float* output, const float* input, long long frames
                 rc = cuda_fail(h, e, "input copy");
                 break;
             }
-            const float* din = h->d_big_in + (planar ? c0 : c0 * h->n_in);
-            float* dout = h->d_big_out + (planar ? c0 : c0 * h->n_out);
-            IOView v = make_view(h, din, dout, n, layout, h->frame_num, frames);
-            rc = run_steps(h, v, n / h->N0, h->stream);
+            rc = run_steps(h, v, n / h->N0, h->stream, i > 0, i + 1 < nch);
             if (rc) break;
             e = cudaEventRecord(edone, h->stream);
             if (e == cudaSuccess) e = cudaStreamWaitEvent(h->cout, edone, 0);
@@ -1527,7 +1664,7 @@ int pc_profile_kernels(pc_handle* h, long long nsteps, pc_kernel_stats* out, int
             cudaEventCreate(&r.a);
             cudaEventCreate(&r.b);
             cudaEventRecord(r.a, h->stream);
-            cudaError_t e = launch_side_spreads(h->sp_cnt[ph], h->d_tasks + h->sp_off[ph], rs, nullptr, 0, h->stream);
+            cudaError_t e = launch_side_spreads(h->sp_cnt[ph], h->d_tasks + h->sp_off[ph], rs.step_base, h->stream);
             cudaEventRecord(r.b, h->stream);
             recs.push_back(r);
             h->launches += 1;
@@ -1541,8 +1678,7 @@ int pc_profile_kernels(pc_handle* h, long long nsteps, pc_kernel_stats* out, int
             cudaEventCreate(&r.a);
             cudaEventCreate(&r.b);
             cudaEventRecord(r.a, h->stream);
-            cudaError_t e = launch_step_class(cls, n, h->class_maxN[cls], h->bank, h->d_tasks + h->off[cls][ph], rs,
-                                              nullptr, 0, h->stream, false);
+            cudaError_t e = launch_step_class(cls, n, h->class_maxN[cls], h->bank, h->d_tasks + h->off[cls][ph], rs, h->stream, false);
             cudaEventRecord(r.b, h->stream);
             recs.push_back(r);
             h->launches += 1;
@@ -1555,8 +1691,7 @@ int pc_profile_kernels(pc_handle* h, long long nsteps, pc_kernel_stats* out, int
             cudaEventCreate(&r.a);
             cudaEventCreate(&r.b);
             cudaEventRecord(r.a, h->stream);
-            cudaError_t e = launch_step_class(gr.cls, gr.cnt, h->class_maxN[gr.cls], h->bank, h->d_tasks + gr.off, rs,
-                                              nullptr, 0, h->stream, false);
+            cudaError_t e = launch_step_class(gr.cls, gr.cnt, h->class_maxN[gr.cls], h->bank, h->d_tasks + gr.off, rs, h->stream, false);
             cudaEventRecord(r.b, h->stream);
             recs.push_back(r);
             h->launches += 1;

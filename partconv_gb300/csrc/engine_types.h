@@ -4,7 +4,8 @@
 // Data layout in HBM (one arena per handle, 256-byte aligned carve-outs):
 //   per PC:    input ring xring[Rin]           (time domain, Rin = pow2 >= 2 N_max)
 //   per level: H[P][cs]  filter spectra        (float2, cs = N + 2 row stride)
-//              X[P][cs]  input-spectrum ring   (slot b mod P holds block b)
+//              X[slots][cs]  input-spectrum ring (row b mod slots holds block b;
+//                        slots = P, plus a chunk of blocks in the engine's handles)
 //              Yp[rows][2][cs] partial sums of the FDL MAC for the next block
 //                        (level 0 with K base blocks per step: [rows][2K][cs])
 //              yring[R]  output ring            (levels >= 1; R = pow2 >= s_L + N0)
@@ -32,8 +33,9 @@ struct DevLevel {
     int rmask;      // output ring size - 1 (levels >= 1)
     int pc;         // owning PC
     int npart;      // partial-sum rows (a spread task covers at most the handle's parts per task)
+    int slots;      // rows of the spectrum ring
     float2* H;      // [P][cs]
-    float2* X;      // [P][cs]
+    float2* X;      // [slots][cs]
     float2* Yp;     // [npart][2][cs]: row q, block parity ([npart][2K][cs], block mod 2K, for
                     // level 0 with K base blocks per step)
     float* yring;   // [rmask + 1]
@@ -83,8 +85,11 @@ struct Task {
     float* pcout;
     float* eyring[kEmitLevels];   // level-0 fire: output rings of levels 1..4
     int emask[kEmitLevels];
+    int slots;                    // rows of the spectrum ring (block b in row b mod slots), >= P
+    int pad_[3];
 };
-static_assert(sizeof(Task) == 192, "Task record is loaded as 12 x 16 bytes");
+constexpr int kTaskVec = 13;   // a Task record is loaded as 13 x 16 bytes
+static_assert(sizeof(Task) == 16 * kTaskVec, "Task record size");
 
 // One CTA of a serving pool's step: descriptor slot and sub-task (0: the
 // level's fire, s >= 1: the s-th bin tile of its spread slice).
@@ -103,12 +108,11 @@ struct IOView {
     long long out_step, out_sample, out_ch;
 };
 
-// Per-run state read by every step kernel.
+// What a step kernel needs to know about its call.
 struct RunState {
-    long long step_base;   // global step of step_in_batch == 0
+    long long step_base;   // global step
     IOView io;
 };
-static_assert(sizeof(RunState) == 80, "RunState is loaded as 5 x 16 bytes");
 
 // Static tables the step kernels read.
 struct Bank {

@@ -26,8 +26,17 @@
 
 namespace pcg {
 
+// Rounding is spelled out (one product, one fused multiply-add per component),
+// so every kernel that inlines it gives the same bits: the one-block steps and
+// the block-parallel path must agree exactly.
 __device__ __forceinline__ float2 cmul(float2 a, float2 b) {
-    return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
+    return make_float2(__fmaf_rn(a.x, b.x, -__fmul_rn(a.y, b.y)), __fmaf_rn(a.x, b.y, __fmul_rn(a.y, b.x)));
+}
+// acc + a b, two fused multiply-adds per component
+__device__ __forceinline__ float2 cmac(float2 acc, float2 a, float2 b) {
+    acc.x = __fmaf_rn(-a.y, b.y, __fmaf_rn(a.x, b.x, acc.x));
+    acc.y = __fmaf_rn(a.y, b.x, __fmaf_rn(a.x, b.y, acc.y));
+    return acc;
 }
 __device__ __forceinline__ float2 cadd(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
 __device__ __forceinline__ float2 csub(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
@@ -399,27 +408,43 @@ __device__ __noinline__ float2* fft_smem_batch_c(float2* a, float2* b, int K, co
     return a;
 }
 
-// Split post-pass for the pair (k, N-k), 0 <= k <= N/2, on Z = FFT_N(z).
-// Returns X[k] in xk and X[N-k] in xnk (for k == 0: X[0] and X[N]).
-template <bool SW = false>
-__device__ __forceinline__ void rfft_split(float2 zk, float2 znk, int k, int logN, const Twiddles& tw, float2& xk,
-                                           float2& xnk) {
-    if (k == 0) {
-        xk = make_float2(zk.x + zk.y, 0.0f);
-        xnk = make_float2(zk.x - zk.y, 0.0f);
-        return;
-    }
+// Split post-pass for the pair (k, N-k), 0 < k <= N/2, on Z = FFT_N(z), with
+// w = e^{-i pi k / N}; k == 0 gives X[0] and X[N] (split_zero).
+__device__ __forceinline__ void split_zero(float2 z0, float2& x0, float2& xn) {
+    x0 = make_float2(z0.x + z0.y, 0.0f);
+    xn = make_float2(z0.x - z0.y, 0.0f);
+}
+__device__ __forceinline__ void split_w(float2 zk, float2 znk, float2 w, float2& xk, float2& xnk) {
+    // the halvings are exact, so no rounding depends on how they are fused
     const float2 E = make_float2(0.5f * (zk.x + znk.x), 0.5f * (zk.y - znk.y));
     const float2 O = make_float2(0.5f * (zk.y + znk.y), -0.5f * (zk.x - znk.x));
-    const float2 w = tw.get<SW>(k, logN + 1, false);   // e^{-i pi k / N}
     const float2 wO = cmul(w, O);
     xk = cadd(E, wO);
     xnk = cconj(csub(E, wO));
 }
 
-// Inverse pre-pass for the pair (k, N-k) from Y[k] (yk) and Y[N-k] (ynk);
-// for k == 0 yk = Y[0], ynk = Y[N] and only zk (= Z'[0]) is meaningful.
-// Imaginary parts of Y[0] and Y[N] are ignored, as FFTW's c2r does.
+// Split post-pass for the pair (k, N-k), 0 <= k <= N/2, on Z = FFT_N(z).
+// Returns X[k] in xk and X[N-k] in xnk (for k == 0: X[0] and X[N]).
+template <bool SW = false>
+__device__ __forceinline__ void rfft_split(float2 zk, float2 znk, int k, int logN, const Twiddles& tw, float2& xk,
+                                           float2& xnk) {
+    if (k == 0) split_zero(zk, xk, xnk);
+    else split_w(zk, znk, tw.get<SW>(k, logN + 1, false), xk, xnk);
+}
+
+// Inverse pre-pass for the pair (k, N-k) from Y[k] (yk) and Y[N-k] (ynk),
+// w = e^{-i pi k / N}; for k == 0 yk = Y[0], ynk = Y[N] and only zk (= Z'[0])
+// is meaningful.  Imaginary parts of Y[0] and Y[N] are ignored, as FFTW's
+// c2r does (the caller passes zero for them).
+__device__ __forceinline__ void merge_w(float2 yk, float2 ynk, float2 w, float2& zk, float2& znk) {
+    const float2 A = make_float2(yk.x + ynk.x, yk.y - ynk.y);   // Y[k] + conj(Y[N-k])
+    const float2 B = make_float2(yk.x - ynk.x, yk.y + ynk.y);   // Y[k] - conj(Y[N-k])
+    const float2 cB = cmul(cconj(w), B);                          // conj(w^k) B
+    zk = make_float2(A.x - cB.y, A.y + cB.x);                     // A + i conj(w^k) B
+    const float2 wcB = cmul(w, cconj(B));                         // w^k conj(B)
+    znk = make_float2(A.x - wcB.y, -A.y + wcB.x);                 // conj(A) + i w^k conj(B)
+}
+
 template <bool SW = false>
 __device__ __forceinline__ void irfft_merge(float2 yk, float2 ynk, int k, int logN, const Twiddles& tw, float2& zk,
                                             float2& znk) {
@@ -427,13 +452,7 @@ __device__ __forceinline__ void irfft_merge(float2 yk, float2 ynk, int k, int lo
         yk.y = 0.0f;
         ynk.y = 0.0f;
     }
-    const float2 A = make_float2(yk.x + ynk.x, yk.y - ynk.y);   // Y[k] + conj(Y[N-k])
-    const float2 B = make_float2(yk.x - ynk.x, yk.y + ynk.y);   // Y[k] - conj(Y[N-k])
-    const float2 w = tw.get<SW>(k, logN + 1, false);
-    const float2 cB = cmul(cconj(w), B);                          // conj(w^k) B
-    zk = make_float2(A.x - cB.y, A.y + cB.x);                     // A + i conj(w^k) B
-    const float2 wcB = cmul(w, cconj(B));                         // w^k conj(B)
-    znk = make_float2(A.x - wcB.y, -A.y + wcB.x);                 // conj(A) + i w^k conj(B)
+    merge_w(yk, ynk, tw.get<SW>(k, logN + 1, false), zk, znk);
 }
 
 // 8-point DFT in registers (used by the cluster transforms and the warp
@@ -450,11 +469,11 @@ __device__ __forceinline__ void dft8(float2 v[8], bool inv) {
     for (int i = 0; i < 4; ++i) {
         const float2 a = cadd(v[i], v[i + 4]);
         float2 d = csub(v[i], v[i + 4]);
-        if (i == 1) d = inv ? make_float2(kSqrtHalf8 * (d.x - d.y), kSqrtHalf8 * (d.x + d.y))
-                            : make_float2(kSqrtHalf8 * (d.x + d.y), kSqrtHalf8 * (d.y - d.x));
+        if (i == 1) d = inv ? make_float2(__fmul_rn(kSqrtHalf8, d.x - d.y), __fmul_rn(kSqrtHalf8, d.x + d.y))
+                            : make_float2(__fmul_rn(kSqrtHalf8, d.x + d.y), __fmul_rn(kSqrtHalf8, d.y - d.x));
         if (i == 2) d = inv ? mul_pi(d) : mul_mi(d);
-        if (i == 3) d = inv ? make_float2(-kSqrtHalf8 * (d.x + d.y), kSqrtHalf8 * (d.x - d.y))
-                            : make_float2(kSqrtHalf8 * (d.y - d.x), -kSqrtHalf8 * (d.x + d.y));
+        if (i == 3) d = inv ? make_float2(__fmul_rn(-kSqrtHalf8, d.x + d.y), __fmul_rn(kSqrtHalf8, d.x - d.y))
+                            : make_float2(__fmul_rn(kSqrtHalf8, d.y - d.x), __fmul_rn(-kSqrtHalf8, d.x + d.y));
         v[i] = a;
         v[i + 4] = d;
     }

@@ -48,27 +48,21 @@ int multi_fire_parts(int N0, int K);
 cudaError_t prepare_kernels();
 // pdl: let the launch overlap the previous kernel in the stream, which must
 // be a step kernel of the same handle (or nothing)
-// prio: 0 = the stream's priority, 1 = the device's highest, -1 = its lowest.
-// whole_sm: request enough shared memory that no other CTA fits beside one
-// of these (classes 1 and 2).
 cudaError_t launch_step_class(int cls, int grid, int maxN, const Bank& bank, const Task* tasks, const RunState& rs,
-                              const RunState* rs_dev, int step_in_batch, cudaStream_t st, bool pdl, int prio = 0,
-                              bool whole_sm = false);
+                              cudaStream_t st, bool pdl);
 // spread tasks of levels >= 1 (several base blocks per step) as their own launch
-cudaError_t launch_side_spreads(int grid, const Task* tasks, const RunState& rs, const RunState* rs_dev,
-                                int step_in_batch, cudaStream_t st);
+cudaError_t launch_side_spreads(int grid, const Task* tasks, long long step, cudaStream_t st);
 cudaError_t launch_pool_class(int cls, int grid, int maxN, const Bank& bank, const Task* slots, const PoolCta* map,
                               const RunState& rs, cudaStream_t st);
 cudaError_t launch_spectra(int cls, int njobs, int maxN, const SpectraJob* jobs, const float2* W, int wlog,
                            cudaStream_t st);
-cudaError_t launch_set_state(RunState* dst, const RunState& v, cudaStream_t st);
 
 // class 3 (cluster_fire.cu): fires and filter spectra of levels with
 // 16384 < N <= 65536, one cluster of kClusterCtas CTAs per task or job
 size_t cluster_smem_bytes();
 cudaError_t prepare_cluster_kernels();
-cudaError_t launch_cluster_fire(int ntasks, const Bank& bank, const Task* tasks, const RunState& rs,
-                                const RunState* rs_dev, int step_in_batch, cudaStream_t st, bool pdl, int prio);
+cudaError_t launch_cluster_fire(int ntasks, const Bank& bank, const Task* tasks, const RunState& rs, cudaStream_t st,
+                                bool pdl);
 cudaError_t launch_cluster_spectra(int njobs, const SpectraJob* jobs, const float2* W, int wlog, cudaStream_t st);
 // PartConvFilter's runLevel for such a level (filter.cu), one cluster
 cudaError_t launch_cluster_filter_level(int N, int P, int cs, unsigned bcurr, const float2* H, float2* X,

@@ -108,6 +108,7 @@ __global__ void noalloc_tables_kernel(TableArgs a) {
         t.N = a.N;
         t.logN = a.logN;
         t.P = a.P;
+        t.slots = a.P;
         t.T = 1;
         t.cs = a.cs;
         t.M = 1;
@@ -125,6 +126,7 @@ __global__ void noalloc_tables_kernel(TableArgs a) {
         u.kind = 1;
         u.N = a.N;
         u.P = a.P;
+        u.slots = a.P;
         u.T = 1;
         u.cs = a.cs;
         u.k0 = s * a.spread_bins;
@@ -266,7 +268,7 @@ extern "C" int pc_convolve_noalloc(const float* d_x, long long n_frames, const f
     for (long long c = 0; c < nsteps; ++c) {
         rs.step_base = c;
         // the first step follows the spectra kernel, so it must not overlap it
-        e = launch_step_class(cls, ntasks, N, bank, d_tasks, rs, nullptr, 0, st, c > 0);
+        e = launch_step_class(cls, ntasks, N, bank, d_tasks, rs, st, c > 0);
         if (e != cudaSuccess) return fail(PC_ERR_CUDA, std::string("step launch: ") + cudaGetErrorString(e));
     }
     pcg_set_global_error("");

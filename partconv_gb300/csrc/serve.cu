@@ -369,6 +369,7 @@ int pcs_admit_async(pcs_handle* h, const float* ir, int ir_len, int M, const int
         t.N = n;
         t.logN = logN;
         t.P = Pv[L];
+        t.slots = Pv[L];
         t.T = n / h->N0;
         t.s_blocks = (int)(s / h->N0);
         t.cs = cs;

@@ -35,6 +35,7 @@
 #include "engine_types.h"
 #include "fft_smem.cuh"
 #include "kernels.h"
+#include "wide.h"
 
 namespace pcg {
 
@@ -45,13 +46,10 @@ __device__ __forceinline__ long long imod(long long a, long long m) {
 
 __device__ __forceinline__ float4 f4mac(float4 acc, float4 x, float4 h) {
     // two complex multiply-adds: (x.x + i x.y)(h.x + i h.y), (x.z + i x.w)(h.z + i h.w)
-    acc.x += x.x * h.x - x.y * h.y;
-    acc.y += x.x * h.y + x.y * h.x;
-    acc.z += x.z * h.z - x.w * h.w;
-    acc.w += x.z * h.w + x.w * h.z;
-    return acc;
+    const float2 lo = cmac(make_float2(acc.x, acc.y), make_float2(x.x, x.y), make_float2(h.x, h.y));
+    const float2 hi = cmac(make_float2(acc.z, acc.w), make_float2(x.z, x.w), make_float2(h.z, h.w));
+    return make_float4(lo.x, lo.y, hi.x, hi.y);
 }
-__device__ __forceinline__ float4 f4mul(float4 x, float4 h) { return f4mac(make_float4(0.f, 0.f, 0.f, 0.f), x, h); }
 __device__ __forceinline__ float4 f4add(float4 a, float4 b) {
     return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w);
 }
@@ -70,9 +68,6 @@ struct Cls {
     static constexpr int SPLIT_CH = 4;                           // post-FFT pairs loaded per batch
     static_assert(MAXB >= 1, "class too small");
 };
-// dynamic shared memory that leaves no room for a level-0 CTA beside it on
-// an SM (228 KB per SM, 1 KB reserved per CTA, 227 KB per CTA at most)
-constexpr size_t kWholeSmSmem = 220 * 1024;
 using Cls0 = Cls<256, 1024, true>;
 using Cls1 = Cls<512, 4096, false>;
 // 1024 threads: four radix-4 butterflies per thread per stage at N = 16384
@@ -138,8 +133,9 @@ __device__ __forceinline__ void spread_lanes(const Task& tk, long long c, float4
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
     if (active) {
         constexpr int U = 4;   // parts whose loads are in flight together
-        const int Gm = G % P;  // slot step between a group's consecutive parts
-        int sl0 = (int)imod(bt - (tk.p_lo + g), P);   // slot of part p0
+        const int R = tk.slots;
+        const int Gm = G % R;  // slot step between a group's consecutive parts
+        int sl0 = (int)imod(bt - (tk.p_lo + g), R);   // slot of part p0
         for (int p0 = tk.p_lo + g; p0 < p_hi; p0 += U * G) {
             float4 xv[U], hv[U];
             int sl = sl0;
@@ -151,7 +147,7 @@ __device__ __forceinline__ void spread_lanes(const Task& tk, long long c, float4
                     hv[u] = __ldg(H4 + (size_t)p * rs4);
                 }
                 sl -= Gm;
-                if (sl < 0) sl += P;
+                if (sl < 0) sl += R;
             }
             sl0 = sl;
 #pragma unroll
@@ -208,8 +204,9 @@ __device__ __forceinline__ void spread_multi(const Task& tk, long long c, float4
 #pragma unroll
     for (int j = 0; j < KM; ++j) acc[j] = make_float4(0.f, 0.f, 0.f, 0.f);
     if (active) {
-        const int Gm = G % P;
-        int sl0 = (int)imod(bt0 - (tk.p_lo + g), P);   // slot of block bt0 - p for the group's part p
+        const int R = tk.slots;
+        const int Gm = G % R;
+        int sl0 = (int)imod(bt0 - (tk.p_lo + g), R);   // slot of block bt0 - p for the group's part p
         for (int p0 = tk.p_lo + g; p0 < p_hi; p0 += U * G) {
             float4 xv[U][KM], hv[U];
             int sl = sl0;
@@ -221,11 +218,11 @@ __device__ __forceinline__ void spread_multi(const Task& tk, long long c, float4
 #pragma unroll
                     for (int j = 0; j < KM; ++j) {   // blocks bt0 + j - p: consecutive slots
                         xv[u][j] = __ldcg(X4 + (size_t)sj * rs4);
-                        sj = (sj + 1 == P) ? 0 : sj + 1;
+                        sj = (sj + 1 == R) ? 0 : sj + 1;
                     }
                 }
                 sl -= Gm;
-                if (sl < 0) sl += P;
+                if (sl < 0) sl += R;
             }
             sl0 = sl;
 #pragma unroll
@@ -314,13 +311,13 @@ __device__ __forceinline__ void fire_body(const Bank& bank, const Task& tk, cons
     c -= tk.origin;                              // schedule and rings by the PC's own steps
     const long long q = c + 1 + tk.s_blocks;
     const long long b = q / tk.T - 1;
-    const int slot = (int)imod(b, P);
+    const int slot = (int)imod(b, tk.slots);
     const long long t_new = c * (long long)N0;
     const long long t_end = t_new + N0;
     const float* in = rs.io.in + io_step * rs.io.in_step + (long long)tk.in_ch * rs.io.in_ch;
     const long long isamp = rs.io.in_sample;
     const float scale = tk.scale;
-    const float2* X1 = tk.X + (size_t)imod(b - 1, P) * cs;   // block b-1 (level 0, p = 1)
+    const float2* X1 = tk.X + (size_t)imod(b - 1, tk.slots) * cs;   // block b-1 (level 0, p = 1)
     const float2* Ypb = tk.Yp + (two ? (size_t)(b & 1) * cs : 0);   // row 0; row q at + 2 q cs
     const int npart = tk.k0 > 0 ? tk.k0 : 1;
     const size_t rstride = 2 * (size_t)cs;
@@ -333,7 +330,7 @@ __device__ __forceinline__ void fire_body(const Bank& bank, const Task& tk, cons
     const bool early = EARLY && C::PREFETCH && l0 && io_step >= 1;
     const int Le = tk.M - 1 < kEmitLevels ? tk.M - 1 : kEmitLevels;
     // the other levels' due output slices, summed in level order into `emit`
-    // (their fires completed before this launch: full graph/stream edges)
+    // (their fires completed before this launch: full stream edges)
     auto gather_emit = [&]() {
         if constexpr (C::PREFETCH) {
             float4 ev[C::PREFETCH ? C::MAXE : 1][kEmitLevels];
@@ -750,8 +747,9 @@ __device__ __forceinline__ void fire_multi(const Bank& bank, const Task& tk, con
     const long long io_step = c - rs.io.step0;
     c -= tk.origin;
     const long long b = c;                        // level-0 block of the first base block
-    const int sold0 = (int)imod(b - (Q - 1), P);  // ring slot of the oldest spectrum read
-    const int snew0 = (int)imod(b, P);            // ring slot of block b
+    const int R = tk.slots;
+    const int sold0 = (int)imod(b - (Q - 1), R);  // ring slot of the oldest spectrum read
+    const int snew0 = (int)imod(b, R);            // ring slot of block b
     const float scale = tk.scale;
     float2* sb = smem;                                   // K N: transform data
     float2* sc = sb + (size_t)K * N;                     // K N: transform scratch
@@ -791,10 +789,10 @@ __device__ __forceinline__ void fire_multi(const Bank& bank, const Task& tk, con
             sb[(bi - 1) * N + half + 2 * w + 1] = make_float2(v.z, v.w);
         }
     };
-    // rows [r0, r0 + n) of a ring starting at slot s0 (wrapping at P): two
+    // rows [r0, r0 + n) of a ring starting at slot s0 (wrapping at R): two
     // contiguous runs; f(ring_row, first_local_row, rows)
     auto ring_runs = [&](int s0, int n, auto&& f) {
-        const int n1 = min(n, P - s0);
+        const int n1 = min(n, R - s0);
         f(s0, 0, n1);
         if (n > n1) f(0, n1, n - n1);
     };
@@ -929,9 +927,9 @@ __device__ __forceinline__ void fire_multi(const Bank& bank, const Task& tk, con
     // them.  With fewer parts than blocks (one-level PCs) only the newest P
     // blocks keep a slot.
     {
-        const int t_keep = K > P ? K - P : 0;
+        const int t_keep = K > R ? K - R : 0;
         int s0 = snew0 + t_keep;
-        if (s0 >= P) s0 -= P;
+        if (s0 >= R) s0 -= R;
         ring_runs(s0, K - t_keep, [&](int sr, int r0, int n) {
             float4* dst = reinterpret_cast<float4*>(tk.X + (size_t)sr * cs);
             const float4* src = reinterpret_cast<const float4*>(xs + (size_t)(Q - 1 + t_keep + r0) * cs);
@@ -1031,8 +1029,8 @@ __device__ __forceinline__ void fire_multi(const Bank& bank, const Task& tk, con
 // LANES: threads per spread part-group (bins per spread task / 2), the tile
 // width of the handle, one instance per width.
 template <class C, bool MULTI = false, int LANES = 64>
-__global__ void __launch_bounds__(C::NT, C::PREFETCH ? 3 : 1) step_kernel(Bank bank, const Task* __restrict__ tasks, RunState rs_val,
-                                                     const RunState* rs_dev, int step_in_batch) {
+__global__ void __launch_bounds__(C::NT, C::PREFETCH ? 3 : 1) step_kernel(Bank bank, const Task* __restrict__ tasks,
+                                                                          RunState rs_val) {
     extern __shared__ float4 dyn_smem[];
     __shared__ __align__(16) Task tk;
     __shared__ __align__(16) RunState rs;
@@ -1041,15 +1039,10 @@ __global__ void __launch_bounds__(C::NT, C::PREFETCH ? 3 : 1) step_kernel(Bank b
     // the next step's CTAs may start their independent part now; they wait in
     // cudaGridDependencySynchronize() until this grid has completed
     cudaTriggerProgrammaticLaunchCompletion();
-    if (tid < 12) {
-        reinterpret_cast<int4*>(&tk)[tid] = __ldg(reinterpret_cast<const int4*>(tasks + blockIdx.x) + tid);
-    } else if (tid >= 32 && tid < 37) {
-        const int j = tid - 32;
-        if (rs_dev) reinterpret_cast<int4*>(&rs)[j] = __ldcg(reinterpret_cast<const int4*>(rs_dev) + j);
-    }
-    if (!rs_dev && tid == 64) rs = rs_val;
+    if (tid < kTaskVec) reinterpret_cast<int4*>(&tk)[tid] = __ldg(reinterpret_cast<const int4*>(tasks + blockIdx.x) + tid);
+    if (tid == 64) rs = rs_val;
     __syncthreads();
-    const long long c = rs.step_base + step_in_batch;
+    const long long c = rs.step_base;
     const int kb = MULTI ? bank.kb : 1;
     if (tk.kind == 1) {
         cudaGridDependencySynchronize();
@@ -1090,7 +1083,7 @@ __global__ void __launch_bounds__(C::NT) pool_kernel(Bank bank, const Task* __re
     __shared__ int s_last;
     const int tid = threadIdx.x;
     const PoolCta pm = map[blockIdx.x];
-    if (tid < 12) reinterpret_cast<int4*>(&tk)[tid] = __ldg(reinterpret_cast<const int4*>(slots + pm.slot) + tid);
+    if (tid < kTaskVec) reinterpret_cast<int4*>(&tk)[tid] = __ldg(reinterpret_cast<const int4*>(slots + pm.slot) + tid);
     if (tid == 64) rs = rs_val;
     __syncthreads();
     const long long c = rs.step_base;
@@ -1185,26 +1178,96 @@ __global__ void __launch_bounds__(NT) spectra_kernel(const SpectraJob* __restric
 // Spread tasks of levels >= 1 with several base blocks per step: their own
 // launch beside the step chain (they feed only the levels' deferred fires).
 constexpr int kSideNT = 256;
-__global__ void __launch_bounds__(kSideNT) spread_kernel(const Task* __restrict__ tasks, RunState rs_val,
-                                                        const RunState* rs_dev, int step_in_batch) {
+__global__ void __launch_bounds__(kSideNT) spread_kernel(const Task* __restrict__ tasks, long long step) {
     __shared__ float4 red[kSideNT];
     __shared__ __align__(16) Task tk;
-    __shared__ long long step_base;
     const int tid = threadIdx.x;
-    if (tid < 12) reinterpret_cast<int4*>(&tk)[tid] = __ldg(reinterpret_cast<const int4*>(tasks + blockIdx.x) + tid);
-    if (tid == 32) step_base = rs_dev ? __ldcg(&rs_dev->step_base) : rs_val.step_base;
+    if (tid < kTaskVec) reinterpret_cast<int4*>(&tk)[tid] = __ldg(reinterpret_cast<const int4*>(tasks + blockIdx.x) + tid);
     __syncthreads();
-    spread_body<kSideNT>(tk, step_base + step_in_batch, red, 1);
+    spread_body<kSideNT>(tk, step, red, 1);
 }
 
-cudaError_t launch_side_spreads(int grid, const Task* tasks, const RunState& rs, const RunState* rs_dev,
-                                int step_in_batch, cudaStream_t st) {
+cudaError_t launch_side_spreads(int grid, const Task* tasks, long long step, cudaStream_t st) {
     if (grid <= 0) return cudaSuccess;
-    spread_kernel<<<grid, kSideNT, 0, st>>>(tasks, rs, rs_dev, step_in_batch);
+    spread_kernel<<<grid, kSideNT, 0, st>>>(tasks, step);
     return cudaGetLastError();
 }
 
-__global__ void set_state_kernel(RunState* dst, RunState v) { *dst = v; }
+// End of a block-parallel call (wide.cu): the partial sums that the spread
+// tasks of the steps up to c1 - 1 would have built for the blocks in
+// progress, by the same code (one CTA per tile of bins and row; a tile whose
+// slices all come later has nothing to do).  NT, LANES: as the handle's
+// spread tasks.
+template <int NT, int LANES>
+__global__ void __launch_bounds__(NT) wide_partials_kernel(const int4* __restrict__ map, const WLevel* __restrict__ lv,
+                                                           int tp, long long c1, int kb) {
+    extern __shared__ float4 dyn_smem[];
+    __shared__ __align__(16) Task tk;
+    const int4 e = map[blockIdx.x];
+    const WLevel& l = lv[e.x];
+    const int T = 1 << l.logT, cs = l.cs;
+    if (T > 1) {
+        // bins of slice j of n start at (j cs / n) & ~1
+        auto start = [&](long long j, int n) { return j >= n ? cs : (int)((j * cs / n) & ~1LL); };
+        const long long q = c1 + l.s_blocks;
+        const int phi = (int)(q & (T - 1));
+        bool need;
+        if (kb > 1) {   // slices since the step in which the level's previous block completed
+            const long long bt = q >> l.logT, x = bt * T - l.s_blocks - 1;
+            const long long sprev = x >= 0 ? x / kb : -((-x + kb - 1) / kb);
+            const int n = T / kb;
+            const long long j = c1 / kb - 1 - sprev;
+            need = j > 0 && e.y < start(j, n);
+        } else if (l.dfer) {   // slice T - 1 at the previous fire's step, then 0, 1, ...
+            need = e.y < start(phi, T) || e.w > start(T - 1, T);
+        } else {
+            need = phi > 0 && e.y < start(phi, T - 1);
+        }
+        if (!need) return;
+    }
+    if (threadIdx.x == 0) {
+        Task t{};
+        t.kind = 1;
+        t.N = l.N;
+        t.P = l.P;
+        t.slots = l.slots;
+        t.T = T;
+        t.s_blocks = l.s_blocks;
+        t.cs = cs;
+        t.k0 = e.y;
+        t.k1 = e.w;
+        t.p_lo = l.p_lo + e.z * tp;
+        t.in_ch = min(l.P, t.p_lo + tp);
+        t.out_ch = e.z;
+        t.dfer = l.dfer;
+        t.H = const_cast<float2*>(l.H);
+        t.X = l.X;
+        t.Yp = l.Yp;
+        tk = t;
+    }
+    __syncthreads();
+    if constexpr (NT == 256) {
+        if (kb > 1 && T == 1) {
+            if (kb == 2) spread_multi<NT, 2>(tk, c1 - 1, dyn_smem);
+            else spread_multi<NT, 4>(tk, c1 - 1, dyn_smem);
+            return;
+        }
+    }
+    spread_lanes<NT, LANES>(tk, c1 - 1, dyn_smem, 1);
+}
+
+cudaError_t launch_wide_partials(int nt, int lanes, int grid, const int4* map, const WLevel* lv, int tp, long long c1,
+                                 int kb, cudaStream_t st) {
+    if (grid <= 0) return cudaSuccess;
+    const size_t red = sizeof(float4) * (size_t)nt;
+    if (nt == 512) wide_partials_kernel<512, 64><<<grid, 512, red, st>>>(map, lv, tp, c1, kb);
+    else if (nt == 1024) wide_partials_kernel<1024, 64><<<grid, 1024, red, st>>>(map, lv, tp, c1, kb);
+    else if (lanes == 32) wide_partials_kernel<256, 32><<<grid, 256, red, st>>>(map, lv, tp, c1, kb);
+    else if (lanes == 128) wide_partials_kernel<256, 128><<<grid, 256, red, st>>>(map, lv, tp, c1, kb);
+    else if (lanes == 256) wide_partials_kernel<256, 256><<<grid, 256, red, st>>>(map, lv, tp, c1, kb);
+    else wide_partials_kernel<256, 64><<<grid, 256, red, st>>>(map, lv, tp, c1, kb);
+    return cudaGetLastError();
+}
 
 // ---------------------------------------------------------------------------
 // Host-side launchers.
@@ -1259,10 +1322,10 @@ cudaError_t prepare_kernels() {
     e = cudaFuncSetAttribute(step_kernel<Cls0, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s0);
     if (e != cudaSuccess) return e;
     e = cudaFuncSetAttribute(step_kernel<Cls1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)std::max(class_smem_bytes(1, Cls1::MAXN), kWholeSmSmem));
+                             (int)class_smem_bytes(1, Cls1::MAXN));
     if (e != cudaSuccess) return e;
     e = cudaFuncSetAttribute(step_kernel<Cls2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)std::max(class_smem_bytes(2, Cls2::MAXN), kWholeSmSmem));
+                             (int)class_smem_bytes(2, Cls2::MAXN));
     if (e != cudaSuccess) return e;
     e = cudaFuncSetAttribute(spectra_kernel<512, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)(12 * 16384));
@@ -1279,49 +1342,34 @@ cudaError_t prepare_kernels() {
 }
 
 cudaError_t launch_step_class(int cls, int grid, int maxN, const Bank& bank, const Task* tasks, const RunState& rs,
-                              const RunState* rs_dev, int step_in_batch, cudaStream_t st, bool pdl, int prio,
-                              bool whole_sm) {
+                              cudaStream_t st, bool pdl) {
     if (grid <= 0) return cudaSuccess;
-    if (cls == 3) return launch_cluster_fire(grid, bank, tasks, rs, rs_dev, step_in_batch, st, pdl, prio);
-    static int least = 0, greatest = 0;
-    static const bool have_range = cudaDeviceGetStreamPriorityRange(&least, &greatest) == cudaSuccess;
+    if (cls == 3) return launch_cluster_fire(grid, bank, tasks, rs, st, pdl);
     // programmatic dependent launch: this step's CTAs may be scheduled while
     // the previous step kernel in the stream finishes (their static prologue
     // reads only data no step writes; see cudaGridDependencySynchronize).
     // Callers pass pdl = false when the preceding work is anything else.
-    // A priority lets the block scheduler place the step chain's CTAs ahead
-    // of deferred fires that run beside it.
-    cudaLaunchAttribute attr[2];
-    int na = 0;
-    if (pdl) {
-        attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[na].val.programmaticStreamSerializationAllowed = 1;
-        ++na;
-    }
-    if (prio != 0 && have_range) {
-        attr[na].id = cudaLaunchAttributePriority;
-        attr[na].val.priority = prio > 0 ? greatest : least;
-        ++na;
-    }
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(kNT[cls]);
     cfg.dynamicSmemBytes = step_smem_bytes(cls, maxN, bank);
-    if (whole_sm && cls != 0) cfg.dynamicSmemBytes = std::max(cfg.dynamicSmemBytes, kWholeSmSmem);
     cfg.stream = st;
     cfg.attrs = attr;
-    cfg.numAttrs = na;
+    cfg.numAttrs = pdl ? 1 : 0;
     switch (cls) {
         case 0:
-            if (bank.kb > 1) return cudaLaunchKernelEx(&cfg, step_kernel<Cls0, true>, bank, tasks, rs, rs_dev, step_in_batch);
+            if (bank.kb > 1) return cudaLaunchKernelEx(&cfg, step_kernel<Cls0, true>, bank, tasks, rs);
             switch (bank.tb) {   // the handle's spread tile width
-                case 64: return cudaLaunchKernelEx(&cfg, step_kernel<Cls0, false, 32>, bank, tasks, rs, rs_dev, step_in_batch);
-                case 256: return cudaLaunchKernelEx(&cfg, step_kernel<Cls0, false, 128>, bank, tasks, rs, rs_dev, step_in_batch);
-                case 512: return cudaLaunchKernelEx(&cfg, step_kernel<Cls0, false, 256>, bank, tasks, rs, rs_dev, step_in_batch);
-                default: return cudaLaunchKernelEx(&cfg, step_kernel<Cls0>, bank, tasks, rs, rs_dev, step_in_batch);
+                case 64: return cudaLaunchKernelEx(&cfg, step_kernel<Cls0, false, 32>, bank, tasks, rs);
+                case 256: return cudaLaunchKernelEx(&cfg, step_kernel<Cls0, false, 128>, bank, tasks, rs);
+                case 512: return cudaLaunchKernelEx(&cfg, step_kernel<Cls0, false, 256>, bank, tasks, rs);
+                default: return cudaLaunchKernelEx(&cfg, step_kernel<Cls0>, bank, tasks, rs);
             }
-        case 1: return cudaLaunchKernelEx(&cfg, step_kernel<Cls1>, bank, tasks, rs, rs_dev, step_in_batch);
-        default: return cudaLaunchKernelEx(&cfg, step_kernel<Cls2>, bank, tasks, rs, rs_dev, step_in_batch);
+        case 1: return cudaLaunchKernelEx(&cfg, step_kernel<Cls1>, bank, tasks, rs);
+        default: return cudaLaunchKernelEx(&cfg, step_kernel<Cls2>, bank, tasks, rs);
     }
 }
 
@@ -1335,11 +1383,6 @@ cudaError_t launch_spectra(int cls, int njobs, int maxN, const SpectraJob* jobs,
         case 1: spectra_kernel<256, 4><<<njobs, 256, smem, st>>>(jobs, W, wlog); break;
         default: spectra_kernel<512, 8><<<njobs, 512, smem, st>>>(jobs, W, wlog); break;
     }
-    return cudaGetLastError();
-}
-
-cudaError_t launch_set_state(RunState* dst, const RunState& v, cudaStream_t st) {
-    set_state_kernel<<<1, 1, 0, st>>>(dst, v);
     return cudaGetLastError();
 }
 
