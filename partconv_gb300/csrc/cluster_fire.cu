@@ -237,11 +237,13 @@ __global__ void __cluster_dims__(kC, 1, 1) __launch_bounds__(kNT)
     const int npart = tk.k0 > 0 ? tk.k0 : 1;
     const size_t rstride = 2 * (size_t)cs;
     auto mac = [&](int pos, float2 x) {
-        float2 y = cmul(x, __ldg(&tk.H[pos]));
-        if (use_x1) y = cadd(y, cmul(__ldcg(&X1[pos]), __ldg(&tk.H[cs + pos])));
-        if (use_yp)
-            for (int qr = 0; qr < npart; ++qr) y = cadd(y, __ldcg(&Ypb[qr * rstride + pos]));
-        return y;
+        float2 a = make_float2(0.f, 0.f);
+        if (use_yp) {
+            a = __ldcg(&Ypb[pos]);
+            for (int qr = 1; qr < npart; ++qr) a = cadd(a, __ldcg(&Ypb[qr * rstride + pos]));
+        }
+        if (use_x1) a = cadd(a, cmul(__ldcg(&X1[pos]), __ldg(&tk.H[cs + pos])));
+        return cadd(cmul(x, __ldg(&tk.H[pos])), a);
     };
     const int np = pair_count(g);
     float2 zo[kMaxPairs][2];
@@ -294,8 +296,10 @@ __global__ void __cluster_dims__(kC, 1, 1) __launch_bounds__(kNT)
     extern __shared__ float4 dyn_smem[];
     cg::cluster_group cl = cg::this_cluster();
     const int tid = threadIdx.x;
+    cudaTriggerProgrammaticLaunchCompletion();
     const int2 e = map[blockIdx.x / kC];
     const WLevel& l = a.lv[e.x];
+    cudaGridDependencySynchronize();
     const long long b0 = (a.c0 + l.s_blocks) >> l.logT;
     const int nb = (int)(((a.c0 + a.nsteps + l.s_blocks) >> l.logT) - b0);
     if (e.y >= nb) return;   // the whole cluster
@@ -511,9 +515,18 @@ cudaError_t prepare_cluster_kernels() {
 
 cudaError_t launch_wide_cluster(bool inverse, int grid, const int2* map, const WArgs& a, cudaStream_t st) {
     if (grid <= 0) return cudaSuccess;
-    if (inverse) wide_cluster_kernel<true><<<grid * kC, kNT, cluster_smem_bytes(), st>>>(map, a);
-    else wide_cluster_kernel<false><<<grid * kC, kNT, cluster_smem_bytes(), st>>>(map, a);
-    return cudaGetLastError();
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid * kC);
+    cfg.blockDim = dim3(kNT);
+    cfg.dynamicSmemBytes = cluster_smem_bytes();
+    cfg.stream = st;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return inverse ? cudaLaunchKernelEx(&cfg, wide_cluster_kernel<true>, map, a)
+                   : cudaLaunchKernelEx(&cfg, wide_cluster_kernel<false>, map, a);
 }
 
 cudaError_t launch_cluster_filter_level(int N, int P, int cs, unsigned bcurr, const float2* H, float2* X,

@@ -42,7 +42,7 @@ constexpr int kWideMinSteps = 8;
 // (one ring row per block of every level) within kWideBytes, so that they and
 // the summed spectra, as many again, are still in the 129 MB L2 when the next
 // kernel reads them.
-constexpr size_t kWideBytes = (size_t)32 << 20;
+constexpr size_t kWideBytes = (size_t)256 << 20;
 constexpr int kWideMinChunk = 32, kWideMaxChunk = 4096;
 constexpr int kMinN0 = 16;
 constexpr int kClasses = kNumClasses;
@@ -198,18 +198,15 @@ struct pc_handle {
         std::vector<int> upto;   // upto[n]: CTAs whose first block can complete within n + 1 steps
     };
     std::vector<WGroup> wgroups;
-    struct WMac {           // one launch of the sum over parts
-        int G;
-        const int2* map;
-        std::vector<int> upto;
-    };
-    std::vector<WMac> wmacs;
+    const int4* wmac_map[2] = {};     // the sum over parts: default tiles, any
+    std::vector<int> wmac_upto[2];
     int w_part_nt = 0, w_part_lanes = 0, w_part_n = 0;   // partial sums at the end of a call
     const int4* w_part_map = nullptr;
     const WLevel* d_wlv = nullptr;
     const float2* d_wtab = nullptr;
     const int* d_lv0 = nullptr;    // level-0 index of every PC
     int n_zero = 0, max_ring = 0;
+    bool wide_ok = true;           // every ring's element offsets fit 32 bits
     bool mixed = false;
 
     // run() staging and Relaxed carry (planar [n_out][N0])
@@ -324,6 +321,19 @@ int launch_step_direct(pc_handle* h, const RunState& rs, cudaStream_t st, bool f
     return PC_OK;
 }
 
+// Thread groups of the handle's spread tasks (they fix the order of the
+// partial sums): step_kernel runs them with the level-0 class's threads over
+// the tile width's lanes; with several base blocks per step the levels' run
+// in spread_kernel, level 0's (spread_multi) with the default width.
+int spread_threads(const pc_handle* h) { return h->KB > 1 ? 256 : class_threads(h->l0_class); }
+int spread_lane_count(const pc_handle* h) { return h->l0_class == 0 ? h->TB / 2 : spread_task_bins() / 2; }
+// parts each thread group of a full spread task sums
+int parts_per_group(const pc_handle* h, bool l0) {
+    const int lanes = l0 && h->KB > 1 ? spread_task_bins() / 2 : spread_lane_count(h);
+    const int G = spread_threads(h) / lanes;
+    return (h->TP + G - 1) / G;
+}
+
 // CTA maps of the block-parallel kernels, built on the host in the order in
 // which their first blocks complete, so a short call launches a prefix.
 struct WideMaps {
@@ -333,20 +343,16 @@ struct WideMaps {
         std::vector<std::pair<int, int2>> e;   // (first relative step at which the entry may have work, entry)
     };
     std::vector<G> groups;
-    struct Mc {
-        int G;
-        std::vector<std::pair<int, int2>> e;
-    };
-    std::vector<Mc> macs;
+    std::vector<std::pair<int, int4>> mac[2];
     std::vector<int4> part;
 
     size_t bytes() const {
-        size_t n = sizeof(int4) * part.size() + 256;
+        size_t n = sizeof(int4) * (part.size() + mac[0].size() + mac[1].size()) + 3 * 256;
         for (auto& g : groups) n += sizeof(int2) * g.e.size() + 256;
-        for (auto& m : macs) n += sizeof(int2) * m.e.size() + 256;
         return n;
     }
-    static std::vector<int> prefix(const std::vector<std::pair<int, int2>>& e, int C) {
+    template <class E>
+    static std::vector<int> prefix(const std::vector<std::pair<int, E>>& e, int C) {
         std::vector<int> u(C, 0);
         size_t j = 0;
         for (int n = 0; n < C; ++n) {   // a call of n + 1 steps: entries that start at step n or before
@@ -364,12 +370,13 @@ struct WideMaps {
             off += (n + 255) & ~(size_t)255;
             return dst;
         };
-        auto entries = [&](std::vector<std::pair<int, int2>>& e) {
+        auto entries = [&](auto& e) {
+            using E = decltype(e[0].second);
             std::stable_sort(e.begin(), e.end(), [](auto& a, auto& b) { return a.first < b.first; });
-            std::vector<int2> v;
+            std::vector<E> v;
             v.reserve(e.size());
             for (auto& x : e) v.push_back(x.second);
-            const int2* d = reinterpret_cast<const int2*>(put(v.data(), sizeof(int2) * v.size()));
+            const E* d = reinterpret_cast<const E*>(put(v.data(), sizeof(E) * v.size()));
             if (err == cudaSuccess) err = cudaStreamSynchronize(h->stream);
             return d;
         };
@@ -378,10 +385,9 @@ struct WideMaps {
             const int2* d = entries(g.e);
             h->wgroups.push_back({g.N, g.l0, g.cluster, d, prefix(g.e, h->C)});
         }
-        h->wmacs.clear();
-        for (auto& m : macs) {
-            const int2* d = entries(m.e);
-            h->wmacs.push_back({m.G, d, prefix(m.e, h->C)});
+        for (int x = 0; x < 2; ++x) {
+            h->wmac_map[x] = entries(mac[x]);
+            h->wmac_upto[x] = prefix(mac[x], h->C);
         }
         h->w_part_map = reinterpret_cast<const int4*>(put(part.data(), sizeof(int4) * part.size()));
         h->w_part_n = (int)part.size();
@@ -390,12 +396,7 @@ struct WideMaps {
 };
 
 void build_wide_maps(pc_handle* h, WideMaps& m) {
-    // thread groups of the handle's spread tasks (they fix the order of the
-    // partial sums): step_kernel runs them with the level-0 class's threads
-    // over the tile width's lanes; with several base blocks per step the
-    // levels' run in spread_kernel, level 0's with the default width
-    const int nt = h->KB > 1 ? 256 : class_threads(h->l0_class);
-    const int lanes = h->l0_class == 0 ? h->TB / 2 : spread_task_bins() / 2;
+    const int nt = spread_threads(h), lanes = spread_lane_count(h);
     const int nlv = (int)h->h_lv.size();
     h->w_part_nt = nt;
     h->w_part_lanes = lanes;
@@ -405,12 +406,6 @@ void build_wide_maps(pc_handle* h, WideMaps& m) {
         m.groups.push_back({N, l0, cluster, {}});
         return m.groups.back();
     };
-    auto mac = [&](int G) -> WideMaps::Mc& {
-        for (auto& x : m.macs)
-            if (x.G == G) return x;
-        m.macs.push_back({G, {}});
-        return m.macs.back();
-    };
     for (int li = 0; li < nlv; ++li) {
         const DevLevel& l = h->h_lv[li];
         const bool l0 = l.T == 1, cluster = h->lv_cls[li] == 3;
@@ -418,10 +413,15 @@ void build_wide_maps(pc_handle* h, WideMaps& m) {
         const int per = cluster ? 1 : wide_transforms_per_cta(l.N);
         auto& g = group(l.N, l0, cluster);
         for (int i = 0; i < nb; i += per) g.e.push_back({i * l.T, make_int2(li, i)});
-        const int G = l0 && h->KB > 1 ? 4 : nt / lanes, run = wide_run(G);
-        const int items = (nb + run - 1) / run * l.cs;
-        auto& mc = mac(G);
-        for (int i = 0; i < items; i += kWideMacNT) mc.e.push_back({i / l.cs * run * l.T, make_int2(li, i)});
+        if (h->TP == spread_task_parts() && parts_per_group(h, l0) == 4 && !(l0 && h->KB > 1)) {
+            for (int i = 0; i < nb; i += kMacSeg)
+                for (int k = 0; k < l.cs; k += kMacTile)
+                    m.mac[0].push_back({i * l.T, make_int4(li, k, i, std::min(nb, i + kMacSeg))});
+        } else {
+            const int items = (nb + kWideRun - 1) / kWideRun * l.cs;
+            for (int i = 0; i < items; i += kMacAnyNT)
+                m.mac[1].push_back({i / l.cs * kWideRun * l.T, make_int4(li, i, 0, 0)});
+        }
         // partial sums: one CTA per tile of bins and row
         const int QC = h->KB > 1 ? multi_fire_parts(h->N0, h->KB) : 2;
         const int p_lo = l0 ? (h->KB > 1 ? std::min(l.P, QC) : 2) : (h->dfl[li] ? 2 : 1);
@@ -535,7 +535,7 @@ int do_setup(pc_handle* h, int fs, int buffer_size, int n_in, int n_out, std::ve
 
     // state (zeroed by reset), laid out after the task table below
     struct StateOffsets {
-        std::vector<size_t> xring, pcout, X, Yp, yr;
+        std::vector<size_t> xring, pcout, X, Yp, yr;   // X, yr: cleared in part
         size_t mix = 0, carry = 0;
     } so;
     // Deferral window of each level (0: fires within its step).  Level L's
@@ -556,6 +556,7 @@ int do_setup(pc_handle* h, int fs, int buffer_size, int n_in, int n_out, std::ve
     std::vector<int> rin(npc), rl(nlv), dwin(nlv, 0);
     std::vector<int>& dfl = h->dfl;
     dfl.assign(nlv, 0);
+    h->wide_ok = true;
     {
         int li = 0;
         for (int i = 0; i < npc; ++i) {
@@ -647,7 +648,8 @@ int do_setup(pc_handle* h, int fs, int buffer_size, int n_in, int n_out, std::ve
                 l.cs = p.N[L] + 2;
                 l.rmask = rl[li] - 1;
                 l.pc = i;
-                l.slots = l.P + std::max((h->C + l.T - 1) / l.T, wide_run());
+                l.slots = l.P + std::max((h->C + l.T - 1) / l.T, kWideRun);
+                if ((long long)l.slots * l.cs >= (1LL << 31)) h->wide_ok = false;
                 {   // spread tasks sum parts >= 2 KB (level 0), >= 2 (deferred levels) or >= 1
                     const int p_lo = L == 0 ? (KB > 1 ? std::min(p.P[L], QC) : 2) : (dfl[li] ? 2 : 1);
                     const int np = p.P[L] - p_lo;
@@ -766,6 +768,7 @@ int do_setup(pc_handle* h, int fs, int buffer_size, int n_in, int n_out, std::ve
                     t.p_lo = p_lo + r * TP;
                     t.in_ch = std::min(l.P, p_lo + (r + 1) * TP);
                     t.out_ch = r;
+                    t.rmask = parts_per_group(h, l.T == 1);
                     t.lv_index = li;
                     t.dfer = dwin[li] > 0;
                     lists[sc][g].push_back(t);
@@ -858,6 +861,7 @@ int do_setup(pc_handle* h, int fs, int buffer_size, int n_in, int n_out, std::ve
                         t.p_lo = p_lo + q * TP;
                         t.in_ch = std::min(l.P, p_lo + (q + 1) * TP);
                         t.out_ch = q;
+                        t.rmask = parts_per_group(h, l.T == 1);
                         t.lv_index = li;
                         t.dfer = l.T > 1;
                         t.origin = origin;
@@ -933,13 +937,17 @@ int do_setup(pc_handle* h, int fs, int buffer_size, int n_in, int n_out, std::ve
     so.yr.resize(nlv);
     for (int li = 0; li < nlv; ++li) {
         const DevLevel& l = h->h_lv[li];
-        so.X[li] = cv.take(sizeof(float2) * (size_t)l.slots * l.cs);
         so.Yp[li] = cv.take(sizeof(float2) * 2 * (l.T == 1 ? KB : 1) * (size_t)l.npart * l.cs);
-        so.yr[li] = cv.take(sizeof(float) * (size_t)(l.rmask + 1));
     }
     so.mix = cv.take(sizeof(int) * n_out);
     so.carry = cv.take(sizeof(float) * (size_t)N0 * n_out);
     const size_t state_end = cv.take(0);
+    // spectrum and output rings: cleared in part (launch_wide_reset)
+    for (int li = 0; li < nlv; ++li) {
+        const DevLevel& l = h->h_lv[li];
+        so.X[li] = cv.take(sizeof(float2) * (size_t)l.slots * l.cs);
+        so.yr[li] = cv.take(sizeof(float) * (size_t)(l.rmask + 1));
+    }
 
     // block-parallel workspace: summed spectra of a chunk's blocks, mixed
     // outputs' samples, and the CTA maps
@@ -1032,7 +1040,9 @@ int do_setup(pc_handle* h, int fs, int buffer_size, int n_in, int n_out, std::ve
                 w.two = L == 0 || dfl[li];
                 w.p_lo = L == 0 && KB > 1 ? std::min(l.P, QC) : (w.two ? 2 : 1);
                 w.nrows = l.npart;
-                w.form = L == 0 && KB > 1 ? kFormMulti : (h->lv_cls[li] == 3 ? kFormCluster : kFormFire);
+                w.multi = L == 0 && KB > 1;
+                w.tp = TP;
+                w.tpg = parts_per_group(h, L == 0);
                 w.in_ch = d.in_ch;
                 w.out_ch = d.out_ch;
                 w.mix_mode = d.mix_mode;
@@ -1059,6 +1069,7 @@ int do_setup(pc_handle* h, int fs, int buffer_size, int n_in, int n_out, std::ve
         h->d_lv0 = reinterpret_cast<const int*>(A + off_lv0);
         h->d_wtab = reinterpret_cast<const float2*>(A + off_wtab);
         CK(wm.place(h, A + off_wmap), "upload maps");
+        CK(launch_wide_reset(h->d_wlv, nlv, h->stream), "clear rings");
     }
     // the level-0 class also runs spread tasks; its smem must fit its fires
     if (h->class_maxN[h->l0_class] == 0) h->class_maxN[h->l0_class] = N0;
@@ -1225,9 +1236,11 @@ int run_chunk(pc_handle* h, const IOView& view, int n, cudaStream_t st) {
            "window transforms");
         h->launches += grid > 0;
     }
-    for (auto& m : h->wmacs) {
-        CK(launch_wide_mac(m.G, h->TP, m.upto[n - 1], m.map, a, st), "sum over parts");
-        h->launches += 1;
+    for (int x = 0; x < 2; ++x) {
+        if (h->wmac_upto[x].empty()) continue;
+        const int grid = h->wmac_upto[x][n - 1];
+        CK(launch_wide_mac(x == 1, grid, h->wmac_map[x], a, st), "sum over parts");
+        h->launches += grid > 0;
     }
     for (auto& g : h->wgroups) {
         const int grid = g.upto[n - 1];
@@ -1247,17 +1260,10 @@ int run_chunk(pc_handle* h, const IOView& view, int n, cudaStream_t st) {
 // After a call's last chunk: the state one-block steps would have left.
 int finish_wide(pc_handle* h, const IOView& view, cudaStream_t st) {
     WArgs a = wide_args(h, view, 0);
-    const long long t_end = h->frame_num * (long long)h->N0;
-    CK(launch_wide_ring(h->d_wlv, h->d_lv0, (int)h->h_pcs.size(), a, t_end, t_end - view.step0 * (long long)h->N0,
-                        h->max_ring, st),
-       "input rings");
+    CK(launch_wide_state(h->w_part_nt, h->w_part_lanes, h->w_part_n, h->w_part_map, h->d_lv0,
+                         (int)h->h_pcs.size(), h->max_ring, a, st),
+       "state after the call");
     h->launches += 1;
-    if (h->w_part_n > 0) {
-        CK(launch_wide_partials(h->w_part_nt, h->w_part_lanes, h->w_part_n, h->w_part_map, h->d_wlv, h->TP,
-                                h->frame_num, h->KB, st),
-           "partial sums");
-        h->launches += 1;
-    }
     return PC_OK;
 }
 
@@ -1267,7 +1273,7 @@ int finish_wide(pc_handle* h, const IOView& view, cudaStream_t st) {
 // for all but the last and again = true for all but the first.
 int run_steps(pc_handle* h, const IOView& view, long long nsteps, cudaStream_t st, bool again = false,
               bool more = false) {
-    if (nsteps < kWideMinSteps && !again && !more) {
+    if (!h->wide_ok || (nsteps < kWideMinSteps && !again && !more)) {
         RunState rs;
         rs.io = view;
         for (long long done = 0; done < nsteps; done += h->KB) {
@@ -1582,6 +1588,7 @@ int pc_reset(pc_handle* h) {
     if (!h->ready) return PC_OK;
     CK(cudaSetDevice(h->device), "cudaSetDevice");
     CK(cudaMemsetAsync(h->arena + h->state_off, 0, h->state_bytes, h->stream), "reset");
+    CK(launch_wide_reset(h->d_wlv, (int)h->h_lv.size(), h->stream), "reset");
     CK(cudaStreamSynchronize(h->stream), "reset sync");
     return PC_OK;
 }

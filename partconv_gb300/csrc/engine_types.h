@@ -63,7 +63,8 @@ struct DevPC {
 // number of partial-sum rows to add (0 means 1).  kind 1 (spread): partial
 // FDL MAC over bins [k0, k1) and parts [p_lo, in_ch) (in_ch 0: up to P) of
 // a level's next block, written to partial-sum row out_ch; a spread task
-// keeps its bins per task (the tile width) in M (0: the default).
+// keeps its bins per task (the tile width) in M (0: the default) and its
+// parts per thread group in rmask (0: its parts divided evenly).
 struct Task {
     int kind, N, logN, P;
     int T, s_blocks, cs, rmask;

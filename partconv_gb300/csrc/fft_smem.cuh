@@ -32,11 +32,50 @@ namespace pcg {
 __device__ __forceinline__ float2 cmul(float2 a, float2 b) {
     return make_float2(__fmaf_rn(a.x, b.x, -__fmul_rn(a.y, b.y)), __fmaf_rn(a.x, b.y, __fmul_rn(a.y, b.x)));
 }
-// acc + a b, two fused multiply-adds per component
-__device__ __forceinline__ float2 cmac(float2 acc, float2 a, float2 b) {
-    acc.x = __fmaf_rn(-a.y, b.y, __fmaf_rn(a.x, b.x, acc.x));
-    acc.y = __fmaf_rn(a.y, b.x, __fmaf_rn(a.x, b.y, acc.y));
+// acc + x h, two fused multiply-adds per component: first with h.x, then with
+// h.y, the order in which pairs of components fill packed instructions
+// (cmac2)
+__device__ __forceinline__ float2 cmac(float2 acc, float2 x, float2 h) {
+    acc.x = __fmaf_rn(-x.y, h.y, __fmaf_rn(x.x, h.x, acc.x));
+    acc.y = __fmaf_rn(x.x, h.y, __fmaf_rn(x.y, h.x, acc.y));
     return acc;
+}
+
+// Packed pairs of float32 (one 64-bit register pair, Blackwell's f32x2
+// instructions: half the issue slots of the scalar ones, same rounding)
+using f32x2 = unsigned long long;
+__device__ __forceinline__ f32x2 pack2(float a, float b) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float2 unpack2(f32x2 v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ f32x2 swap2(f32x2 v) {
+    const float2 t = unpack2(v);
+    return pack2(t.y, t.x);
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+    f32x2 d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+// cmac with x as a packed pair, xs = swap2(x), hr = (h.x, h.x), hi = (-h.y, h.y)
+__device__ __forceinline__ f32x2 cmac2(f32x2 acc, f32x2 x, f32x2 xs, f32x2 hr, f32x2 hi) {
+    return fma2(xs, hi, fma2(x, hr, acc));
 }
 __device__ __forceinline__ float2 cadd(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
 __device__ __forceinline__ float2 csub(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }

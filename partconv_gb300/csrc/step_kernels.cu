@@ -86,9 +86,10 @@ __host__ __device__ constexpr size_t fire_smem_bytes(int N, bool prefetch) {
 // ---------------------------------------------------------------------------
 // Spread: the streaming FDL MAC over the task's bins [k0, k1) and parts
 // [p_lo, p_hi).  NT threads form G = NT / LANES part-groups of LANES
-// threads; thread t owns bins k0 + 2 (t mod LANES), +1 (one float4) and sums
-// parts p_lo + g, + G, ... (g = t / LANES); the groups are added in order
-// through shared memory.  Bins per task (2 LANES; a tile shape the autotuner
+// threads; thread t owns bins k0 + 2 (t mod LANES), +1 (one float4) and group
+// g = t / LANES sums the g-th of G runs of consecutive parts; the groups
+// are added in order through shared memory (the block-parallel sum, wide.cu,
+// keeps this order with one running sum at a time).  Bins per task (2 LANES; a tile shape the autotuner
 // picks per handle) travel in the task's M field, 0 meaning kSpreadBins;
 // each width is its own instantiation (constant strides): the step kernel
 // is instantiated per width and launched for the handle's width.  Parts per task
@@ -134,25 +135,23 @@ __device__ __forceinline__ void spread_lanes(const Task& tk, long long c, float4
     if (active) {
         constexpr int U = 4;   // parts whose loads are in flight together
         const int R = tk.slots;
-        const int Gm = G % R;  // slot step between a group's consecutive parts
-        int sl0 = (int)imod(bt - (tk.p_lo + g), R);   // slot of part p0
-        for (int p0 = tk.p_lo + g; p0 < p_hi; p0 += U * G) {
+        const int tg = tk.rmask > 0 ? tk.rmask : (p_hi - tk.p_lo + G - 1) / G;   // parts per group
+        const int pb = tk.p_lo + g * tg, pe = min(p_hi, pb + tg);
+        int sl = (int)imod(bt - pb, R);   // slot of part p
+        for (int p0 = pb; p0 < pe; p0 += U) {
             float4 xv[U], hv[U];
-            int sl = sl0;
 #pragma unroll
             for (int u = 0; u < U; ++u) {
-                const int p = p0 + u * G;
-                if (p < p_hi) {
+                const int p = p0 + u;
+                if (p < pe) {
                     xv[u] = __ldcg(X4 + (size_t)sl * rs4);
                     hv[u] = __ldg(H4 + (size_t)p * rs4);
                 }
-                sl -= Gm;
-                if (sl < 0) sl += R;
+                sl = sl == 0 ? R - 1 : sl - 1;
             }
-            sl0 = sl;
 #pragma unroll
             for (int u = 0; u < U; ++u)
-                if (p0 + u * G < p_hi) acc = f4mac(acc, xv[u], hv[u]);
+                if (p0 + u < pe) acc = f4mac(acc, xv[u], hv[u]);
         }
     }
     if (G > 1) {
@@ -182,8 +181,8 @@ __device__ __forceinline__ void spread_body(const Task& tk, long long c, float4*
 // Level 0 with K base blocks per step: parts [p_lo, p_hi) of the next
 // step's K blocks bt_j = c + 1 + j (the task's c is the step's last base
 // step) over one slice of bins: each filter row is loaded once for the K
-// blocks.  Group g sums parts p_lo + g, p_lo + g + G, ...; groups are added
-// in order, per block.
+// blocks.  Groups of consecutive parts as in spread_lanes, added in order,
+// per block.
 template <int NT, int KM>
 __device__ __forceinline__ void spread_multi(const Task& tk, long long c, float4* red) {
     constexpr int G = NT / kSpreadLanes;
@@ -205,15 +204,15 @@ __device__ __forceinline__ void spread_multi(const Task& tk, long long c, float4
     for (int j = 0; j < KM; ++j) acc[j] = make_float4(0.f, 0.f, 0.f, 0.f);
     if (active) {
         const int R = tk.slots;
-        const int Gm = G % R;
-        int sl0 = (int)imod(bt0 - (tk.p_lo + g), R);   // slot of block bt0 - p for the group's part p
-        for (int p0 = tk.p_lo + g; p0 < p_hi; p0 += U * G) {
+        const int tg = tk.rmask > 0 ? tk.rmask : (p_hi - tk.p_lo + G - 1) / G;
+        const int pb = tk.p_lo + g * tg, pe = min(p_hi, pb + tg);
+        int sl = (int)imod(bt0 - pb, R);   // slot of block bt0 - p for the group's part p
+        for (int p0 = pb; p0 < pe; p0 += U) {
             float4 xv[U][KM], hv[U];
-            int sl = sl0;
 #pragma unroll
             for (int u = 0; u < U; ++u) {
-                if (p0 + u * G < p_hi) {
-                    hv[u] = __ldg(H4 + (size_t)(p0 + u * G) * rs4);
+                if (p0 + u < pe) {
+                    hv[u] = __ldg(H4 + (size_t)(p0 + u) * rs4);
                     int sj = sl;
 #pragma unroll
                     for (int j = 0; j < KM; ++j) {   // blocks bt0 + j - p: consecutive slots
@@ -221,13 +220,11 @@ __device__ __forceinline__ void spread_multi(const Task& tk, long long c, float4
                         sj = (sj + 1 == R) ? 0 : sj + 1;
                     }
                 }
-                sl -= Gm;
-                if (sl < 0) sl += R;
+                sl = sl == 0 ? R - 1 : sl - 1;
             }
-            sl0 = sl;
 #pragma unroll
             for (int u = 0; u < U; ++u)
-                if (p0 + u * G < p_hi) {
+                if (p0 + u < pe) {
 #pragma unroll
                     for (int j = 0; j < KM; ++j) acc[j] = f4mac(acc[j], xv[u][j], hv[u]);
                 }
@@ -1118,6 +1115,7 @@ __global__ void __launch_bounds__(C::NT) pool_kernel(Bank bank, const Task* __re
         tk.k0 = k0;
         tk.k1 = min(hi, k0 + kSpreadBins);
         tk.M = 0;        // default bins per task
+        tk.rmask = 0;    // parts divided evenly over the thread groups
         tk.p_lo = p_lo;
         tk.in_ch = 0;    // all parts from p_lo
         tk.out_ch = 0;   // partial-sum row 0
@@ -1196,15 +1194,30 @@ cudaError_t launch_side_spreads(int grid, const Task* tasks, long long step, cud
 // End of a block-parallel call (wide.cu): the partial sums that the spread
 // tasks of the steps up to c1 - 1 would have built for the blocks in
 // progress, by the same code (one CTA per tile of bins and row; a tile whose
-// slices all come later has nothing to do).  NT, LANES: as the handle's
-// spread tasks.
+// slices all come later has nothing to do), and, by ring_ctas CTAs per PC,
+// the call's newest samples (at most a ring's worth) in the input rings.
+// NT, LANES: as the handle's spread tasks.
 template <int NT, int LANES>
-__global__ void __launch_bounds__(NT) wide_partials_kernel(const int4* __restrict__ map, const WLevel* __restrict__ lv,
-                                                           int tp, long long c1, int kb) {
+__global__ void __launch_bounds__(NT) wide_state_kernel(const int4* __restrict__ map, int n_part,
+                                                        const int* __restrict__ lv0, int ring_ctas, WArgs a) {
     extern __shared__ float4 dyn_smem[];
     __shared__ __align__(16) Task tk;
+    cudaTriggerProgrammaticLaunchCompletion();
+    cudaGridDependencySynchronize();
+    const long long c1 = a.c0;
+    const int kb = a.kb;
+    if ((int)blockIdx.x >= n_part) {
+        const int j = (int)blockIdx.x - n_part;
+        const WLevel& l = a.lv[lv0[j / ring_ctas]];
+        const long long t_end = c1 * a.N0, t_in0 = a.io.step0 * (long long)a.N0;
+        const int n = (int)min(t_end - t_in0, (long long)l.rin_mask + 1);
+        const float* in = a.io.in + (long long)l.in_ch * a.io.in_ch + (t_end - n - t_in0) * a.io.in_sample;
+        for (int i = (j % ring_ctas) * NT + (int)threadIdx.x; i < n; i += ring_ctas * NT)
+            l.xring[(t_end - n + i) & l.rin_mask] = in[i * a.io.in_sample] * l.scale;
+        return;
+    }
     const int4 e = map[blockIdx.x];
-    const WLevel& l = lv[e.x];
+    const WLevel& l = a.lv[e.x];
     const int T = 1 << l.logT, cs = l.cs;
     if (T > 1) {
         // bins of slice j of n start at (j cs / n) & ~1
@@ -1236,9 +1249,10 @@ __global__ void __launch_bounds__(NT) wide_partials_kernel(const int4* __restric
         t.cs = cs;
         t.k0 = e.y;
         t.k1 = e.w;
-        t.p_lo = l.p_lo + e.z * tp;
-        t.in_ch = min(l.P, t.p_lo + tp);
+        t.p_lo = l.p_lo + e.z * l.tp;
+        t.in_ch = min(l.P, t.p_lo + l.tp);
         t.out_ch = e.z;
+        t.rmask = l.tpg;
         t.dfer = l.dfer;
         t.H = const_cast<float2*>(l.H);
         t.X = l.X;
@@ -1256,17 +1270,34 @@ __global__ void __launch_bounds__(NT) wide_partials_kernel(const int4* __restric
     spread_lanes<NT, LANES>(tk, c1 - 1, dyn_smem, 1);
 }
 
-cudaError_t launch_wide_partials(int nt, int lanes, int grid, const int4* map, const WLevel* lv, int tp, long long c1,
-                                 int kb, cudaStream_t st) {
-    if (grid <= 0) return cudaSuccess;
-    const size_t red = sizeof(float4) * (size_t)nt;
-    if (nt == 512) wide_partials_kernel<512, 64><<<grid, 512, red, st>>>(map, lv, tp, c1, kb);
-    else if (nt == 1024) wide_partials_kernel<1024, 64><<<grid, 1024, red, st>>>(map, lv, tp, c1, kb);
-    else if (lanes == 32) wide_partials_kernel<256, 32><<<grid, 256, red, st>>>(map, lv, tp, c1, kb);
-    else if (lanes == 128) wide_partials_kernel<256, 128><<<grid, 256, red, st>>>(map, lv, tp, c1, kb);
-    else if (lanes == 256) wide_partials_kernel<256, 256><<<grid, 256, red, st>>>(map, lv, tp, c1, kb);
-    else wide_partials_kernel<256, 64><<<grid, 256, red, st>>>(map, lv, tp, c1, kb);
-    return cudaGetLastError();
+template <int NT, int LANES>
+static cudaError_t launch_state(int n_part, const int4* map, const int* lv0, int npc, int ring_ctas,
+                                const WArgs& a, cudaStream_t st) {
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(n_part + npc * ring_ctas));
+    cfg.blockDim = dim3(NT);
+    cfg.dynamicSmemBytes = sizeof(float4) * NT;
+    cfg.stream = st;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, wide_state_kernel<NT, LANES>, map, n_part, lv0, ring_ctas, a);
+}
+
+cudaError_t launch_wide_state(int nt, int lanes, int n_part, const int4* map, const int* lv0, int npc, int max_ring,
+                              const WArgs& a, cudaStream_t st) {
+    // about four samples per thread, fewer CTAs for many PCs
+    const int ring_ctas = std::max(1, std::min(max_ring / (4 * nt), 4096 / npc));
+    if (nt == 512) return launch_state<512, 64>(n_part, map, lv0, npc, ring_ctas, a, st);
+    if (nt == 1024) return launch_state<1024, 64>(n_part, map, lv0, npc, ring_ctas, a, st);
+    switch (lanes) {
+        case 32: return launch_state<256, 32>(n_part, map, lv0, npc, ring_ctas, a, st);
+        case 128: return launch_state<256, 128>(n_part, map, lv0, npc, ring_ctas, a, st);
+        case 256: return launch_state<256, 256>(n_part, map, lv0, npc, ring_ctas, a, st);
+        default: return launch_state<256, 64>(n_part, map, lv0, npc, ring_ctas, a, st);
+    }
 }
 
 // ---------------------------------------------------------------------------

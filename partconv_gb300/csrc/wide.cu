@@ -6,22 +6,26 @@
 // block.  A chunk of base steps is
 //   1. wide_fft   per block size: the window of every block that completes in
 //                 the chunk, real FFT, spectrum ring row b mod slots;
-//   2. wide_mac   all levels: Y_b = sum_p X_{b-p} H_p for runs of a few
-//                 consecutive blocks per thread and bin, with the run's window
-//                 of spectra in registers (each spectrum row is read once per
-//                 run and part instead of once per block and part, each
-//                 filter row once per run);
+//   2. wide_mac   all levels: Y_b = sum_p X_{b-p} H_p, a tile of bins through
+//                 a segment of blocks per CTA, filter and spectrum rows in
+//                 shared memory and the window of a run of blocks in registers
+//                 (each row is read once per segment instead of once per block
+//                 and part);
 //   3. wide_ifft  per block size, level 0 last: inverse FFT, output ring, and
 //                 for level 0 the sum of the levels' due samples and the output;
 //   4. wide_mix   outputs fed by several PCs, in PC order.
 // After the last chunk of a call the input rings and the partial sums of the
 // blocks in progress are brought to where one-block steps would have left
-// them (wide_ring, wide_partials), so pc_run can continue.
+// them (wide_state_kernel in step_kernels.cu), so pc_run can continue.
 //
 // Every block is computed with the float operations of the one-block steps
 // (step_kernels.cu) in the same order -- same butterflies and twiddles
 // (fft_reg.cuh), same grouping of the parts -- so a call's result does not
 // depend on how its steps were executed, bit for bit.
+//
+// The launches of a call overlap by programmatic dependent launch: a kernel
+// reads its CTA map and level descriptor, which no kernel writes, and then
+// waits for the kernel before it, in every CTA and before anything else.
 //
 // (the reference's counterpart of a long call is a loop over
 // PartConvMulti::run, src/partconvMulti.cpp:815-928 of ebattenberg/partconv)
@@ -39,6 +43,7 @@ namespace pcg {
 namespace {
 
 __device__ __forceinline__ int wmod(long long a, int m) {
+    if ((unsigned long long)a < 0x80000000ULL) return (int)((unsigned)a % (unsigned)m);   // a 32-bit division
     const long long r = a % m;
     return (int)(r < 0 ? r + m : r);
 }
@@ -54,8 +59,10 @@ __global__ void __launch_bounds__(RegFft<LOGN>::NT) wide_fft_kernel(const int2* 
     using F = RegFft<LOGN>;
     constexpr int N = F::N, TPT = F::TPT;
     extern __shared__ float4 dyn_smem[];
+    cudaTriggerProgrammaticLaunchCompletion();
     const int2 e = map[blockIdx.x];
     const WLevel& l = a.lv[e.x];
+    cudaGridDependencySynchronize();
     const int t = threadIdx.x % TPT, tr = threadIdx.x / TPT;
     float2* s = reinterpret_cast<float2*>(dyn_smem) + tr * F::SM;
     const long long b0 = blocks_before(l, a.c0);
@@ -117,17 +124,253 @@ __global__ void __launch_bounds__(RegFft<LOGN>::NT) wide_fft_kernel(const int2* 
 }
 
 // ---------------------------------------------------------------------------
-// 2. the sum over parts.  G: part groups per partial-sum row of the handle's
-// spread tasks (the parts p_lo + q tp + g, + G, ... of row q form one running
-// sum; a row is its groups added in order).
+// 2. the sum over parts: one thread per bin and run of RB consecutive blocks.
 // ---------------------------------------------------------------------------
-template <int G>
-__global__ void __launch_bounds__(kWideMacNT) wide_mac_kernel(const int2* __restrict__ map, WArgs a, int tp) {
-    constexpr int RB = wide_run(G);
-    constexpr int U = G > 8 ? G : 8;   // parts per unrolled batch
-    static_assert(U % RB == 0 && U % G == 0, "constant window rotation and groups");
-    const int2 e = map[blockIdx.x];
+// One bin's column of a level: filter rows and spectrum rows, walked from one
+// part to the next (offsets in elements).  SH: rows staged in shared memory,
+// else the level's own (L2).
+template <bool SH>
+struct MacCol {
+    const float2* H;   // row of the part at hand
+    const float2* X;
+    int cs, wrap;      // row stride; ring size in elements
+    int ox;            // spectrum of block (run's first) - p, for the part p at hand
+    __device__ __forceinline__ int back(int o) const {   // the block before
+        o -= cs;
+        return o < 0 ? o + wrap : o;
+    }
+    __device__ __forceinline__ int fwd(int o) const {
+        o += cs;
+        return o >= wrap ? o - wrap : o;
+    }
+    __device__ __forceinline__ f32x2 x(int o) const {
+        const f32x2* p = reinterpret_cast<const f32x2*>(X + o);
+        if constexpr (SH) return *p;
+        else return __ldcg(p);
+    }
+    __device__ __forceinline__ float2 h() const {
+        if constexpr (SH) return *H;
+        else return __ldg(H);
+    }
+};
+
+// Sums X_{b+j-p} H_p, j < RB, over n consecutive parts in groups of tg (one
+// running sum each, the groups added in order into row); c stands at the first
+// part on entry and after the last one on return.  The run's RB spectra under
+// part p stay in registers: part p + 1 needs one new one.  The loads of four
+// parts go together; with tg = 4 (TG4, the default tiles) they are a group.
+template <int RB, bool TG4, bool SH>
+__device__ __forceinline__ void sum_parts(MacCol<SH>& c, int n, int tg, f32x2 (&row)[RB]) {
+    constexpr int U = 4;
+    static_assert(RB % U == 0, "constant window rotation");
+    f32x2 acc[RB], w[RB], ws[RB];   // window: block (run's first) + d - first part at w[d mod RB], and its swapped pairs
+    {
+        int o = c.ox;
+#pragma unroll
+        for (int j = 0; j < RB; ++j) {
+            row[j] = acc[j] = 0;
+            w[j] = c.x(o);
+            ws[j] = swap2(w[j]);
+            o = c.fwd(o);
+        }
+    }
+    int left = tg;
+    for (int i0 = 0; i0 < n; i0 += RB) {
+#pragma unroll
+        for (int s = 0; s < RB / U; ++s) {
+            if (i0 + s * U >= n) break;
+            float2 h[U];
+            f32x2 nx[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (i0 + s * U + u < n) {
+                    h[u] = c.h();
+                    c.H += c.cs;
+                    c.ox = c.back(c.ox);
+                    nx[u] = c.x(c.ox);
+                }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                if (i0 + s * U + u >= n) break;
+                const int r = s * U + u;   // part index mod RB
+                const f32x2 hr = pack2(h[u].x, h[u].x), hi = pack2(-h[u].y, h[u].y);
+#pragma unroll
+                for (int j = 0; j < RB; ++j) {
+                    const int q = (j - r + RB) % RB;
+                    acc[j] = TG4 && u == 0 ? fma2(ws[q], hi, mul2(w[q], hr)) : cmac2(acc[j], w[q], ws[q], hr, hi);
+                }
+                const int q = (RB - 1 - r + RB) % RB;
+                w[q] = nx[u];
+                ws[q] = swap2(nx[u]);
+                if constexpr (!TG4) {
+                    if (--left == 0) {
+                        left = tg;
+#pragma unroll
+                        for (int j = 0; j < RB; ++j) {
+                            row[j] = add2(row[j], acc[j]);
+                            acc[j] = 0;
+                        }
+                    }
+                }
+            }
+            if constexpr (TG4) {
+#pragma unroll
+                for (int j = 0; j < RB; ++j) row[j] = i0 + s == 0 ? acc[j] : add2(row[j], acc[j]);
+            }
+        }
+    }
+    if constexpr (!TG4) {
+        if (left != tg) {
+#pragma unroll
+            for (int j = 0; j < RB; ++j) row[j] = add2(row[j], acc[j]);
+        }
+    }
+}
+
+// y = X_b H_0 + (X_{b-1} H_1 + rows) for the run's blocks, c at part 0
+template <int RB, bool SH>
+__device__ __forceinline__ void finish_run(const MacCol<SH>& c, const WLevel& l, const f32x2 (&ys)[RB], float2* Y,
+                                           int live) {
+    const bool rows = l.P > l.p_lo, x1 = l.two && l.P >= 2;
+    const float2 h0 = c.h();
+    const float2 h1 = x1 ? MacCol<SH>{c.H + c.cs, nullptr, 0, 0, 0}.h() : make_float2(0.f, 0.f);
+    float2 xm = x1 ? unpack2(c.x(c.back(c.ox))) : make_float2(0.f, 0.f);
+    int o = c.ox;
+#pragma unroll
+    for (int j = 0; j < RB; ++j) {
+        const float2 x = unpack2(c.x(o));
+        float2 s = unpack2(ys[j]);
+        if (x1) s = rows ? cadd(cmul(xm, h1), s) : cmul(xm, h1);
+        const float2 y = cadd(cmul(x, h0), s);
+        if (j < live) Y[(size_t)j * l.cs] = y;
+        xm = x;
+        o = c.fwd(o);
+    }
+}
+
+__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
+}
+
+// The default tiles: a CTA takes a tile of at most kMacTile bins of one level
+// through a segment of blocks, kWideRun at a time, from shared memory.  With
+// at most kMacRes parts the filter rows of the tile stay there for the whole
+// segment and each spectrum row is copied in once, a run ahead of its use;
+// with more, every run takes the parts a partial-sum row at a time.
+__global__ void __launch_bounds__(kMacTile) wide_mac_kernel(const int4* __restrict__ map, WArgs a) {
+    constexpr int RB = kWideRun, W = kMacTile;
+    extern __shared__ float4 dyn_smem[];
+    cudaTriggerProgrammaticLaunchCompletion();
+    const int4 e = map[blockIdx.x];   // level, first bin, blocks [z, w) of the chunk
     const WLevel& l = a.lv[e.x];
+    cudaGridDependencySynchronize();
+    const long long bf = blocks_before(l, a.c0);
+    const int nb = min(e.w, (int)(blocks_before(l, a.c0 + a.nsteps) - bf));
+    if (e.z >= nb) return;
+    const int cs = l.cs, P = l.P, R = l.slots, k0 = e.y;
+    const int w2 = min(W, cs - k0) >> 1;   // pairs of bins in the tile
+    const int tid = threadIdx.x, lr = tid / (W / 2), lc = tid % (W / 2);
+    const bool live = tid < 2 * w2;
+    const float2* Hg = l.H + k0;
+    const float2* Xg = l.X + k0;
+    float2* Y = l.Yw + k0 + tid;
+    int sl = wmod(bf, R) + e.z;   // ring row of block e.z of the chunk
+    if (sl >= R) sl -= R;
+    // rows [0, n) of the filter / of blocks starting at ring row s, to shared rows dst + ((p + i) mod m) W
+    auto copy_h = [&](float2* dst, int p, int n) {
+        if (lc < w2)
+            for (int i = lr; i < n; i += 2) cp_async16(dst + i * W + 2 * lc, Hg + (size_t)(p + i) * cs + 2 * lc);
+    };
+    auto copy_x = [&](float2* dst, int p, int m, int s, int n) {
+        if (s < 0) s += R;
+        if (s >= R) s -= R;
+        if (lc < w2)
+            for (int i = lr; i < n; i += 2) {
+                int r = s + i;
+                if (r >= R) r -= R;
+                int q = p + i;
+                if (q >= m) q -= m;
+                cp_async16(dst + q * W + 2 * lc, Xg + (size_t)r * cs + 2 * lc);
+            }
+    };
+    float2* Hs = reinterpret_cast<float2*>(dyn_smem);
+    f32x2 ys[RB];
+    if (P <= kMacRes) {
+        float2* Xs = Hs + kMacRes * W;
+        const int RX = P - 1 + 2 * RB;   // ring rows: the history of a run, the run, the next run
+        copy_h(Hs, 0, P);
+        copy_x(Xs, 0, RX, sl - (P - 1), P - 1 + RB);
+        cp_async_commit();
+        int pos = P - 1;                 // shared row of the run's first block
+        for (int i0 = e.z; i0 < nb; i0 += RB) {
+            if (i0 + RB < nb) {
+                int q = pos + RB;
+                if (q >= RX) q -= RX;
+                copy_x(Xs, q, RX, sl + RB, RB);
+            }
+            cp_async_commit();
+            cp_async_wait<1>();
+            __syncthreads();
+            if (live) {
+                MacCol<true> c{Hs + l.p_lo * W + tid, Xs + tid, W, RX * W, 0};
+                int q = pos - l.p_lo;
+                c.ox = (q < 0 ? q + RX : q) * W;
+#pragma unroll
+                for (int j = 0; j < RB; ++j) ys[j] = 0;
+                if (P > l.p_lo) sum_parts<RB, true>(c, P - l.p_lo, 4, ys);
+                c.H = Hs + tid;
+                c.ox = pos * W;
+                finish_run(c, l, ys, Y + (size_t)i0 * cs, nb - i0);
+            }
+            __syncthreads();   // the next run's copies overwrite rows read here
+            pos += RB;
+            if (pos >= RX) pos -= RX;
+            sl += RB;
+            if (sl >= R) sl -= R;
+        }
+        return;
+    }
+    constexpr int TP = kMacRes - 2;      // parts per partial-sum row at most
+    float2* Xs = Hs + TP * W;
+    for (int i0 = e.z; i0 < nb; i0 += RB) {
+        for (int q = 0; q < l.nrows; ++q) {
+            const int pb = l.p_lo + q * l.tp, n = min(l.tp, P - pb);
+            // blocks (run's first) - pb - n .. (run's first) - pb + RB - 1
+            copy_h(Hs, pb, n);
+            copy_x(Xs, 0, TP + RB, sl - pb - n, n + RB);
+            cp_async_commit();
+            cp_async_wait<0>();
+            __syncthreads();
+            if (live) {
+                f32x2 row[RB];
+                MacCol<true> c{Hs + tid, Xs + tid, W, (TP + RB) * W, n * W};
+                sum_parts<RB, true>(c, n, 4, row);
+#pragma unroll
+                for (int j = 0; j < RB; ++j) ys[j] = q == 0 ? row[j] : add2(ys[j], row[j]);
+            }
+            __syncthreads();
+        }
+        if (live)
+            finish_run(MacCol<false>{Hg + tid, Xg + tid, cs, R * cs, sl * cs}, l, ys, Y + (size_t)i0 * cs, nb - i0);
+        sl += RB;
+        if (sl >= R) sl -= R;
+    }
+}
+
+// Other tile shapes and several base blocks per step: one thread per bin and
+// run, rows from L2.
+__global__ void __launch_bounds__(kMacAnyNT, 3) wide_mac_any_kernel(const int4* __restrict__ map, WArgs a) {
+    constexpr int RB = kWideRun;
+    cudaTriggerProgrammaticLaunchCompletion();
+    const int4 e = map[blockIdx.x];   // level, first (run, bin) item
+    const WLevel& l = a.lv[e.x];
+    cudaGridDependencySynchronize();
     const long long bf = blocks_before(l, a.c0);
     const int nb = (int)(blocks_before(l, a.c0 + a.nsteps) - bf);
     const int cs = l.cs, P = l.P, R = l.slots;
@@ -135,109 +378,34 @@ __global__ void __launch_bounds__(kWideMacNT) wide_mac_kernel(const int2* __rest
     const int run = item / cs, k = item - run * cs;
     const int i0 = run * RB;
     if (i0 >= nb) return;
-    const float2* __restrict__ H = l.H + k;
-    const float2* X = l.X + k;
-    const int sl0 = wmod(bf + i0, R);
-    // row of block (run's first) + d, -R <= d < R
-    auto xat = [&](int d) {
-        int sl = sl0 + d;
-        if (sl < 0) sl += R;
-        if (sl >= R) sl -= R;
-        return __ldcg(X + (size_t)sl * cs);
-    };
+    int sl = wmod(bf, R) + i0;   // ring row of the run's first block
+    if (sl >= R) sl -= R;
+    MacCol<false> c{l.H + (size_t)l.p_lo * cs + k, l.X + k, cs, R * cs, 0};
+    f32x2 ys[RB];   // partial-sum rows of the parts >= p_lo
+#pragma unroll
+    for (int j = 0; j < RB; ++j) ys[j] = 0;
     const bool rows = P > l.p_lo;
-    float2 y[RB];
-    float2 part[RB];   // kFormFire: the part the fire adds to X_b H_0
-    if (l.form == kFormMulti) {
-        // p < p_lo in one running sum
-#pragma unroll
-        for (int j = 0; j < RB; ++j) y[j] = make_float2(0.f, 0.f);
-        float2 w[RB];
-#pragma unroll
-        for (int j = 0; j < RB; ++j) w[j] = xat(j);
-        const int Q = l.p_lo;
-        for (int p0 = 0; p0 < Q; p0 += RB) {
-            float2 h[RB], nx[RB];
-#pragma unroll
-            for (int u = 0; u < RB; ++u)
-                if (p0 + u < Q) {
-                    h[u] = __ldg(H + (size_t)(p0 + u) * cs);
-                    nx[u] = xat(-(p0 + u + 1));
-                }
-#pragma unroll
-            for (int u = 0; u < RB; ++u)
-                if (p0 + u < Q) {
-#pragma unroll
-                    for (int j = 0; j < RB; ++j) y[j] = cmac(y[j], w[(j - u + RB) % RB], h[u]);
-                    w[(RB - 1 - u + RB) % RB] = nx[u];
-                }
-        }
-    } else {
-        const float2 h0 = __ldg(H);
-        const bool x1 = l.two && P >= 2;
-        float2 w[RB + 1];
-#pragma unroll
-        for (int j = 0; j < RB; ++j) w[j + 1] = xat(j);
-        w[0] = x1 ? xat(-1) : make_float2(0.f, 0.f);
-        const float2 h1 = x1 ? __ldg(H + cs) : make_float2(0.f, 0.f);
-#pragma unroll
-        for (int j = 0; j < RB; ++j) {
-            y[j] = cmul(w[j + 1], h0);
-            part[j] = x1 ? cmul(w[j], h1) : make_float2(0.f, 0.f);
-            if (l.form == kFormCluster && x1) y[j] = cadd(y[j], part[j]);
-        }
-    }
     if (rows) {
-        float2 ys[RB];
+        const int o = sl - l.p_lo;
+        c.ox = (o < 0 ? o + R : o) * cs;
         for (int q = 0; q < l.nrows; ++q) {
-            const int pb = l.p_lo + q * tp, n = min(tp, P - pb);
-            float2 acc[G][RB];
+            f32x2 row[RB];
+            sum_parts<RB, false>(c, min(l.tp, P - l.p_lo - q * l.tp), l.tpg, row);
 #pragma unroll
-            for (int g = 0; g < G; ++g)
-#pragma unroll
-                for (int j = 0; j < RB; ++j) acc[g][j] = make_float2(0.f, 0.f);
-            float2 w[RB];   // block (run's first) + d at w[d mod RB]
-#pragma unroll
-            for (int j = 0; j < RB; ++j) w[j] = xat(j - pb);
-            for (int p0 = 0; p0 < n; p0 += U) {
-                float2 h[U], nx[U];
-#pragma unroll
-                for (int u = 0; u < U; ++u)
-                    if (p0 + u < n) {
-                        h[u] = __ldg(H + (size_t)(pb + p0 + u) * cs);
-                        nx[u] = xat(-(pb + p0 + u + 1));
-                    }
-#pragma unroll
-                for (int u = 0; u < U; ++u)
-                    if (p0 + u < n) {
-#pragma unroll
-                        for (int j = 0; j < RB; ++j) acc[u % G][j] = cmac(acc[u % G][j], w[(j - u + U) % RB], h[u]);
-                        w[(RB - 1 - u + U) % RB] = nx[u];
-                    }
-            }
-#pragma unroll
-            for (int j = 0; j < RB; ++j) {
-                float2 r = acc[0][j];
-#pragma unroll
-                for (int g = 1; g < G; ++g) r = cadd(r, acc[g][j]);
-                if (l.form == kFormCluster) y[j] = cadd(y[j], r);
-                else ys[j] = q == 0 ? r : cadd(ys[j], r);
-            }
-        }
-        if (l.form == kFormFire) {
-#pragma unroll
-            for (int j = 0; j < RB; ++j) part[j] = cadd(part[j], ys[j]);
-        } else if (l.form == kFormMulti) {
-#pragma unroll
-            for (int j = 0; j < RB; ++j) y[j] = cadd(y[j], ys[j]);
+            for (int j = 0; j < RB; ++j) ys[j] = q == 0 ? row[j] : add2(ys[j], row[j]);
         }
     }
+    c.H = l.H + k;
+    c.ox = sl * cs;
     float2* Y = l.Yw + (size_t)i0 * cs + k;
+    if (l.multi) {   // parts < p_lo in one running sum
+        f32x2 y[RB];
+        sum_parts<RB, false>(c, l.p_lo, l.p_lo, y);
 #pragma unroll
-    for (int j = 0; j < RB; ++j) {
-        if (i0 + j >= nb) break;
-        if (l.form == kFormFire) y[j] = cadd(y[j], part[j]);
-        Y[(size_t)j * cs] = y[j];
+        for (int j = 0; j < RB; ++j)
+            if (i0 + j < nb) Y[(size_t)j * cs] = unpack2(rows ? add2(y[j], ys[j]) : y[j]);
+    } else {
+        finish_run(c, l, ys, Y, nb - i0);
     }
 }
 
@@ -249,8 +417,10 @@ __global__ void __launch_bounds__(RegFft<LOGN>::NT) wide_ifft_kernel(const int2*
     using F = RegFft<LOGN>;
     constexpr int N = F::N, TPT = F::TPT;
     extern __shared__ float4 dyn_smem[];
+    cudaTriggerProgrammaticLaunchCompletion();
     const int2 e = map[blockIdx.x];
     const WLevel& l = a.lv[e.x];
+    cudaGridDependencySynchronize();
     const int t = threadIdx.x % TPT, tr = threadIdx.x / TPT;
     float2* s = reinterpret_cast<float2*>(dyn_smem) + tr * F::SM;
     const long long b0 = blocks_before(l, a.c0);
@@ -333,6 +503,8 @@ __global__ void __launch_bounds__(RegFft<LOGN>::NT) wide_ifft_kernel(const int2*
 
 // 4. outputs fed by several PCs (summed in PC order) and outputs without any
 __global__ void wide_mix_kernel(Bank bank, int n_zero, int mixed, WArgs a) {
+    cudaTriggerProgrammaticLaunchCompletion();
+    cudaGridDependencySynchronize();
     const int len = a.nsteps * a.N0;
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= len) return;
@@ -349,17 +521,39 @@ __global__ void wide_mix_kernel(Bank bank, int n_zero, int mixed, WArgs a) {
     for (int z = 0; z < n_zero; ++z) o[(long long)bank.zero_list[z] * a.io.out_ch] = 0.0f;
 }
 
-// the call's newest samples (at most a ring's worth) to every PC's input ring
-__global__ void wide_ring_kernel(const WLevel* __restrict__ lv, const int* __restrict__ lv0, WArgs a, long long t_end,
-                                 long long frames) {
-    const WLevel& l = lv[lv0[blockIdx.y]];
-    const long long n = min(frames, (long long)l.rin_mask + 1);
-    const float* in = a.io.in + (long long)l.in_ch * a.io.in_ch;
-    const long long t_in0 = a.io.step0 * (long long)a.N0;
-    for (long long j = blockIdx.x * (long long)blockDim.x + threadIdx.x; j < n; j += (long long)gridDim.x * blockDim.x) {
-        const long long ta = t_end - n + j;
-        l.xring[ta & l.rin_mask] = in[(ta - t_in0) * a.io.in_sample] * l.scale;
+// What a run from the start reads before writing it: the spectrum rows of
+// the P - 1 blocks before the first one, and the output ring up to the first
+// block's samples.  (The rest of both is written first.)
+__global__ void wide_reset_kernel(const WLevel* __restrict__ lv) {
+    const WLevel& l = lv[blockIdx.x];
+    const long long b0 = blocks_before(l, 0);
+    const int nt = gridDim.y * blockDim.x, t = blockIdx.y * blockDim.x + threadIdx.x;
+    const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+    const int n4 = l.cs >> 1;   // float4 per row (rows are 16-byte aligned)
+    int sl = wmod(b0, l.slots);
+    for (int p = 1; p < l.P; ++p) {
+        sl = sl == 0 ? l.slots - 1 : sl - 1;
+        float4* row = reinterpret_cast<float4*>(l.X + (size_t)sl * l.cs);
+        for (int i = t; i < n4; i += nt) row[i] = z;
     }
+    const int ny = (int)min((long long)l.rmask + 1, b0 << l.logN) >> 2;
+    for (int i = t; i < ny; i += nt) reinterpret_cast<float4*>(l.yring)[i] = z;
+}
+
+// launch that may overlap the previous kernel's tail (see above)
+template <class... KA, class... A>
+cudaError_t launch_dep(void (*k)(KA...), int grid, int nt, size_t smem, cudaStream_t st, A&&... args) {
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(nt);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, k, KA(args)...);
 }
 
 template <int LOGN>
@@ -420,8 +614,7 @@ struct WideFft {
     cudaStream_t st;
     template <int L>
     cudaError_t operator()() const {
-        wide_fft_kernel<L><<<grid, RegFft<L>::NT, reg_smem<L>(), st>>>(map, a);
-        return cudaGetLastError();
+        return launch_dep(wide_fft_kernel<L>, grid, RegFft<L>::NT, reg_smem<L>(), st, map, a);
     }
 };
 cudaError_t launch_wide_fft(int N, int grid, const int2* map, const WArgs& a, cudaStream_t st) {
@@ -436,41 +629,30 @@ struct WideIfft {
     cudaStream_t st;
     template <int L>
     cudaError_t operator()() const {
-        if (l0) wide_ifft_kernel<L, true><<<grid, RegFft<L>::NT, reg_smem<L>(), st>>>(map, a);
-        else wide_ifft_kernel<L, false><<<grid, RegFft<L>::NT, reg_smem<L>(), st>>>(map, a);
-        return cudaGetLastError();
+        return l0 ? launch_dep(wide_ifft_kernel<L, true>, grid, RegFft<L>::NT, reg_smem<L>(), st, map, a)
+                  : launch_dep(wide_ifft_kernel<L, false>, grid, RegFft<L>::NT, reg_smem<L>(), st, map, a);
     }
 };
 cudaError_t launch_wide_ifft(int N, bool l0, int grid, const int2* map, const WArgs& a, cudaStream_t st) {
     return grid > 0 ? by_log(N, WideIfft{l0, grid, map, a, st}) : cudaSuccess;
 }
 
-cudaError_t launch_wide_mac(int G, int tp, int grid, const int2* map, const WArgs& a, cudaStream_t st) {
+// filter rows and ring of a tile (the staged form needs less)
+constexpr size_t kMacSmem = sizeof(float2) * kMacTile * (size_t)(kMacRes + kMacRes - 1 + 2 * kWideRun);
+
+cudaError_t launch_wide_mac(bool any, int grid, const int4* map, const WArgs& a, cudaStream_t st) {
     if (grid <= 0) return cudaSuccess;
-    switch (G) {
-        case 1: wide_mac_kernel<1><<<grid, kWideMacNT, 0, st>>>(map, a, tp); break;
-        case 2: wide_mac_kernel<2><<<grid, kWideMacNT, 0, st>>>(map, a, tp); break;
-        case 4: wide_mac_kernel<4><<<grid, kWideMacNT, 0, st>>>(map, a, tp); break;
-        case 8: wide_mac_kernel<8><<<grid, kWideMacNT, 0, st>>>(map, a, tp); break;
-        case 16: wide_mac_kernel<16><<<grid, kWideMacNT, 0, st>>>(map, a, tp); break;
-        default: return cudaErrorInvalidValue;
-    }
-    return cudaGetLastError();
+    return any ? launch_dep(wide_mac_any_kernel, grid, kMacAnyNT, 0, st, map, a)
+               : launch_dep(wide_mac_kernel, grid, kMacTile, kMacSmem, st, map, a);
 }
 
 cudaError_t launch_wide_mix(const Bank& bank, int n_zero, bool mixed, const WArgs& a, cudaStream_t st) {
     const int len = a.nsteps * a.N0;
-    wide_mix_kernel<<<(len + 255) / 256, 256, 0, st>>>(bank, n_zero, mixed ? 1 : 0, a);
-    return cudaGetLastError();
+    return launch_dep(wide_mix_kernel, (len + 255) / 256, 256, 0, st, bank, n_zero, mixed ? 1 : 0, a);
 }
 
-cudaError_t launch_wide_ring(const WLevel* lv, const int* lv0, int npc, const WArgs& a, long long t_end,
-                             long long frames, int max_ring, cudaStream_t st) {
-    const long long n = std::min<long long>(frames, max_ring);
-    for (int p = 0; p < npc; p += 65535) {
-        const dim3 grid((unsigned)std::min<long long>((n + 1023) / 1024, 64), (unsigned)std::min(npc - p, 65535));
-        wide_ring_kernel<<<grid, 256, 0, st>>>(lv, lv0 + p, a, t_end, frames);
-    }
+cudaError_t launch_wide_reset(const WLevel* lv, int nlv, cudaStream_t st) {
+    wide_reset_kernel<<<dim3(nlv, nlv > 512 ? 4 : 64), 256, 0, st>>>(lv);
     return cudaGetLastError();
 }
 

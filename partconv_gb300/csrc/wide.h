@@ -15,12 +15,12 @@ struct WLevel {
     int s_blocks, cs, slots, rmask;
     int nrows;      // partial-sum rows (groups of parts >= p_lo)
     int p_lo;       // first part of the rows
-    int form;       // order of the sum over parts: kFormFire, kFormCluster or kFormMulti
+    int multi;      // level 0 with several base blocks per step: parts < p_lo are one running sum
     int two;        // the fire adds X_{b-1} H_1 itself
     int in_ch, out_ch, mix_mode, M;
-    int rin_mask, lv0, dfer, pad;
+    int rin_mask, lv0, dfer;
+    int tp, tpg;    // parts per partial-sum row, and per running sum within one
     float scale;
-    float pad2;
     const float2* H;
     float2* X;
     float2* Yw;     // [blocks of a chunk][cs]
@@ -29,7 +29,6 @@ struct WLevel {
     float* xring;
     float* pcw;     // [chunk samples], mixed outputs only
 };
-enum { kFormFire = 0, kFormCluster = 1, kFormMulti = 2 };
 
 struct WArgs {
     const WLevel* lv;
@@ -42,31 +41,33 @@ struct WArgs {
     IOView io;
 };
 
-constexpr int kWideMacNT = 128;
-// consecutive blocks a thread of the sum over parts takes together; G is the
-// number of running sums per block (fewer blocks where there are more sums,
-// so that all stay in registers)
-__host__ __device__ constexpr int wide_run(int G = 1) { return G <= 4 ? 8 : 32 / G; }
+constexpr int kWideRun = 8;       // consecutive blocks a thread of the sum over parts takes together
+constexpr int kMacTile = 96;      // bins per CTA of the sum over parts (three warps: 258 bins are three tiles of 86)
+constexpr int kMacSeg = 32;       // ... and blocks
+constexpr int kMacRes = 18;       // most parts whose filter rows stay in shared memory (the default 16 per row and 2)
+constexpr int kMacAnyNT = 128;    // threads of the general form
 
-// CTA maps: (level, first block of the chunk) for the transforms, (level,
-// first of kWideMacNT (run, bin) items) for the sum over parts.
+// CTA maps: (level, first block of the chunk) for the transforms; for the sum
+// over parts (level, first bin, first block, end block) of a tile and segment,
+// or (level, first of kMacAnyNT (run, bin) items) in the general form.
 int wide_transforms_per_cta(int N);
 cudaError_t prepare_wide_kernels();
 cudaError_t launch_wide_fft(int N, int grid, const int2* map, const WArgs& a, cudaStream_t st);
 // l0: level 0 (writes the output), else a larger level (writes its output ring)
 cudaError_t launch_wide_ifft(int N, bool l0, int grid, const int2* map, const WArgs& a, cudaStream_t st);
-// G: part groups of the handle's spread tasks, tp: parts per task
-cudaError_t launch_wide_mac(int G, int tp, int grid, const int2* map, const WArgs& a, cudaStream_t st);
+// any: tile shapes other than the default, or level 0 with several base blocks per step
+cudaError_t launch_wide_mac(bool any, int grid, const int4* map, const WArgs& a, cudaStream_t st);
 // outputs fed by several PCs, and outputs without any
 cudaError_t launch_wide_mix(const Bank& bank, int n_zero, bool mixed, const WArgs& a, cudaStream_t st);
-// the newest samples of a call of `frames` samples appended to every PC's input ring
-cudaError_t launch_wide_ring(const WLevel* lv, const int* lv0, int npc, const WArgs& a, long long t_end,
-                             long long frames, int max_ring, cudaStream_t st);
+// clears what a run from the start reads before it writes it (spectrum rows, output rings)
+cudaError_t launch_wide_reset(const WLevel* lv, int nlv, cudaStream_t st);
 // class-3 levels (cluster_fire.cu)
 cudaError_t launch_wide_cluster(bool inverse, int grid, const int2* map, const WArgs& a, cudaStream_t st);
-// partial sums of the blocks in progress after step c1 - 1 (step_kernels.cu);
-// map: (level, first bin, row, end bin) of a tile
-cudaError_t launch_wide_partials(int nt, int lanes, int grid, const int4* map, const WLevel* lv, int tp, long long c1,
-                                 int kb, cudaStream_t st);
+// the state one-block steps would have left after step a.c0 - 1
+// (step_kernels.cu): the partial sums of the blocks in progress, by n_part
+// CTAs of map (level, first bin, row, end bin), and the newest samples of the
+// call (which began at step a.io.step0) in the input rings of npc PCs
+cudaError_t launch_wide_state(int nt, int lanes, int n_part, const int4* map, const int* lv0, int npc, int max_ring,
+                              const WArgs& a, cudaStream_t st);
 
 }  // namespace pcg
