@@ -37,7 +37,7 @@ namespace {
 
 constexpr int kWlog = 17;          // twiddle table 2^17 entries: real FFTs up to 2 * 65536
 // Calls of at least this many base steps run block-parallel (wide.cu).
-constexpr int kWideMinSteps = 8;
+constexpr int kWideMinSteps = 4;
 // Base steps per block-parallel chunk: as many as keep the chunk's spectra
 // (one ring row per block of every level) within kWideBytes, so that they and
 // the summed spectra, as many again, are still in the 129 MB L2 when the next
@@ -191,13 +191,16 @@ struct pc_handle {
     int class_maxN[kClasses] = {};
 
     // block-parallel processing (wide.cu)
-    struct WGroup {         // levels of one block size: CTAs in order of their first block's step
-        int N;
-        bool l0, cluster;
-        const int2* map;
+    struct WMap {                // CTAs in order of their first block's step
+        const int2* map = nullptr;
         std::vector<int> upto;   // upto[n]: CTAs whose first block can complete within n + 1 steps
     };
-    std::vector<WGroup> wgroups;
+    // windows of all one-CTA levels, inverse transforms of those >= 1, level 0's, cluster levels
+    // (each of the first two: all block sizes together, or those above 2048 and
+    // those up to 2048 by themselves)
+    WMap w_fwd[3], w_inv[3], w_out, w_cl;
+    int w_nt[3] = {};            // threads per CTA of w_fwd and w_inv
+    int w_split = 0;             // chunks of at least this many steps launch the block sizes apart
     const int4* wmac_map[2] = {};     // the sum over parts: default tiles, any
     std::vector<int> wmac_upto[2];
     int w_part_nt = 0, w_part_lanes = 0, w_part_n = 0;   // partial sums at the end of a call
@@ -337,18 +340,14 @@ int parts_per_group(const pc_handle* h, bool l0) {
 // CTA maps of the block-parallel kernels, built on the host in the order in
 // which their first blocks complete, so a short call launches a prefix.
 struct WideMaps {
-    struct G {
-        int N;
-        bool l0, cluster;
-        std::vector<std::pair<int, int2>> e;   // (first relative step at which the entry may have work, entry)
-    };
-    std::vector<G> groups;
+    using Entries = std::vector<std::pair<int, int2>>;   // (first relative step at which the entry may have work, entry)
+    Entries fwd[3], inv[3], out, cl;
     std::vector<std::pair<int, int4>> mac[2];
     std::vector<int4> part;
 
     size_t bytes() const {
         size_t n = sizeof(int4) * (part.size() + mac[0].size() + mac[1].size()) + 3 * 256;
-        for (auto& g : groups) n += sizeof(int2) * g.e.size() + 256;
+        for (auto* e : {&fwd[0], &fwd[1], &fwd[2], &inv[0], &inv[1], &inv[2], &out, &cl}) n += sizeof(int2) * e->size() + 256;
         return n;
     }
     template <class E>
@@ -380,11 +379,16 @@ struct WideMaps {
             if (err == cudaSuccess) err = cudaStreamSynchronize(h->stream);
             return d;
         };
-        h->wgroups.clear();
-        for (auto& g : groups) {
-            const int2* d = entries(g.e);
-            h->wgroups.push_back({g.N, g.l0, g.cluster, d, prefix(g.e, h->C)});
+        auto put_map = [&](Entries& e, pc_handle::WMap& m) {
+            m.map = entries(e);
+            m.upto = prefix(e, h->C);
+        };
+        for (int g = 0; g < 3; ++g) {
+            put_map(fwd[g], h->w_fwd[g]);
+            put_map(inv[g], h->w_inv[g]);
         }
+        put_map(out, h->w_out);
+        put_map(cl, h->w_cl);
         for (int x = 0; x < 2; ++x) {
             h->wmac_map[x] = entries(mac[x]);
             h->wmac_upto[x] = prefix(mac[x], h->C);
@@ -400,19 +404,36 @@ void build_wide_maps(pc_handle* h, WideMaps& m) {
     const int nlv = (int)h->h_lv.size();
     h->w_part_nt = nt;
     h->w_part_lanes = lanes;
-    auto group = [&](int N, bool l0, bool cluster) -> WideMaps::G& {
-        for (auto& g : m.groups)
-            if (g.N == N && g.l0 == l0 && g.cluster == cluster) return g;
-        m.groups.push_back({N, l0, cluster, {}});
-        return m.groups.back();
-    };
+    int big = 0, one = 0;
+    for (int li = 0; li < nlv; ++li)
+        if (h->lv_cls[li] != 3) {
+            big = std::max(big, h->h_lv[li].N);
+            ++one;
+        }
+    // One launch for all block sizes, so that a call of little work fills the
+    // GPU with all its levels at once.  With work for more than four waves of
+    // 1024-thread CTAs (16384 points each) the blocks up to 2048 samples run
+    // in 128-thread CTAs of their own, eight per SM, which hide one another's
+    // loads (32 streams of 2^18 samples, ten waves: 454 against 469 us per
+    // call; 12 paths, 1001 blocks, two waves: 153 us apart, 137 together;
+    // six-level stereo ladder, half a wave: 285 and 238).
+    h->w_nt[0] = h->w_nt[1] = wide_threads(big);
+    h->w_nt[2] = wide_threads(1);
+    h->w_split = h->w_nt[0] == h->w_nt[2] ? h->C + 1 : (int)std::min(4.0 * 152 * 16384 / ((double)one * h->N0) + 1, 1e9);
     for (int li = 0; li < nlv; ++li) {
         const DevLevel& l = h->h_lv[li];
         const bool l0 = l.T == 1, cluster = h->lv_cls[li] == 3;
         const int nb = (h->C + l.T - 1) / l.T;   // most blocks of the level in a chunk
-        const int per = cluster ? 1 : wide_transforms_per_cta(l.N);
-        auto& g = group(l.N, l0, cluster);
-        for (int i = 0; i < nb; i += per) g.e.push_back({i * l.T, make_int2(li, i)});
+        for (int g = 0; g < 3 && !cluster; ++g) {
+            if (g > 0 && (l.N <= 16 * h->w_nt[2]) != (g == 2)) continue;
+            for (int i = 0; i < nb; i += 16 * h->w_nt[g] / l.N) {
+                m.fwd[g].push_back({i * l.T, make_int2(li, i)});
+                if (!l0) m.inv[g].push_back({i * l.T, make_int2(li, i)});
+            }
+        }
+        for (int i = 0; i < nb && cluster; ++i) m.cl.push_back({i * l.T, make_int2(li, i)});
+        if (l0)
+            for (int i = 0; i < nb; i += wide_out_blocks(l.N)) m.out.push_back({i, make_int2(li, i)});
         if (h->TP == spread_task_parts() && parts_per_group(h, l0) == 4 && !(l0 && h->KB > 1)) {
             for (int i = 0; i < nb; i += kMacSeg)
                 for (int k = 0; k < l.cs; k += kMacTile)
@@ -430,8 +451,6 @@ void build_wide_maps(pc_handle* h, WideMaps& m) {
             for (int k = 0; k < l.cs; k += tile)
                 for (int r = 0; r < l.npart; ++r) m.part.push_back(make_int4(li, k, r, std::min(l.cs, k + tile)));
     }
-    // larger blocks first (their inverse transforms feed level 0's output)
-    std::stable_sort(m.groups.begin(), m.groups.end(), [](auto& a, auto& b) { return a.N > b.N; });
 }
 
 int do_setup(pc_handle* h, int fs, int buffer_size, int n_in, int n_out, std::vector<PCSpec>&& specs) {
@@ -970,7 +989,6 @@ int do_setup(pc_handle* h, int fs, int buffer_size, int n_in, int n_out, std::ve
     char* A = h->arena;
     h->state_off = state_begin;
     h->state_bytes = state_end - state_begin;
-    CK(cudaMemsetAsync(A + state_begin, 0, h->state_bytes, h->stream), "memset state");
 
     // pointers into the arena
     for (int i = 0; i < npc; ++i) {
@@ -1069,7 +1087,7 @@ int do_setup(pc_handle* h, int fs, int buffer_size, int n_in, int n_out, std::ve
         h->d_lv0 = reinterpret_cast<const int*>(A + off_lv0);
         h->d_wtab = reinterpret_cast<const float2*>(A + off_wtab);
         CK(wm.place(h, A + off_wmap), "upload maps");
-        CK(launch_wide_reset(h->d_wlv, nlv, h->stream), "clear rings");
+        CK(launch_wide_reset(h->d_wlv, nlv, A + h->state_off, h->state_bytes, h->stream), "clear state");
     }
     // the level-0 class also runs spread tasks; its smem must fit its fires
     if (h->class_maxN[h->l0_class] == 0) h->class_maxN[h->l0_class] = N0;
@@ -1230,25 +1248,24 @@ IOView make_view(const pc_handle* h, const float* in, float* out, long long fram
 // One chunk of n <= h->C base steps from h->frame_num, block-parallel.
 int run_chunk(pc_handle* h, const IOView& view, int n, cudaStream_t st) {
     WArgs a = wide_args(h, view, n);
-    for (auto& g : h->wgroups) {
-        const int grid = g.upto[n - 1];
-        CK(g.cluster ? launch_wide_cluster(false, grid, g.map, a, st) : launch_wide_fft(g.N, grid, g.map, a, st),
-           "window transforms");
-        h->launches += grid > 0;
+    auto grid = [n](const pc_handle::WMap& m) { return m.upto[n - 1]; };
+    CK(launch_wide_cluster(false, grid(h->w_cl), h->w_cl.map, a, st), "window transforms");
+    const int g0 = n >= h->w_split ? 1 : 0, g1 = g0 ? 3 : 1;
+    for (int g = g0; g < g1; ++g) {
+        CK(launch_wide_fft(false, h->w_nt[g], grid(h->w_fwd[g]), h->w_fwd[g].map, a, st), "window transforms");
+        h->launches += (grid(h->w_fwd[g]) > 0) + (grid(h->w_inv[g]) > 0);
     }
     for (int x = 0; x < 2; ++x) {
         if (h->wmac_upto[x].empty()) continue;
-        const int grid = h->wmac_upto[x][n - 1];
-        CK(launch_wide_mac(x == 1, grid, h->wmac_map[x], a, st), "sum over parts");
-        h->launches += grid > 0;
+        const int cnt = h->wmac_upto[x][n - 1];
+        CK(launch_wide_mac(x == 1, cnt, h->wmac_map[x], a, st), "sum over parts");
+        h->launches += cnt > 0;
     }
-    for (auto& g : h->wgroups) {
-        const int grid = g.upto[n - 1];
-        CK(g.cluster ? launch_wide_cluster(true, grid, g.map, a, st)
-                     : launch_wide_ifft(g.N, g.l0, grid, g.map, a, st),
-           "inverse transforms");
-        h->launches += grid > 0;
-    }
+    CK(launch_wide_cluster(true, grid(h->w_cl), h->w_cl.map, a, st), "inverse transforms");
+    for (int g = g0; g < g1; ++g)
+        CK(launch_wide_fft(true, h->w_nt[g], grid(h->w_inv[g]), h->w_inv[g].map, a, st), "inverse transforms");
+    CK(launch_wide_out(h->N0, grid(h->w_out), h->w_out.map, a, st), "output");
+    h->launches += 2 * (grid(h->w_cl) > 0) + (grid(h->w_out) > 0);
     if (h->mixed || h->n_zero) {
         CK(launch_wide_mix(h->bank, h->n_zero, h->mixed, a, st), "mix");
         h->launches += 1;
@@ -1587,8 +1604,7 @@ int pc_reset(pc_handle* h) {
     h->frame_num = 0;
     if (!h->ready) return PC_OK;
     CK(cudaSetDevice(h->device), "cudaSetDevice");
-    CK(cudaMemsetAsync(h->arena + h->state_off, 0, h->state_bytes, h->stream), "reset");
-    CK(launch_wide_reset(h->d_wlv, (int)h->h_lv.size(), h->stream), "reset");
+    CK(launch_wide_reset(h->d_wlv, (int)h->h_lv.size(), h->arena + h->state_off, h->state_bytes, h->stream), "reset");
     CK(cudaStreamSynchronize(h->stream), "reset sync");
     return PC_OK;
 }

@@ -71,18 +71,26 @@ inline std::vector<float2> build_fft_tables(const std::vector<float2>& W, int wl
 // writes of a pass (16 or 16 Ns apart) spread over the banks.
 __device__ __forceinline__ int rpad(int i) { return i + (i >> 4); }
 
-// Threads per transform, and the barrier among them.
-template <int LOGN>
+// Threads per transform, and the barrier among them (a named one per transform
+// where a CTA of NT threads runs several, so transforms do not wait for one
+// another; at most 16, 1024 threads / 64).
+template <int LOGN, int NT>
 struct RegFft {
     static constexpr int N = 1 << LOGN;
-    static constexpr int TPT = N / 16;                    // threads per transform
-    static constexpr int NT = TPT < 128 ? 128 : TPT;      // threads per CTA
-    static constexpr int TPC = NT / TPT;                  // transforms per CTA
-    static constexpr int SM = N + N / 16;                 // shared float2 per transform
-    static constexpr bool FULL = LOGN <= 10;              // all three factors of a butterfly from the table
+    static constexpr int TPT = N / 16;          // threads per transform
+    static constexpr int SM = N + N / 16;       // shared float2 per transform
+    static constexpr bool FULL = LOGN <= 10;    // all three factors of a butterfly from the table
     __device__ static __forceinline__ void sync() {
-        if constexpr (TPT <= 32) __syncwarp();
-        else __syncthreads();
+        if constexpr (TPT <= 32) {
+            __syncwarp();
+        } else if constexpr (TPT == NT) {
+            __syncthreads();
+        } else if constexpr (2 * TPT == NT) {   // constant names: a CTA then holds two barriers, not sixteen
+            if ((int)threadIdx.x < TPT) asm volatile("bar.sync 0, %0;" ::"n"(TPT) : "memory");
+            else asm volatile("bar.sync 1, %0;" ::"n"(TPT) : "memory");
+        } else {
+            asm volatile("bar.sync %0, %1;" ::"r"((int)threadIdx.x / TPT), "n"(TPT) : "memory");
+        }
     }
 };
 
@@ -119,10 +127,10 @@ __device__ __forceinline__ void stage_tw(const float2* __restrict__ T, int k, fl
 
 // Stages S and S + 1 on v[m] = a[t + m TPT]; afterwards v[r + 4 e] is the
 // element 16 (t - k) + k + (r + 4 e) Ns, k = t mod Ns.
-template <int LOGN, int S, bool INV>
+template <int LOGN, int NT, int S, bool INV>
 __device__ __forceinline__ void pass16(float2 (&v)[16], int t, const float2* __restrict__ T) {
     constexpr int Ns = 1 << (2 * S);
-    constexpr bool FULL = RegFft<LOGN>::FULL;
+    constexpr bool FULL = RegFft<LOGN, NT>::FULL;
     const int k = t & (Ns - 1);
     if constexpr (S > 0) {
         float2 w1, w2, w3;
@@ -159,11 +167,11 @@ __device__ __forceinline__ void pass16(float2 (&v)[16], int t, const float2* __r
 
 // The last stages after the radix-16 passes, in place on v[m] = a[t + m TPT]
 // (the results lie at the same places): radix 8 (4 then 2), 4 or 2.
-template <int LOGN, bool INV>
+template <int LOGN, int NT, bool INV>
 __device__ __forceinline__ void pass_tail(float2 (&v)[16], int t, const float2* __restrict__ T) {
-    constexpr int N4 = LOGN / 2, TPT = RegFft<LOGN>::TPT;
+    constexpr int N4 = LOGN / 2, TPT = RegFft<LOGN, NT>::TPT;
     constexpr bool odd4 = (N4 & 1) != 0, r2 = (LOGN & 1) != 0;
-    constexpr bool FULL = RegFft<LOGN>::FULL;
+    constexpr bool FULL = RegFft<LOGN, NT>::FULL;
     if constexpr (odd4) {   // the last radix-4 stage, Ns = 4^(N4 - 1)
         constexpr int S = N4 - 1;
         constexpr int Ns = 1 << (2 * S);
@@ -212,9 +220,9 @@ __device__ __forceinline__ void pass_tail(float2 (&v)[16], int t, const float2* 
 }
 
 // write a radix-16 pass's results, read the next pass's points
-template <int LOGN, int S>
+template <int LOGN, int NT, int S>
 __device__ __forceinline__ void exchange(float2 (&v)[16], int t, float2* s) {
-    using F = RegFft<LOGN>;
+    using F = RegFft<LOGN, NT>;
     constexpr int Ns = 1 << (2 * S);
     const int k = t & (Ns - 1);
     const int base = 16 * (t - k) + k;
@@ -228,25 +236,25 @@ __device__ __forceinline__ void exchange(float2 (&v)[16], int t, float2* s) {
 // N-point transform of one group of TPT threads: in and out v[m] = a[t + m TPT].
 // s: this transform's shared memory (RegFft::SM float2), free on entry; a
 // caller that writes it afterwards syncs first.
-template <int LOGN, bool INV>
+template <int LOGN, int NT, bool INV>
 __device__ __forceinline__ void fft_reg(float2 (&v)[16], int t, float2* s, const float2* __restrict__ T) {
-    using F = RegFft<LOGN>;
+    using F = RegFft<LOGN, NT>;
     constexpr int NP = LOGN / 4;   // radix-16 passes (LOGN / 2 radix-4 stages in pairs)
     constexpr bool tail = (LOGN & 3) != 0;
-    pass16<LOGN, 0, INV>(v, t, T);
+    pass16<LOGN, NT, 0, INV>(v, t, T);
     if constexpr (NP > 1) {
-        exchange<LOGN, 0>(v, t, s);
-        pass16<LOGN, 2, INV>(v, t, T);
+        exchange<LOGN, NT, 0>(v, t, s);
+        pass16<LOGN, NT, 2, INV>(v, t, T);
     }
     if constexpr (NP > 2) {
         F::sync();
-        exchange<LOGN, 2>(v, t, s);
-        pass16<LOGN, 4, INV>(v, t, T);
+        exchange<LOGN, NT, 2>(v, t, s);
+        pass16<LOGN, NT, 4, INV>(v, t, T);
     }
     if constexpr (tail) {
         if constexpr (NP > 1) F::sync();
-        exchange<LOGN, 2 * (NP - 1)>(v, t, s);
-        pass_tail<LOGN, INV>(v, t, T);
+        exchange<LOGN, NT, 2 * (NP - 1)>(v, t, s);
+        pass_tail<LOGN, NT, INV>(v, t, T);
     }
 }
 

@@ -4,15 +4,15 @@
 // nothing in partitioned convolution feeds back, so the blocks of every level
 // can be computed side by side instead of one dependent launch per base
 // block.  A chunk of base steps is
-//   1. wide_fft   per block size: the window of every block that completes in
+//   1. wide_fft   all block sizes: the window of every block that completes in
 //                 the chunk, real FFT, spectrum ring row b mod slots;
 //   2. wide_mac   all levels: Y_b = sum_p X_{b-p} H_p, a tile of bins through
 //                 a segment of blocks per CTA, filter and spectrum rows in
 //                 shared memory and the window of a run of blocks in registers
 //                 (each row is read once per segment instead of once per block
 //                 and part);
-//   3. wide_ifft  per block size, level 0 last: inverse FFT, output ring, and
-//                 for level 0 the sum of the levels' due samples and the output;
+//   3. wide_ifft  levels >= 1: inverse FFT, output ring;
+//      wide_out   level 0: inverse FFT, the levels' due samples, the output;
 //   4. wide_mix   outputs fed by several PCs, in PC order.
 // After the last chunk of a call the input rings and the partial sums of the
 // blocks in progress are brought to where one-block steps would have left
@@ -52,24 +52,21 @@ __device__ __forceinline__ int wmod(long long a, int m) {
 __device__ __forceinline__ long long blocks_before(const WLevel& l, long long c) { return (c + l.s_blocks) >> l.logT; }
 
 // ---------------------------------------------------------------------------
-// 1. window, forward real FFT, spectrum row
+// 1. window, forward real FFT, spectrum row: one launch for all block sizes.
+// A CTA of NT threads runs 16 NT / N transforms of one level; every CTA has
+// the same amount of work whatever its block size.
 // ---------------------------------------------------------------------------
-template <int LOGN>
-__global__ void __launch_bounds__(RegFft<LOGN>::NT) wide_fft_kernel(const int2* __restrict__ map, WArgs a) {
-    using F = RegFft<LOGN>;
+template <int LOGN, int NT>
+__device__ __forceinline__ void fft_body(const WLevel& l, int first, const WArgs& a, float2* smem) {
+    using F = RegFft<LOGN, NT>;
     constexpr int N = F::N, TPT = F::TPT;
-    extern __shared__ float4 dyn_smem[];
-    cudaTriggerProgrammaticLaunchCompletion();
-    const int2 e = map[blockIdx.x];
-    const WLevel& l = a.lv[e.x];
-    cudaGridDependencySynchronize();
     const int t = threadIdx.x % TPT, tr = threadIdx.x / TPT;
-    float2* s = reinterpret_cast<float2*>(dyn_smem) + tr * F::SM;
+    float2* s = smem + tr * F::SM;
     const long long b0 = blocks_before(l, a.c0);
     const int nb = (int)(blocks_before(l, a.c0 + a.nsteps) - b0);
-    if (e.y >= nb) return;                     // the whole CTA
-    const bool live = e.y + tr < nb;
-    const long long b = b0 + min(e.y + tr, nb - 1);
+    const bool live = first + tr < nb;
+    if (TPT >= 32 && !live) return;            // whole warps, whole barriers
+    const long long b = b0 + min(first + tr, nb - 1);
     // window [t_end - 2 N, t_end) of the channel; samples before t_in0 (the
     // call's first) are in the PC's input ring, already scaled
     const long long t_end = ((b + 1) << LOGN) - (long long)l.s_blocks * a.N0;
@@ -97,7 +94,7 @@ __global__ void __launch_bounds__(RegFft<LOGN>::NT) wide_fft_kernel(const int2* 
             }
         }
     }
-    fft_reg<LOGN, false>(v, t, s, a.tab);
+    fft_reg<LOGN, NT, false>(v, t, s, a.tab);
     // the split pairs k < N / 2 (this thread's v[0 .. 7]) with N - k, which
     // lies in another thread's upper half
     F::sync();
@@ -121,6 +118,47 @@ __global__ void __launch_bounds__(RegFft<LOGN>::NT) wide_fft_kernel(const int2* 
         split_w(v[8], v[8], __ldg(sp + N / 2), xk, xnk);
         Xs[N / 2] = xk;
     }
+}
+
+// f.template operator()<LOGN>() for log2 N, up to 16 NT points
+template <int NT, class Fn>
+__device__ __forceinline__ void by_log_dev(int logN, Fn&& f) {
+    switch (logN) {
+        case 4: f.template operator()<4>(); break;
+        case 5: f.template operator()<5>(); break;
+        case 6: f.template operator()<6>(); break;
+        case 7: f.template operator()<7>(); break;
+        case 8: f.template operator()<8>(); break;
+        case 9: f.template operator()<9>(); break;
+        case 10: f.template operator()<10>(); break;
+        case 11: f.template operator()<11>(); break;
+        default:
+            if constexpr (NT >= 1024) {
+                if (logN == 12) f.template operator()<12>();
+                else if (logN == 13) f.template operator()<13>();
+                else f.template operator()<14>();
+            }
+    }
+}
+
+template <int NT>
+struct FftBody {
+    const WLevel& l;
+    int first;
+    const WArgs& a;
+    float2* smem;
+    template <int LOGN>
+    __device__ __forceinline__ void operator()() const { fft_body<LOGN, NT>(l, first, a, smem); }
+};
+template <int NT>
+__global__ void __launch_bounds__(NT) wide_fft_kernel(const int2* __restrict__ map, WArgs a) {
+    extern __shared__ float4 dyn_smem[];
+    cudaTriggerProgrammaticLaunchCompletion();
+    const int2 e = map[blockIdx.x];
+    const WLevel& l = a.lv[e.x];
+    cudaGridDependencySynchronize();
+    if (e.y >= (int)(blocks_before(l, a.c0 + a.nsteps) - blocks_before(l, a.c0))) return;
+    by_log_dev<NT>(l.logN, FftBody<NT>{l, e.y, a, reinterpret_cast<float2*>(dyn_smem)});
 }
 
 // ---------------------------------------------------------------------------
@@ -410,24 +448,20 @@ __global__ void __launch_bounds__(kMacAnyNT, 3) wide_mac_any_kernel(const int4* 
 }
 
 // ---------------------------------------------------------------------------
-// 3. inverse merge, inverse FFT, output ring or the call's output
+// 3. inverse merge, inverse FFT, output ring (levels >= 1, one launch for all
+// block sizes) or the call's output (level 0, after them)
 // ---------------------------------------------------------------------------
-template <int LOGN, bool L0>
-__global__ void __launch_bounds__(RegFft<LOGN>::NT) wide_ifft_kernel(const int2* __restrict__ map, WArgs a) {
-    using F = RegFft<LOGN>;
+template <int LOGN, int NT, bool L0>
+__device__ __forceinline__ void ifft_body(const WLevel& l, int first, const WArgs& a, float2* smem) {
+    using F = RegFft<LOGN, NT>;
     constexpr int N = F::N, TPT = F::TPT;
-    extern __shared__ float4 dyn_smem[];
-    cudaTriggerProgrammaticLaunchCompletion();
-    const int2 e = map[blockIdx.x];
-    const WLevel& l = a.lv[e.x];
-    cudaGridDependencySynchronize();
     const int t = threadIdx.x % TPT, tr = threadIdx.x / TPT;
-    float2* s = reinterpret_cast<float2*>(dyn_smem) + tr * F::SM;
+    float2* s = smem + tr * F::SM;
     const long long b0 = blocks_before(l, a.c0);
     const int nb = (int)(blocks_before(l, a.c0 + a.nsteps) - b0);
-    if (e.y >= nb) return;
-    const bool live = e.y + tr < nb;
-    const int i = min(e.y + tr, nb - 1);
+    const bool live = first + tr < nb;
+    if (TPT >= 32 && !live) return;
+    const int i = min(first + tr, nb - 1);
     const long long b = b0 + i;
     const float2* Y = l.Yw + (size_t)i * l.cs;
     const float2* sp = a.tab + ft_sp(LOGN);
@@ -444,7 +478,7 @@ __global__ void __launch_bounds__(RegFft<LOGN>::NT) wide_ifft_kernel(const int2*
             merge_w(yc, yn, __ldg(sp + N - n), other, v[m]);
         }
     }
-    fft_reg<LOGN, true>(v, t, s, a.tab);
+    fft_reg<LOGN, NT, true>(v, t, s, a.tab);
     if (!live) return;
     // real samples 2 n, 2 n + 1 of the block in v[m], n = t + m TPT < N / 2
     if constexpr (!L0) {
@@ -501,6 +535,38 @@ __global__ void __launch_bounds__(RegFft<LOGN>::NT) wide_ifft_kernel(const int2*
     }
 }
 
+template <int NT>
+struct IfftBody {
+    const WLevel& l;
+    int first;
+    const WArgs& a;
+    float2* smem;
+    template <int LOGN>
+    __device__ __forceinline__ void operator()() const { ifft_body<LOGN, NT, false>(l, first, a, smem); }
+};
+template <int NT>
+__global__ void __launch_bounds__(NT) wide_ifft_kernel(const int2* __restrict__ map, WArgs a) {
+    extern __shared__ float4 dyn_smem[];
+    cudaTriggerProgrammaticLaunchCompletion();
+    const int2 e = map[blockIdx.x];
+    const WLevel& l = a.lv[e.x];
+    cudaGridDependencySynchronize();
+    if (e.y >= (int)(blocks_before(l, a.c0 + a.nsteps) - blocks_before(l, a.c0))) return;
+    by_log_dev<NT>(l.logN, IfftBody<NT>{l, e.y, a, reinterpret_cast<float2*>(dyn_smem)});
+}
+
+__host__ __device__ constexpr int out_threads(int logN) { return logN <= 11 ? 128 : 1 << (logN - 4); }
+template <int LOGN>
+__global__ void __launch_bounds__(out_threads(LOGN)) wide_out_kernel(const int2* __restrict__ map, WArgs a) {
+    extern __shared__ float4 dyn_smem[];
+    cudaTriggerProgrammaticLaunchCompletion();
+    const int2 e = map[blockIdx.x];
+    const WLevel& l = a.lv[e.x];
+    cudaGridDependencySynchronize();
+    if (e.y >= a.nsteps) return;
+    ifft_body<LOGN, out_threads(LOGN), true>(l, e.y, a, reinterpret_cast<float2*>(dyn_smem));
+}
+
 // 4. outputs fed by several PCs (summed in PC order) and outputs without any
 __global__ void wide_mix_kernel(Bank bank, int n_zero, int mixed, WArgs a) {
     cudaTriggerProgrammaticLaunchCompletion();
@@ -523,12 +589,18 @@ __global__ void wide_mix_kernel(Bank bank, int n_zero, int mixed, WArgs a) {
 
 // What a run from the start reads before writing it: the spectrum rows of
 // the P - 1 blocks before the first one, and the output ring up to the first
-// block's samples.  (The rest of both is written first.)
-__global__ void wide_reset_kernel(const WLevel* __restrict__ lv) {
-    const WLevel& l = lv[blockIdx.x];
-    const long long b0 = blocks_before(l, 0);
+// block's samples (the rest of both is written first); and the state region
+// of n16 16-byte words, cleared by the CTAs after the levels'.
+__global__ void wide_reset_kernel(const WLevel* __restrict__ lv, int nlv, float4* state, size_t n16) {
     const int nt = gridDim.y * blockDim.x, t = blockIdx.y * blockDim.x + threadIdx.x;
     const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+    if ((int)blockIdx.x >= nlv) {
+        const size_t step = (size_t)(gridDim.x - nlv) * nt;
+        for (size_t i = (size_t)(blockIdx.x - nlv) * nt + t; i < n16; i += step) state[i] = z;
+        return;
+    }
+    const WLevel& l = lv[blockIdx.x];
+    const long long b0 = blocks_before(l, 0);
     const int n4 = l.cs >> 1;   // float4 per row (rows are 16-byte aligned)
     int sl = wmod(b0, l.slots);
     for (int p = 1; p < l.P; ++p) {
@@ -556,21 +628,8 @@ cudaError_t launch_dep(void (*k)(KA...), int grid, int nt, size_t smem, cudaStre
     return cudaLaunchKernelEx(&cfg, k, KA(args)...);
 }
 
-template <int LOGN>
-size_t reg_smem() {
-    return sizeof(float2) * (size_t)RegFft<LOGN>::SM * RegFft<LOGN>::TPC;
-}
-
-template <int LOGN>
-cudaError_t prepare_one() {
-    const int b = (int)reg_smem<LOGN>();
-    cudaError_t e = cudaFuncSetAttribute(wide_fft_kernel<LOGN>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(wide_ifft_kernel<LOGN, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(wide_ifft_kernel<LOGN, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
-    return e;
-}
+// shared memory of a CTA of nt threads, 16 points each
+constexpr size_t fft_smem_of(int nt) { return sizeof(float2) * 17 * (size_t)nt; }
 
 // f.template operator()<LOGN>() for log2 N
 template <class Fn>
@@ -591,50 +650,51 @@ cudaError_t by_log(int N, Fn&& f) {
     }
 }
 
+struct OutPrepare {
+    template <int L>
+    cudaError_t operator()() const {
+        return cudaFuncSetAttribute(wide_out_kernel<L>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)fft_smem_of(out_threads(L)));
+    }
+};
+
 }  // namespace
 
-int wide_transforms_per_cta(int N) { return N >= 2048 ? 1 : 2048 / N; }
-
-struct WidePrepare {
-    template <int L>
-    cudaError_t operator()() const { return prepare_one<L>(); }
-};
 cudaError_t prepare_wide_kernels() {
-    for (int N = 8192; N <= 16384; N *= 2) {   // the others fit the default shared memory
-        cudaError_t e = by_log(N, WidePrepare{});
-        if (e != cudaSuccess) return e;
-    }
-    return cudaSuccess;
+    cudaError_t e = cudaFuncSetAttribute(wide_fft_kernel<1024>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)fft_smem_of(1024));
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(wide_ifft_kernel<1024>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)fft_smem_of(1024));
+    for (int N = 8192; N <= 16384 && e == cudaSuccess; N *= 2) e = by_log(N, OutPrepare{});
+    return e;
 }
 
-struct WideFft {
+int wide_threads(int max_n) { return max_n <= 2048 ? 128 : 1024; }
+int wide_out_blocks(int N0) { return N0 <= 2048 ? 2048 / N0 : 1; }
+
+cudaError_t launch_wide_fft(bool inverse, int nt, int grid, const int2* map, const WArgs& a, cudaStream_t st) {
+    if (grid <= 0) return cudaSuccess;
+    const size_t sm = fft_smem_of(nt);
+    if (nt == 128)
+        return inverse ? launch_dep(wide_ifft_kernel<128>, grid, nt, sm, st, map, a)
+                       : launch_dep(wide_fft_kernel<128>, grid, nt, sm, st, map, a);
+    return inverse ? launch_dep(wide_ifft_kernel<1024>, grid, nt, sm, st, map, a)
+                   : launch_dep(wide_fft_kernel<1024>, grid, nt, sm, st, map, a);
+}
+
+struct WideOut {
     int grid;
     const int2* map;
     const WArgs& a;
     cudaStream_t st;
     template <int L>
     cudaError_t operator()() const {
-        return launch_dep(wide_fft_kernel<L>, grid, RegFft<L>::NT, reg_smem<L>(), st, map, a);
+        return launch_dep(wide_out_kernel<L>, grid, out_threads(L), fft_smem_of(out_threads(L)), st, map, a);
     }
 };
-cudaError_t launch_wide_fft(int N, int grid, const int2* map, const WArgs& a, cudaStream_t st) {
-    return grid > 0 ? by_log(N, WideFft{grid, map, a, st}) : cudaSuccess;
-}
-
-struct WideIfft {
-    bool l0;
-    int grid;
-    const int2* map;
-    const WArgs& a;
-    cudaStream_t st;
-    template <int L>
-    cudaError_t operator()() const {
-        return l0 ? launch_dep(wide_ifft_kernel<L, true>, grid, RegFft<L>::NT, reg_smem<L>(), st, map, a)
-                  : launch_dep(wide_ifft_kernel<L, false>, grid, RegFft<L>::NT, reg_smem<L>(), st, map, a);
-    }
-};
-cudaError_t launch_wide_ifft(int N, bool l0, int grid, const int2* map, const WArgs& a, cudaStream_t st) {
-    return grid > 0 ? by_log(N, WideIfft{l0, grid, map, a, st}) : cudaSuccess;
+cudaError_t launch_wide_out(int N0, int grid, const int2* map, const WArgs& a, cudaStream_t st) {
+    return grid > 0 ? by_log(N0, WideOut{grid, map, a, st}) : cudaSuccess;
 }
 
 // filter rows and ring of a tile (the staged form needs less)
@@ -651,8 +711,11 @@ cudaError_t launch_wide_mix(const Bank& bank, int n_zero, bool mixed, const WArg
     return launch_dep(wide_mix_kernel, (len + 255) / 256, 256, 0, st, bank, n_zero, mixed ? 1 : 0, a);
 }
 
-cudaError_t launch_wide_reset(const WLevel* lv, int nlv, cudaStream_t st) {
-    wide_reset_kernel<<<dim3(nlv, nlv > 512 ? 4 : 64), 256, 0, st>>>(lv);
+cudaError_t launch_wide_reset(const WLevel* lv, int nlv, void* state, size_t bytes, cudaStream_t st) {
+    // about 16 KB per CTA for the region
+    const int gy = nlv > 512 ? 4 : 64;
+    const int extra = (int)std::min<size_t>(64, bytes / ((size_t)gy << 14) + 1);
+    wide_reset_kernel<<<dim3(nlv + extra, gy), 256, 0, st>>>(lv, nlv, static_cast<float4*>(state), bytes >> 4);
     return cudaGetLastError();
 }
 

@@ -50,17 +50,21 @@ constexpr int kMacAnyNT = 128;    // threads of the general form
 // CTA maps: (level, first block of the chunk) for the transforms; for the sum
 // over parts (level, first bin, first block, end block) of a tile and segment,
 // or (level, first of kMacAnyNT (run, bin) items) in the general form.
-int wide_transforms_per_cta(int N);
 cudaError_t prepare_wide_kernels();
-cudaError_t launch_wide_fft(int N, int grid, const int2* map, const WArgs& a, cudaStream_t st);
-// l0: level 0 (writes the output), else a larger level (writes its output ring)
-cudaError_t launch_wide_ifft(int N, bool l0, int grid, const int2* map, const WArgs& a, cudaStream_t st);
+// threads per CTA of the transform kernels for blocks up to max_n (a CTA runs
+// 16 threads / N transforms), and blocks per CTA of wide_out
+int wide_threads(int max_n);
+int wide_out_blocks(int N0);
+cudaError_t launch_wide_fft(bool inverse, int nt, int grid, const int2* map, const WArgs& a, cudaStream_t st);
+// level 0: inverse transforms and the call's output
+cudaError_t launch_wide_out(int N0, int grid, const int2* map, const WArgs& a, cudaStream_t st);
 // any: tile shapes other than the default, or level 0 with several base blocks per step
 cudaError_t launch_wide_mac(bool any, int grid, const int4* map, const WArgs& a, cudaStream_t st);
 // outputs fed by several PCs, and outputs without any
 cudaError_t launch_wide_mix(const Bank& bank, int n_zero, bool mixed, const WArgs& a, cudaStream_t st);
-// clears what a run from the start reads before it writes it (spectrum rows, output rings)
-cudaError_t launch_wide_reset(const WLevel* lv, int nlv, cudaStream_t st);
+// clears what a run from the start reads before it writes it: spectrum rows,
+// output rings, and the state region (16-byte aligned)
+cudaError_t launch_wide_reset(const WLevel* lv, int nlv, void* state, size_t bytes, cudaStream_t st);
 // class-3 levels (cluster_fire.cu)
 cudaError_t launch_wide_cluster(bool inverse, int grid, const int2* map, const WArgs& a, cudaStream_t st);
 // the state one-block steps would have left after step a.c0 - 1
