@@ -1092,16 +1092,12 @@ int do_setup(pc_handle* h, int fs, int buffer_size, int n_in, int n_out, std::ve
     // the level-0 class also runs spread tasks; its smem must fit its fires
     if (h->class_maxN[h->l0_class] == 0) h->class_maxN[h->l0_class] = N0;
 
-    // twiddles, computed in double
+    // twiddles
     {
-        std::vector<float2> W((size_t)1 << kWlog);
-        for (size_t m = 0; m < W.size(); ++m) {
-            const double a = -2.0 * M_PI * (double)m / (double)W.size();
-            W[m] = make_float2((float)std::cos(a), (float)std::sin(a));
-        }
+        const std::vector<float2>& W = host_twiddles(kWlog);
         CK(cudaMemcpyAsync(A + off_W, W.data(), sizeof(float2) * W.size(), cudaMemcpyHostToDevice, h->stream),
            "upload twiddles");
-        const std::vector<float2> tab = build_fft_tables(W, kWlog);
+        const std::vector<float2>& tab = host_fft_tables();
         CK(cudaMemcpyAsync(A + off_wtab, tab.data(), sizeof(float2) * tab.size(), cudaMemcpyHostToDevice, h->stream),
            "upload twiddles");
         CK(cudaStreamSynchronize(h->stream), "sync");

@@ -28,15 +28,16 @@ constexpr int kRegMaxLog = 14;
 
 // ---- layout of the table (float2 entries) ---------------------------------------
 // w1(s): exp(-2 pi i k / 4^(s+1)), k < 4^s, stages s = 1 .. 6
-// w2(s), w3(s): its squares and cubes, s = 1 .. 4 (blocks up to 1024 points
-//   read all three factors; larger ones form them by products)
+// w2(s), w3(s): its squares and cubes (blocks up to 1024 points read all three
+//   factors; larger ones do with `full`, else they form them by products as
+//   fft_smem's conflict-free stages do, with about one rounding more each)
 // r2(a): exp(-2 pi i k / (2 4^a)), k < 4^a, a = 2 .. 6 (the radix-2 stage)
 // sp(l): exp(-2 pi i k / 2^(l+1)), k <= 2^(l-1), l = 4 .. 14 (the real split)
 __host__ __device__ constexpr int ft_pow4(int s) { return 1 << (2 * s); }
 __host__ __device__ constexpr int ft_w1(int s) { return (ft_pow4(s) - 4) / 3; }                // sum of 4^j, 1 <= j < s
 __host__ __device__ constexpr int ft_w2(int s) { return ft_w1(7) + (ft_pow4(s) - 4) / 3; }
-__host__ __device__ constexpr int ft_w3(int s) { return ft_w2(5) + (ft_pow4(s) - 4) / 3; }
-__host__ __device__ constexpr int ft_r2(int a) { return ft_w3(5) + (ft_pow4(a) - 16) / 3; }
+__host__ __device__ constexpr int ft_w3(int s) { return ft_w2(7) + (ft_pow4(s) - 4) / 3; }
+__host__ __device__ constexpr int ft_r2(int a) { return ft_w3(7) + (ft_pow4(a) - 16) / 3; }
 __host__ __device__ constexpr int ft_sp(int l) { return ft_r2(7) + (1 << (l - 1)) - 8 + 2 * (l - 4); }
 constexpr int kFftTabEntries = ft_sp(15);
 
@@ -55,10 +56,8 @@ inline std::vector<float2> build_fft_tables(const std::vector<float2>& W, int wl
     for (int s = 1; s <= 6; ++s)
         for (int k = 0; k < ft_pow4(s); ++k) {
             t[ft_w1(s) + k] = w(k, 2 * s + 2);
-            if (s <= 4) {
-                t[ft_w2(s) + k] = w(2 * k, 2 * s + 2);
-                t[ft_w3(s) + k] = w(3 * k, 2 * s + 2);
-            }
+            t[ft_w2(s) + k] = w(2 * k, 2 * s + 2);
+            t[ft_w3(s) + k] = w(3 * k, 2 * s + 2);
         }
     for (int a = 2; a <= 6; ++a)
         for (int k = 0; k < ft_pow4(a); ++k) t[ft_r2(a) + k] = w(k, 2 * a + 1);
@@ -114,9 +113,10 @@ __device__ __forceinline__ void bfly4(float2& v0, float2& v1, float2& v2, float2
 
 // the three factors of stage S (Ns = 4^S) at index k
 template <int S, bool FULL, bool INV>
-__device__ __forceinline__ void stage_tw(const float2* __restrict__ T, int k, float2& w1, float2& w2, float2& w3) {
+__device__ __forceinline__ void stage_tw(const float2* __restrict__ T, bool full, int k, float2& w1, float2& w2,
+                                         float2& w3) {
     w1 = tw_dir<INV>(__ldg(T + ft_w1(S) + k));
-    if constexpr (FULL) {
+    if (FULL || full) {
         w2 = tw_dir<INV>(__ldg(T + ft_w2(S) + k));
         w3 = tw_dir<INV>(__ldg(T + ft_w3(S) + k));
     } else {
@@ -128,13 +128,13 @@ __device__ __forceinline__ void stage_tw(const float2* __restrict__ T, int k, fl
 // Stages S and S + 1 on v[m] = a[t + m TPT]; afterwards v[r + 4 e] is the
 // element 16 (t - k) + k + (r + 4 e) Ns, k = t mod Ns.
 template <int LOGN, int NT, int S, bool INV>
-__device__ __forceinline__ void pass16(float2 (&v)[16], int t, const float2* __restrict__ T) {
+__device__ __forceinline__ void pass16(float2 (&v)[16], int t, const float2* __restrict__ T, bool full) {
     constexpr int Ns = 1 << (2 * S);
     constexpr bool FULL = RegFft<LOGN, NT>::FULL;
     const int k = t & (Ns - 1);
     if constexpr (S > 0) {
         float2 w1, w2, w3;
-        stage_tw<S, FULL, INV>(T, k, w1, w2, w3);
+        stage_tw<S, FULL, INV>(T, full, k, w1, w2, w3);
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
             v[q + 4] = cmul(v[q + 4], w1);
@@ -150,7 +150,7 @@ __device__ __forceinline__ void pass16(float2 (&v)[16], int t, const float2* __r
         float2 a0 = v[4 * r], a1 = v[4 * r + 1], a2 = v[4 * r + 2], a3 = v[4 * r + 3];
         if (S > 0 || r > 0) {
             float2 w1, w2, w3;
-            stage_tw<S + 1, FULL, INV>(T, k + r * Ns, w1, w2, w3);
+            stage_tw<S + 1, FULL, INV>(T, full, k + r * Ns, w1, w2, w3);
             a1 = cmul(a1, w1);
             a2 = cmul(a2, w2);
             a3 = cmul(a3, w3);
@@ -168,7 +168,7 @@ __device__ __forceinline__ void pass16(float2 (&v)[16], int t, const float2* __r
 // The last stages after the radix-16 passes, in place on v[m] = a[t + m TPT]
 // (the results lie at the same places): radix 8 (4 then 2), 4 or 2.
 template <int LOGN, int NT, bool INV>
-__device__ __forceinline__ void pass_tail(float2 (&v)[16], int t, const float2* __restrict__ T) {
+__device__ __forceinline__ void pass_tail(float2 (&v)[16], int t, const float2* __restrict__ T, bool full) {
     constexpr int N4 = LOGN / 2, TPT = RegFft<LOGN, NT>::TPT;
     constexpr bool odd4 = (N4 & 1) != 0, r2 = (LOGN & 1) != 0;
     constexpr bool FULL = RegFft<LOGN, NT>::FULL;
@@ -182,7 +182,7 @@ __device__ __forceinline__ void pass_tail(float2 (&v)[16], int t, const float2* 
         for (int g = 0; g < G; ++g) {
             float2 w1, w2, w3;
             const int k = (t + g * TPT) & (Ns - 1);
-            if constexpr (S > 0) stage_tw<S, FULL, INV>(T, k, w1, w2, w3);
+            if constexpr (S > 0) stage_tw<S, FULL, INV>(T, full, k, w1, w2, w3);
 #pragma unroll
             for (int q = 0; q < (r2 ? 2 : 1); ++q) {
                 const int b = g + 2 * q;   // inputs b + 4 r
@@ -235,26 +235,26 @@ __device__ __forceinline__ void exchange(float2 (&v)[16], int t, float2* s) {
 
 // N-point transform of one group of TPT threads: in and out v[m] = a[t + m TPT].
 // s: this transform's shared memory (RegFft::SM float2), free on entry; a
-// caller that writes it afterwards syncs first.
+// caller that writes it afterwards syncs first.  full: see the table above.
 template <int LOGN, int NT, bool INV>
-__device__ __forceinline__ void fft_reg(float2 (&v)[16], int t, float2* s, const float2* __restrict__ T) {
+__device__ __forceinline__ void fft_reg(float2 (&v)[16], int t, float2* s, const float2* __restrict__ T, bool full) {
     using F = RegFft<LOGN, NT>;
     constexpr int NP = LOGN / 4;   // radix-16 passes (LOGN / 2 radix-4 stages in pairs)
     constexpr bool tail = (LOGN & 3) != 0;
-    pass16<LOGN, NT, 0, INV>(v, t, T);
+    pass16<LOGN, NT, 0, INV>(v, t, T, full);
     if constexpr (NP > 1) {
         exchange<LOGN, NT, 0>(v, t, s);
-        pass16<LOGN, NT, 2, INV>(v, t, T);
+        pass16<LOGN, NT, 2, INV>(v, t, T, full);
     }
     if constexpr (NP > 2) {
         F::sync();
         exchange<LOGN, NT, 2>(v, t, s);
-        pass16<LOGN, NT, 4, INV>(v, t, T);
+        pass16<LOGN, NT, 4, INV>(v, t, T, full);
     }
     if constexpr (tail) {
         if constexpr (NP > 1) F::sync();
         exchange<LOGN, NT, 2 * (NP - 1)>(v, t, s);
-        pass_tail<LOGN, NT, INV>(v, t, T);
+        pass_tail<LOGN, NT, INV>(v, t, T, full);
     }
 }
 

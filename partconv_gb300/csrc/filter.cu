@@ -286,11 +286,7 @@ int pcf_setup(pcf_handle* h, int M, const int* N, int* P, const float* ir, int i
     }
     // twiddles
     {
-        std::vector<float2> W((size_t)1 << kWlog);
-        for (size_t m = 0; m < W.size(); ++m) {
-            const double a = -2.0 * M_PI * (double)m / (double)W.size();
-            W[m] = make_float2((float)std::cos(a), (float)std::sin(a));
-        }
+        const std::vector<float2>& W = host_twiddles(kWlog);
         FCK(dalloc(h, &h->W, W.size()), "alloc");
         FCK(cudaMemcpyAsync(h->W, W.data(), sizeof(float2) * W.size(), cudaMemcpyHostToDevice, h->stream), "upload");
         FCK(cudaStreamSynchronize(h->stream), "sync");

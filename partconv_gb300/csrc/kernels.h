@@ -4,6 +4,7 @@
 
 #include <cstddef>
 #include <string>
+#include <vector>
 
 #include "engine_types.h"
 
@@ -17,6 +18,11 @@ struct SpectraJob {
     int logN;
     float2* dst;
 };
+
+// W[m] = exp(-2 pi i m / 2^wlog), computed in double (wlog 15 or 17), and the
+// transform tables of fft_reg.cuh; computed once per process
+const std::vector<float2>& host_twiddles(int wlog);
+const std::vector<float2>& host_fft_tables();
 
 // kernel class by block size: 0 (N <= 1024), 1 (N <= 4096), 2 (N <= 16384),
 // 3 (N <= 65536: a cluster of kClusterCtas CTAs per fire, cluster_fire.cu)

@@ -29,6 +29,17 @@
 // so one MAC task streams one contiguous range of H (about 40 KB: its inputs'
 // rows of the tile, parts adjacent, in the order it sums them) instead of a
 // 0.4 KB segment of every (input, part) row.
+//
+// A call of many base steps runs block-parallel (wide.cu's transforms): the
+// sum over inputs and parts is then, per bin, a product of the outputs' filter
+// matrix with the spectra of many blocks, and H is read once per chunk of
+// blocks instead of once per block (mimo_wide_mac_kernel).  It reads a second
+// copy of H laid out for it, Hw: [output pair][tile of kTile bins][input][part]
+// [bins of the tile] of (re0, re1, im0, im1), operands of packed (f32x2)
+// multiply-adds as they lie (an odd last output is paired with zeros).  One
+// layout for both was slower for one of them: the one-block kernel on the
+// pairs ran 29.7 instead of 25.5 us per launch, the block-parallel one on the
+// tiles of single outputs 727 instead of 640 us per 128 blocks.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -40,8 +51,9 @@
 
 #include "../../include/partconv_gb300.h"
 #include "engine_types.h"
-#include "fft_smem.cuh"
+#include "fft_reg.cuh"
 #include "kernels.h"
+#include "wide.h"
 
 using namespace pcg;
 
@@ -50,17 +62,31 @@ namespace {
 constexpr int kWlog = 15;
 constexpr int kMacNT = 128;        // MAC CTA: threads = (bin-pair column, term group) pairs
 constexpr int kMacMaxBins = 128;   // widest bin tile (64 columns of two bins: two term groups)
+constexpr int kTile = 32;          // bins per tile of Hw (a warp's lanes); a row's last two bins, N
+                                   // and its padding, belong to the tile before them
 constexpr int kMaxMimoLevels = 8;
 constexpr int kMaxMacTerms = 2048;  // (input, part) terms one MAC task sums
+// block-parallel calls: from this many base steps on; base steps per chunk, as
+// many as keep the chunk's spectra within kWideBytes
+constexpr int kWideMinSteps = 8;
+constexpr size_t kWideBytes = (size_t)64 << 20;
+constexpr int kWideMinChunk = 32, kWideMaxChunk = 4096;
+constexpr int kOB = 4;             // outputs a warp sums together
+constexpr int kBB = 8;             // ... and consecutive blocks
+constexpr int kSegBlocks = 2 * kBB;   // blocks per CTA of mimo_wide_mac_kernel (8, 16 or 32)
 
 struct MLevel {
     int N, logN, P, T, s_blocks, cs, rmask, npart;
-    int ntile;           // bin tiles of a row
+    int ntile;           // bin tiles of a row of H
     const int* tstart;   // [ntile + 1]: first bin of each tile (the last entry is cs)
+    int slots;      // rows of an input's spectrum ring (block b in row b mod slots)
+    int nbw;        // most blocks of a block-parallel chunk
     float2* H;      // [nO][tile][nI][P][tile width]
-    float2* X;      // [nI][P][cs]
+    float4* Hw;     // [output pair][tile of kTile][nI][P][tile width] (null: one-block steps only)
+    float2* X;      // [nI][slots][cs]
     float2* Yp;     // [nO][npart][2][cs]
     float2* Yf;     // [nO][cs]
+    float2* Yw;     // [nO][nbw][cs]
     float* yring;   // [nO][rmask + 1]
 };
 
@@ -69,6 +95,16 @@ struct MBank {
     int wlog, N0, nI, nO, M, pad;
     MLevel lv[kMaxMimoLevels];
 };
+
+// tiles of Hw for a row of cs = N + 2 bins, and the tile that holds bin k: first bin, bins
+__host__ __device__ __forceinline__ int tile_count(int cs) { return cs - 2 < kTile ? 1 : (cs - 2) / kTile; }
+__host__ __device__ __forceinline__ int tile_start(int cs, int k) {
+    const int t = k / kTile, n = tile_count(cs);
+    return (t < n ? t : n - 1) * kTile;
+}
+__host__ __device__ __forceinline__ int tile_width(int cs, int k0) {
+    return k0 == (tile_count(cs) - 1) * kTile ? cs - k0 : kTile;
+}
 
 // one task of one stage; kind: 0 input FFT, 1 fire sum, 2 spread, 3 output IFFT
 struct MTask {
@@ -80,12 +116,12 @@ __device__ __forceinline__ long long imod(long long a, long long m) {
     long long r = a % m;
     return r < 0 ? r + m : r;
 }
+__device__ __forceinline__ f32x2 neg2(f32x2 v) { return v ^ 0x8000000080000000ULL; }
 __device__ __forceinline__ float4 f4mac(float4 acc, float4 x, float4 h) {
-    acc.x += x.x * h.x - x.y * h.y;
-    acc.y += x.x * h.y + x.y * h.x;
-    acc.z += x.z * h.z - x.w * h.w;
-    acc.w += x.z * h.w + x.w * h.z;
-    return acc;
+    // the products rounded before they are added: one rounding of the long sum each
+    const float2 lo = cmul(make_float2(x.x, x.y), make_float2(h.x, h.y));
+    const float2 hi = cmul(make_float2(x.z, x.w), make_float2(h.z, h.w));
+    return make_float4(acc.x + lo.x, acc.y + lo.y, acc.z + hi.x, acc.w + hi.y);
 }
 __device__ __forceinline__ float4 f4add(float4 a, float4 b) {
     return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w);
@@ -136,7 +172,7 @@ __global__ void __launch_bounds__(NT) mimo_xfft_kernel(const MBank* __restrict__
     load_twiddles<NT>(twt, logN, bank.W, bank.wlog);
     const long long isamp = rs.io.in_sample;
     const long long b = block_of(l, c);
-    float2* Xs = l.X + ((size_t)t.ch * l.P + (size_t)imod(b, l.P)) * l.cs;
+    float2* Xs = l.X + ((size_t)t.ch * l.slots + (size_t)imod(b, l.slots)) * l.cs;
     // A window that lies wholly in this call's input is transformed before
     // the dependency wait (it reads only the input), its spectrum held in
     // registers until after the wait, when the spectrum ring may be written.
@@ -275,13 +311,13 @@ __global__ void __launch_bounds__(kMacNT, 8) mimo_mac_kernel(const MBank* __rest
     // row offsets (in float4 units) of every (input, part) term, computed
     // once per CTA so the streaming loop carries no index arithmetic
     __shared__ int xoff[kMaxMacTerms], hoff[kMaxMacTerms];
-    const int slot_bt = (int)imod(bt, P);
+    const int R = l.slots, slot_bt = (int)imod(bt, R);
     for (int j = threadIdx.x; j < J; j += kMacNT) {
         const int i = i0 + j / np;
         const int p = p_lo + j % np;
         int sl = slot_bt - p;
-        if (sl < 0) sl += P;
-        xoff[j] = ((i * P + sl) * cs) >> 1;
+        if (sl < 0) sl += R;
+        xoff[j] = ((i * R + sl) * cs) >> 1;
         hoff[j] = ((i * P + p) * (t.k1 - t.k0)) >> 1;
     }
     __syncthreads();
@@ -328,6 +364,216 @@ __global__ void __launch_bounds__(kMacNT, 8) mimo_mac_kernel(const MBank* __rest
     } else {
         const int buf = (l.T == 1) ? (int)(bt & 1) : 0;
         *reinterpret_cast<float4*>(l.Yp + (((size_t)o * l.npart + t.part) * 2 + buf) * cs + k) = acc;
+    }
+}
+
+// ---------------------------------------------------------------------------
+// Block-parallel sum over inputs and parts, Y_o[b] = sum_i sum_p X_i[b-p]
+// H_{i,o,p} per bin.  Lane = bin; a warp keeps kOB outputs x kBB consecutive
+// blocks in registers (packed pairs), so an H value loaded once serves kBB
+// blocks and an X value kOB outputs, and the window of kBB spectra moves by
+// one row per part.  The CTA's four warps take four groups of blocks (the same
+// H, from L1), or with fewer blocks split the inputs; a tile of 2 bins splits
+// the inputs over the lanes instead.  An input's parts are summed last to first
+// (a response decays, so the small terms come first) and folded into a second
+// sum in shared memory: a plain chain over 64 inputs x 16 parts would round
+// four times as much as the one-block kernel's short ones.
+// Bound: float32 multiply-adds (8.3 us per billion cmacs at the packed rate)
+// where H is reused over many blocks, else HBM reading H.
+// ---------------------------------------------------------------------------
+constexpr int kOP = kOB / 2;            // pairs of outputs a warp sums together
+constexpr int kStages = 4;              // pipeline stages of two parts (or an input's window)
+constexpr int kStageBytes = 2 * (16 * kOP + 8) * 32;   // per warp: H and X of two parts
+static_assert(8 * 32 * kBB <= kStageBytes, "a window is one stage");
+struct WideMacSmem {
+    char ring[4][kStages][kStageBytes];
+    f32x2 so[4][kOB * kBB][32];
+};
+// global -> shared copies, each lane its own column; X zero-filled when !on
+__device__ __forceinline__ void cp_async8(unsigned dst, const void* src, bool on) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(dst), "l"(src), "r"(on ? 8 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_async16(unsigned dst, const void* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(src) : "memory");
+}
+
+__global__ void __launch_bounds__(128, 3) mimo_wide_mac_kernel(const MBank* __restrict__ bank_p,
+                                                               const int4* __restrict__ map, long long c0, int nsteps) {
+    extern __shared__ float4 dyn_smem[];
+    WideMacSmem& sm = *reinterpret_cast<WideMacSmem*>(dyn_smem);
+    cudaTriggerProgrammaticLaunchCompletion();
+    const MBank& bank = *bank_p;
+    const int4 e = map[blockIdx.x];   // level, first bin, first output, first block of the chunk
+    const MLevel& l = bank.lv[e.x];
+    const int nI = bank.nI, nO = bank.nO, P = l.P, cs = l.cs, R = l.slots;
+    const long long bf = (c0 + l.s_blocks) / l.T;
+    const int nb = (int)((c0 + nsteps + l.s_blocks) / l.T - bf) - e.w;   // blocks from the CTA's first on
+    cudaGridDependencySynchronize();
+    if (nb <= 0) return;
+    const int t0 = tile_start(cs, e.y), tw = tile_width(cs, t0);   // the tile in memory
+    const int w = min(min(kTile, t0 + tw - e.y), cs - 2 > kTile && e.y < cs - 2 ? cs - 2 - e.y : kTile);
+    const int wl = w > 2 ? 32 : 2, nsub = 32 / wl;   // lanes per set of bins, input split over lanes
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int bin = lane & (wl - 1), sub = lane / wl;
+    const int nbg = min(kSegBlocks / kBB, nb > 2 * kBB ? 4 : (nb > kBB ? 2 : 1)), ks = 4 / nbg;
+    const int g = warp % nbg, kq = warp / nbg;
+    const bool live = bin < w;
+    const int col = min(bin, w - 1);
+    f32x2 re[kOP][kBB], im[kOP][kBB];   // (output 2 q, output 2 q + 1) of pair q
+#pragma unroll
+    for (int q = 0; q < kOP; ++q)
+#pragma unroll
+        for (int j = 0; j < kBB; ++j) {
+            re[q][j] = im[q][j] = 0;
+            sm.so[warp][(2 * q) * kBB + j][lane] = 0;
+            sm.so[warp][(2 * q + 1) * kBB + j][lane] = 0;
+        }
+    // filter rows of the tile, [input][part][tw]; the pairs after the first one
+    // pair_stride further (the last pair again beyond the outputs)
+    const size_t pair_elems = (size_t)nI * P * cs;
+    const int op0 = e.z >> 1, npair = (nO + 1) >> 1;
+    const float4* H0 = l.Hw + op0 * pair_elems + (size_t)t0 * nI * P + (e.y - t0) + col;
+    size_t pair_off[kOP];
+#pragma unroll
+    for (int q = 0; q < kOP; ++q) pair_off[q] = (size_t)(min(op0 + q, npair - 1) - op0) * pair_elems * sizeof(float4);
+    int sl0 = (int)(bf % R) + e.w + g * kBB;   // ring row of the group's first block
+    sl0 %= R;
+    const int step = ks * nsub, wrap = R * cs;
+    const int nit = g * kBB < nb ? (nI - kq * nsub + step - 1) / step : 0;
+    // The copies run kStages - 1 stages ahead of the sums, through every input:
+    // a stage is an input's window under its last part or two parts' filter
+    // values with the two spectra that enter the window after them.
+    const unsigned ring0 = (unsigned)__cvta_generic_to_shared(sm.ring[warp][0]);
+    int p_it = 0, p_part = -1, p_ox = 0;   // the producer: input, part (-1: the window)
+    unsigned p_slot = ring0;
+    bool p_on = false;
+    const float2* p_X = l.X;
+    const char* p_H = reinterpret_cast<const char*>(H0);
+    auto next_slot = [&](unsigned sl) { return sl == ring0 + (kStages - 1) * kStageBytes ? ring0 : sl + kStageBytes; };
+    auto produce = [&]() {
+        if (p_it < nit) {
+            if (p_part < 0) {
+                const int i0 = kq * nsub + p_it * step + sub, i = min(i0, nI - 1);
+                p_on = live && i0 < nI;
+                p_X = l.X + (size_t)i * R * cs + e.y + col;
+                p_H = reinterpret_cast<const char*>(H0 + ((size_t)i * P + P - 1) * tw);
+                p_ox = sl0 - (P - 1);   // the window under the last part
+                p_ox = (p_ox < 0 ? p_ox + R : p_ox) * cs;
+                int o = p_ox;
+#pragma unroll
+                for (int j = 0; j < kBB; ++j) {
+                    cp_async8(p_slot + (j * 32 + lane) * 8, p_X + o, p_on);
+                    o += cs;
+                    if (o >= wrap) o -= wrap;
+                }
+                p_ox = o;               // the block that enters next
+                p_part = 0;
+            } else {
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                    if (p_part + u < P) {
+#pragma unroll
+                        for (int q = 0; q < kOP; ++q)
+                            cp_async16(p_slot + ((u * kOP + q) * 32 + lane) * 16, p_H + pair_off[q]);
+                        p_H -= tw * sizeof(float4);
+                        cp_async8(p_slot + 2 * kOP * 512 + (u * 32 + lane) * 8, p_X + p_ox, p_on);
+                        p_ox += cs;
+                        if (p_ox >= wrap) p_ox -= wrap;
+                    }
+                }
+                p_part += 2;
+                if (p_part >= P) {
+                    p_part = -1;
+                    ++p_it;
+                }
+            }
+        }
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+        p_slot = next_slot(p_slot);
+    };
+    auto landed = [&]() { asm volatile("cp.async.wait_group %0;\n" ::"n"(kStages - 2) : "memory"); };
+#pragma unroll
+    for (int q = 0; q < kStages - 1; ++q) produce();
+    int c_slot = 0;
+    for (int it = 0; it < nit; ++it) {
+        // (re, re) and (im, im) of the window: block (first) + j under the r-th part at [(j + r) mod kBB]
+        f32x2 xr[kBB], xi[kBB];
+        auto put = [&](int q, f32x2 v) {
+            const float2 t = unpack2(v);
+            xr[q] = pack2(t.x, t.x);
+            xi[q] = pack2(t.y, t.y);
+        };
+        landed();
+        {
+            const f32x2* d = reinterpret_cast<const f32x2*>(sm.ring[warp][c_slot]);
+#pragma unroll
+            for (int j = 0; j < kBB; ++j) put(j, d[j * 32 + lane]);
+        }
+        c_slot = (c_slot + 1) & (kStages - 1);
+        produce();
+        for (int p0 = 0; p0 < P; p0 += kBB) {
+#pragma unroll
+            for (int s = 0; s < kBB / 2; ++s) {
+                if (p0 + 2 * s >= P) break;
+                landed();
+                const char* d = sm.ring[warp][c_slot];
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                    const int r = 2 * s + u;   // r-th part from the last, mod kBB
+                    if (p0 + r >= P) break;
+#pragma unroll
+                    for (int q = 0; q < kOP; ++q) {
+                        const ulonglong2 h = reinterpret_cast<const ulonglong2*>(d)[(u * kOP + q) * 32 + lane];
+                        const f32x2 hr = h.x, hi = h.y, hn = neg2(h.y);
+                        // (sixteen independent sums between the two products of one)
+#pragma unroll
+                        for (int j = 0; j < kBB; ++j) {
+                            const int m = (j + r) % kBB;
+                            re[q][j] = fma2(xr[m], hr, re[q][j]);
+                            im[q][j] = fma2(xr[m], hi, im[q][j]);
+                        }
+#pragma unroll
+                        for (int j = 0; j < kBB; ++j) {
+                            const int m = (j + r) % kBB;
+                            re[q][j] = fma2(xi[m], hn, re[q][j]);
+                            im[q][j] = fma2(xi[m], hr, im[q][j]);
+                        }
+                    }
+                    put(r % kBB,
+                        reinterpret_cast<const f32x2*>(d + 2 * kOP * 512)[u * 32 + lane]);   // (unused after the last part)
+                }
+                c_slot = (c_slot + 1) & (kStages - 1);
+                produce();
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < kOP; ++q)
+#pragma unroll
+            for (int j = 0; j < kBB; ++j) {
+                f32x2& dr = sm.so[warp][(2 * q) * kBB + j][lane];
+                f32x2& di = sm.so[warp][(2 * q + 1) * kBB + j][lane];
+                dr = add2(dr, re[q][j]);
+                di = add2(di, im[q][j]);
+                re[q][j] = im[q][j] = 0;
+            }
+    }
+    __syncthreads();
+    // the input ranges in order: lanes, then warps
+    const int items = nbg * kOP * kBB * wl;
+    for (int x = threadIdx.x; x < items; x += 128) {
+        const int bi = x & (wl - 1), r = x / wl, j = r % kBB, q = r / kBB % kOP, gg = r / (kBB * kOP);
+        const int o = e.z + 2 * q, b = gg * kBB + j;
+        if (bi >= w || o >= nO || b >= nb) continue;
+        f32x2 vr = sm.so[gg][(2 * q) * kBB + j][bi], vi = sm.so[gg][(2 * q + 1) * kBB + j][bi];
+        for (int p = 1; p < ks * nsub; ++p) {
+            const int ww = (p / nsub) * nbg + gg, ll = (p % nsub) * wl + bi;
+            vr = add2(vr, sm.so[ww][(2 * q) * kBB + j][ll]);
+            vi = add2(vi, sm.so[ww][(2 * q + 1) * kBB + j][ll]);
+        }
+        const float2 yr = unpack2(vr), yi = unpack2(vi);
+        float2* Y = l.Yw + ((size_t)o * l.nbw + e.w + b) * cs + e.y + bi;
+        Y[0] = make_float2(yr.x, yi.x);
+        if (o + 1 < nO) Y[(size_t)l.nbw * cs] = make_float2(yr.y, yi.y);
     }
 }
 
@@ -381,7 +627,7 @@ __global__ void __launch_bounds__(NT) mimo_yifft_kernel(const MBank* __restrict_
 // filter spectra of one path row: H[o][i][p] = rfft([0_N, h_{i,o}[start + pN ...]]) / 2N
 template <int NT, int MAXB>
 __global__ void __launch_bounds__(NT) mimo_spectra_kernel(const float* __restrict__ irs, int ir_len, int nI, int nO,
-                                                          int N, int logN, int P, int cs, long long start, float2* H,
+                                                          int N, int logN, int P, int cs, long long start, float2* H, float4* Hw,
                                                           const int* __restrict__ tstart, int ntile,
                                                           const float2* W, int wlog) {
     extern __shared__ float4 dyn_smem[];
@@ -406,7 +652,9 @@ __global__ void __launch_bounds__(NT) mimo_spectra_kernel(const float* __restric
     fft_smem<NT, MAXB>(s, N, logN, tw, false);
     const float inv = 1.0f / (float)(2 * N);
     // bin k of path (i, o), part p goes to its tile: H[o][tile][i][p][k - tile start]
+    // and to Hw[o / 2][tile][i][p][k - tile start], (re, im) of output o mod 2
     float2* Ho = H + (size_t)o * nI * P * cs;
+    float* Hwo = reinterpret_cast<float*>(Hw + (size_t)(o >> 1) * nI * P * cs) + (o & 1);
     const int ip = i * P + p;
     auto put = [&](int kb, float2 v) {
         int lo = 0, hi = ntile;   // tile t with tstart[t] <= kb < tstart[t + 1]
@@ -417,6 +665,12 @@ __global__ void __launch_bounds__(NT) mimo_spectra_kernel(const float* __restric
         }
         const int k0 = tstart[lo], w = tstart[lo + 1] - k0;
         Ho[(size_t)k0 * nI * P + (size_t)ip * w + (kb - k0)] = v;
+        if (Hw) {
+            const int t0 = tile_start(cs, kb);
+            float* d = Hwo + 4 * ((size_t)t0 * nI * P + (size_t)ip * tile_width(cs, t0) + (kb - t0));
+            d[0] = v.x;
+            d[2] = v.y;
+        }
     };
     for (int k = threadIdx.x; k <= N / 2; k += NT) {
         const int nk = (k == 0) ? 0 : N - k;
@@ -462,6 +716,22 @@ struct pcm_handle {
     std::vector<int> off[3], cnt[3];
     std::vector<double> mac_bytes;   // algorithmic bytes of K2 per phase
     std::vector<std::vector<int>> tiles;   // per level: bin tile starts (last entry cs)
+    // block-parallel calls (wide.cu): descriptors of every (level, input) and
+    // (output, level), CTA maps in order of their first block's step and the
+    // prefix of each that a chunk of n + 1 steps needs
+    int C = 32;       // base steps per chunk
+    bool wide_ok = true;
+    const float2* d_tab = nullptr;
+    const WLevel* d_wlv = nullptr;
+    const int* d_lv0 = nullptr;   // level-0 descriptor of every input
+    int n_wlv = 0, w_nt = 0;
+    const int2* w_map[3] = {};    // windows, inverse transforms of levels >= 1, output
+    const int4* w_mac = nullptr;
+    std::vector<int> w_upto[4];
+    // spread tasks that rebuild the partial sums after such a call: per level,
+    // first task and tasks of the first j slices
+    std::vector<int> state_off;
+    std::vector<std::vector<int>> state_cnt;
     size_t state_bytes_total = 0;
     std::vector<std::pair<void*, size_t>> state;   // zeroed by reset
     long long frame_num = 0;
@@ -483,12 +753,19 @@ int mfail(pcm_handle* h, int code, const std::string& m) {
     } while (0)
 
 template <class T>
-cudaError_t malloc_zero(pcm_handle* h, T** p, size_t n, bool is_state) {
+cudaError_t malloc_raw(pcm_handle* h, T** p, size_t n) {
     const size_t bytes = sizeof(T) * std::max<size_t>(n, 1);
     cudaError_t e = cudaMalloc((void**)p, bytes);
     if (e != cudaSuccess) return e;
     h->allocs.push_back(*p);
     h->device_bytes += bytes;
+    return e;
+}
+template <class T>
+cudaError_t malloc_zero(pcm_handle* h, T** p, size_t n, bool is_state) {
+    cudaError_t e = malloc_raw(h, p, n);
+    if (e != cudaSuccess) return e;
+    const size_t bytes = sizeof(T) * std::max<size_t>(n, 1);
     if (is_state) h->state.push_back({*p, bytes});
     return cudaMemsetAsync(*p, 0, bytes, h->stream);
 }
@@ -527,6 +804,156 @@ cudaError_t launch_mac(pcm_handle* h, int grid, const MTask* tasks, const RunSta
     cudaLaunchAttribute attr[1];
     cudaLaunchConfig_t cfg = pdl_cfg(grid, kMacNT, 0, st, attr, pdl);
     return cudaLaunchKernelEx(&cfg, mimo_mac_kernel, (const MBank*)h->d_bank, tasks, rs);
+}
+
+// descriptors and CTA maps of the block-parallel kernels, cleared rings
+int setup_wide(pcm_handle* h) {
+    const MBank& B = h->hbank;
+    const int M = h->M, nI = h->nI, nO = h->nO;
+    std::vector<WLevel> wl;
+    std::vector<int> lv0(nI);
+    auto common = [&](int L) {
+        const MLevel& l = B.lv[L];
+        WLevel w{};
+        w.N = l.N;
+        w.logN = l.logN;
+        w.P = 1;
+        for (int t = l.T; t > 1; t >>= 1) ++w.logT;
+        w.s_blocks = l.s_blocks;
+        w.cs = l.cs;
+        w.slots = l.slots;
+        w.M = M;
+        w.scale = 1.0f;
+        return w;
+    };
+    for (int i = 0; i < nI; ++i) {   // inputs: window transforms
+        lv0[i] = (int)wl.size();
+        for (int L = 0; L < M; ++L) {
+            WLevel w = common(L);
+            w.P = B.lv[L].P;
+            w.in_ch = i;
+            w.rin_mask = h->rin_mask;
+            w.X = B.lv[L].X + (size_t)i * w.slots * w.cs;
+            w.xring = h->xring + (size_t)i * (h->rin_mask + 1);
+            wl.push_back(w);
+        }
+    }
+    const int out0 = (int)wl.size();
+    for (int o = 0; o < nO; ++o)     // outputs: inverse transforms
+        for (int L = 0; L < M; ++L) {
+            WLevel w = common(L);
+            const MLevel& l = B.lv[L];
+            w.out_ch = o;
+            w.mix_mode = 1;
+            w.lv0 = out0 + o * M;
+            w.rmask = l.rmask;
+            w.Yw = l.Yw + (size_t)o * l.nbw * l.cs;
+            w.yring = l.yring + (size_t)o * (l.rmask + 1);
+            wl.push_back(w);
+        }
+    h->n_wlv = (int)wl.size();
+    h->w_nt = wide_threads(h->maxN);
+    std::vector<std::pair<int, int2>> e[3];
+    std::vector<std::pair<int, int4>> mac;
+    for (int L = 0; L < M; ++L) {
+        const MLevel& l = B.lv[L];
+        for (int b = 0; b < l.nbw; b += 16 * h->w_nt / l.N) {
+            for (int i = 0; i < nI; ++i) e[0].push_back({b * l.T, make_int2(i * M + L, b)});
+            for (int o = 0; o < nO && L > 0; ++o) e[1].push_back({b * l.T, make_int2(out0 + o * M + L, b)});
+        }
+        for (int b = 0; b < l.nbw && L == 0; b += wide_out_blocks(l.N))
+            for (int o = 0; o < nO; ++o) e[2].push_back({b, make_int2(out0 + o * M, b)});
+        for (int b = 0; b < l.nbw; b += kSegBlocks)
+            for (int k = 0; k < l.cs; k += kTile)   // (the last two bins by themselves)
+                for (int o = 0; o < nO; o += kOB) mac.push_back({b * l.T, make_int4(L, k, o, b)});
+    }
+    // one allocation and one upload for all the tables
+    std::vector<char> blob;
+    auto put = [&](const void* src, size_t bytes) {
+        const size_t at = blob.size();
+        blob.resize(at + ((bytes + 255) & ~(size_t)255));
+        if (bytes) std::memcpy(blob.data() + at, src, bytes);
+        return at;
+    };
+    auto put_map = [&](auto& v, std::vector<int>& upto) {
+        using E = std::remove_reference_t<decltype(v[0].second)>;
+        std::stable_sort(v.begin(), v.end(), [](auto& a, auto& b) { return a.first < b.first; });
+        std::vector<E> flat;
+        for (auto& x : v) flat.push_back(x.second);
+        upto.assign(h->C, 0);
+        size_t j = 0;
+        for (int n = 0; n < h->C; ++n) {
+            while (j < v.size() && v[j].first <= n) ++j;
+            upto[n] = (int)j;
+        }
+        return put(flat.data(), sizeof(E) * flat.size());
+    };
+    size_t at[7];
+    for (int m = 0; m < 3; ++m) at[m] = put_map(e[m], h->w_upto[m]);
+    at[3] = put_map(mac, h->w_upto[3]);
+    at[4] = put(wl.data(), sizeof(WLevel) * wl.size());
+    at[5] = put(lv0.data(), sizeof(int) * lv0.size());
+    at[6] = put(host_fft_tables().data(), sizeof(float2) * host_fft_tables().size());
+    char* d = nullptr;
+    MCK(cudaMalloc(&d, blob.size()), "alloc tables");
+    h->allocs.push_back(d);
+    h->device_bytes += blob.size();
+    MCK(cudaMemcpyAsync(d, blob.data(), blob.size(), cudaMemcpyHostToDevice, h->stream), "upload tables");
+    MCK(cudaStreamSynchronize(h->stream), "sync");
+    for (int m = 0; m < 3; ++m) h->w_map[m] = reinterpret_cast<const int2*>(d + at[m]);
+    h->w_mac = reinterpret_cast<const int4*>(d + at[3]);
+    h->d_wlv = reinterpret_cast<const WLevel*>(d + at[4]);
+    h->d_lv0 = reinterpret_cast<const int*>(d + at[5]);
+    h->d_tab = reinterpret_cast<const float2*>(d + at[6]);
+    MCK(launch_wide_reset(h->d_wlv, h->n_wlv, nullptr, 0, h->stream), "clear rings");
+    return PC_OK;
+}
+
+// nsteps base steps from h->frame_num, block-parallel
+int mimo_wide(pcm_handle* h, const IOView& io, long long nsteps, cudaStream_t st) {
+    WArgs a{};
+    a.lv = h->d_wlv;
+    a.tab = h->d_tab;
+    a.N0 = h->N0;
+    a.kb = 1;
+    a.full = 1;   // as the one-block kernels here
+    a.io = io;
+    a.vec_in = io.in_sample == 1 && (h->nI == 1 || io.in_ch % 2 == 0) && (reinterpret_cast<uintptr_t>(io.in) & 7) == 0;
+    a.vec_out =
+        io.out_sample == 1 && (h->nO == 1 || io.out_ch % 2 == 0) && (reinterpret_cast<uintptr_t>(io.out) & 7) == 0;
+    while (nsteps > 0) {
+        const int n = (int)std::min<long long>(nsteps, h->C);
+        a.c0 = h->frame_num;
+        a.nsteps = n;
+        MCK(launch_wide_fft(false, h->w_nt, h->w_upto[0][n - 1], h->w_map[0], a, st), "MIMO windows");
+        cudaLaunchAttribute attr[1];
+        cudaLaunchConfig_t cfg = pdl_cfg(h->w_upto[3][n - 1], 128, sizeof(WideMacSmem), st, attr, true);
+        MCK(cudaLaunchKernelEx(&cfg, mimo_wide_mac_kernel, (const MBank*)h->d_bank, h->w_mac, a.c0, n),
+            "MIMO sums");
+        MCK(launch_wide_fft(true, h->w_nt, h->w_upto[1][n - 1], h->w_map[1], a, st), "MIMO inverse");
+        MCK(launch_wide_out(h->N0, h->w_upto[2][n - 1], h->w_map[2], a, st), "MIMO output");
+        h->launches += 3 + (h->w_upto[1][n - 1] > 0);
+        h->frame_num += n;
+        nsteps -= n;
+    }
+    // the input rings and partial sums one-block steps would have left
+    a.c0 = h->frame_num;
+    a.nsteps = 0;
+    MCK(launch_wide_state(256, 64, 0, nullptr, h->d_lv0, h->nI, h->rin_mask + 1, a, st), "MIMO input rings");
+    h->launches += 1;
+    RunState rs{};
+    rs.step_base = h->frame_num - 1;
+    rs.io = io;
+    for (int L = 0; L < h->M; ++L) {
+        const MLevel& l = h->hbank.lv[L];
+        const auto& cnt = h->state_cnt[L];
+        const int phi = (int)((h->frame_num + l.s_blocks) % l.T);   // slices built since the level's last block
+        const int n = cnt.size() < 2 ? 0 : cnt[l.T == 1 ? 1 : phi];
+        if (n <= 0) continue;
+        MCK(launch_mac(h, n, h->d_tasks + h->state_off[L], rs, st, true), "MIMO partial sums");
+        h->launches += 1;
+    }
+    return PC_OK;
 }
 
 // one base step; kernel k of the step is timed by ev[k] pairs when given
@@ -589,17 +1016,24 @@ int pcm_setup(pcm_handle* h, int fs, int buffer_size, int n_in, int n_out, int M
         MCK(cudaFuncSetAttribute(mimo_yifft_kernel<512, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, 12 * 16384), "attr");
         MCK(cudaFuncSetAttribute(mimo_spectra_kernel<512, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, 12 * 16384), "attr");
     }
+    {
+        const double row = sizeof(float2) * (double)buffer_size * M * std::max(n_in, n_out);   // per base step
+        h->wide_ok = true;
+        h->tiles.clear();
+        h->C = kWideMaxChunk;
+        while (h->C > kWideMinChunk && h->C * row > (double)kWideBytes) h->C >>= 1;
+    }
     // twiddles
     float2* W = nullptr;
     {
-        std::vector<float2> Wh((size_t)1 << kWlog);
-        for (size_t m = 0; m < Wh.size(); ++m) {
-            const double a = -2.0 * M_PI * (double)m / (double)Wh.size();
-            Wh[m] = make_float2((float)std::cos(a), (float)std::sin(a));
-        }
+        const std::vector<float2>& Wh = host_twiddles(kWlog);
         MCK(malloc_zero(h, &W, Wh.size(), false), "alloc");
         MCK(cudaMemcpyAsync(W, Wh.data(), sizeof(float2) * Wh.size(), cudaMemcpyHostToDevice, h->stream), "upload");
         MCK(cudaStreamSynchronize(h->stream), "sync");
+        MCK(prepare_wide_kernels(), "kernel attributes");
+        MCK(cudaFuncSetAttribute(mimo_wide_mac_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)sizeof(WideMacSmem)),
+            "kernel attributes");
     }
     int rin = 1;
     while (rin < 2 * h->maxN) rin <<= 1;
@@ -626,7 +1060,7 @@ int pcm_setup(pcm_handle* h, int fs, int buffer_size, int n_in, int n_out, int M
         l.s_blocks = (int)(s / buffer_size);
         l.cs = Nv[L] + 2;
         long R = Nv[L];
-        while (R < s + buffer_size) R <<= 1;
+        while (R < s + (long)h->C * buffer_size) R <<= 1;   // a chunk's samples in flight
         l.rmask = (int)R - 1;
         // input ranges per spread task (about 8 inputs each, more ranges when
         // a range times the older parts exceeds what one MAC task sums)
@@ -649,8 +1083,9 @@ int pcm_setup(pcm_handle* h, int fs, int buffer_size, int n_in, int n_out, int M
             auto tiles_of = [&](int lo, int hi) {
                 const int n = hi - lo;
                 int best_nt = 0;
-                double best = -1.0;
-                for (int nt = (n + kMacMaxBins - 1) / kMacMaxBins; nt <= 16; ++nt) {
+                double best = -1e30;
+                const int nt0 = (n + kMacMaxBins - 1) / kMacMaxBins;
+                for (int nt = nt0; nt <= std::max(nt0, 16); ++nt) {
                     const int per = ((n + nt - 1) / nt + 1) & ~1;
                     if (per < 2 || (nt - 1) * per >= n) continue;
                     double busy = 0.0;
@@ -687,24 +1122,39 @@ int pcm_setup(pcm_handle* h, int fs, int buffer_size, int n_in, int n_out, int M
             h->tiles.push_back(ts);
         }
         MCK(malloc_zero(h, &l.H, (size_t)n_out * n_in * l.P * l.cs, false), "alloc H");
-        MCK(malloc_zero(h, &l.X, (size_t)n_in * l.P * l.cs, true), "alloc");
+        // the copy for block-parallel calls; without room for it every call runs one-block steps
+        if (h->wide_ok &&
+            malloc_zero(h, &l.Hw, (size_t)((n_out + 1) / 2) * n_in * l.P * l.cs, false) != cudaSuccess) {
+            cudaGetLastError();
+            l.Hw = nullptr;
+            h->wide_ok = false;
+        }
+        l.nbw = (h->C + l.T - 1) / l.T;
+        l.slots = l.P + std::max(l.nbw, kBB);
+        if ((long long)n_in * l.slots * l.cs >= (1LL << 31)) {   // 32-bit offsets: one-block steps only
+            l.slots = l.P;
+            h->wide_ok = false;
+        }
+        // (cleared in part by setup_wide)
+        MCK(malloc_raw(h, &l.X, (size_t)n_in * l.slots * l.cs), "alloc");
+        MCK(malloc_raw(h, &l.Yw, (size_t)n_out * l.nbw * l.cs), "alloc");
         MCK(malloc_zero(h, &l.Yp, (size_t)n_out * l.npart * 2 * l.cs, true), "alloc");
         MCK(malloc_zero(h, &l.Yf, (size_t)n_out * l.cs, true), "alloc");
-        MCK(malloc_zero(h, &l.yring, (size_t)n_out * R, true), "alloc");
+        MCK(malloc_raw(h, &l.yring, (size_t)n_out * R), "alloc");
         const size_t smem = (size_t)12 * l.N;
         const int rows = n_out * n_in * l.P;
         switch (cls_of(l.N)) {
             case 0:
                 mimo_spectra_kernel<256, 1><<<rows, 256, smem, h->stream>>>(d_irs, ir_len, n_in, n_out, l.N, l.logN, l.P,
-                                                                            l.cs, s, l.H, l.tstart, l.ntile, W, kWlog);
+                                                                            l.cs, s, l.H, l.Hw, l.tstart, l.ntile, W, kWlog);
                 break;
             case 1:
                 mimo_spectra_kernel<512, 2><<<rows, 512, smem, h->stream>>>(d_irs, ir_len, n_in, n_out, l.N, l.logN, l.P,
-                                                                            l.cs, s, l.H, l.tstart, l.ntile, W, kWlog);
+                                                                            l.cs, s, l.H, l.Hw, l.tstart, l.ntile, W, kWlog);
                 break;
             default:
                 mimo_spectra_kernel<512, 8><<<rows, 512, smem, h->stream>>>(d_irs, ir_len, n_in, n_out, l.N, l.logN, l.P,
-                                                                            l.cs, s, l.H, l.tstart, l.ntile, W, kWlog);
+                                                                            l.cs, s, l.H, l.Hw, l.tstart, l.ntile, W, kWlog);
                 break;
         }
         MCK(cudaGetLastError(), "MIMO spectra");
@@ -715,6 +1165,22 @@ int pcm_setup(pcm_handle* h, int fs, int buffer_size, int n_in, int n_out, int M
     MCK(cudaMemcpyAsync(h->d_bank, &B, sizeof(MBank), cudaMemcpyHostToDevice, h->stream), "upload bank");
 
     // ---- per-phase task lists --------------------------------------------------------
+    // spread tasks of slice j of level L's row (level 0: the whole row); returns its bins
+    auto spread_tasks = [&](const MLevel& l, int L, int j, std::vector<MTask>& dst) {
+        const int nch = l.T == 1 ? 1 : l.T - 1;
+        const int lo = (int)(((long)j * l.cs / nch) & ~1L);
+        const int hi = (j == nch - 1) ? l.cs : (int)(((long)(j + 1) * l.cs / nch) & ~1L);
+        const std::vector<int>& ts = h->tiles[L];
+        for (int o = 0; o < n_out; ++o)
+            for (size_t t = 0; t + 1 < ts.size(); ++t) {
+                if (ts[t] < lo || ts[t + 1] > hi) continue;
+                for (int q = 0; q < l.npart; ++q) {
+                    const int i0 = (int)((long)q * n_in / l.npart), i1 = (int)((long)(q + 1) * n_in / l.npart);
+                    dst.push_back(MTask{2, L, o, ts[t], ts[t + 1], i0, i1, q});
+                }
+            }
+        return hi - lo;
+    };
     std::vector<std::vector<MTask>> lists[3];
     for (auto& v : lists) v.assign(h->H, {});
     h->mac_bytes.assign(h->H, 0.0);
@@ -735,33 +1201,28 @@ int pcm_setup(pcm_handle* h, int fs, int buffer_size, int n_in, int n_out, int M
                 h->mac_bytes[g] += 8.0 * C * ((double)n_out * n_in * np + (double)n_in * np);
             }
             // spread: level 0 every step over parts >= 2; other levels in the
-            // T-1 steps after their block, a slice of bins per step
-            int lo = 0, hi = 0, p_lo = 1;
-            if (l.T == 1) {
-                if (l.P < 3) continue;
-                lo = 0;
-                hi = l.cs;
-                p_lo = 2;
-            } else {
-                if (l.P < 2) continue;
-                const int phi = (g + 1 + l.s_blocks) % l.T;
-                if (phi == 0) continue;
-                const int j = phi - 1, nch = l.T - 1;
-                lo = (int)(((long)j * l.cs / nch) & ~1L);
-                hi = (j == nch - 1) ? l.cs : (int)(((long)(j + 1) * l.cs / nch) & ~1L);
-            }
-            if (hi <= lo) continue;
-            std::vector<std::pair<int, int>> tl;   // the level's fixed tiles within [lo, hi)
-            const std::vector<int>& ts = h->tiles[L];
-            for (size_t t = 0; t + 1 < ts.size(); ++t)
-                if (ts[t] >= lo && ts[t + 1] <= hi) tl.push_back({ts[t], ts[t + 1]});
-            for (int o = 0; o < n_out; ++o)
-                for (auto& kk : tl)
-                    for (int q = 0; q < l.npart; ++q) {
-                        const int i0 = (int)((long)q * n_in / l.npart), i1 = (int)((long)(q + 1) * n_in / l.npart);
-                        lists[1][g].push_back(MTask{2, L, o, kk.first, kk.second, i0, i1, q});
-                    }
-            h->mac_bytes[g] += 8.0 * (hi - lo) * ((double)n_out * n_in * (l.P - p_lo) + (double)n_in * (l.P - p_lo));
+            // T-1 steps after their block, a slice of bins (whole tiles) per step
+            const int p_lo = l.T == 1 ? 2 : 1;
+            if (l.P <= p_lo) continue;
+            const int phi = (g + 1 + l.s_blocks) % l.T;
+            if (l.T > 1 && phi == 0) continue;
+            const int bins = spread_tasks(l, L, l.T == 1 ? 0 : phi - 1, lists[1][g]);
+            h->mac_bytes[g] += 8.0 * bins * ((double)n_out * n_in * (l.P - p_lo) + (double)n_in * (l.P - p_lo));
+        }
+    }
+    // after a block-parallel call: the spread tasks of the steps since each
+    // level's last block, in slice order
+    std::vector<MTask> state;
+    h->state_off.assign(M, 0);
+    h->state_cnt.assign(M, {});
+    for (int L = 0; L < M; ++L) {
+        const MLevel& l = B.lv[L];
+        h->state_off[L] = (int)state.size();
+        h->state_cnt[L].push_back(0);
+        if (l.P <= (l.T == 1 ? 2 : 1)) continue;
+        for (int j = 0; j < std::max(1, l.T - 1); ++j) {
+            spread_tasks(l, L, j, state);
+            h->state_cnt[L].push_back((int)state.size() - h->state_off[L]);
         }
     }
     size_t ntask = 0;
@@ -775,12 +1236,18 @@ int pcm_setup(pcm_handle* h, int fs, int buffer_size, int n_in, int n_out, int M
         }
     }
     std::vector<MTask> all;
-    all.reserve(ntask);
+    all.reserve(ntask + state.size());
     for (int st = 0; st < 3; ++st)
         for (int g = 0; g < h->H; ++g) all.insert(all.end(), lists[st][g].begin(), lists[st][g].end());
+    for (int& o : h->state_off) o += (int)ntask;
+    all.insert(all.end(), state.begin(), state.end());
     MCK(malloc_zero(h, &h->d_tasks, all.size(), false), "alloc tasks");
     MCK(cudaMemcpyAsync(h->d_tasks, all.data(), sizeof(MTask) * all.size(), cudaMemcpyHostToDevice, h->stream),
         "upload tasks");
+    {
+        int r2 = setup_wide(h);
+        if (r2) return r2;
+    }
     MCK(cudaStreamSynchronize(h->stream), "setup sync");
     cudaFree(d_irs);
     h->allocs.erase(std::find(h->allocs.begin(), h->allocs.end(), (void*)d_irs));
@@ -817,6 +1284,7 @@ int pcm_process_device(pcm_handle* h, float* d_out, const float* d_in, long long
         rs.io.out_ch = 1;
     }
     const long long nsteps = frames / h->N0;
+    if (nsteps >= kWideMinSteps && h->wide_ok) return mimo_wide(h, rs.io, nsteps, st);
     for (long long s = 0; s < nsteps; ++s) {
         rs.step_base = h->frame_num + s;
         int r = mimo_step(h, rs, st, s == 0, nullptr);
@@ -832,6 +1300,7 @@ int pcm_reset(pcm_handle* h) {
     if (!h->ready) return PC_OK;
     cudaSetDevice(h->device);
     for (auto& z : h->state) MCK(cudaMemsetAsync(z.first, 0, z.second, h->stream), "reset");
+    MCK(launch_wide_reset(h->d_wlv, h->n_wlv, nullptr, 0, h->stream), "reset");
     MCK(cudaStreamSynchronize(h->stream), "reset sync");
     return PC_OK;
 }

@@ -210,11 +210,7 @@ extern "C" int pc_convolve_noalloc(const float* d_x, long long n_frames, const f
                 return fail(PC_ERR_CUDA, std::string("cudaGetSymbolAddress: ") + cudaGetErrorString(e));
             e = prepare_kernels();
             if (e != cudaSuccess) return fail(PC_ERR_CUDA, std::string("kernel attributes: ") + cudaGetErrorString(e));
-            std::vector<float2> W((size_t)1 << kWlog);
-            for (size_t m = 0; m < W.size(); ++m) {
-                const double a = -2.0 * M_PI * (double)m / (double)W.size();
-                W[m] = make_float2((float)std::cos(a), (float)std::sin(a));
-            }
+            const std::vector<float2>& W = host_twiddles(kWlog);
             e = cudaMemcpy(p, W.data(), sizeof(float2) * W.size(), cudaMemcpyHostToDevice);
             if (e != cudaSuccess) return fail(PC_ERR_CUDA, std::string("twiddle upload: ") + cudaGetErrorString(e));
             g_scratch_addr[dev] = static_cast<unsigned char*>(p);

@@ -252,11 +252,7 @@ pcs_handle* pcs_create(int buffer_size, long long hbm_budget_bytes, int max_pcs)
         return bad();
     }
     h->fl.init(h->budget);
-    std::vector<float2> W((size_t)1 << kWlog);
-    for (size_t m = 0; m < W.size(); ++m) {
-        const double a = -2.0 * M_PI * (double)m / (double)W.size();
-        W[m] = make_float2((float)std::cos(a), (float)std::sin(a));
-    }
+    const std::vector<float2>& W = host_twiddles(kWlog);
     if (smalloc(h, &h->d_W, W.size()) != cudaSuccess) return bad();
     if (cudaMemcpyAsync(h->d_W, W.data(), sizeof(float2) * W.size(), cudaMemcpyHostToDevice, h->stream) != cudaSuccess)
         return bad();

@@ -44,14 +44,21 @@ __device__ __forceinline__ long long imod(long long a, long long m) {
     return r < 0 ? r + m : r;
 }
 
+// two complex multiply-adds: (x.x + i x.y)(h.x + i h.y), (x.z + i x.w)(h.z + i h.w),
+// fused with the sum (two roundings of it per product: for chains of a few)
 __device__ __forceinline__ float4 f4mac(float4 acc, float4 x, float4 h) {
-    // two complex multiply-adds: (x.x + i x.y)(h.x + i h.y), (x.z + i x.w)(h.z + i h.w)
     const float2 lo = cmac(make_float2(acc.x, acc.y), make_float2(x.x, x.y), make_float2(h.x, h.y));
     const float2 hi = cmac(make_float2(acc.z, acc.w), make_float2(x.z, x.w), make_float2(h.z, h.w));
     return make_float4(lo.x, lo.y, hi.x, hi.y);
 }
 __device__ __forceinline__ float4 f4add(float4 a, float4 b) {
     return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w);
+}
+// acc + x h with the product rounded first (one rounding of the sum: for long chains)
+__device__ __forceinline__ float4 f4mul_add(float4 acc, float4 x, float4 h) {
+    const float2 lo = cmul(make_float2(x.x, x.y), make_float2(h.x, h.y));
+    const float2 hi = cmul(make_float2(x.z, x.w), make_float2(h.z, h.w));
+    return f4add(acc, make_float4(lo.x, lo.y, hi.x, hi.y));
 }
 
 // Kernel class: threads per CTA, largest block size, operand prefetch.
@@ -87,9 +94,11 @@ __host__ __device__ constexpr size_t fire_smem_bytes(int N, bool prefetch) {
 // Spread: the streaming FDL MAC over the task's bins [k0, k1) and parts
 // [p_lo, p_hi).  NT threads form G = NT / LANES part-groups of LANES
 // threads; thread t owns bins k0 + 2 (t mod LANES), +1 (one float4) and group
-// g = t / LANES sums the g-th of G runs of consecutive parts; the groups
-// are added in order through shared memory (the block-parallel sum, wide.cu,
-// keeps this order with one running sum at a time).  Bins per task (2 LANES; a tile shape the autotuner
+// g = t / LANES sums the g-th of G runs of consecutive parts, in running sums
+// of four added in order (short chains: the sum of a long response does not
+// round more often than its parts); the groups are added in order through
+// shared memory (the block-parallel sum, wide.cu, keeps this order with one
+// running sum at a time).  Bins per task (2 LANES; a tile shape the autotuner
 // picks per handle) travel in the task's M field, 0 meaning kSpreadBins;
 // each width is its own instantiation (constant strides): the step kernel
 // is instantiated per width and launched for the handle's width.  Parts per task
@@ -149,9 +158,11 @@ __device__ __forceinline__ void spread_lanes(const Task& tk, long long c, float4
                 }
                 sl = sl == 0 ? R - 1 : sl - 1;
             }
+            float4 s4 = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
             for (int u = 0; u < U; ++u)
-                if (p0 + u < pe) acc = f4mac(acc, xv[u], hv[u]);
+                if (p0 + u < pe) s4 = f4mac(s4, xv[u], hv[u]);
+            acc = p0 == pb ? s4 : f4add(acc, s4);
         }
     }
     if (G > 1) {
@@ -223,11 +234,13 @@ __device__ __forceinline__ void spread_multi(const Task& tk, long long c, float4
                 sl = sl == 0 ? R - 1 : sl - 1;
             }
 #pragma unroll
-            for (int u = 0; u < U; ++u)
-                if (p0 + u < pe) {
+            for (int j = 0; j < KM; ++j) {   // running sums of two parts
+                float4 s2 = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-                    for (int j = 0; j < KM; ++j) acc[j] = f4mac(acc[j], xv[u][j], hv[u]);
-                }
+                for (int u = 0; u < U; ++u)
+                    if (p0 + u < pe) s2 = f4mac(s2, xv[u][j], hv[u]);
+                acc[j] = p0 == pb ? s2 : f4add(acc[j], s2);
+            }
         }
     }
 #pragma unroll
@@ -855,7 +868,7 @@ __device__ __forceinline__ void fire_multi(const Bank& bank, const Task& tk, con
             if (it < nitem) {
                 int t, col;
                 item(it, t, col);
-                for (int p = 0; p <= t && p < Q; ++p) acc[i] = f4mac(acc[i], X4(Q - 1 + t - p, col), H4(p, col));
+                for (int p = 0; p <= t && p < Q; ++p) acc[i] = f4mul_add(acc[i], X4(Q - 1 + t - p, col), H4(p, col));
             }
         }
     }
@@ -948,7 +961,7 @@ __device__ __forceinline__ void fire_multi(const Bank& bank, const Task& tk, con
         for (int p = 1; p < Q; ++p) {
 #pragma unroll
             for (int i = 0; i < MAXI; ++i)
-                if (p > ti[i]) acc[i] = f4mac(acc[i], X4(Q - 1 + ti[i] - p, ci[i]), H4(p, ci[i]));
+                if (p > ti[i]) acc[i] = f4mul_add(acc[i], X4(Q - 1 + ti[i] - p, ci[i]), H4(p, ci[i]));
         }
 #pragma unroll
         for (int i = 0; i < MAXI; ++i) {

@@ -32,6 +32,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 
 #include "engine_types.h"
 #include "fft_reg.cuh"
@@ -94,7 +95,7 @@ __device__ __forceinline__ void fft_body(const WLevel& l, int first, const WArgs
             }
         }
     }
-    fft_reg<LOGN, NT, false>(v, t, s, a.tab);
+    fft_reg<LOGN, NT, false>(v, t, s, a.tab, a.full != 0);
     // the split pairs k < N / 2 (this thread's v[0 .. 7]) with N - k, which
     // lies in another thread's upper half
     F::sync();
@@ -192,27 +193,30 @@ struct MacCol {
     }
 };
 
-// Sums X_{b+j-p} H_p, j < RB, over n consecutive parts in groups of tg (one
-// running sum each, the groups added in order into row); c stands at the first
-// part on entry and after the last one on return.  The run's RB spectra under
-// part p stay in registers: part p + 1 needs one new one.  The loads of four
-// parts go together; with tg = 4 (TG4, the default tiles) they are a group.
+// Sums X_{b+j-p} H_p, j < RB, over n consecutive parts in groups of tg, a group
+// in running sums of `unit` parts (running sums added in order into the group,
+// groups in order into row); c stands at the first part on entry and after the
+// last one on return.  The run's RB spectra under part p stay in registers:
+// part p + 1 needs one new one.  The loads of four parts go together; TG4:
+// tg = unit = 4 (the default tiles), they are a group.
 template <int RB, bool TG4, bool SH>
-__device__ __forceinline__ void sum_parts(MacCol<SH>& c, int n, int tg, f32x2 (&row)[RB]) {
+__device__ __forceinline__ void sum_parts(MacCol<SH>& c, int n, int tg, int unit, f32x2 (&row)[RB]) {
     constexpr int U = 4;
     static_assert(RB % U == 0, "constant window rotation");
     f32x2 acc[RB], w[RB], ws[RB];   // window: block (run's first) + d - first part at w[d mod RB], and its swapped pairs
+    f32x2 grp[TG4 ? 1 : RB];
     {
         int o = c.ox;
 #pragma unroll
         for (int j = 0; j < RB; ++j) {
             row[j] = acc[j] = 0;
+            if constexpr (!TG4) grp[j] = 0;
             w[j] = c.x(o);
             ws[j] = swap2(w[j]);
             o = c.fwd(o);
         }
     }
-    int left = tg;
+    int left = tg, run = unit;   // parts until the group and the running sum end
     for (int i0 = 0; i0 < n; i0 += RB) {
 #pragma unroll
         for (int s = 0; s < RB / U; ++s) {
@@ -241,12 +245,21 @@ __device__ __forceinline__ void sum_parts(MacCol<SH>& c, int n, int tg, f32x2 (&
                 w[q] = nx[u];
                 ws[q] = swap2(nx[u]);
                 if constexpr (!TG4) {
-                    if (--left == 0) {
-                        left = tg;
+                    --left;
+                    if (--run == 0 || left == 0 || i0 + r + 1 == n) {
+                        run = unit;
 #pragma unroll
                         for (int j = 0; j < RB; ++j) {
-                            row[j] = add2(row[j], acc[j]);
+                            grp[j] = add2(grp[j], acc[j]);
                             acc[j] = 0;
+                        }
+                        if (left == 0 || i0 + r + 1 == n) {
+                            left = tg;
+#pragma unroll
+                            for (int j = 0; j < RB; ++j) {
+                                row[j] = add2(row[j], grp[j]);
+                                grp[j] = 0;
+                            }
                         }
                     }
                 }
@@ -257,11 +270,24 @@ __device__ __forceinline__ void sum_parts(MacCol<SH>& c, int n, int tg, f32x2 (&
             }
         }
     }
-    if constexpr (!TG4) {
-        if (left != tg) {
+}
+
+// row[j] = sum of X_{b+j-p} H_p over the first n parts, one by one with each
+// product rounded before it is added (fire_multi's sum)
+template <int RB, bool SH>
+__device__ __forceinline__ void chain_parts(MacCol<SH> c, int n, float2 (&y)[RB]) {
 #pragma unroll
-            for (int j = 0; j < RB; ++j) row[j] = add2(row[j], acc[j]);
+    for (int j = 0; j < RB; ++j) y[j] = make_float2(0.f, 0.f);
+    for (int p = 0; p < n; ++p) {
+        const float2 h = c.h();
+        int o = c.ox;
+#pragma unroll
+        for (int j = 0; j < RB; ++j) {
+            y[j] = cadd(y[j], cmul(unpack2(c.x(o)), h));
+            o = c.fwd(o);
         }
+        c.H += c.cs;
+        c.ox = c.back(c.ox);
     }
 }
 
@@ -361,7 +387,7 @@ __global__ void __launch_bounds__(kMacTile) wide_mac_kernel(const int4* __restri
                 c.ox = (q < 0 ? q + RX : q) * W;
 #pragma unroll
                 for (int j = 0; j < RB; ++j) ys[j] = 0;
-                if (P > l.p_lo) sum_parts<RB, true>(c, P - l.p_lo, 4, ys);
+                if (P > l.p_lo) sum_parts<RB, true>(c, P - l.p_lo, 4, 4, ys);
                 c.H = Hs + tid;
                 c.ox = pos * W;
                 finish_run(c, l, ys, Y + (size_t)i0 * cs, nb - i0);
@@ -388,7 +414,7 @@ __global__ void __launch_bounds__(kMacTile) wide_mac_kernel(const int4* __restri
             if (live) {
                 f32x2 row[RB];
                 MacCol<true> c{Hs + tid, Xs + tid, W, (TP + RB) * W, n * W};
-                sum_parts<RB, true>(c, n, 4, row);
+                sum_parts<RB, true>(c, n, 4, 4, row);
 #pragma unroll
                 for (int j = 0; j < RB; ++j) ys[j] = q == 0 ? row[j] : add2(ys[j], row[j]);
             }
@@ -428,7 +454,7 @@ __global__ void __launch_bounds__(kMacAnyNT, 3) wide_mac_any_kernel(const int4* 
         c.ox = (o < 0 ? o + R : o) * cs;
         for (int q = 0; q < l.nrows; ++q) {
             f32x2 row[RB];
-            sum_parts<RB, false>(c, min(l.tp, P - l.p_lo - q * l.tp), l.tpg, row);
+            sum_parts<RB, false>(c, min(l.tp, P - l.p_lo - q * l.tp), l.tpg, l.multi ? 2 : 4, row);
 #pragma unroll
             for (int j = 0; j < RB; ++j) ys[j] = q == 0 ? row[j] : add2(ys[j], row[j]);
         }
@@ -436,12 +462,12 @@ __global__ void __launch_bounds__(kMacAnyNT, 3) wide_mac_any_kernel(const int4* 
     c.H = l.H + k;
     c.ox = sl * cs;
     float2* Y = l.Yw + (size_t)i0 * cs + k;
-    if (l.multi) {   // parts < p_lo in one running sum
-        f32x2 y[RB];
-        sum_parts<RB, false>(c, l.p_lo, l.p_lo, y);
+    if (l.multi) {   // parts < p_lo one by one
+        float2 y[RB];
+        chain_parts<RB>(c, l.p_lo, y);
 #pragma unroll
         for (int j = 0; j < RB; ++j)
-            if (i0 + j < nb) Y[(size_t)j * cs] = unpack2(rows ? add2(y[j], ys[j]) : y[j]);
+            if (i0 + j < nb) Y[(size_t)j * cs] = rows ? cadd(y[j], unpack2(ys[j])) : y[j];
     } else {
         finish_run(c, l, ys, Y, nb - i0);
     }
@@ -478,7 +504,7 @@ __device__ __forceinline__ void ifft_body(const WLevel& l, int first, const WArg
             merge_w(yc, yn, __ldg(sp + N - n), other, v[m]);
         }
     }
-    fft_reg<LOGN, NT, true>(v, t, s, a.tab);
+    fft_reg<LOGN, NT, true>(v, t, s, a.tab, a.full != 0);
     if (!live) return;
     // real samples 2 n, 2 n + 1 of the block in v[m], n = t + m TPT < N / 2
     if constexpr (!L0) {
@@ -659,6 +685,23 @@ struct OutPrepare {
 };
 
 }  // namespace
+
+static std::vector<float2> make_twiddles(int wlog) {
+    std::vector<float2> W((size_t)1 << wlog);
+    for (size_t m = 0; m < W.size(); ++m) {
+        const double a = -2.0 * M_PI * (double)m / (double)W.size();
+        W[m] = make_float2((float)std::cos(a), (float)std::sin(a));
+    }
+    return W;
+}
+const std::vector<float2>& host_twiddles(int wlog) {
+    static const std::vector<float2> w15 = make_twiddles(15), w17 = make_twiddles(17);
+    return wlog == 15 ? w15 : w17;
+}
+const std::vector<float2>& host_fft_tables() {
+    static const std::vector<float2> t = build_fft_tables(host_twiddles(15), 15);
+    return t;
+}
 
 cudaError_t prepare_wide_kernels() {
     cudaError_t e = cudaFuncSetAttribute(wide_fft_kernel<1024>, cudaFuncAttributeMaxDynamicSharedMemorySize,

@@ -19,7 +19,7 @@ struct WLevel {
     int two;        // the fire adds X_{b-1} H_1 itself
     int in_ch, out_ch, mix_mode, M;
     int rin_mask, lv0, dfer;
-    int tp, tpg;    // parts per partial-sum row, and per running sum within one
+    int tp, tpg;    // parts per partial-sum row, and per group within one
     float scale;
     const float2* H;
     float2* X;
@@ -38,6 +38,7 @@ struct WArgs {
     long long c0;         // first base step of the chunk
     int nsteps, kb;       // base steps of the chunk; base blocks per step of the handle
     int vec_in, vec_out;  // contiguous channels, 8-byte aligned: float2 loads and stores
+    int full;             // every twiddle factor from the table (fft_reg.cuh)
     IOView io;
 };
 
