@@ -93,7 +93,8 @@ constexpr int kTaskVec = 13;   // a Task record is loaded as 13 x 16 bytes
 static_assert(sizeof(Task) == 16 * kTaskVec, "Task record size");
 
 // One CTA of a serving pool's step: descriptor slot and sub-task (0: the
-// level's fire, s >= 1: the s-th bin tile of its spread slice).
+// level's fire, s >= 1: the s-th bin tile of its spread slice).  A slot < 0
+// stands for the channel -1 - slot, which has no PC: its output is zero.
 struct PoolCta {
     int slot;
     int sub;

@@ -106,6 +106,10 @@ struct pcs_handle {
     PoolCta* d_map[3] = {nullptr, nullptr, nullptr};
     size_t map_cap = 0;
     int map_n[3] = {0, 0, 0};
+    int channels = 0;                        // 1 + the largest live id: the channels the map writes
+    // levels of a class that fire within steps congruent to i modulo the table's
+    // length (a power of two): a class whose levels have nothing due is not launched
+    std::vector<int> due[3];
     bool map_dirty = false;
     float* d_in = nullptr;                   // [max_pcs][N0] staging
     float* d_out = nullptr;
@@ -190,13 +194,30 @@ size_t pc_bytes(int N0, const std::vector<int>& N, const std::vector<int>& P, si
 
 int rebuild_map(pcs_handle* h) {
     std::vector<PoolCta> m[3];
-    for (int id = 0; id < (int)h->pcs.size(); ++id) {
+    const int c0 = fire_class_of(h->N0);
+    h->channels = 0;
+    int tmax = 1;
+    for (int id = 0; id < (int)h->pcs.size(); ++id)
+        if (h->pcs[id].live) {
+            h->channels = id + 1;
+            tmax = std::max(tmax, h->pcs[id].N.back() / h->N0);
+        }
+    for (auto& d : h->due) d.assign(tmax, 0);
+    for (int id = 0; id < h->channels; ++id) {
         const PoolPC& p = h->pcs[id];
-        if (!p.live) continue;
+        if (!p.live) {
+            m[c0].push_back({-1 - id, 0});
+            continue;
+        }
         for (int L = 0; L < p.M; ++L) {
             const int slot = id * kPoolMaxLevels + L;
-            m[fire_class_of(p.N[L])].push_back({slot, 0});
-            for (int t = 1; t <= p.spread_tiles[L]; ++t) m[fire_class_of(h->N0)].push_back({slot, t});
+            const int cls = fire_class_of(p.N[L]);
+            m[cls].push_back({slot, 0});
+            for (int t = 1; t <= p.spread_tiles[L]; ++t) m[c0].push_back({slot, t});
+            // the level fires at steps c with (c - origin + 1 + s) % T == 0
+            const Task& t = h->h_slots[slot];
+            long long r = (t.origin - 1 - t.s_blocks) % t.T;
+            for (int i = (int)(r < 0 ? r + t.T : r); i < tmax; i += t.T) h->due[cls][i]++;
         }
     }
     size_t need = std::max({m[0].size(), m[1].size(), m[2].size(), (size_t)1});
@@ -522,11 +543,29 @@ int pcs_step(pcs_handle* h, const float* in, float* out, int n_channels) {
     if (n_channels < 0 || n_channels > h->max_pcs) return sfail(h, PC_ERR_ARG, "bad channel count");
     SCK(cudaSetDevice(h->device), "cudaSetDevice");
     const size_t nb = sizeof(float) * (size_t)n_channels * h->N0;
-    if (nb) SCK(cudaMemcpyAsync(h->d_in, in, nb, cudaMemcpyHostToDevice, h->stream), "input copy");
+    // Pinned buffers of exactly the pool's channels are read and written by the
+    // kernels themselves (no copy engine start-up per block on either side);
+    // others, which the caller may change once this returns, go through copies.
+    bool direct = n_channels == h->channels && n_channels > 0;
+    const float* src = h->d_in;
+    float* dst = h->d_out;
+    if (direct) {
+        cudaPointerAttributes ai, ao;
+        direct = cudaPointerGetAttributes(&ai, in) == cudaSuccess && ai.type == cudaMemoryTypeHost &&
+                 cudaPointerGetAttributes(&ao, out) == cudaSuccess && ao.type == cudaMemoryTypeHost &&
+                 ai.devicePointer && ao.devicePointer;
+        if (direct) {
+            src = static_cast<const float*>(ai.devicePointer);
+            dst = static_cast<float*>(ao.devicePointer);
+        } else {
+            cudaGetLastError();
+        }
+    }
+    if (nb && !direct) SCK(cudaMemcpyAsync(h->d_in, in, nb, cudaMemcpyHostToDevice, h->stream), "input copy");
     RunState rs{};
     rs.step_base = h->step;
-    rs.io.in = h->d_in;
-    rs.io.out = h->d_out;
+    rs.io.in = src;
+    rs.io.out = dst;
     rs.io.step0 = h->step;
     rs.io.in_step = 0;
     rs.io.in_sample = 1;
@@ -538,12 +577,13 @@ int pcs_step(pcs_handle* h, const float* in, float* out, int n_channels) {
     for (int k = 0; k < 3; ++k) {
         const int cls = (c0 + k) % 3;
         if (h->map_n[cls] <= 0) continue;
+        if (cls != c0 && h->due[cls][h->step & (long long)(h->due[cls].size() - 1)] == 0) continue;
         SCK(launch_pool_class(cls, h->map_n[cls], std::max(h->class_maxN[cls], 16), h->bank, h->d_slots, h->d_map[cls],
                               rs, h->stream),
             "pool step");
         h->launches++;
     }
-    if (nb) SCK(cudaMemcpyAsync(out, h->d_out, nb, cudaMemcpyDeviceToHost, h->stream), "output copy");
+    if (nb && !direct) SCK(cudaMemcpyAsync(out, h->d_out, nb, cudaMemcpyDeviceToHost, h->stream), "output copy");
     SCK(cudaEventRecord(h->done, h->stream), "event");
     h->step++;
     return PC_OK;

@@ -1093,6 +1093,11 @@ __global__ void __launch_bounds__(C::NT) pool_kernel(Bank bank, const Task* __re
     __shared__ int s_last;
     const int tid = threadIdx.x;
     const PoolCta pm = map[blockIdx.x];
+    if (pm.slot < 0) {
+        for (int i = tid; i < bank.N0; i += C::NT)
+            rs_val.io.out[i * rs_val.io.out_sample + (-1 - pm.slot) * rs_val.io.out_ch] = 0.0f;
+        return;
+    }
     if (tid < kTaskVec) reinterpret_cast<int4*>(&tk)[tid] = __ldg(reinterpret_cast<const int4*>(slots + pm.slot) + tid);
     if (tid == 64) rs = rs_val;
     __syncthreads();
