@@ -41,10 +41,10 @@ __host__ __device__ constexpr int ft_r2(int a) { return ft_w3(7) + (ft_pow4(a) -
 __host__ __device__ constexpr int ft_sp(int l) { return ft_r2(7) + (1 << (l - 1)) - 8 + 2 * (l - 4); }
 constexpr int kFftTabEntries = ft_sp(15);
 
-// The table, from W[m] = exp(-2 pi i m / 2^wlog) (quarter-turn symmetry as in
-// Twiddles::get, so the values are the ones fft_smem's stages use).
-inline std::vector<float2> build_fft_tables(const std::vector<float2>& W, int wlog) {
-    std::vector<float2> t((size_t)kFftTabEntries, make_float2(1.f, 0.f));
+// The entries for transforms up to 2^max_log points, from W[m] =
+// exp(-2 pi i m / 2^wlog) (quarter-turn symmetry as in Twiddles::get, so the
+// values are the ones fft_smem's stages use), by thread t of nt.
+__host__ __device__ inline void fill_fft_tables(float2* tab, const float2* W, int wlog, int max_log, int t, int nt) {
     auto w = [&](long long a, int lg) {   // exp(-2 pi i a / 2^lg)
         const long long i = a << (wlog - lg);
         const int q = (int)(i >> (wlog - 2));
@@ -53,17 +53,21 @@ inline std::vector<float2> build_fft_tables(const std::vector<float2>& W, int wl
         const float sg = (q & 2) ? -1.0f : 1.0f;
         return make_float2(sg * (odd ? v.y : v.x), sg * (odd ? -v.x : v.y));
     };
-    for (int s = 1; s <= 6; ++s)
-        for (int k = 0; k < ft_pow4(s); ++k) {
-            t[ft_w1(s) + k] = w(k, 2 * s + 2);
-            t[ft_w2(s) + k] = w(2 * k, 2 * s + 2);
-            t[ft_w3(s) + k] = w(3 * k, 2 * s + 2);
+    for (int s = 1; s <= 6 && 2 * s + 2 <= max_log; ++s)
+        for (int k = t; k < ft_pow4(s); k += nt) {
+            tab[ft_w1(s) + k] = w(k, 2 * s + 2);
+            tab[ft_w2(s) + k] = w(2 * k, 2 * s + 2);
+            tab[ft_w3(s) + k] = w(3 * k, 2 * s + 2);
         }
-    for (int a = 2; a <= 6; ++a)
-        for (int k = 0; k < ft_pow4(a); ++k) t[ft_r2(a) + k] = w(k, 2 * a + 1);
-    for (int l = kRegMinLog; l <= kRegMaxLog; ++l)
-        for (int k = 0; k <= (1 << (l - 1)); ++k) t[ft_sp(l) + k] = w(k, l + 1);
-    return t;
+    for (int a = 2; a <= 6 && 2 * a + 1 <= max_log; ++a)
+        for (int k = t; k < ft_pow4(a); k += nt) tab[ft_r2(a) + k] = w(k, 2 * a + 1);
+    for (int l = kRegMinLog; l <= max_log; ++l)
+        for (int k = t; k <= (1 << (l - 1)); k += nt) tab[ft_sp(l) + k] = w(k, l + 1);
+}
+inline std::vector<float2> build_fft_tables(const std::vector<float2>& W, int wlog) {
+    std::vector<float2> tab((size_t)kFftTabEntries, make_float2(1.f, 0.f));
+    fill_fft_tables(tab.data(), W.data(), wlog, kRegMaxLog, 0, 1);
+    return tab;
 }
 
 // Shared-memory index of point i: one spare element per 16, so the strided

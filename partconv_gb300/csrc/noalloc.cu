@@ -18,11 +18,14 @@
 // with a one-CTA kernel from scalar launch arguments, so a call reads no
 // host memory and makes no host-to-device copy.
 //
-// The work is the step kernel of the multi-level engine run on a one-level
-// layout (block size N0, P = ceil(len(h) / N0) parts), so the result equals
-// pc_run over the same samples with a fresh handle.
+// The work is that of the multi-level engine on a one-level layout (block size
+// N0, P = ceil(len(h) / N0) parts), so the result equals pc_run over the same
+// samples with a fresh handle: block-parallel (wide.cu) in chunks of as many
+// blocks as the rest of the array holds, or, for a few blocks or a response
+// that leaves no room, one step kernel per block.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -32,7 +35,9 @@
 
 #include "../../include/partconv_gb300.h"
 #include "engine_types.h"
+#include "fft_reg.cuh"
 #include "kernels.h"
+#include "wide.h"
 
 using namespace pcg;
 
@@ -42,6 +47,10 @@ constexpr size_t kScratchBytes = (size_t)32 << 20;   // PC_NOALLOC_SCRATCH_BYTES
 static_assert(kScratchBytes == (size_t)PC_NOALLOC_SCRATCH_BYTES, "header and implementation disagree");
 constexpr int kWlog = 15;
 constexpr int kMaxDevices = 64;
+constexpr int kWideMinBlocks = 4;   // calls of at least this many blocks run block-parallel ...
+constexpr int kWideMinChunk = 8;    // ... if the array holds a chunk of this many
+constexpr int kWideMaxChunk = 4096;
+constexpr int kSeg = kWideRun;      // blocks per CTA of the sum over parts: one response has few tiles
 
 // The scratch array.  In host code its name is only a host-side stand-in;
 // the device address comes from cudaGetSymbolAddress, once per device.
@@ -149,6 +158,69 @@ __global__ void noalloc_tables_kernel(TableArgs a) {
     }
 }
 
+// The block-parallel form: where its tables and rows sit, in place of the step
+// path's after the filter spectra and their jobs.
+struct WideTables {
+    unsigned char* base;
+    const float* h;
+    int h_len, N, logN, P, cs, C, slots, nfwd, nmac;
+    size_t o_W, o_jobs, o_H, o_tab, o_lv, o_fwd, o_mac, o_xr, o_X, o_Yw;
+};
+
+// Writes the level descriptor, the CTA maps, the spectrum jobs and the transform
+// table, and clears the spectrum rows before the first block and the silence
+// before the first sample.
+__global__ void noalloc_wide_tables_kernel(WideTables a) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, nt = gridDim.x * blockDim.x;
+    float2* H = reinterpret_cast<float2*>(a.base + a.o_H);
+    float2* X = reinterpret_cast<float2*>(a.base + a.o_X);
+    float* xr = reinterpret_cast<float*>(a.base + a.o_xr);
+    if (t == 0) {
+        WLevel l{};
+        l.N = a.N;
+        l.logN = a.logN;
+        l.P = a.P;
+        l.cs = a.cs;
+        l.slots = a.slots;
+        l.p_lo = 2;
+        l.tp = 16;
+        l.tpg = 4;
+        l.nrows = a.P > 2 ? (a.P - 2 + 15) / 16 : 0;
+        l.two = 1;
+        l.mix_mode = 1;
+        l.M = 1;
+        l.rin_mask = 2 * a.N - 1;
+        l.scale = 1.0f;
+        l.H = H;
+        l.X = X;
+        l.Yw = reinterpret_cast<float2*>(a.base + a.o_Yw);
+        l.xring = xr;
+        *reinterpret_cast<WLevel*>(a.base + a.o_lv) = l;
+    }
+    const int per = 2048 / a.N;   // transforms per CTA
+    for (int i = t; i < a.nfwd; i += nt) reinterpret_cast<int2*>(a.base + a.o_fwd)[i] = make_int2(0, i * per);
+    const int tiles = (a.cs + kMacTile - 1) / kMacTile;
+    for (int i = t; i < a.nmac; i += nt)
+        reinterpret_cast<int4*>(a.base + a.o_mac)[i] =
+            make_int4(0, i % tiles * kMacTile, i / tiles * kSeg, min(a.C, (i / tiles + 1) * kSeg));
+    for (int p = t; p < a.P; p += nt) {
+        const long start = (long)p * a.N;
+        SpectraJob j;
+        j.src = a.h + start;
+        j.len = (int)min((long)a.N, (long)a.h_len - start);
+        j.N = a.N;
+        j.logN = a.logN;
+        j.dst = H + (size_t)p * a.cs;
+        reinterpret_cast<SpectraJob*>(a.base + a.o_jobs)[p] = j;
+    }
+    // the table's values are those of W, which the host wrote
+    fill_fft_tables(reinterpret_cast<float2*>(a.base + a.o_tab), reinterpret_cast<const float2*>(a.base + a.o_W), kWlog,
+                    a.logN, t, nt);
+    for (int i = t; i < 2 * a.N; i += nt) xr[i] = 0.0f;
+    const size_t z0 = (size_t)(a.slots - (a.P - 1)) * a.cs, z1 = (size_t)a.slots * a.cs;   // blocks -(P - 1) .. -1
+    for (size_t i = z0 + t; i < z1; i += nt) X[i] = make_float2(0.f, 0.f);
+}
+
 }  // namespace
 
 extern "C" int pc_convolve_noalloc(const float* d_x, long long n_frames, const float* d_h, int h_len, float* d_y,
@@ -209,6 +281,7 @@ extern "C" int pc_convolve_noalloc(const float* d_x, long long n_frames, const f
             if (e != cudaSuccess)
                 return fail(PC_ERR_CUDA, std::string("cudaGetSymbolAddress: ") + cudaGetErrorString(e));
             e = prepare_kernels();
+            if (e == cudaSuccess) e = prepare_wide_kernels();
             if (e != cudaSuccess) return fail(PC_ERR_CUDA, std::string("kernel attributes: ") + cudaGetErrorString(e));
             const std::vector<float2>& W = host_twiddles(kWlog);
             e = cudaMemcpy(p, W.data(), sizeof(float2) * W.size(), cudaMemcpyHostToDevice);
@@ -216,6 +289,74 @@ extern "C" int pc_convolve_noalloc(const float* d_x, long long n_frames, const f
             g_scratch_addr[dev] = static_cast<unsigned char*>(p);
         }
         base = g_scratch_addr[dev];
+    }
+
+    // ---- many blocks: block-parallel chunks ------------------------------------------------
+    const long long nblocks = n_frames / N;
+    if (nblocks >= kWideMinBlocks) {
+        size_t o = 0;
+        WideTables wt{};
+        wt.o_W = take(o, sizeof(float2) << kWlog);
+        wt.o_jobs = take(o, sizeof(SpectraJob) * (size_t)P);
+        wt.o_H = take(o, sizeof(float2) * (size_t)P * cs);
+        wt.o_tab = take(o, sizeof(float2) * kFftTabEntries);
+        wt.o_lv = take(o, sizeof(WLevel));
+        wt.o_xr = take(o, sizeof(float) * 2 * N);
+        // a block of a chunk takes a spectrum row, a summed row and its share of the maps
+        const int tiles = (cs + kMacTile - 1) / kMacTile, per = 2048 / N;
+        const long long rows = ((long long)kScratchBytes - (long long)o - 4096) / (long long)(sizeof(float2) * cs);
+        const long long map_rows = (long long)((sizeof(int4) * tiles + sizeof(int2)) / (sizeof(float2) * cs) + 1);
+        const long long C = std::min<long long>({(rows - P - kWideRun) / (2 + map_rows), nblocks, kWideMaxChunk});
+        if (C >= kWideMinChunk || (C >= nblocks && C > 0)) {
+            wt.base = base;
+            wt.h = d_h;
+            wt.h_len = h_len;
+            wt.N = N;
+            wt.logN = logN;
+            wt.P = P;
+            wt.cs = cs;
+            wt.C = (int)C;
+            wt.slots = P + (int)std::max<long long>(C, kWideRun);
+            wt.nfwd = (int)((C + per - 1) / per);
+            wt.nmac = (int)((C + kSeg - 1) / kSeg) * tiles;
+            wt.o_fwd = take(o, sizeof(int2) * (size_t)wt.nfwd);
+            wt.o_mac = take(o, sizeof(int4) * (size_t)wt.nmac);
+            wt.o_X = take(o, sizeof(float2) * (size_t)wt.slots * cs);
+            wt.o_Yw = take(o, sizeof(float2) * (size_t)C * cs);
+        }
+        if (wt.base && o <= kScratchBytes) {
+            noalloc_wide_tables_kernel<<<96, 256, 0, st>>>(wt);
+            if ((e = cudaGetLastError()) != cudaSuccess)
+                return fail(PC_ERR_CUDA, std::string("scratch tables: ") + cudaGetErrorString(e));
+            e = launch_spectra(cls, P, N, reinterpret_cast<const SpectraJob*>(base + wt.o_jobs),
+                               reinterpret_cast<const float2*>(base + wt.o_W), kWlog, st);
+            if (e != cudaSuccess) return fail(PC_ERR_CUDA, std::string("filter spectra: ") + cudaGetErrorString(e));
+            WArgs a{};
+            a.lv = reinterpret_cast<const WLevel*>(base + wt.o_lv);
+            a.tab = reinterpret_cast<const float2*>(base + wt.o_tab);
+            a.N0 = N;
+            a.kb = 1;
+            a.vec_in = (reinterpret_cast<uintptr_t>(d_x) & 7) == 0;
+            a.vec_out = (reinterpret_cast<uintptr_t>(d_y) & 7) == 0;
+            a.io.in = d_x;
+            a.io.out = d_y;
+            a.io.in_step = a.io.out_step = N;
+            a.io.in_sample = a.io.out_sample = 1;
+            const int2* fwd = reinterpret_cast<const int2*>(base + wt.o_fwd);
+            const int4* mac = reinterpret_cast<const int4*>(base + wt.o_mac);
+            for (long long c = 0; c < nblocks; c += C) {
+                const int n = (int)std::min<long long>(C, nblocks - c);
+                a.c0 = c;
+                a.nsteps = n;
+                // (the maps were written by this call: the first kernel that reads them must not start early)
+                if ((e = launch_wide_fft(false, 128, (n + per - 1) / per, fwd, a, st, c > 0)) != cudaSuccess ||
+                    (e = launch_wide_mac(false, (n + kSeg - 1) / kSeg * tiles, mac, a, st)) != cudaSuccess ||
+                    (e = launch_wide_out(N, (n + per - 1) / per, fwd, a, st)) != cudaSuccess)
+                    return fail(PC_ERR_CUDA, std::string("block-parallel launch: ") + cudaGetErrorString(e));
+            }
+            pcg_set_global_error("");
+            return PC_OK;
+        }
     }
 
     // ---- descriptor tables (a kernel: no host memory is read), cleared state,

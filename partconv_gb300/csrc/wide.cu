@@ -716,9 +716,13 @@ cudaError_t prepare_wide_kernels() {
 int wide_threads(int max_n) { return max_n <= 2048 ? 128 : 1024; }
 int wide_out_blocks(int N0) { return N0 <= 2048 ? 2048 / N0 : 1; }
 
-cudaError_t launch_wide_fft(bool inverse, int nt, int grid, const int2* map, const WArgs& a, cudaStream_t st) {
+cudaError_t launch_wide_fft(bool inverse, int nt, int grid, const int2* map, const WArgs& a, cudaStream_t st, bool dep) {
     if (grid <= 0) return cudaSuccess;
     const size_t sm = fft_smem_of(nt);
+    if (nt == 128 && !dep && !inverse) {
+        wide_fft_kernel<128><<<grid, nt, sm, st>>>(map, a);
+        return cudaGetLastError();
+    }
     if (nt == 128)
         return inverse ? launch_dep(wide_ifft_kernel<128>, grid, nt, sm, st, map, a)
                        : launch_dep(wide_fft_kernel<128>, grid, nt, sm, st, map, a);

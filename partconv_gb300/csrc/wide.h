@@ -56,7 +56,9 @@ cudaError_t prepare_wide_kernels();
 // 16 threads / N transforms), and blocks per CTA of wide_out
 int wide_threads(int max_n);
 int wide_out_blocks(int N0);
-cudaError_t launch_wide_fft(bool inverse, int nt, int grid, const int2* map, const WArgs& a, cudaStream_t st);
+// (dep = false: tables that the kernel reads are still being written by the stream's last kernel)
+cudaError_t launch_wide_fft(bool inverse, int nt, int grid, const int2* map, const WArgs& a, cudaStream_t st,
+                            bool dep = true);
 // level 0: inverse transforms and the call's output
 cudaError_t launch_wide_out(int N0, int grid, const int2* map, const WArgs& a, cudaStream_t st);
 // any: tile shapes other than the default, or level 0 with several base blocks per step
