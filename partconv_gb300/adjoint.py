@@ -95,7 +95,7 @@ class PartitionedConvFunction(torch.autograd.Function):
         stream = torch.cuda.current_stream(gy.device).cuda_stream
         ws = ctx.ws if ctx.ws is not None else plan.new_workspace(gy.device)
         gx = torch.empty_like(x) if ctx.needs_input_grad[0] else None
-        gh = torch.zeros_like(h) if ctx.needs_input_grad[1] else None
+        gh = torch.empty_like(h) if ctx.needs_input_grad[1] else None
         plan.backward(x, h, gy, gx, gh, ws, ctx.ws is None, stream)
         ctx.ws = None
         return gx, gh, None, None

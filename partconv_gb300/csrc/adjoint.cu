@@ -1,29 +1,35 @@
 // adjoint.cu -- differentiable partitioned convolution: block-parallel FDL
 // forward pass and hand-written adjoint kernels.
 //
-// For a batch of signals x_s (length T) and one IR h, y_s = (x_s * h)[0:T]
-// with the IR cut into the levels of a partition layout (level L: N_L-sample
-// blocks, P_L parts, taps [s_L, s_L + N_L P_L)).  The whole signal is known,
-// so every block of a level is computed in parallel (offline form of the
-// streaming FDL of PartConvFilter::runLevel, src/partconv.cpp:354-490):
-//   X_b  = rfft(x_L window [(b-1)N, (b+1)N)),  x_L[m] = x[m - s_L]
-//   Y_b  = sum_p X_{b-p} H_p,  H_p = rfft([0_N, h_p]) / 2N
-//   y_L block b = irfft(Y_b)[0:N]
+// For a batch of signals x_s (length T) and one IR h, y_s = (x_s * h)[0:T].
+// The whole signal is known, so nothing calls for the small blocks that a
+// layout's first levels keep for latency: the layout given at creation is
+// validated (src/partconv.cpp:87-181) and reported, and the computation takes
+// one level of N-sample blocks, N the smallest power of two that covers the IR
+// with at most 16 parts (256 .. 16384), with every block in parallel (the
+// offline form of the streaming FDL of PartConvFilter::runLevel,
+// src/partconv.cpp:354-490, run by wide.cu):
+//   X_b = rfft(x[(b-1)N, (b+1)N)),  Y_b = sum_p X_{b-p} H_p,
+//   H_p = rfft([0_N, h part p]) / 2N,  y block b = irfft(Y_b)[0:N]
 // Backward with g = dL/dy:
-//   dL/dx (adjoint, anti-causal, conjugated spectra):
-//     G'_c = rfft(g[cN + s_L, cN + s_L + 2N)),
-//     gx_L block b = irfft(sum_p (-1)^k conj(H_p) G'_{b+p})[0:N]
+//   dL/dx (adjoint, anti-causal): dL/dx[i] = sum_j h[j] g[i + j], the same
+//     convolution run backwards in time over g, written backwards;
 //   dL/dh (partitioned cross-correlation of the input with the gradient):
 //     GP_b = rfft([g block b, 0_N]),  D_p = sum_s sum_b conj(GP_b) X_{b-p},
-//     dh[s_L + pN + q] = irfft(D_p)[N - q] / 2N,  0 <= q < N.
-// Levels are summed in ascending order (PartConvFilter::output,
-// src/partconv.cpp:616-631).  The caller provides the workspace (no
-// allocation here); the input spectra X can be kept from the forward pass or
-// recomputed in the backward pass.
+//     dh[pN + q] = irfft(D_p)[N - q] / 2N,  0 <= q < N.
+// Sixteen parts: the products of T samples with an IR of L taps take
+// (L / N)(T / N) N multiply-adds, so they fall with N while a transform's work
+// per sample grows with log N only; below 16 parts the partial sums of D and the
+// zero padding of short signals outweigh what is left.  Eight signals of 2^18
+// samples, 2^16 taps, forward and backward: 463 us with the layout's own levels
+// (512 and 4096: 8 + 15 parts, a walk per level), 222 us so, of which 142 us on
+// the device and the rest in autograd's host path; three of 20011 samples,
+// 4999 taps: 310 to 236 us, bound by that host path.
+// The caller provides the workspace (no allocation here); the input spectra X
+// can be kept from the forward pass or recomputed in the backward pass.
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <array>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -32,327 +38,288 @@
 
 #include "../../include/partconv_gb300.h"
 #include "engine_types.h"
+#include "fft_reg.cuh"
 #include "fft_smem.cuh"
 #include "kernels.h"
+#include "wide.h"
 
 using namespace pcg;
 
 namespace {
 
-constexpr int kWlog = 15;
 constexpr int kMaxDLevels = 8;
-constexpr int kDhChunks = 16;   // partial sums of the dL/dh reduction (fixed order)
+constexpr int kMaxParts = 16;     // parts the block size is chosen for (and of one dL/dh pass)
+constexpr int kMinBlock = 256;
+constexpr int kRun = 16;          // blocks a thread of the dL/dh correlation sums
 
-// Job tables are built once per plan with addresses relative to the call's
-// buffers (DPtrs), so a call only launches kernels over tables already on
-// the device.
-enum { kSrcX = 0, kSrcH = 1, kSrcG = 2 };     // FJob sources: x, h, dL/dy
-enum { kDstY = 0, kDstGH = 1, kDstGX = 2 };   // IJob targets: y, dL/dh, dL/dx
-struct DPtrs {
-    const float* in[3];
-    float* out[3];
-    char* ws;   // workspace: spectra rows are byte offsets into it
-};
-// window FFT job: row at ws + dst_off = rfft(w) * scale, w[n] = src[start + n]
-// for n < 2N with src = in[src] + src_off, zero outside [0, len); half == 1
-// zeroes the second half ([g block, 0_N]), half == 2 the first ([0_N, h part])
-struct FJob {
-    long long src_off, len, start, dst_off;
+__host__ __device__ constexpr int job_threads(int logN) { return logN <= 11 ? 128 : 1 << (logN - 4); }
+
+// Transforms of windows with one zero half: rows of H (h part p in the second
+// half, scaled) or of GP (g block b in the first half).
+struct WinArgs {
+    const float* src;     // h, or dL/dy
+    float2* dst;          // rows of cs
+    const float2* tab;
+    long long len;        // samples per signal
+    int rows, per_sig;    // rows in all, per signal
+    int cs, second;       // live half of the window
     float scale;
-    int src, half, pad;
 };
-// inverse FFT job: o = irfft(row at ws + src_off), dst = out[dst] + dst_off;
-// mode 0: dst[i] = o[i], 1: dst[i] += o[i] (i < min(N, limit)); mode 2:
-// dst[q] = o[N - q] * scale (q < min(N, limit))
-struct IJob {
-    long long src_off, dst_off, limit;
-    float scale;
-    int dst, mode, pad;
-};
-
-// (the 512-thread, two-butterfly instances here and in difft_kernel are held
-// to 32 registers so that four CTAs fit an SM: the 512 windows of a
-// 4096-sample level over a batch of 8 then run in one wave instead of two)
-template <int NT, int MAXB>
-__global__ void __launch_bounds__(NT, NT * MAXB == 1024 ? 4 : 1) dfft_kernel(const FJob* __restrict__ jobs, DPtrs ptr, int N, int logN,
-                                                  const float2* W, int wlog) {
+template <int LOGN>
+__global__ void __launch_bounds__(job_threads(LOGN)) dwin_fft_kernel(WinArgs a) {
+    constexpr int NT = job_threads(LOGN);
+    using F = RegFft<LOGN, NT>;
+    constexpr int N = F::N, TPT = F::TPT;
     extern __shared__ float4 dyn_smem[];
-    float2* s = reinterpret_cast<float2*>(dyn_smem);
-    float2* twt = s + N;
-    const FJob jb = jobs[blockIdx.x];
-    const float* src = ptr.in[jb.src] + jb.src_off;
-    float2* dst = reinterpret_cast<float2*>(ptr.ws + jb.dst_off);
-    const int lo = jb.half == 2 ? N : 0, hi = jb.half == 1 ? N : 2 * N;   // live window samples [lo, hi)
-    for (int n = threadIdx.x; n < N; n += NT) {
-        const long long i = jb.start + 2LL * n;
-        float a = 0.f, b = 0.f;
-        if (2 * n >= lo && 2 * n < hi && i >= 0 && i < jb.len) a = src[i];
-        if (2 * n + 1 >= lo && 2 * n + 1 < hi && i + 1 >= 0 && i + 1 < jb.len) b = src[i + 1];
-        s[sidx<true>(n)] = make_float2(a, b);
-    }
-    load_twiddles_sw<NT>(twt, logN, W, wlog);
-    __syncthreads();
-    const Twiddles tw{twt, logN};
-    // transform buffer and twiddles in the conflict-free placement
-    fft_smem<NT, MAXB, true>(s, N, logN, tw, false);
-    for (int k = threadIdx.x; k <= N / 2; k += NT) {
-        const int nk = (k == 0) ? 0 : N - k;
-        float2 xk, xnk;
-        rfft_split<true>(s[sidx<true>(k)], s[sidx<true>(nk)], k, logN, tw, xk, xnk);
-        dst[k] = make_float2(xk.x * jb.scale, xk.y * jb.scale);
-        if (N - k != k) dst[N - k] = make_float2(xnk.x * jb.scale, xnk.y * jb.scale);
-    }
-}
-
-template <int NT, int MAXB>
-__global__ void __launch_bounds__(NT, NT * MAXB == 1024 ? 4 : 1) difft_kernel(const IJob* __restrict__ jobs, DPtrs ptr, int N, int logN,
-                                                   const float2* W, int wlog) {
-    extern __shared__ float4 dyn_smem[];
-    float2* s = reinterpret_cast<float2*>(dyn_smem);
-    float2* twt = s + N;
-    const IJob jb = jobs[blockIdx.x];
-    const float2* src = reinterpret_cast<const float2*>(ptr.ws + jb.src_off);
-    float* dst = ptr.out[jb.dst] + jb.dst_off;
-    load_twiddles_sw<NT>(twt, logN, W, wlog);
-    __syncthreads();
-    const Twiddles tw{twt, logN};
-    for (int k = threadIdx.x; k <= N / 2; k += NT) {
-        float2 zk, znk;
-        irfft_merge<true>(src[k], src[N - k], k, logN, tw, zk, znk);
-        s[sidx<true>(k)] = zk;
-        if (k != 0 && k != N / 2) s[sidx<true>(N - k)] = znk;
-    }
-    __syncthreads();
-    fft_smem<NT, MAXB, true>(s, N, logN, tw, true);
-    // real sample i is component i & 1 of complex element i >> 1
-    auto y = [&](int i) { return reinterpret_cast<const float*>(s + sidx<true>(i >> 1))[i & 1]; };
-    const int n = jb.limit < N ? (int)jb.limit : N;
-    for (int i = threadIdx.x; i < n; i += NT) {
-        if (jb.mode == 0) dst[i] = y(i);
-        else if (jb.mode == 1) dst[i] += y(i);
-        else dst[i] = y(N - i) * jb.scale;
-    }
-}
-
-// Y[s][b] = sum_p X[s][b-p] H[p]                       (forward, mode 0)
-// Y[s][b] = sum_p (-1)^k conj(H[p]) X[s][b+p]          (adjoint, mode 1)
-// X has nxb blocks per signal; Y has nyb.
-__global__ void dmac_kernel(const float2* __restrict__ X, const float2* __restrict__ H, float2* __restrict__ Y, int nsig,
-                            int nxb, int nyb, int P, int cs, int mode) {
-    const long long total = (long long)nsig * nyb * cs;
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
-         t += (long long)gridDim.x * blockDim.x) {
-        const int k = (int)(t % cs);
-        const long long sb = t / cs;
-        const int b = (int)(sb % nyb);
-        const int sg = (int)(sb / nyb);
-        float2 acc = make_float2(0.f, 0.f);
-        for (int p = 0; p < P; ++p) {
-            const int xb = mode == 0 ? b - p : b + p;
-            if (xb < 0 || xb >= nxb) continue;
-            const float2 x = X[((long long)sg * nxb + xb) * cs + k];
-            float2 h = H[(long long)p * cs + k];
-            if (mode == 1) h = (k & 1) ? make_float2(-h.x, h.y) : make_float2(h.x, -h.y);   // (-1)^k conj(h)
-            acc = cadd(acc, cmul(x, h));
-        }
-        Y[t] = acc;
-    }
-}
-
-// Dpart[chunk][p][k] = sum over (s, b) of chunk of conj(GP[s][b][k]) X[s][b-p][k]
-__global__ void ddh_partial_kernel(const float2* __restrict__ X, const float2* __restrict__ GP,
-                                   float2* __restrict__ Dpart, int nsig, int nb, int P, int cs, int nchunk) {
-    const long long total = (long long)nchunk * P * cs;
-    const long long nsb = (long long)nsig * nb;
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
-         t += (long long)gridDim.x * blockDim.x) {
-        const int k = (int)(t % cs);
-        const int p = (int)((t / cs) % P);
-        const int ch = (int)(t / ((long long)cs * P));
-        const long long j0 = ch * nsb / nchunk, j1 = (ch + 1) * nsb / nchunk;
-        float2 acc = make_float2(0.f, 0.f);
-        for (long long j = j0; j < j1; ++j) {
-            const int sg = (int)(j / nb), b = (int)(j % nb);
-            if (b - p < 0) continue;
-            const float2 g = GP[((long long)sg * nb + b) * cs + k];
-            const float2 x = X[((long long)sg * nb + (b - p)) * cs + k];
-            acc = cadd(acc, cmul(cconj(g), x));
-        }
-        Dpart[t] = acc;
-    }
-}
-
-// Sliding forms of the two FDL sums for P <= kSlideP: a thread owns one bin
-// of one signal over a run of kSlideRun consecutive blocks and keeps the last
-// P input spectra of that bin in registers, so each block's spectrum is
-// loaded once instead of once per part.  Same sums in the same part order as
-// dmac_kernel / ddh_partial_kernel.
-constexpr int kSlideP = 16;
-constexpr int kSlideRun = 32;
-
-// Y[s][b] = sum_p X[s][b-p] H[p] (mode 0); Y[s][b] = sum_p (-1)^k conj(H[p]) X[s][b+p] (mode 1)
-__global__ void dmac_slide_kernel(const float2* __restrict__ X, const float2* __restrict__ H, float2* __restrict__ Y,
-                                  int nsig, int nxb, int nyb, int P, int cs, int mode) {
-    const int nrun = (nyb + kSlideRun - 1) / kSlideRun;
-    const long long total = (long long)nsig * nrun * cs;
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
-         t += (long long)gridDim.x * blockDim.x) {
-        const int k = (int)(t % cs);
-        const long long sr = t / cs;
-        const int run = (int)(sr % nrun), sg = (int)(sr / nrun);
-        float2 h[kSlideP], w[kSlideP];   // filter bin per part; window of input spectra
+    const int t = threadIdx.x % TPT, tr = threadIdx.x / TPT;
+    float2* s = reinterpret_cast<float2*>(dyn_smem) + tr * F::SM;
+    const int row = blockIdx.x * (NT / TPT) + tr;
+    const bool live = row < a.rows;
+    if (TPT >= 32 && !live) return;
+    const int r = min(row, a.rows - 1), sig = r / a.per_sig, b = r - sig * a.per_sig;
+    const float* src = a.src + sig * a.len + (long long)b * N;
+    const long long left = a.len - (long long)b * N;   // live samples of the block
+    float2 v[16];
 #pragma unroll
-        for (int p = 0; p < kSlideP; ++p) {
-            h[p] = make_float2(0.f, 0.f);
-            w[p] = make_float2(0.f, 0.f);
-            if (p < P) {
-                float2 v = H[(long long)p * cs + k];
-                if (mode == 1) v = (k & 1) ? make_float2(-v.x, v.y) : make_float2(v.x, -v.y);   // (-1)^k conj
-                h[p] = v;
+    for (int m = 0; m < 16; ++m) v[m] = make_float2(0.f, 0.f);
+    // window pairs n < N / 2 are the first half, v[0 .. 7]
+    float2 u[8];
+#pragma unroll
+    for (int m = 0; m < 8; ++m) {
+        const int i = 2 * (t + m * TPT);
+        u[m] = make_float2(i < left ? src[i] : 0.0f, i + 1 < left ? src[i + 1] : 0.0f);
+    }
+#pragma unroll
+    for (int m = 0; m < 8; ++m) {
+        if (a.second) v[m + 8] = u[m];
+        else v[m] = u[m];
+    }
+    fft_reg<LOGN, NT, false, true>(v, t, s, a.tab);
+    F::sync();
+#pragma unroll
+    for (int m = 8; m < 16; ++m) s[rpad(t + m * TPT)] = v[m];
+    F::sync();
+    if (!live) return;
+    float2* d = a.dst + (size_t)r * a.cs;
+    const float2* sp = a.tab + ft_sp(LOGN);
+    auto put = [&](int k, float2 x) { d[k] = make_float2(x.x * a.scale, x.y * a.scale); };
+#pragma unroll
+    for (int m = 0; m < 8; ++m) {
+        const int k = t + m * TPT;
+        float2 xk, xnk;
+        if (m == 0 && t == 0) split_zero(v[0], xk, xnk);
+        else split_w(v[m], s[rpad(N - k)], __ldg(sp + k), xk, xnk);
+        put(k, xk);
+        put(N - k, xnk);
+    }
+    if (t == 0) {
+        float2 xk, xnk;
+        split_w(v[8], v[8], __ldg(sp + N / 2), xk, xnk);
+        put(N / 2, xk);
+    }
+}
+
+// dh[p N + q] = irfft(D_p)[N - q] / 2N, q < N, p N + q < len
+template <int LOGN>
+__global__ void __launch_bounds__(job_threads(LOGN)) dtap_ifft_kernel(const float2* __restrict__ D, int P, int cs,
+                                                                      const float2* __restrict__ tab, float* gh, int len) {
+    constexpr int NT = job_threads(LOGN);
+    using F = RegFft<LOGN, NT>;
+    constexpr int N = F::N, TPT = F::TPT;
+    extern __shared__ float4 dyn_smem[];
+    const int t = threadIdx.x % TPT, tr = threadIdx.x / TPT;
+    float2* s = reinterpret_cast<float2*>(dyn_smem) + tr * F::SM;
+    const int row = blockIdx.x * (NT / TPT) + tr;
+    const bool live = row < P;
+    if (TPT >= 32 && !live) return;
+    const int p = min(row, P - 1);
+    const float2* Y = D + (size_t)p * cs;
+    const float2* sp = tab + ft_sp(LOGN);
+    float2 v[16];
+#pragma unroll
+    for (int m = 0; m < 16; ++m) {
+        const int n = t + m * TPT;
+        float2 yn = __ldcg(Y + n), yc = __ldcg(Y + N - n), other;
+        if (m < 8) {
+            if (m == 0 && t == 0) yn.y = yc.y = 0.0f;
+            merge_w(yn, yc, __ldg(sp + n), v[m], other);
+        } else {
+            merge_w(yc, yn, __ldg(sp + N - n), other, v[m]);
+        }
+    }
+    fft_reg<LOGN, NT, true, true>(v, t, s, tab);
+    if (!live) return;
+    // real samples 2 n, 2 n + 1 in v[m], n = t + m TPT; taps q = N - i, 0 < i <= N
+    const float scale = 1.0f / (2.0f * N);
+    float* d = gh + (size_t)p * N;
+    const int live_taps = min(N, len - p * N);
+    auto put = [&](int i, float y) {
+        const int q = N - i;
+        if (q >= 0 && q < live_taps) d[q] = y * scale;
+    };
+#pragma unroll
+    for (int m = 0; m < 9; ++m) {
+        const int i = 2 * (t + m * TPT);
+        if (i <= N) {
+            put(i, v[m].x);
+            put(i + 1, v[m].y);
+        }
+    }
+}
+
+// Dpart[sig * nrun + run][p][k] = sum over the run's blocks b of
+// conj(GP[sig][b][k]) X[sig][b-p][k], parts p0 <= p < p0 + 16 (blockIdx.y), the
+// bin's last 16 input spectra in registers: each spectrum is loaded once per
+// pass instead of once per part, four blocks' loads in flight.  The products
+// are rounded before they are added (one rounding of the sum each).
+// Bound: latency of two rows per block (63 of 8 x 64 blocks x 4098 bins x 16
+// parts are 34 M products, 15 us of packed arithmetic; measured 26 us).
+__global__ void __launch_bounds__(128) ddh_slide_kernel(const float2* __restrict__ X, const float2* __restrict__ GP,
+                                                        float2* __restrict__ Dpart, int nsig, int nb, int slots, int P,
+                                                        int cs) {
+    constexpr int U = 4;
+    const int nrun = (nb + kRun - 1) / kRun;
+    const long long t = blockIdx.x * 128LL + threadIdx.x;
+    if (t >= (long long)nsig * nrun * cs) return;
+    const int k = (int)(t % cs);
+    const int sr = (int)(t / cs), run = sr % nrun, sg = sr / nrun;
+    const int p0 = blockIdx.y * kMaxParts;
+    const f32x2* Xs = reinterpret_cast<const f32x2*>(X + (size_t)sg * slots * cs + k);
+    const float2* Gs = GP + (size_t)sg * nb * cs + k;
+    const int b0 = run * kRun, b1 = min(nb, b0 + kRun);
+    auto xat = [&](int b) { return b >= 0 ? __ldcg(Xs + (size_t)b * cs) : 0ULL; };
+    // w[(p + i) mod 16 from the newest]: block b - p0 - p at step i of the unrolled sixteen
+    f32x2 w[kMaxParts], acc[kMaxParts];
+#pragma unroll
+    for (int p = 0; p < kMaxParts; ++p) {
+        acc[p] = 0;
+        w[(kMaxParts - 1 - p)] = p < kMaxParts - 1 ? xat(b0 - 1 - p0 - p) : 0;   // slot (15 - p): the block p before b0 - 1
+    }
+    // at step i the newest block goes to slot i, the block p older to slot (i - p) mod 16
+    for (int bb = b0; bb < b1; bb += kMaxParts) {
+#pragma unroll
+        for (int i0 = 0; i0 < kMaxParts; i0 += U) {
+            if (bb + i0 >= b1) break;
+            f32x2 xn[U];
+            float2 g[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int b = bb + i0 + u;
+                if (b < b1) {
+                    xn[u] = xat(b - p0);
+                    g[u] = __ldcg(Gs + (size_t)b * cs);
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                if (bb + i0 + u >= b1) break;
+                const int i = i0 + u;
+                w[i] = xn[u];
+                // conj(g) x = (g.re x.re + g.im x.im, g.re x.im - g.im x.re)
+                const f32x2 gr = pack2(g[u].x, g[u].x), gi = pack2(g[u].y, -g[u].y);
+#pragma unroll
+                for (int p = 0; p < kMaxParts; ++p)
+                    if (p0 + p < P) {
+                        const f32x2 x = w[(i - p + kMaxParts) % kMaxParts];
+                        acc[p] = add2(acc[p], fma2(x, gr, mul2(swap2(x), gi)));
+                    }
             }
         }
-        const float2* Xs = X + (long long)sg * nxb * cs + k;
-        float2* Ys = Y + (long long)sg * nyb * cs + k;
-        const int b0 = run * kSlideRun, b1 = min(nyb, b0 + kSlideRun);
-        auto xat = [&](int xb) { return (xb >= 0 && xb < nxb) ? Xs[(long long)xb * cs] : make_float2(0.f, 0.f); };
-        // mode 0 walks b upwards with w[p] = X[b - p]; mode 1 walks it
-        // downwards with w[p] = X[b + p].  Each step shifts the window by one
-        // and loads the newest block into w[0].
-        const int dir = mode == 0 ? 1 : -1;
-        const int start = mode == 0 ? b0 : b1 - 1;
-#pragma unroll
-        for (int p = 0; p < kSlideP - 1; ++p)   // the window one step before `start`
-            if (p < P - 1) w[p] = xat(start - dir * (p + 1));
-        for (int i = 0, b = start; i < b1 - b0; ++i, b += dir) {
-#pragma unroll
-            for (int p = kSlideP - 1; p > 0; --p) w[p] = w[p - 1];
-            w[0] = xat(b);
-            float2 acc = make_float2(0.f, 0.f);
-#pragma unroll
-            for (int p = 0; p < kSlideP; ++p)
-                if (p < P) acc = cadd(acc, cmul(w[p], h[p]));
-            Ys[(long long)b * cs] = acc;
-        }
     }
+    float2* D = Dpart + ((size_t)sr * P + p0) * cs + k;
+#pragma unroll
+    for (int p = 0; p < kMaxParts; ++p)
+        if (p0 + p < P) D[(size_t)p * cs] = unpack2(acc[p]);
 }
 
-// Dpart[s * nrun + run][p][k] = sum over blocks b of the run of
-// conj(GP[s][b][k]) X[s][b-p][k], p < P <= kSlideP (the dL/dh correlation),
-// with the last P input spectra of the bin kept in registers.
-__global__ void ddh_slide_kernel(const float2* __restrict__ X, const float2* __restrict__ GP,
-                                 float2* __restrict__ Dpart, int nsig, int nb, int P, int cs) {
-    const int nrun = (nb + kSlideRun - 1) / kSlideRun;
-    const long long total = (long long)nsig * nrun * cs;
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
-         t += (long long)gridDim.x * blockDim.x) {
-        const int k = (int)(t % cs);
-        const long long sr = t / cs;
-        const int run = (int)(sr % nrun), sg = (int)(sr / nrun);
-        const float2* Xs = X + (long long)sg * nb * cs + k;
-        const float2* Gs = GP + (long long)sg * nb * cs + k;
-        const int b0 = run * kSlideRun, b1 = min(nb, b0 + kSlideRun);
-        float2 w[kSlideP], acc[kSlideP];
+// D[p][k] = sum of the nchunk partial rows, in order, eight loads in flight
+__global__ void ddh_reduce_kernel(const float2* __restrict__ Dpart, float2* __restrict__ D, int total, int nchunk) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= total) return;
+    constexpr int U = 8;
+    float2 acc = make_float2(0.f, 0.f);
+    for (int c0 = 0; c0 < nchunk; c0 += U) {
+        float2 v[U];
 #pragma unroll
-        for (int p = 0; p < kSlideP; ++p) {
-            acc[p] = make_float2(0.f, 0.f);
-            const int xb = b0 - 1 - p;   // the window one block before b0
-            w[p] = (p < P - 1 && xb >= 0) ? Xs[(long long)xb * cs] : make_float2(0.f, 0.f);
-        }
-        for (int b = b0; b < b1; ++b) {
+        for (int u = 0; u < U; ++u)
+            if (c0 + u < nchunk) v[u] = __ldcg(Dpart + (size_t)(c0 + u) * total + t);
 #pragma unroll
-            for (int p = kSlideP - 1; p > 0; --p) w[p] = w[p - 1];
-            w[0] = Xs[(long long)b * cs];
-            const float2 g = cconj(Gs[(long long)b * cs]);
-#pragma unroll
-            for (int p = 0; p < kSlideP; ++p)
-                if (p < P) acc[p] = cadd(acc[p], cmul(g, w[p]));
-        }
-        float2* D = Dpart + (sr * P) * cs + k;
-#pragma unroll
-        for (int p = 0; p < kSlideP; ++p)
-            if (p < P) D[(long long)p * cs] = acc[p];
+        for (int u = 0; u < U; ++u)
+            if (c0 + u < nchunk) acc = cadd(acc, v[u]);
     }
+    D[t] = acc;
 }
 
-__global__ void ddh_reduce_kernel(const float2* __restrict__ Dpart, float2* __restrict__ D, int P, int cs, int nchunk) {
-    const int total = P * cs;
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
-        float2 acc = make_float2(0.f, 0.f);
-        for (int c = 0; c < nchunk; ++c) acc = cadd(acc, Dpart[(long long)c * total + t]);
-        D[t] = acc;
+// f.template operator()<LOGN>() for block sizes 256 .. 16384
+template <class Fn>
+cudaError_t by_block(int N, Fn&& f) {
+    switch (N) {
+        case 256: return f.template operator()<8>();
+        case 512: return f.template operator()<9>();
+        case 1024: return f.template operator()<10>();
+        case 2048: return f.template operator()<11>();
+        case 4096: return f.template operator()<12>();
+        case 8192: return f.template operator()<13>();
+        case 16384: return f.template operator()<14>();
+        default: return cudaErrorInvalidValue;
     }
 }
+constexpr size_t job_smem(int nt) { return sizeof(float2) * 17 * (size_t)nt; }
 
-int cls_of(int N) { return N <= 1024 ? 0 : (N <= 4096 ? 1 : 2); }
-
-// the FDL sum over parts, sliding for P <= kSlideP
-int launch_mac(const float2* X, const float2* H, float2* Y, int nsig, int nxb, int nyb, int P, int cs, int mode,
-               cudaStream_t st) {
-    if (P <= kSlideP) {
-        const long long total = (long long)nsig * ((nyb + kSlideRun - 1) / kSlideRun) * cs;
-        dmac_slide_kernel<<<(int)std::min<long long>((total + 255) / 256, 152 * 16), 256, 0, st>>>(X, H, Y, nsig, nxb,
-                                                                                                    nyb, P, cs, mode);
-    } else {
-        const long long total = (long long)nsig * nyb * cs;
-        dmac_kernel<<<(int)std::min<long long>((total + 255) / 256, 152 * 16), 256, 0, st>>>(X, H, Y, nsig, nxb, nyb,
-                                                                                              P, cs, mode);
+struct WinFft {
+    const WinArgs& a;
+    cudaStream_t st;
+    template <int L>
+    cudaError_t operator()() const {
+        constexpr int NT = job_threads(L), per = NT * 16 >> L;
+        dwin_fft_kernel<L><<<(a.rows + per - 1) / per, NT, job_smem(NT), st>>>(a);
+        return cudaGetLastError();
     }
-    return 0;
-}
-
-cudaError_t launch_fft(int N, int logN, const FJob* jobs, int njobs, const DPtrs& ptr, const float2* W,
-                       cudaStream_t st) {
-    if (njobs <= 0) return cudaSuccess;
-    const size_t smem = (size_t)12 * N;
-    switch (cls_of(N)) {
-        case 0:   // one radix-4 butterfly per thread and stage: N / 4 threads
-            if (N <= 512) dfft_kernel<128, 1><<<njobs, 128, smem, st>>>(jobs, ptr, N, logN, W, kWlog);
-            else dfft_kernel<256, 1><<<njobs, 256, smem, st>>>(jobs, ptr, N, logN, W, kWlog);
-            break;
-        case 1: dfft_kernel<512, 2><<<njobs, 512, smem, st>>>(jobs, ptr, N, logN, W, kWlog); break;
-        default: dfft_kernel<512, 8><<<njobs, 512, smem, st>>>(jobs, ptr, N, logN, W, kWlog); break;
+};
+struct TapIfft {
+    const float2* D;
+    int P, cs;
+    const float2* tab;
+    float* gh;
+    int len;
+    cudaStream_t st;
+    template <int L>
+    cudaError_t operator()() const {
+        constexpr int NT = job_threads(L), per = NT * 16 >> L;
+        dtap_ifft_kernel<L><<<(P + per - 1) / per, NT, job_smem(NT), st>>>(D, P, cs, tab, gh, len);
+        return cudaGetLastError();
     }
-    return cudaGetLastError();
-}
-
-cudaError_t launch_ifft(int N, int logN, const IJob* jobs, int njobs, const DPtrs& ptr, const float2* W,
-                        cudaStream_t st) {
-    if (njobs <= 0) return cudaSuccess;
-    const size_t smem = (size_t)12 * N;
-    switch (cls_of(N)) {
-        case 0:
-            if (N <= 512) difft_kernel<128, 1><<<njobs, 128, smem, st>>>(jobs, ptr, N, logN, W, kWlog);
-            else difft_kernel<256, 1><<<njobs, 256, smem, st>>>(jobs, ptr, N, logN, W, kWlog);
-            break;
-        case 1: difft_kernel<512, 2><<<njobs, 512, smem, st>>>(jobs, ptr, N, logN, W, kWlog); break;
-        default: difft_kernel<512, 8><<<njobs, 512, smem, st>>>(jobs, ptr, N, logN, W, kWlog); break;
+};
+struct Prepare {
+    template <int L>
+    cudaError_t operator()() const {
+        const int b = (int)job_smem(job_threads(L));
+        cudaError_t e = cudaFuncSetAttribute(dwin_fft_kernel<L>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(dtap_ifft_kernel<L>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
+        return e;
     }
-    return cudaGetLastError();
-}
+};
 
 }  // namespace
 
 struct pcd_plan {
-    int M = 0, B = 0, ir_len = 0;
+    int B = 0, ir_len = 0;
     long long T = 0;
-    std::vector<int> N, P, logN, cs, nb, nbg;
-    std::vector<long long> s;
+    int N = 0, logN = 0, P = 0, cs = 0, nb = 0, slots = 0, nrun = 0;   // P: parts that reach the output
     // workspace offsets (bytes)
-    size_t o_W = 0, total = 0;
-    std::vector<size_t> o_H, o_X, o_Y, o_Dp, o_D;
-    // job tables (device, built at creation): per level and kind, byte offset
-    // into d_tab and job count
-    struct Tab {
-        size_t off = 0;
-        int n = 0;
-    };
-    enum Kind { kFH, kFX, kIY, kFGP, kIGH, kFGX, kIGX, kKinds };
-    std::vector<std::array<Tab, kKinds>> tab;
+    size_t o_H = 0, o_X = 0, o_Y = 0, o_Dp = 0, o_D = 0, total = 0;
+    // device tables (built at creation): transform factors, level descriptors of
+    // the signals (pointers relative to the workspace), CTA maps
     char* d_tab = nullptr;
+    const float2* tab = nullptr;
+    const WLevel* lv = nullptr;
+    const int2 *m_fft = nullptr, *m_out = nullptr;
+    const int4* m_mac = nullptr;
+    int n_fft = 0, n_out = 0, n_mac = 0, nt = 0;
     int device = -1;
     std::string err;
     long long launches = 0;
-    bool attrs_set = false;   // large-FFT shared memory attributes applied
     ~pcd_plan() {
         if (d_tab) {
             int cur = -1;
@@ -383,117 +350,115 @@ int dfail(pcd_plan* p, int code, const std::string& m) {
         if (e_ != cudaSuccess) return dfail(p, PC_ERR_CUDA, std::string(where) + ": " + cudaGetErrorString(e_)); \
     } while (0)
 
-struct WS {
-    char* base;
-    template <class T>
-    T* at(size_t off) const {
-        return reinterpret_cast<T*>(base + off);
-    }
-};
+template <class T>
+T* at(void* ws, size_t off) {
+    return reinterpret_cast<T*>(static_cast<char*>(ws) + off);
+}
 
-// launch the table of one kind for level L over the call's buffers
-int run_tab(pcd_plan* p, int L, int kind, const DPtrs& ptr, cudaStream_t st) {
-    const pcd_plan::Tab& t = p->tab[L][kind];
-    if (t.n <= 0) return PC_OK;
-    const float2* W = reinterpret_cast<const float2*>(ptr.ws + p->o_W);
-    const bool fwd = kind == pcd_plan::kFH || kind == pcd_plan::kFX || kind == pcd_plan::kFGP || kind == pcd_plan::kFGX;
-    if (fwd)
-        DCK(launch_fft(p->N[L], p->logN[L], reinterpret_cast<const FJob*>(p->d_tab + t.off), t.n, ptr, W, st),
-            "window FFT");
-    else
-        DCK(launch_ifft(p->N[L], p->logN[L], reinterpret_cast<const IJob*>(p->d_tab + t.off), t.n, ptr, W, st),
-            "inverse FFT");
+// in -> in * h over every signal, or with rev both read and written backwards
+// in time; spectra of `in` stay in the workspace's X rows
+int convolve(pcd_plan* p, const float* in, float* out, void* ws, bool rev, bool windows, cudaStream_t st) {
+    WArgs a{};
+    a.lv = p->lv;
+    a.tab = p->tab;
+    a.N0 = p->N;
+    a.kb = 1;
+    a.full = 1;
+    a.nsteps = p->nb;
+    a.rel = (long long)reinterpret_cast<unsigned long long>(ws);
+    a.len = p->T;
+    const long long last = rev ? p->T - 1 : 0;
+    a.io.in = in + last;
+    a.io.out = out + last;
+    a.io.in_sample = a.io.out_sample = rev ? -1 : 1;
+    a.io.in_ch = a.io.out_ch = p->T;
+    a.vec_in = !rev && (p->B == 1 || p->T % 2 == 0) && (reinterpret_cast<uintptr_t>(in) & 7) == 0;
+    a.vec_out = !rev && (p->B == 1 || p->T % 2 == 0) && (reinterpret_cast<uintptr_t>(out) & 7) == 0;
+    if (windows) {
+        DCK(launch_wide_fft(false, p->nt, p->n_fft, p->m_fft, a, st), "window FFT");
+        p->launches++;
+    }
+    if (out) {
+        DCK(launch_wide_mac(false, p->n_mac, p->m_mac, a, st), "sum over parts");
+        DCK(launch_wide_out(p->N, p->n_out, p->m_out, a, st), "inverse FFT");
+        p->launches += 2;
+    }
+    return PC_OK;
+}
+
+int filter_spectra(pcd_plan* p, const float* h, void* ws, cudaStream_t st) {
+    WinArgs a{h, at<float2>(ws, p->o_H), p->tab, p->ir_len, p->P, p->P, p->cs, 1, 1.0f / (2.0f * p->N)};
+    DCK(by_block(p->N, WinFft{a, st}), "filter spectra");
     p->launches++;
     return PC_OK;
 }
 
-int filter_spectra(pcd_plan* p, const DPtrs& ptr, cudaStream_t st) {
-    for (int L = 0; L < p->M; ++L) {
-        int r = run_tab(p, L, pcd_plan::kFH, ptr, st);
-        if (r) return r;
-    }
-    return PC_OK;
-}
-
-int input_spectra(pcd_plan* p, const DPtrs& ptr, cudaStream_t st) {
-    for (int L = 0; L < p->M; ++L) {
-        int r = run_tab(p, L, pcd_plan::kFX, ptr, st);
-        if (r) return r;
-    }
-    return PC_OK;
-}
-
-// every job table of the plan, relative to the call's buffers (see DPtrs)
+// level descriptors, maps and transform factors on the device
 int build_tables(pcd_plan* p) {
-    std::vector<char> host;
-    auto add = [&](auto&& jobs) -> pcd_plan::Tab {
-        pcd_plan::Tab t;
-        t.off = host.size();
-        t.n = (int)jobs.size();
-        const size_t bytes = sizeof(jobs[0]) * jobs.size();
-        host.resize(host.size() + ((bytes + 255) & ~(size_t)255));
-        if (bytes) std::memcpy(host.data() + t.off, jobs.data(), bytes);
-        return t;
+    std::vector<char> blob;
+    auto put = [&](const void* src, size_t bytes) {
+        const size_t o = blob.size();
+        blob.resize(o + ((bytes + 255) & ~(size_t)255));
+        if (bytes) std::memcpy(blob.data() + o, src, bytes);
+        return o;
     };
-    const long long T = p->T;
-    p->tab.assign(p->M, {});
-    for (int L = 0; L < p->M; ++L) {
-        const int N = p->N[L], P = p->P[L], nb = p->nb[L], nbg = p->nbg[L];
-        const long long row = (long long)sizeof(float2) * p->cs[L];
-        const long long sL = p->s[L];
-        auto& tb = p->tab[L];
-        std::vector<FJob> f;
-        std::vector<IJob> v;
-        for (int q = 0; q < P; ++q)   // H_q = rfft([0_N, h part q]) / 2N: the window starts N before the part
-            f.push_back(FJob{0, p->ir_len, sL + (long long)q * N - N, (long long)p->o_H[L] + q * row,
-                             1.0f / (2.0f * N), kSrcH, 2, 0});
-        tb[pcd_plan::kFH] = add(f);
-        f.clear();
-        for (int sg = 0; sg < p->B; ++sg)   // X_b = rfft(x[(b-1)N - s_L, (b+1)N - s_L))
-            for (int b = 0; b < nb; ++b)
-                f.push_back(FJob{sg * T, T, (long long)(b - 1) * N - sL,
-                                 (long long)p->o_X[L] + ((long long)sg * nb + b) * row, 1.0f, kSrcX, 0, 0});
-        tb[pcd_plan::kFX] = add(f);
-        f.clear();
-        for (int sg = 0; sg < p->B; ++sg)   // y block b (level 0 stores, larger levels add)
-            for (int b = 0; b < nb; ++b) {
-                const long long t0 = (long long)b * N;
-                v.push_back(IJob{(long long)p->o_Y[L] + ((long long)sg * nb + b) * row, sg * T + t0, T - t0, 1.0f,
-                                 kDstY, L == 0 ? 0 : 1, 0});
-            }
-        tb[pcd_plan::kIY] = add(v);
-        v.clear();
-        for (int sg = 0; sg < p->B; ++sg)   // GP_b = rfft([g block b, 0_N])
-            for (int b = 0; b < nb; ++b)
-                f.push_back(FJob{sg * T, T, (long long)b * N, (long long)p->o_Y[L] + ((long long)sg * nb + b) * row,
-                                 1.0f, kSrcG, 1, 0});
-        tb[pcd_plan::kFGP] = add(f);
-        f.clear();
-        for (int q = 0; q < P; ++q) {   // dh[s_L + qN + t] = irfft(D_q)[N - t] / 2N
-            const long long t0 = sL + (long long)q * N;
-            if (t0 >= p->ir_len) break;
-            v.push_back(IJob{(long long)p->o_D[L] + q * row, t0, p->ir_len - t0, 1.0f / (2.0f * N), kDstGH, 2, 0});
-        }
-        tb[pcd_plan::kIGH] = add(v);
-        v.clear();
-        for (int sg = 0; sg < p->B; ++sg)   // G'_c = rfft(g[cN + s_L, cN + s_L + 2N)), c < nb + P - 1
-            for (int c = 0; c < nbg; ++c)
-                f.push_back(FJob{sg * T, T, (long long)c * N + sL,
-                                 (long long)p->o_Y[L] + ((long long)sg * nbg + c) * row, 1.0f, kSrcG, 0, 0});
-        tb[pcd_plan::kFGX] = add(f);
-        f.clear();
-        for (int sg = 0; sg < p->B; ++sg)   // dx block b from the adjoint sums (kept in the X rows)
-            for (int b = 0; b < nb; ++b) {
-                const long long t0 = (long long)b * N;
-                v.push_back(IJob{(long long)p->o_X[L] + ((long long)sg * nb + b) * row, sg * T + t0, T - t0, 1.0f,
-                                 kDstGX, L == 0 ? 0 : 1, 0});
-            }
-        tb[pcd_plan::kIGX] = add(v);
-        v.clear();
+    std::vector<WLevel> lv;
+    std::vector<int2> fft, out;
+    std::vector<int4> mac;
+    auto rel = [](size_t off) { return reinterpret_cast<float2*>(off); };   // completed by WArgs::rel
+    const size_t row = sizeof(float2) * (size_t)p->cs;
+    p->nt = p->N <= 2048 ? 128 : (p->N <= 4096 ? 256 : 1024);
+    for (int s = 0; s < p->B; ++s) {
+        WLevel w{};
+        w.N = p->N;
+        w.logN = p->logN;
+        w.P = p->P;
+        w.cs = p->cs;
+        w.slots = p->slots;
+        w.p_lo = 2;
+        w.tp = 16;
+        w.tpg = 4;
+        w.nrows = p->P > 2 ? (p->P - 2 + 15) / 16 : 0;
+        w.two = 1;
+        w.in_ch = w.out_ch = s;
+        w.mix_mode = 1;
+        w.M = 1;
+        w.lv0 = s;
+        w.scale = 1.0f;
+        w.H = rel(p->o_H);
+        w.X = rel(p->o_X + row * p->slots * s);
+        w.Yw = rel(p->o_Y + row * p->nb * s);
+        lv.push_back(w);
     }
+    // a segment of few enough blocks that there are CTAs for every SM
+    int seg = kMacSeg;
+    const long long tiles = (p->cs + kMacTile - 1) / kMacTile;
+    while (seg > kWideRun && tiles * p->B * ((p->nb + seg - 1) / seg) < 4 * 152) seg >>= 1;
+    for (int s = 0; s < p->B; ++s) {
+        for (int b = 0; b < p->nb; b += 16 * p->nt / p->N) fft.push_back(make_int2(s, b));
+        for (int b = 0; b < p->nb; b += wide_out_blocks(p->N)) out.push_back(make_int2(s, b));
+        for (int b = 0; b < p->nb; b += seg)
+            for (int k = 0; k < p->cs; k += kMacTile) mac.push_back(make_int4(s, k, b, std::min(p->nb, b + seg)));
+    }
+    p->n_fft = (int)fft.size();
+    p->n_out = (int)out.size();
+    p->n_mac = (int)mac.size();
+    const auto& t = host_fft_tables();
+    const size_t o_t = put(t.data(), sizeof(float2) * t.size());
+    const size_t o_lv = put(lv.data(), sizeof(WLevel) * lv.size());
+    const size_t o_f = put(fft.data(), sizeof(int2) * fft.size());
+    const size_t o_o = put(out.data(), sizeof(int2) * out.size());
+    const size_t o_m = put(mac.data(), sizeof(int4) * mac.size());
     DCK(cudaGetDevice(&p->device), "cudaGetDevice");
-    DCK(cudaMalloc(&p->d_tab, std::max<size_t>(host.size(), 256)), "job table allocation");
-    DCK(cudaMemcpy(p->d_tab, host.data(), host.size(), cudaMemcpyHostToDevice), "job table upload");
+    DCK(cudaMalloc(&p->d_tab, blob.size()), "table allocation");
+    DCK(cudaMemcpy(p->d_tab, blob.data(), blob.size(), cudaMemcpyHostToDevice), "table upload");
+    p->tab = reinterpret_cast<const float2*>(p->d_tab + o_t);
+    p->lv = reinterpret_cast<const WLevel*>(p->d_tab + o_lv);
+    p->m_fft = reinterpret_cast<const int2*>(p->d_tab + o_f);
+    p->m_out = reinterpret_cast<const int2*>(p->d_tab + o_o);
+    p->m_mac = reinterpret_cast<const int4*>(p->d_tab + o_m);
+    DCK(prepare_wide_kernels(), "kernel attributes");
+    if (p->N > 2048) DCK(by_block(p->N, Prepare{}), "kernel attributes");
     return PC_OK;
 }
 
@@ -526,36 +491,28 @@ pcd_plan* pcd_create(int M, const int* N, int* P, int ir_len, int batch, long lo
     for (int i = 0; i < M; ++i) P[i] = Pv[i];
     pcd_plan* p = new (std::nothrow) pcd_plan();
     if (!p) return nullptr;
-    p->M = M;
     p->B = batch;
     p->ir_len = ir_len;
     p->T = length;
-    p->N = Nv;
-    p->P = Pv;
-    long long s = 0;
+    // the smallest block with at most kMaxParts parts, no larger than the signal needs
+    p->N = kMinBlock;
+    while (p->N < kMaxBlockOneCta && p->N < length && (long long)p->N * kMaxParts < ir_len) p->N <<= 1;
+    while ((1 << p->logN) < p->N) ++p->logN;
+    p->cs = p->N + 2;
+    p->nb = (int)((length + p->N - 1) / p->N);
+    p->P = std::min((ir_len + p->N - 1) / p->N, p->nb);   // later parts reach no output sample
+    p->slots = p->P + std::max(p->nb, kWideRun);
+    p->nrun = (p->nb + kRun - 1) / kRun;
+    const size_t row = sizeof(float2) * (size_t)p->cs;
     size_t off = 0;
-    p->o_W = take(off, sizeof(float2) << kWlog);
-    for (int L = 0; L < M; ++L) {
-        p->s.push_back(s);
-        p->logN.push_back((int)std::lround(std::log2((double)Nv[L])));
-        p->cs.push_back(Nv[L] + 2);
-        const int nb = (int)((length + Nv[L] - 1) / Nv[L]);
-        p->nb.push_back(nb);
-        p->nbg.push_back(nb + Pv[L] - 1);   // adjoint windows reach P-1 blocks past the end
-        s += (long long)Nv[L] * Pv[L];
-    }
-    for (int L = 0; L < M; ++L) {
-        const size_t cs = p->cs[L];
-        p->o_H.push_back(take(off, sizeof(float2) * Pv[L] * cs));
-        p->o_X.push_back(take(off, sizeof(float2) * (size_t)batch * p->nb[L] * cs));
-        p->o_Y.push_back(take(off, sizeof(float2) * (size_t)batch * p->nbg[L] * cs));
-        const size_t nrun = (size_t)(p->nb[L] + kSlideRun - 1) / kSlideRun;
-        p->o_Dp.push_back(take(off, sizeof(float2) * std::max<size_t>(kDhChunks, (size_t)batch * nrun) * Pv[L] * cs));
-        p->o_D.push_back(take(off, sizeof(float2) * (size_t)Pv[L] * cs));
-    }
+    p->o_H = take(off, row * p->P);
+    p->o_X = take(off, row * p->slots * batch);
+    p->o_Y = take(off, row * p->nb * batch);
+    p->o_Dp = take(off, row * p->P * p->nrun * batch);
+    p->o_D = take(off, row * p->P);
     p->total = off;
-    if (build_tables(p) != PC_OK) {
-        put(p->err.c_str());
+    if ((long long)p->slots * p->cs >= (1LL << 31) || build_tables(p) != PC_OK) {
+        put(p->err.empty() ? "signal too long for one plan" : p->err.c_str());
         delete p;
         return nullptr;
     }
@@ -568,95 +525,40 @@ long long pcd_workspace_bytes(const pcd_plan* p) { return p ? (long long)p->tota
 int pcd_forward(pcd_plan* p, const float* d_x, const float* d_h, float* d_y, void* d_ws, void* stream) {
     if (!p || !d_x || !d_h || !d_y || !d_ws) return dfail(p, PC_ERR_ARG, "null pointer");
     cudaStream_t st = (cudaStream_t)stream;
-    WS w{static_cast<char*>(d_ws)};
-    const DPtrs ptr{{d_x, d_h, nullptr}, {d_y, nullptr, nullptr}, w.base};
-    {
-        static thread_local std::vector<float2> Wh;
-        if (Wh.empty()) {
-            Wh.resize((size_t)1 << kWlog);
-            for (size_t m = 0; m < Wh.size(); ++m) {
-                const double a = -2.0 * M_PI * (double)m / (double)Wh.size();
-                Wh[m] = make_float2((float)std::cos(a), (float)std::sin(a));
-            }
-        }
-        DCK(cudaMemcpyAsync(w.at<float2>(p->o_W), Wh.data(), sizeof(float2) * Wh.size(), cudaMemcpyHostToDevice, st),
-            "twiddles");
-    }
-    if (!p->attrs_set) {
-        DCK(cudaFuncSetAttribute(dfft_kernel<512, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, 12 * 16384), "attr");
-        DCK(cudaFuncSetAttribute(difft_kernel<512, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, 12 * 16384), "attr");
-        p->attrs_set = true;
-    }
-    int r = filter_spectra(p, ptr, st);
-    if (r) return r;
-    r = input_spectra(p, ptr, st);
-    if (r) return r;
-    for (int L = 0; L < p->M; ++L) {
-        const int cs = p->cs[L], nb = p->nb[L];
-        float2* Y = w.at<float2>(p->o_Y[L]);
-        r = launch_mac(w.at<float2>(p->o_X[L]), w.at<float2>(p->o_H[L]), Y, p->B, nb, nb, p->P[L], cs, 0, st);
-        DCK(cudaGetLastError(), "forward MAC");
-        p->launches++;
-        r = run_tab(p, L, pcd_plan::kIY, ptr, st);
-        if (r) return r;
-    }
-    return PC_OK;
+    int r = filter_spectra(p, d_h, d_ws, st);
+    return r ? r : convolve(p, d_x, d_y, d_ws, false, true, st);
 }
 
 int pcd_backward(pcd_plan* p, const float* d_x, const float* d_h, const float* d_gy, float* d_gx, float* d_gh,
                  void* d_ws, int recompute, void* stream) {
     if (!p || !d_gy || !d_ws) return dfail(p, PC_ERR_ARG, "null pointer");
     cudaStream_t st = (cudaStream_t)stream;
-    WS w{static_cast<char*>(d_ws)};
-    const DPtrs ptr{{d_x, d_h, d_gy}, {nullptr, d_gh, d_gx}, w.base};
     int r;
     if (recompute) {   // rebuild what the forward pass left in the workspace
         if (!d_x || !d_h) return dfail(p, PC_ERR_ARG, "recompute needs x and h");
-        r = filter_spectra(p, ptr, st);
-        if (r) return r;
-        r = input_spectra(p, ptr, st);
-        if (r) return r;
+        if (d_gx && (r = filter_spectra(p, d_h, d_ws, st))) return r;
+        if (d_gh && (r = convolve(p, d_x, nullptr, d_ws, false, true, st))) return r;
     }
-    for (int L = 0; L < p->M; ++L) {
-        const int cs = p->cs[L], nb = p->nb[L], nbg = p->nbg[L], P = p->P[L];
-        float2* Y = w.at<float2>(p->o_Y[L]);
-        // dL/dh first: it needs the input spectra X, which the adjoint pass
-        // below overwrites with its own result
-        if (d_gh) {
-            r = run_tab(p, L, pcd_plan::kFGP, ptr, st);   // GP_b = rfft([g block b, 0_N]) into Y
-            if (r) return r;
-            float2* Dp = w.at<float2>(p->o_Dp[L]);
-            float2* D = w.at<float2>(p->o_D[L]);
-            int nchunk = kDhChunks;
-            if (P <= kSlideP) {
-                const int nrun = (nb + kSlideRun - 1) / kSlideRun;
-                nchunk = p->B * nrun;
-                const long long tot = (long long)nchunk * cs;
-                ddh_slide_kernel<<<(int)std::min<long long>((tot + 255) / 256, 152 * 16), 256, 0, st>>>(
-                    w.at<float2>(p->o_X[L]), Y, Dp, p->B, nb, P, cs);
-            } else {
-                const long long tot = (long long)kDhChunks * P * cs;
-                ddh_partial_kernel<<<(int)std::min<long long>((tot + 255) / 256, 152 * 16), 256, 0, st>>>(
-                    w.at<float2>(p->o_X[L]), Y, Dp, p->B, nb, P, cs, kDhChunks);
-            }
-            ddh_reduce_kernel<<<(P * cs + 255) / 256, 256, 0, st>>>(Dp, D, P, cs, nchunk);
-            DCK(cudaGetLastError(), "dL/dh reduction");
-            p->launches += 2;
-            r = run_tab(p, L, pcd_plan::kIGH, ptr, st);   // dh[s_L + qN + t] = irfft(D_q)[N - t] / 2N
-            if (r) return r;
-        }
-        if (d_gx) {
-            r = run_tab(p, L, pcd_plan::kFGX, ptr, st);   // G'_c into Y
-            if (r) return r;
-            float2* Z = w.at<float2>(p->o_X[L]);   // adjoint sums replace the input spectra
-            launch_mac(Y, w.at<float2>(p->o_H[L]), Z, p->B, nbg, nb, P, cs, 1, st);
-            DCK(cudaGetLastError(), "adjoint MAC");
-            p->launches++;
-            r = run_tab(p, L, pcd_plan::kIGX, ptr, st);
-            if (r) return r;
-        }
+    // dL/dh first: it needs the input spectra X, which the adjoint pass below
+    // overwrites with those of the gradient
+    if (d_gh) {
+        float2* GP = at<float2>(d_ws, p->o_Y);
+        float2 *Dp = at<float2>(d_ws, p->o_Dp), *D = at<float2>(d_ws, p->o_D);
+        const WinArgs a{d_gy, GP, p->tab, p->T, p->B * p->nb, p->nb, p->cs, 0, 1.0f};   // GP_b = rfft([g block b, 0_N])
+        DCK(by_block(p->N, WinFft{a, st}), "gradient windows");
+        const long long tot = (long long)p->B * p->nrun * p->cs;
+        const int total = p->P * p->cs;
+        ddh_slide_kernel<<<dim3((unsigned)((tot + 127) / 128), (p->P + kMaxParts - 1) / kMaxParts), 128, 0, st>>>(
+            at<float2>(d_ws, p->o_X), GP, Dp, p->B, p->nb, p->slots, p->P, p->cs);
+        ddh_reduce_kernel<<<(total + 127) / 128, 128, 0, st>>>(Dp, D, total, p->B * p->nrun);
+        DCK(cudaGetLastError(), "dL/dh correlation");
+        DCK(by_block(p->N, TapIfft{D, p->P, p->cs, p->tab, d_gh, p->ir_len, st}), "dL/dh taps");
+        p->launches += 4;
+        const long long done = (long long)p->P * p->N;
+        if (done < p->ir_len)   // taps beyond the signal's length
+            DCK(cudaMemsetAsync(d_gh + done, 0, sizeof(float) * (p->ir_len - done), st), "dL/dh taps");
     }
-    return PC_OK;
+    return d_gx ? convolve(p, d_gy, d_gx, d_ws, true, true, st) : PC_OK;
 }
 
 void pcd_destroy(pcd_plan* p) { delete p; }

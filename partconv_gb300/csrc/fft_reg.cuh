@@ -29,7 +29,7 @@ constexpr int kRegMaxLog = 14;
 // ---- layout of the table (float2 entries) ---------------------------------------
 // w1(s): exp(-2 pi i k / 4^(s+1)), k < 4^s, stages s = 1 .. 6
 // w2(s), w3(s): its squares and cubes (blocks up to 1024 points read all three
-//   factors; larger ones do with `full`, else they form them by products as
+//   factors; larger ones do with FULL, else they form them by products as
 //   fft_smem's conflict-free stages do, with about one rounding more each)
 // r2(a): exp(-2 pi i k / (2 4^a)), k < 4^a, a = 2 .. 6 (the radix-2 stage)
 // sp(l): exp(-2 pi i k / 2^(l+1)), k <= 2^(l-1), l = 4 .. 14 (the real split)
@@ -82,7 +82,6 @@ struct RegFft {
     static constexpr int N = 1 << LOGN;
     static constexpr int TPT = N / 16;          // threads per transform
     static constexpr int SM = N + N / 16;       // shared float2 per transform
-    static constexpr bool FULL = LOGN <= 10;    // all three factors of a butterfly from the table
     __device__ static __forceinline__ void sync() {
         if constexpr (TPT <= 32) {
             __syncwarp();
@@ -117,10 +116,9 @@ __device__ __forceinline__ void bfly4(float2& v0, float2& v1, float2& v2, float2
 
 // the three factors of stage S (Ns = 4^S) at index k
 template <int S, bool FULL, bool INV>
-__device__ __forceinline__ void stage_tw(const float2* __restrict__ T, bool full, int k, float2& w1, float2& w2,
-                                         float2& w3) {
+__device__ __forceinline__ void stage_tw(const float2* __restrict__ T, int k, float2& w1, float2& w2, float2& w3) {
     w1 = tw_dir<INV>(__ldg(T + ft_w1(S) + k));
-    if (FULL || full) {
+    if constexpr (FULL) {
         w2 = tw_dir<INV>(__ldg(T + ft_w2(S) + k));
         w3 = tw_dir<INV>(__ldg(T + ft_w3(S) + k));
     } else {
@@ -131,14 +129,14 @@ __device__ __forceinline__ void stage_tw(const float2* __restrict__ T, bool full
 
 // Stages S and S + 1 on v[m] = a[t + m TPT]; afterwards v[r + 4 e] is the
 // element 16 (t - k) + k + (r + 4 e) Ns, k = t mod Ns.
-template <int LOGN, int NT, int S, bool INV>
-__device__ __forceinline__ void pass16(float2 (&v)[16], int t, const float2* __restrict__ T, bool full) {
+template <int LOGN, int NT, int S, bool INV, bool F>
+__device__ __forceinline__ void pass16(float2 (&v)[16], int t, const float2* __restrict__ T) {
     constexpr int Ns = 1 << (2 * S);
-    constexpr bool FULL = RegFft<LOGN, NT>::FULL;
+    constexpr bool FULL = F || LOGN <= 10;   // all three factors of a butterfly from the table
     const int k = t & (Ns - 1);
     if constexpr (S > 0) {
         float2 w1, w2, w3;
-        stage_tw<S, FULL, INV>(T, full, k, w1, w2, w3);
+        stage_tw<S, FULL, INV>(T, k, w1, w2, w3);
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
             v[q + 4] = cmul(v[q + 4], w1);
@@ -154,7 +152,7 @@ __device__ __forceinline__ void pass16(float2 (&v)[16], int t, const float2* __r
         float2 a0 = v[4 * r], a1 = v[4 * r + 1], a2 = v[4 * r + 2], a3 = v[4 * r + 3];
         if (S > 0 || r > 0) {
             float2 w1, w2, w3;
-            stage_tw<S + 1, FULL, INV>(T, full, k + r * Ns, w1, w2, w3);
+            stage_tw<S + 1, FULL, INV>(T, k + r * Ns, w1, w2, w3);
             a1 = cmul(a1, w1);
             a2 = cmul(a2, w2);
             a3 = cmul(a3, w3);
@@ -171,11 +169,11 @@ __device__ __forceinline__ void pass16(float2 (&v)[16], int t, const float2* __r
 
 // The last stages after the radix-16 passes, in place on v[m] = a[t + m TPT]
 // (the results lie at the same places): radix 8 (4 then 2), 4 or 2.
-template <int LOGN, int NT, bool INV>
-__device__ __forceinline__ void pass_tail(float2 (&v)[16], int t, const float2* __restrict__ T, bool full) {
+template <int LOGN, int NT, bool INV, bool F>
+__device__ __forceinline__ void pass_tail(float2 (&v)[16], int t, const float2* __restrict__ T) {
     constexpr int N4 = LOGN / 2, TPT = RegFft<LOGN, NT>::TPT;
     constexpr bool odd4 = (N4 & 1) != 0, r2 = (LOGN & 1) != 0;
-    constexpr bool FULL = RegFft<LOGN, NT>::FULL;
+    constexpr bool FULL = F || LOGN <= 10;   // all three factors of a butterfly from the table
     if constexpr (odd4) {   // the last radix-4 stage, Ns = 4^(N4 - 1)
         constexpr int S = N4 - 1;
         constexpr int Ns = 1 << (2 * S);
@@ -186,7 +184,7 @@ __device__ __forceinline__ void pass_tail(float2 (&v)[16], int t, const float2* 
         for (int g = 0; g < G; ++g) {
             float2 w1, w2, w3;
             const int k = (t + g * TPT) & (Ns - 1);
-            if constexpr (S > 0) stage_tw<S, FULL, INV>(T, full, k, w1, w2, w3);
+            if constexpr (S > 0) stage_tw<S, FULL, INV>(T, k, w1, w2, w3);
 #pragma unroll
             for (int q = 0; q < (r2 ? 2 : 1); ++q) {
                 const int b = g + 2 * q;   // inputs b + 4 r
@@ -239,26 +237,26 @@ __device__ __forceinline__ void exchange(float2 (&v)[16], int t, float2* s) {
 
 // N-point transform of one group of TPT threads: in and out v[m] = a[t + m TPT].
 // s: this transform's shared memory (RegFft::SM float2), free on entry; a
-// caller that writes it afterwards syncs first.  full: see the table above.
-template <int LOGN, int NT, bool INV>
-__device__ __forceinline__ void fft_reg(float2 (&v)[16], int t, float2* s, const float2* __restrict__ T, bool full) {
+// caller that writes it afterwards syncs first.  FULL: see the table above.
+template <int LOGN, int NT, bool INV, bool FULL>
+__device__ __forceinline__ void fft_reg(float2 (&v)[16], int t, float2* s, const float2* __restrict__ T) {
     using F = RegFft<LOGN, NT>;
     constexpr int NP = LOGN / 4;   // radix-16 passes (LOGN / 2 radix-4 stages in pairs)
     constexpr bool tail = (LOGN & 3) != 0;
-    pass16<LOGN, NT, 0, INV>(v, t, T, full);
+    pass16<LOGN, NT, 0, INV, FULL>(v, t, T);
     if constexpr (NP > 1) {
         exchange<LOGN, NT, 0>(v, t, s);
-        pass16<LOGN, NT, 2, INV>(v, t, T, full);
+        pass16<LOGN, NT, 2, INV, FULL>(v, t, T);
     }
     if constexpr (NP > 2) {
         F::sync();
         exchange<LOGN, NT, 2>(v, t, s);
-        pass16<LOGN, NT, 4, INV>(v, t, T, full);
+        pass16<LOGN, NT, 4, INV, FULL>(v, t, T);
     }
     if constexpr (tail) {
         if constexpr (NP > 1) F::sync();
         exchange<LOGN, NT, 2 * (NP - 1)>(v, t, s);
-        pass_tail<LOGN, NT, INV>(v, t, T, full);
+        pass_tail<LOGN, NT, INV, FULL>(v, t, T);
     }
 }
 

@@ -57,7 +57,7 @@ __device__ __forceinline__ long long blocks_before(const WLevel& l, long long c)
 // A CTA of NT threads runs 16 NT / N transforms of one level; every CTA has
 // the same amount of work whatever its block size.
 // ---------------------------------------------------------------------------
-template <int LOGN, int NT>
+template <int LOGN, int NT, bool FULL>
 __device__ __forceinline__ void fft_body(const WLevel& l, int first, const WArgs& a, float2* smem) {
     using F = RegFft<LOGN, NT>;
     constexpr int N = F::N, TPT = F::TPT;
@@ -75,7 +75,7 @@ __device__ __forceinline__ void fft_body(const WLevel& l, int first, const WArgs
     const float* in = a.io.in + (long long)l.in_ch * a.io.in_ch;
     const float scale = l.scale;
     float2 v[16];
-    if (w0 >= t_in0 && a.vec_in) {
+    if (w0 >= t_in0 && a.vec_in && (a.len == 0 || t_end - t_in0 <= a.len)) {
         const float2* p = reinterpret_cast<const float2*>(in + (w0 - t_in0));
 #pragma unroll
         for (int m = 0; m < 16; ++m) {
@@ -88,14 +88,17 @@ __device__ __forceinline__ void fft_body(const WLevel& l, int first, const WArgs
         for (int m = 0; m < 16; ++m) {
             const long long ta = w0 + 2LL * (t + m * TPT);
             if (ta >= t_in0) {
-                const float* p = in + (ta - t_in0) * isamp;
-                v[m] = make_float2(p[0] * scale, p[isamp] * scale);
-            } else {
+                const long long i = ta - t_in0, left = a.len == 0 ? 2 : a.len - i;
+                const float* p = in + i * isamp;
+                v[m] = make_float2(left > 0 ? p[0] * scale : 0.0f, left > 1 ? p[isamp] * scale : 0.0f);
+            } else if (l.xring) {
                 v[m] = __ldcg(reinterpret_cast<const float2*>(l.xring + (ta & l.rin_mask)));
+            } else {
+                v[m] = make_float2(0.f, 0.f);
             }
         }
     }
-    fft_reg<LOGN, NT, false>(v, t, s, a.tab, a.full != 0);
+    fft_reg<LOGN, NT, false, FULL>(v, t, s, a.tab);
     // the split pairs k < N / 2 (this thread's v[0 .. 7]) with N - k, which
     // lies in another thread's upper half
     F::sync();
@@ -103,7 +106,7 @@ __device__ __forceinline__ void fft_body(const WLevel& l, int first, const WArgs
     for (int m = 8; m < 16; ++m) s[rpad(t + m * TPT)] = v[m];
     F::sync();
     if (!live) return;
-    float2* Xs = l.X + (size_t)wmod(b, l.slots) * l.cs;
+    float2* Xs = wide_at(l.X, a.rel) + (size_t)wmod(b, l.slots) * l.cs;
     const float2* sp = a.tab + ft_sp(LOGN);
 #pragma unroll
     for (int m = 0; m < 8; ++m) {
@@ -134,7 +137,9 @@ __device__ __forceinline__ void by_log_dev(int logN, Fn&& f) {
         case 10: f.template operator()<10>(); break;
         case 11: f.template operator()<11>(); break;
         default:
-            if constexpr (NT >= 1024) {
+            if constexpr (NT == 256) {
+                f.template operator()<12>();
+            } else if constexpr (NT >= 1024) {
                 if (logN == 12) f.template operator()<12>();
                 else if (logN == 13) f.template operator()<13>();
                 else f.template operator()<14>();
@@ -142,16 +147,16 @@ __device__ __forceinline__ void by_log_dev(int logN, Fn&& f) {
     }
 }
 
-template <int NT>
+template <int NT, bool FULL>
 struct FftBody {
     const WLevel& l;
     int first;
     const WArgs& a;
     float2* smem;
     template <int LOGN>
-    __device__ __forceinline__ void operator()() const { fft_body<LOGN, NT>(l, first, a, smem); }
+    __device__ __forceinline__ void operator()() const { fft_body<LOGN, NT, FULL>(l, first, a, smem); }
 };
-template <int NT>
+template <int NT, bool FULL>
 __global__ void __launch_bounds__(NT) wide_fft_kernel(const int2* __restrict__ map, WArgs a) {
     extern __shared__ float4 dyn_smem[];
     cudaTriggerProgrammaticLaunchCompletion();
@@ -159,7 +164,7 @@ __global__ void __launch_bounds__(NT) wide_fft_kernel(const int2* __restrict__ m
     const WLevel& l = a.lv[e.x];
     cudaGridDependencySynchronize();
     if (e.y >= (int)(blocks_before(l, a.c0 + a.nsteps) - blocks_before(l, a.c0))) return;
-    by_log_dev<NT>(l.logN, FftBody<NT>{l, e.y, a, reinterpret_cast<float2*>(dyn_smem)});
+    by_log_dev<NT>(l.logN, FftBody<NT, FULL>{l, e.y, a, reinterpret_cast<float2*>(dyn_smem)});
 }
 
 // ---------------------------------------------------------------------------
@@ -291,14 +296,15 @@ __device__ __forceinline__ void chain_parts(MacCol<SH> c, int n, float2 (&y)[RB]
     }
 }
 
-// y = X_b H_0 + (X_{b-1} H_1 + rows) for the run's blocks, c at part 0
+// y = X_b H_0 + (X_{b-1} H_1 + rows) for the run's blocks, c at part 0 (first:
+// the run begins with block 0, before which there is silence)
 template <int RB, bool SH>
 __device__ __forceinline__ void finish_run(const MacCol<SH>& c, const WLevel& l, const f32x2 (&ys)[RB], float2* Y,
-                                           int live) {
+                                           int live, bool first = false) {
     const bool rows = l.P > l.p_lo, x1 = l.two && l.P >= 2;
     const float2 h0 = c.h();
     const float2 h1 = x1 ? MacCol<SH>{c.H + c.cs, nullptr, 0, 0, 0}.h() : make_float2(0.f, 0.f);
-    float2 xm = x1 ? unpack2(c.x(c.back(c.ox))) : make_float2(0.f, 0.f);
+    float2 xm = x1 && !first ? unpack2(c.x(c.back(c.ox))) : make_float2(0.f, 0.f);
     int o = c.ox;
 #pragma unroll
     for (int j = 0; j < RB; ++j) {
@@ -312,8 +318,10 @@ __device__ __forceinline__ void finish_run(const MacCol<SH>& c, const WLevel& l,
     }
 }
 
-__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+// (zeros when !on)
+__device__ __forceinline__ void cp_async16(void* dst, const void* src, bool on = true) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)),
+                 "l"(src), "r"(on ? 16 : 0)
                  : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
@@ -341,9 +349,9 @@ __global__ void __launch_bounds__(kMacTile) wide_mac_kernel(const int4* __restri
     const int w2 = min(W, cs - k0) >> 1;   // pairs of bins in the tile
     const int tid = threadIdx.x, lr = tid / (W / 2), lc = tid % (W / 2);
     const bool live = tid < 2 * w2;
-    const float2* Hg = l.H + k0;
-    const float2* Xg = l.X + k0;
-    float2* Y = l.Yw + k0 + tid;
+    const float2* Hg = wide_at(l.H, a.rel) + k0;
+    const float2* Xg = wide_at(l.X, a.rel) + k0;
+    float2* Y = wide_at(l.Yw, a.rel) + k0 + tid;
     int sl = wmod(bf, R) + e.z;   // ring row of block e.z of the chunk
     if (sl >= R) sl -= R;
     // rows [0, n) of the filter / of blocks starting at ring row s, to shared rows dst + ((p + i) mod m) W
@@ -351,7 +359,8 @@ __global__ void __launch_bounds__(kMacTile) wide_mac_kernel(const int4* __restri
         if (lc < w2)
             for (int i = lr; i < n; i += 2) cp_async16(dst + i * W + 2 * lc, Hg + (size_t)(p + i) * cs + 2 * lc);
     };
-    auto copy_x = [&](float2* dst, int p, int m, int s, int n) {
+    // (nz: rows that lie before block 0, zero)
+    auto copy_x = [&](float2* dst, int p, int m, int s, int n, int nz) {
         if (s < 0) s += R;
         if (s >= R) s -= R;
         if (lc < w2)
@@ -360,7 +369,7 @@ __global__ void __launch_bounds__(kMacTile) wide_mac_kernel(const int4* __restri
                 if (r >= R) r -= R;
                 int q = p + i;
                 if (q >= m) q -= m;
-                cp_async16(dst + q * W + 2 * lc, Xg + (size_t)r * cs + 2 * lc);
+                cp_async16(dst + q * W + 2 * lc, Xg + (size_t)r * cs + 2 * lc, i >= nz);
             }
     };
     float2* Hs = reinterpret_cast<float2*>(dyn_smem);
@@ -369,14 +378,14 @@ __global__ void __launch_bounds__(kMacTile) wide_mac_kernel(const int4* __restri
         float2* Xs = Hs + kMacRes * W;
         const int RX = P - 1 + 2 * RB;   // ring rows: the history of a run, the run, the next run
         copy_h(Hs, 0, P);
-        copy_x(Xs, 0, RX, sl - (P - 1), P - 1 + RB);
+        copy_x(Xs, 0, RX, sl - (P - 1), P - 1 + RB, (int)max(0LL, P - 1 - (bf + e.z)));
         cp_async_commit();
         int pos = P - 1;                 // shared row of the run's first block
         for (int i0 = e.z; i0 < nb; i0 += RB) {
             if (i0 + RB < nb) {
                 int q = pos + RB;
                 if (q >= RX) q -= RX;
-                copy_x(Xs, q, RX, sl + RB, RB);
+                copy_x(Xs, q, RX, sl + RB, RB, 0);
             }
             cp_async_commit();
             cp_async_wait<1>();
@@ -407,7 +416,8 @@ __global__ void __launch_bounds__(kMacTile) wide_mac_kernel(const int4* __restri
             const int pb = l.p_lo + q * l.tp, n = min(l.tp, P - pb);
             // blocks (run's first) - pb - n .. (run's first) - pb + RB - 1
             copy_h(Hs, pb, n);
-            copy_x(Xs, 0, TP + RB, sl - pb - n, n + RB);
+            // (before block 0 only in the first blocks of all: the ring holds no more than R of them)
+            copy_x(Xs, 0, TP + RB, sl - pb - n, n + RB, (int)max(0LL, pb + n - (bf + i0)));
             cp_async_commit();
             cp_async_wait<0>();
             __syncthreads();
@@ -421,7 +431,8 @@ __global__ void __launch_bounds__(kMacTile) wide_mac_kernel(const int4* __restri
             __syncthreads();
         }
         if (live)
-            finish_run(MacCol<false>{Hg + tid, Xg + tid, cs, R * cs, sl * cs}, l, ys, Y + (size_t)i0 * cs, nb - i0);
+            finish_run(MacCol<false>{Hg + tid, Xg + tid, cs, R * cs, sl * cs}, l, ys, Y + (size_t)i0 * cs, nb - i0,
+                       bf + i0 == 0);
         sl += RB;
         if (sl >= R) sl -= R;
     }
@@ -477,7 +488,7 @@ __global__ void __launch_bounds__(kMacAnyNT, 3) wide_mac_any_kernel(const int4* 
 // 3. inverse merge, inverse FFT, output ring (levels >= 1, one launch for all
 // block sizes) or the call's output (level 0, after them)
 // ---------------------------------------------------------------------------
-template <int LOGN, int NT, bool L0>
+template <int LOGN, int NT, bool L0, bool FULL>
 __device__ __forceinline__ void ifft_body(const WLevel& l, int first, const WArgs& a, float2* smem) {
     using F = RegFft<LOGN, NT>;
     constexpr int N = F::N, TPT = F::TPT;
@@ -489,7 +500,7 @@ __device__ __forceinline__ void ifft_body(const WLevel& l, int first, const WArg
     if (TPT >= 32 && !live) return;
     const int i = min(first + tr, nb - 1);
     const long long b = b0 + i;
-    const float2* Y = l.Yw + (size_t)i * l.cs;
+    const float2* Y = wide_at(l.Yw, a.rel) + (size_t)i * l.cs;
     const float2* sp = a.tab + ft_sp(LOGN);
     float2 v[16];
 #pragma unroll
@@ -504,7 +515,7 @@ __device__ __forceinline__ void ifft_body(const WLevel& l, int first, const WArg
             merge_w(yc, yn, __ldg(sp + N - n), other, v[m]);
         }
     }
-    fft_reg<LOGN, NT, true>(v, t, s, a.tab, a.full != 0);
+    fft_reg<LOGN, NT, true, FULL>(v, t, s, a.tab);
     if (!live) return;
     // real samples 2 n, 2 n + 1 of the block in v[m], n = t + m TPT < N / 2
     if constexpr (!L0) {
@@ -547,7 +558,15 @@ __device__ __forceinline__ void ifft_body(const WLevel& l, int first, const WArg
         } else if (l.mix_mode == 1) {
             const long long os = a.io.out_sample;
             float* o = a.io.out + (long long)l.out_ch * a.io.out_ch + (t0 - a.io.step0 * (long long)a.N0) * os;
-            if (a.vec_out) {
+            const long long left = a.len == 0 ? N : a.len - (t0 - a.io.step0 * (long long)a.N0);   // samples of the block to write
+            if (left < N) {
+#pragma unroll
+                for (int m = 0; m < 8; ++m) {
+                    const long long i = 2 * (t + m * TPT);
+                    if (i < left) o[i * os] = v[m].x;
+                    if (i + 1 < left) o[(i + 1) * os] = v[m].y;
+                }
+            } else if (a.vec_out) {
 #pragma unroll
                 for (int m = 0; m < 8; ++m) reinterpret_cast<float2*>(o)[t + m * TPT] = v[m];
             } else {
@@ -561,16 +580,16 @@ __device__ __forceinline__ void ifft_body(const WLevel& l, int first, const WArg
     }
 }
 
-template <int NT>
+template <int NT, bool FULL>
 struct IfftBody {
     const WLevel& l;
     int first;
     const WArgs& a;
     float2* smem;
     template <int LOGN>
-    __device__ __forceinline__ void operator()() const { ifft_body<LOGN, NT, false>(l, first, a, smem); }
+    __device__ __forceinline__ void operator()() const { ifft_body<LOGN, NT, false, FULL>(l, first, a, smem); }
 };
-template <int NT>
+template <int NT, bool FULL>
 __global__ void __launch_bounds__(NT) wide_ifft_kernel(const int2* __restrict__ map, WArgs a) {
     extern __shared__ float4 dyn_smem[];
     cudaTriggerProgrammaticLaunchCompletion();
@@ -578,11 +597,11 @@ __global__ void __launch_bounds__(NT) wide_ifft_kernel(const int2* __restrict__ 
     const WLevel& l = a.lv[e.x];
     cudaGridDependencySynchronize();
     if (e.y >= (int)(blocks_before(l, a.c0 + a.nsteps) - blocks_before(l, a.c0))) return;
-    by_log_dev<NT>(l.logN, IfftBody<NT>{l, e.y, a, reinterpret_cast<float2*>(dyn_smem)});
+    by_log_dev<NT>(l.logN, IfftBody<NT, FULL>{l, e.y, a, reinterpret_cast<float2*>(dyn_smem)});
 }
 
 __host__ __device__ constexpr int out_threads(int logN) { return logN <= 11 ? 128 : 1 << (logN - 4); }
-template <int LOGN>
+template <int LOGN, bool FULL>
 __global__ void __launch_bounds__(out_threads(LOGN)) wide_out_kernel(const int2* __restrict__ map, WArgs a) {
     extern __shared__ float4 dyn_smem[];
     cudaTriggerProgrammaticLaunchCompletion();
@@ -590,7 +609,7 @@ __global__ void __launch_bounds__(out_threads(LOGN)) wide_out_kernel(const int2*
     const WLevel& l = a.lv[e.x];
     cudaGridDependencySynchronize();
     if (e.y >= a.nsteps) return;
-    ifft_body<LOGN, out_threads(LOGN), true>(l, e.y, a, reinterpret_cast<float2*>(dyn_smem));
+    ifft_body<LOGN, out_threads(LOGN), true, FULL>(l, e.y, a, reinterpret_cast<float2*>(dyn_smem));
 }
 
 // 4. outputs fed by several PCs (summed in PC order) and outputs without any
@@ -676,11 +695,15 @@ cudaError_t by_log(int N, Fn&& f) {
     }
 }
 
+template <class K>
+cudaError_t allow_smem(K* k, int nt) {
+    return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fft_smem_of(nt));
+}
 struct OutPrepare {
     template <int L>
     cudaError_t operator()() const {
-        return cudaFuncSetAttribute(wide_out_kernel<L>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)fft_smem_of(out_threads(L)));
+        const cudaError_t e = allow_smem(wide_out_kernel<L, false>, out_threads(L));
+        return e == cudaSuccess ? allow_smem(wide_out_kernel<L, true>, out_threads(L)) : e;
     }
 };
 
@@ -704,11 +727,10 @@ const std::vector<float2>& host_fft_tables() {
 }
 
 cudaError_t prepare_wide_kernels() {
-    cudaError_t e = cudaFuncSetAttribute(wide_fft_kernel<1024>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)fft_smem_of(1024));
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(wide_ifft_kernel<1024>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)fft_smem_of(1024));
+    cudaError_t e = allow_smem(wide_fft_kernel<1024, false>, 1024);
+    if (e == cudaSuccess) e = allow_smem(wide_fft_kernel<1024, true>, 1024);
+    if (e == cudaSuccess) e = allow_smem(wide_ifft_kernel<1024, false>, 1024);
+    if (e == cudaSuccess) e = allow_smem(wide_ifft_kernel<1024, true>, 1024);
     for (int N = 8192; N <= 16384 && e == cudaSuccess; N *= 2) e = by_log(N, OutPrepare{});
     return e;
 }
@@ -716,18 +738,24 @@ cudaError_t prepare_wide_kernels() {
 int wide_threads(int max_n) { return max_n <= 2048 ? 128 : 1024; }
 int wide_out_blocks(int N0) { return N0 <= 2048 ? 2048 / N0 : 1; }
 
+template <int NT, bool FULL>
+static cudaError_t launch_fft(bool inverse, bool dep, int grid, const int2* map, const WArgs& a, cudaStream_t st) {
+    if (inverse) {
+        if constexpr (NT != 256) return launch_dep(wide_ifft_kernel<NT, FULL>, grid, NT, fft_smem_of(NT), st, map, a);
+        return cudaErrorInvalidValue;
+    }
+    if (dep) return launch_dep(wide_fft_kernel<NT, FULL>, grid, NT, fft_smem_of(NT), st, map, a);
+    wide_fft_kernel<NT, FULL><<<grid, NT, fft_smem_of(NT), st>>>(map, a);
+    return cudaGetLastError();
+}
 cudaError_t launch_wide_fft(bool inverse, int nt, int grid, const int2* map, const WArgs& a, cudaStream_t st, bool dep) {
     if (grid <= 0) return cudaSuccess;
-    const size_t sm = fft_smem_of(nt);
-    if (nt == 128 && !dep && !inverse) {
-        wide_fft_kernel<128><<<grid, nt, sm, st>>>(map, a);
-        return cudaGetLastError();
-    }
+    if (nt == 256) return launch_fft<256, true>(inverse, dep, grid, map, a, st);
     if (nt == 128)
-        return inverse ? launch_dep(wide_ifft_kernel<128>, grid, nt, sm, st, map, a)
-                       : launch_dep(wide_fft_kernel<128>, grid, nt, sm, st, map, a);
-    return inverse ? launch_dep(wide_ifft_kernel<1024>, grid, nt, sm, st, map, a)
-                   : launch_dep(wide_fft_kernel<1024>, grid, nt, sm, st, map, a);
+        return a.full ? launch_fft<128, true>(inverse, dep, grid, map, a, st)
+                      : launch_fft<128, false>(inverse, dep, grid, map, a, st);
+    return a.full ? launch_fft<1024, true>(inverse, dep, grid, map, a, st)
+                  : launch_fft<1024, false>(inverse, dep, grid, map, a, st);
 }
 
 struct WideOut {
@@ -737,7 +765,9 @@ struct WideOut {
     cudaStream_t st;
     template <int L>
     cudaError_t operator()() const {
-        return launch_dep(wide_out_kernel<L>, grid, out_threads(L), fft_smem_of(out_threads(L)), st, map, a);
+        // (blocks up to 1024 read every factor from the table either way)
+        return L > 10 && a.full ? launch_dep(wide_out_kernel<L, true>, grid, out_threads(L), fft_smem_of(out_threads(L)), st, map, a)
+                                : launch_dep(wide_out_kernel<L, false>, grid, out_threads(L), fft_smem_of(out_threads(L)), st, map, a);
     }
 };
 cudaError_t launch_wide_out(int N0, int grid, const int2* map, const WArgs& a, cudaStream_t st) {

@@ -26,7 +26,7 @@ struct WLevel {
     float2* Yw;     // [blocks of a chunk][cs]
     float2* Yp;
     float* yring;
-    float* xring;
+    float* xring;   // null: silence before the call
     float* pcw;     // [chunk samples], mixed outputs only
 };
 
@@ -39,8 +39,15 @@ struct WArgs {
     int nsteps, kb;       // base steps of the chunk; base blocks per step of the handle
     int vec_in, vec_out;  // contiguous channels, 8-byte aligned: float2 loads and stores
     int full;             // every twiddle factor from the table (fft_reg.cuh)
+    long long rel;        // added (bytes) to the descriptors' H, X and Yw: a workspace given per call
+    long long len;        // samples of the call's input and output; silence after them (0: whole blocks)
     IOView io;
 };
+// descriptor pointer p of a launch with a.rel
+template <class T>
+__host__ __device__ __forceinline__ T* wide_at(T* p, long long rel) {
+    return reinterpret_cast<T*>(reinterpret_cast<unsigned long long>(p) + rel);
+}
 
 constexpr int kWideRun = 8;       // consecutive blocks a thread of the sum over parts takes together
 constexpr int kMacTile = 96;      // bins per CTA of the sum over parts (three warps: 258 bins are three tiles of 86)
@@ -56,7 +63,7 @@ cudaError_t prepare_wide_kernels();
 // 16 threads / N transforms), and blocks per CTA of wide_out
 int wide_threads(int max_n);
 int wide_out_blocks(int N0);
-// (dep = false: tables that the kernel reads are still being written by the stream's last kernel)
+// (nt = 256: forward transforms of blocks up to 4096; dep = false: tables that the kernel reads are still being written by the stream's last kernel)
 cudaError_t launch_wide_fft(bool inverse, int nt, int grid, const int2* map, const WArgs& a, cudaStream_t st,
                             bool dep = true);
 // level 0: inverse transforms and the call's output
