@@ -1215,7 +1215,7 @@ cudaError_t launch_side_spreads(int grid, const Task* tasks, long long step, cud
 // slices all come later has nothing to do), and, by ring_ctas CTAs per PC,
 // the call's newest samples (at most a ring's worth) in the input rings.
 // NT, LANES: as the handle's spread tasks.
-template <int NT, int LANES>
+template <int NT, int LANES, bool MULTI>
 __global__ void __launch_bounds__(NT) wide_state_kernel(const int4* __restrict__ map, int n_part,
                                                         const int* __restrict__ lv0, int ring_ctas, WArgs a) {
     extern __shared__ float4 dyn_smem[];
@@ -1278,8 +1278,8 @@ __global__ void __launch_bounds__(NT) wide_state_kernel(const int4* __restrict__
         tk = t;
     }
     __syncthreads();
-    if constexpr (NT == 256) {
-        if (kb > 1 && T == 1) {
+    if constexpr (MULTI) {
+        if (T == 1) {
             if (kb == 2) spread_multi<NT, 2>(tk, c1 - 1, dyn_smem);
             else spread_multi<NT, 4>(tk, c1 - 1, dyn_smem);
             return;
@@ -1288,7 +1288,7 @@ __global__ void __launch_bounds__(NT) wide_state_kernel(const int4* __restrict__
     spread_lanes<NT, LANES>(tk, c1 - 1, dyn_smem, 1);
 }
 
-template <int NT, int LANES>
+template <int NT, int LANES, bool MULTI = false>
 static cudaError_t launch_state(int n_part, const int4* map, const int* lv0, int npc, int ring_ctas,
                                 const WArgs& a, cudaStream_t st) {
     cudaLaunchAttribute attr[1];
@@ -1301,7 +1301,7 @@ static cudaError_t launch_state(int n_part, const int4* map, const int* lv0, int
     cfg.stream = st;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, wide_state_kernel<NT, LANES>, map, n_part, lv0, ring_ctas, a);
+    return cudaLaunchKernelEx(&cfg, wide_state_kernel<NT, LANES, MULTI>, map, n_part, lv0, ring_ctas, a);
 }
 
 cudaError_t launch_wide_state(int nt, int lanes, int n_part, const int4* map, const int* lv0, int npc, int max_ring,
@@ -1310,12 +1310,20 @@ cudaError_t launch_wide_state(int nt, int lanes, int n_part, const int4* map, co
     const int ring_ctas = std::max(1, std::min(max_ring / (4 * nt), 4096 / npc));
     if (nt == 512) return launch_state<512, 64>(n_part, map, lv0, npc, ring_ctas, a, st);
     if (nt == 1024) return launch_state<1024, 64>(n_part, map, lv0, npc, ring_ctas, a, st);
-    switch (lanes) {
-        case 32: return launch_state<256, 32>(n_part, map, lv0, npc, ring_ctas, a, st);
-        case 128: return launch_state<256, 128>(n_part, map, lv0, npc, ring_ctas, a, st);
-        case 256: return launch_state<256, 256>(n_part, map, lv0, npc, ring_ctas, a, st);
-        default: return launch_state<256, 64>(n_part, map, lv0, npc, ring_ctas, a, st);
-    }
+    auto go = [&](auto multi) {
+        constexpr bool M = decltype(multi)::value;
+        switch (lanes) {
+            case 32: return launch_state<256, 32, M>(n_part, map, lv0, npc, ring_ctas, a, st);
+            case 128: return launch_state<256, 128, M>(n_part, map, lv0, npc, ring_ctas, a, st);
+            case 256: return launch_state<256, 256, M>(n_part, map, lv0, npc, ring_ctas, a, st);
+            default: return launch_state<256, 64, M>(n_part, map, lv0, npc, ring_ctas, a, st);
+        }
+    };
+    // several blocks per step: a kernel of its own, its sums hold twice the
+    // registers (89 a thread; in one kernel with the others, streams of one
+    // block per step took 52 us where they take 37)
+    if (a.kb > 1) return go(std::true_type{});
+    return go(std::false_type{});
 }
 
 // ---------------------------------------------------------------------------
