@@ -461,8 +461,8 @@ __device__ __forceinline__ void fire_body(const Bank& bank, const Task& tk, cons
                 Xs[k] = xk;
                 if (bnk != k) Xs[bnk] = xnk;
             }
-            const float2 pk = cmul(xk, h0s[k]);
-            const float2 pnk = cmul(xnk, h0s[bnk]);
+            const float2 pk = cmul(h0s[k], xk);
+            const float2 pnk = cmul(h0s[bnk], xnk);
             h0s[k] = pk;
             h0s[bnk != k ? bnk : N + 1] = pnk;
         }
@@ -479,8 +479,8 @@ __device__ __forceinline__ void fire_body(const Bank& bank, const Task& tk, cons
             const int bnk = N - k;
             float2 ak = make_float2(0.f, 0.f), ank = ak;
             if (use_x1) {
-                ak = cmul(xp[j][0], yacc[k]);
-                ank = cmul(xp[j][1], yacc[bnk]);
+                ak = cmul(yacc[k], xp[j][0]);
+                ank = cmul(yacc[bnk], xp[j][1]);
             }
             if (use_yp) {
                 ak = cadd(ak, yp[j][0]);
@@ -617,8 +617,8 @@ __device__ __forceinline__ void fire_body(const Bank& bank, const Task& tk, cons
             const int bk = k, bnk = N - k;   // k == 0 pairs bin 0 with bin N
             Xs[bk] = xk;
             if (bnk != bk) Xs[bnk] = xnk;
-            const float2 yk = cadd(cmul(xk, h0k), ak);
-            const float2 ynk = cadd(cmul(xnk, h0nk), ank);
+            const float2 yk = cadd(cmul(h0k, xk), ak);
+            const float2 ynk = cadd(cmul(h0nk, xnk), ank);
             float2 zk, znk;
             irfft_merge<SW>(yk, ynk, k, logN, tw, zk, znk);
             s[sidx<SW>(k)] = zk;
@@ -645,8 +645,8 @@ __device__ __forceinline__ void fire_body(const Bank& bank, const Task& tk, cons
                         }
                     }
                     if (use_x1) {
-                        av[u][0] = cadd(av[u][0], cmul(__ldcg(&X1[k]), __ldg(&tk.H[cs + k])));
-                        av[u][1] = cadd(av[u][1], cmul(__ldcg(&X1[bnk]), __ldg(&tk.H[cs + bnk])));
+                        av[u][0] = cadd(av[u][0], cmul(__ldg(&tk.H[cs + k]), __ldcg(&X1[k])));
+                        av[u][1] = cadd(av[u][1], cmul(__ldg(&tk.H[cs + bnk]), __ldcg(&X1[bnk])));
                     }
                 }
             }

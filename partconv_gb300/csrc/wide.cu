@@ -170,10 +170,8 @@ __global__ void __launch_bounds__(NT) wide_fft_kernel(const int2* __restrict__ m
 // ---------------------------------------------------------------------------
 // 2. the sum over parts: one thread per bin and run of RB consecutive blocks.
 // ---------------------------------------------------------------------------
-// One bin's column of a level: filter rows and spectrum rows, walked from one
-// part to the next (offsets in elements).  SH: rows staged in shared memory,
-// else the level's own (L2).
-template <bool SH>
+// One bin's column of a level in global memory: filter rows and spectrum
+// rows, walked from one part to the next (offsets in elements).
 struct MacCol {
     const float2* H;   // row of the part at hand
     const float2* X;
@@ -187,35 +185,26 @@ struct MacCol {
         o += cs;
         return o >= wrap ? o - wrap : o;
     }
-    __device__ __forceinline__ f32x2 x(int o) const {
-        const f32x2* p = reinterpret_cast<const f32x2*>(X + o);
-        if constexpr (SH) return *p;
-        else return __ldcg(p);
-    }
-    __device__ __forceinline__ float2 h() const {
-        if constexpr (SH) return *H;
-        else return __ldg(H);
-    }
+    __device__ __forceinline__ f32x2 x(int o) const { return __ldcg(reinterpret_cast<const f32x2*>(X + o)); }
+    __device__ __forceinline__ float2 h() const { return __ldg(H); }
 };
 
 // Sums X_{b+j-p} H_p, j < RB, over n consecutive parts in groups of tg, a group
 // in running sums of `unit` parts (running sums added in order into the group,
 // groups in order into row); c stands at the first part on entry and after the
 // last one on return.  The run's RB spectra under part p stay in registers:
-// part p + 1 needs one new one.  The loads of four parts go together; TG4:
-// tg = unit = 4 (the default tiles), they are a group.
-template <int RB, bool TG4, bool SH>
-__device__ __forceinline__ void sum_parts(MacCol<SH>& c, int n, int tg, int unit, f32x2 (&row)[RB]) {
+// part p + 1 needs one new one.  The loads of four parts go together.
+template <int RB>
+__device__ __forceinline__ void sum_parts(MacCol& c, int n, int tg, int unit, f32x2 (&row)[RB]) {
     constexpr int U = 4;
     static_assert(RB % U == 0, "constant window rotation");
     f32x2 acc[RB], w[RB], ws[RB];   // window: block (run's first) + d - first part at w[d mod RB], and its swapped pairs
-    f32x2 grp[TG4 ? 1 : RB];
+    f32x2 grp[RB];
     {
         int o = c.ox;
 #pragma unroll
         for (int j = 0; j < RB; ++j) {
-            row[j] = acc[j] = 0;
-            if constexpr (!TG4) grp[j] = 0;
+            row[j] = acc[j] = grp[j] = 0;
             w[j] = c.x(o);
             ws[j] = swap2(w[j]);
             o = c.fwd(o);
@@ -244,34 +233,28 @@ __device__ __forceinline__ void sum_parts(MacCol<SH>& c, int n, int tg, int unit
 #pragma unroll
                 for (int j = 0; j < RB; ++j) {
                     const int q = (j - r + RB) % RB;
-                    acc[j] = TG4 && u == 0 ? fma2(ws[q], hi, mul2(w[q], hr)) : cmac2(acc[j], w[q], ws[q], hr, hi);
+                    acc[j] = cmac2(acc[j], w[q], ws[q], hr, hi);
                 }
                 const int q = (RB - 1 - r + RB) % RB;
                 w[q] = nx[u];
                 ws[q] = swap2(nx[u]);
-                if constexpr (!TG4) {
-                    --left;
-                    if (--run == 0 || left == 0 || i0 + r + 1 == n) {
-                        run = unit;
+                --left;
+                if (--run == 0 || left == 0 || i0 + r + 1 == n) {
+                    run = unit;
+#pragma unroll
+                    for (int j = 0; j < RB; ++j) {
+                        grp[j] = add2(grp[j], acc[j]);
+                        acc[j] = 0;
+                    }
+                    if (left == 0 || i0 + r + 1 == n) {
+                        left = tg;
 #pragma unroll
                         for (int j = 0; j < RB; ++j) {
-                            grp[j] = add2(grp[j], acc[j]);
-                            acc[j] = 0;
-                        }
-                        if (left == 0 || i0 + r + 1 == n) {
-                            left = tg;
-#pragma unroll
-                            for (int j = 0; j < RB; ++j) {
-                                row[j] = add2(row[j], grp[j]);
-                                grp[j] = 0;
-                            }
+                            row[j] = add2(row[j], grp[j]);
+                            grp[j] = 0;
                         }
                     }
                 }
-            }
-            if constexpr (TG4) {
-#pragma unroll
-                for (int j = 0; j < RB; ++j) row[j] = i0 + s == 0 ? acc[j] : add2(row[j], acc[j]);
             }
         }
     }
@@ -279,8 +262,8 @@ __device__ __forceinline__ void sum_parts(MacCol<SH>& c, int n, int tg, int unit
 
 // row[j] = sum of X_{b+j-p} H_p over the first n parts, one by one with each
 // product rounded before it is added (fire_multi's sum)
-template <int RB, bool SH>
-__device__ __forceinline__ void chain_parts(MacCol<SH> c, int n, float2 (&y)[RB]) {
+template <int RB>
+__device__ __forceinline__ void chain_parts(MacCol c, int n, float2 (&y)[RB]) {
 #pragma unroll
     for (int j = 0; j < RB; ++j) y[j] = make_float2(0.f, 0.f);
     for (int p = 0; p < n; ++p) {
@@ -298,20 +281,20 @@ __device__ __forceinline__ void chain_parts(MacCol<SH> c, int n, float2 (&y)[RB]
 
 // y = X_b H_0 + (X_{b-1} H_1 + rows) for the run's blocks, c at part 0 (first:
 // the run begins with block 0, before which there is silence)
-template <int RB, bool SH>
-__device__ __forceinline__ void finish_run(const MacCol<SH>& c, const WLevel& l, const f32x2 (&ys)[RB], float2* Y,
+template <int RB>
+__device__ __forceinline__ void finish_run(const MacCol& c, const WLevel& l, const f32x2 (&ys)[RB], float2* Y,
                                            int live, bool first = false) {
     const bool rows = l.P > l.p_lo, x1 = l.two && l.P >= 2;
     const float2 h0 = c.h();
-    const float2 h1 = x1 ? MacCol<SH>{c.H + c.cs, nullptr, 0, 0, 0}.h() : make_float2(0.f, 0.f);
+    const float2 h1 = x1 ? __ldg(c.H + c.cs) : make_float2(0.f, 0.f);
     float2 xm = x1 && !first ? unpack2(c.x(c.back(c.ox))) : make_float2(0.f, 0.f);
     int o = c.ox;
 #pragma unroll
     for (int j = 0; j < RB; ++j) {
         const float2 x = unpack2(c.x(o));
         float2 s = unpack2(ys[j]);
-        if (x1) s = rows ? cadd(cmul(xm, h1), s) : cmul(xm, h1);
-        const float2 y = cadd(cmul(x, h0), s);
+        if (x1) s = rows ? cadd(cmul(h1, xm), s) : cmul(h1, xm);
+        const float2 y = cadd(cmul(h0, x), s);
         if (j < live) Y[(size_t)j * l.cs] = y;
         xm = x;
         o = c.fwd(o);
@@ -330,12 +313,92 @@ __device__ __forceinline__ void cp_async_wait() {
     asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
 }
 
+// row[j] = sum of X_{b+j-p} H_p over n consecutive parts in groups of four, from
+// shared memory; x: the spectrum of the run's first block under the first of
+// them, h: that part's row.  The window of a run under one part (RB spectra and
+// their swapped pairs) stays in registers: the next part needs one new one.
+// Shared rows are kMacTile apart, so every row is at a constant offset.  The
+// loads of four parts go together (the one after the last part is not used: it
+// is the shared row before the oldest spectrum).
+template <int RB>
+__device__ __forceinline__ void sum_groups(const f32x2* x, const float2* h, int n, f32x2 (&row)[RB]) {
+    constexpr int U = 4, W = kMacTile;
+    static_assert(RB % U == 0, "constant window rotation");
+    f32x2 w[RB], ws[RB];   // the block of run index j under part r at w[(j - r) mod RB]
+#pragma unroll
+    for (int j = 0; j < RB; ++j) {
+        w[j] = x[j * W];
+        ws[j] = swap2(w[j]);
+    }
+    for (int i0 = 0; i0 < n; i0 += RB, x -= RB * W, h += RB * W) {
+#pragma unroll
+        for (int s = 0; s < RB; s += U) {
+            if (i0 + s >= n) break;
+            float2 hv[U];
+            f32x2 nx[U], acc[RB];
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (i0 + s + u < n) {
+                    hv[u] = h[(s + u) * W];
+                    nx[u] = x[-(s + u + 1) * W];
+                }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                if (i0 + s + u >= n) break;
+                const f32x2 hr = pack2(hv[u].x, hv[u].x), hi = pack2(-hv[u].y, hv[u].y);
+#pragma unroll
+                for (int j = 0; j < RB; ++j) {
+                    const int q = (j + RB - s - u) % RB;
+                    acc[j] = u == 0 ? fma2(ws[q], hi, mul2(w[q], hr)) : cmac2(acc[j], w[q], ws[q], hr, hi);
+                }
+                const int q = RB - 1 - s - u;
+                w[q] = nx[u];
+                ws[q] = swap2(nx[u]);
+            }
+#pragma unroll
+            for (int j = 0; j < RB; ++j) row[j] = i0 + s == 0 ? acc[j] : add2(row[j], acc[j]);
+        }
+    }
+}
+
+// Y = X_b H_0 + (X_{b-1} H_1 + row) for the run, X_{b-1} H_1 with x1 and the row
+// with rows; x, h: the shared rows of the run's first block and of part 0.
+// Products as cmul(H, X).
+template <int RB>
+__device__ __forceinline__ void mac_finish(const f32x2* x, const float2* h, bool x1, bool rows, const f32x2 (&row)[RB],
+                                           float2* Y, int cs, int live) {
+    constexpr int W = kMacTile;
+    const float2 h0 = h[0], h1 = x1 ? h[W] : make_float2(0.f, 0.f);
+    const f32x2 hr0 = pack2(h0.x, h0.x), hi0 = pack2(-h0.y, h0.y), hr1 = pack2(h1.x, h1.x), hi1 = pack2(-h1.y, h1.y);
+    f32x2 xm = x1 ? x[-W] : 0, xms = swap2(xm);
+    f32x2* y = reinterpret_cast<f32x2*>(Y);
+#pragma unroll
+    for (int j = 0; j < RB; ++j) {
+        const f32x2 xj = x[j * W], xs = swap2(xj);
+        f32x2 s = row[j];
+        if (x1) {
+            const f32x2 m1 = fma2(xm, hr1, mul2(xms, hi1));
+            s = rows ? add2(m1, s) : m1;
+        }
+        if (j < live) y[(size_t)j * cs] = add2(fma2(xj, hr0, mul2(xs, hi0)), s);
+        xm = xj;
+        xms = xs;
+    }
+}
+
 // The default tiles: a CTA takes a tile of at most kMacTile bins of one level
-// through a segment of blocks, kWideRun at a time, from shared memory.  With
-// at most kMacRes parts the filter rows of the tile stay there for the whole
-// segment and each spectrum row is copied in once, a run ahead of its use;
-// with more, every run takes the parts a partial-sum row at a time.
-__global__ void __launch_bounds__(kMacTile) wide_mac_kernel(const int4* __restrict__ map, WArgs a) {
+// through a segment of kMacSeg blocks, kWideRun at a time, from shared memory.
+// With at most kMacRes parts the filter rows of the tile stay there, and the
+// segment's spectra with the P - 1 before them (up to 14 parts all 32, then 24)
+// are all on their way before the first run is waited for; with more, every run
+// takes the parts a partial-sum row at a time.
+// Bound: issue slots; half of the instructions are the packed products.  32
+// streams of 2^18 samples (14 | 14 | 1 .. 31 parts, 300 M products, 201 MB of
+// spectra in and out): 154 us with rows in a ring of shared memory walked with
+// wrapped offsets and the first two parts one float at a time, 138 us with
+// constant offsets and packed ends.  Four CTAs per SM with 152 registers a
+// thread beat five with 128 (424 against 432 us for the call).
+__global__ void __launch_bounds__(kMacTile, 4) wide_mac_kernel(const int4* __restrict__ map, WArgs a) {
     constexpr int RB = kWideRun, W = kMacTile;
     extern __shared__ float4 dyn_smem[];
     cudaTriggerProgrammaticLaunchCompletion();
@@ -354,85 +417,94 @@ __global__ void __launch_bounds__(kMacTile) wide_mac_kernel(const int4* __restri
     float2* Y = wide_at(l.Yw, a.rel) + k0 + tid;
     int sl = wmod(bf, R) + e.z;   // ring row of block e.z of the chunk
     if (sl >= R) sl -= R;
-    // rows [0, n) of the filter / of blocks starting at ring row s, to shared rows dst + ((p + i) mod m) W
+    float2* Hs = reinterpret_cast<float2*>(dyn_smem);
+    // filter rows [p, p + n) to shared rows dst ..
     auto copy_h = [&](float2* dst, int p, int n) {
         if (lc < w2)
             for (int i = lr; i < n; i += 2) cp_async16(dst + i * W + 2 * lc, Hg + (size_t)(p + i) * cs + 2 * lc);
     };
-    // (nz: rows that lie before block 0, zero)
-    auto copy_x = [&](float2* dst, int p, int m, int s, int n, int nz) {
+    // ring rows s + i (mod R), i0 <= i < i1, to shared rows dst + i; zeros for i < nz (blocks before 0)
+    auto copy_x = [&](float2* dst, int s, int i0, int i1, int nz) {
         if (s < 0) s += R;
-        if (s >= R) s -= R;
         if (lc < w2)
-            for (int i = lr; i < n; i += 2) {
-                int r = s + i;
-                if (r >= R) r -= R;
-                int q = p + i;
-                if (q >= m) q -= m;
-                cp_async16(dst + q * W + 2 * lc, Xg + (size_t)r * cs + 2 * lc, i >= nz);
+            for (int i = i0 + lr; i < i1; i += 2) {
+                const int r = s + i;
+                cp_async16(dst + i * W + 2 * lc, Xg + (size_t)(r >= R ? r - R : r) * cs + 2 * lc, i >= nz);
             }
     };
-    float2* Hs = reinterpret_cast<float2*>(dyn_smem);
-    f32x2 ys[RB];
     if (P <= kMacRes) {
-        float2* Xs = Hs + kMacRes * W;
-        const int RX = P - 1 + 2 * RB;   // ring rows: the history of a run, the run, the next run
+        float2* Xs = Hs + P * W;
+        const int hist = P - 1;
+        const int S = min(kMacSeg, (kMacRows - P - hist) & -RB);   // blocks whose spectra fit
         copy_h(Hs, 0, P);
-        copy_x(Xs, 0, RX, sl - (P - 1), P - 1 + RB, (int)max(0LL, P - 1 - (bf + e.z)));
-        cp_async_commit();
-        int pos = P - 1;                 // shared row of the run's first block
-        for (int i0 = e.z; i0 < nb; i0 += RB) {
-            if (i0 + RB < nb) {
-                int q = pos + RB;
-                if (q >= RX) q -= RX;
-                copy_x(Xs, q, RX, sl + RB, RB, 0);
-            }
-            cp_async_commit();
-            cp_async_wait<1>();
-            __syncthreads();
-            if (live) {
-                MacCol<true> c{Hs + l.p_lo * W + tid, Xs + tid, W, RX * W, 0};
-                int q = pos - l.p_lo;
-                c.ox = (q < 0 ? q + RX : q) * W;
+        for (int s0 = e.z; s0 < nb; s0 += S) {
+            const int n = min(S, nb - s0);
+            const int nz = (int)max(0LL, hist - (bf + s0));
+            if (s0 > e.z) __syncthreads();   // the rows before are still being read
 #pragma unroll
-                for (int j = 0; j < RB; ++j) ys[j] = 0;
-                if (P > l.p_lo) sum_parts<RB, true>(c, P - l.p_lo, 4, 4, ys);
-                c.H = Hs + tid;
-                c.ox = pos * W;
-                finish_run(c, l, ys, Y + (size_t)i0 * cs, nb - i0);
+            for (int g = 0; g < kMacSeg / RB; ++g) {
+                copy_x(Xs, sl - hist, g == 0 ? 0 : hist + g * RB, hist + min((g + 1) * RB, n), nz);
+                cp_async_commit();
             }
-            __syncthreads();   // the next run's copies overwrite rows read here
-            pos += RB;
-            if (pos >= RX) pos -= RX;
-            sl += RB;
+            const f32x2* x = reinterpret_cast<const f32x2*>(Xs + hist * W) + tid;
+            float2* y = Y + (size_t)s0 * cs;
+            for (int i = 0; i < n; i += RB, x += RB * W, y += (size_t)RB * cs) {
+                switch (i / RB) {   // the copies of the later runs may be under way
+                    case 0: cp_async_wait<kMacSeg / RB - 1>(); break;
+                    case 1: cp_async_wait<kMacSeg / RB - 2>(); break;
+                    case 2: cp_async_wait<kMacSeg / RB - 3>(); break;
+                    default: cp_async_wait<0>();
+                }
+                __syncthreads();
+                if (!live) continue;
+                f32x2 row[RB];
+#pragma unroll
+                for (int j = 0; j < RB; ++j) row[j] = 0;
+                if (P > l.p_lo) sum_groups<RB>(x - l.p_lo * W, Hs + tid + l.p_lo * W, P - l.p_lo, row);
+                mac_finish<RB>(x, Hs + tid, l.two && P > 1, P > l.p_lo, row, y, cs, n - i);
+            }
+            sl += S;
             if (sl >= R) sl -= R;
         }
         return;
     }
-    constexpr int TP = kMacRes - 2;      // parts per partial-sum row at most
-    float2* Xs = Hs + TP * W;
+    // shared rows: filter rows 0 and 1, the run's spectra and the one before them,
+    // its partial sums so far, then the row of parts at hand
+    constexpr int XH = 2, YS = XH + 1 + RB, HS = YS + RB;
+    static_assert(HS + 2 * (kMacRes - 2) - 1 + RB <= kMacRows, "a partial-sum row's parts");
+    f32x2* ys = reinterpret_cast<f32x2*>(Hs + YS * W) + tid;
     for (int i0 = e.z; i0 < nb; i0 += RB) {
         for (int q = 0; q < l.nrows; ++q) {
             const int pb = l.p_lo + q * l.tp, n = min(l.tp, P - pb);
-            // blocks (run's first) - pb - n .. (run's first) - pb + RB - 1
-            copy_h(Hs, pb, n);
+            float2* Xs = Hs + (HS + n) * W;
+            if (q == 0) {
+                if (i0 == e.z) copy_h(Hs, 0, 2);
+                copy_x(Hs + XH * W, sl - 1, 0, 1 + min(RB, nb - i0), bf + i0 == 0 ? 1 : 0);
+            }
+            // blocks (run's first) - pb - (n - 1) .. (run's first) - pb + RB - 1
+            copy_h(Hs + HS * W, pb, n);
             // (before block 0 only in the first blocks of all: the ring holds no more than R of them)
-            copy_x(Xs, 0, TP + RB, sl - pb - n, n + RB, (int)max(0LL, pb + n - (bf + i0)));
+            copy_x(Xs, sl - pb - (n - 1), 0, n - 1 + RB, (int)max(0LL, pb + n - 1 - (bf + i0)));
             cp_async_commit();
             cp_async_wait<0>();
             __syncthreads();
             if (live) {
                 f32x2 row[RB];
-                MacCol<true> c{Hs + tid, Xs + tid, W, (TP + RB) * W, n * W};
-                sum_parts<RB, true>(c, n, 4, 4, row);
+                sum_groups<RB>(reinterpret_cast<const f32x2*>(Xs + (n - 1) * W) + tid, Hs + HS * W + tid, n, row);
+                if (q > 0) {
 #pragma unroll
-                for (int j = 0; j < RB; ++j) ys[j] = q == 0 ? row[j] : add2(ys[j], row[j]);
+                    for (int j = 0; j < RB; ++j) row[j] = add2(ys[j * W], row[j]);
+                }
+                if (q + 1 < l.nrows) {
+#pragma unroll
+                    for (int j = 0; j < RB; ++j) ys[j * W] = row[j];
+                } else {
+                    mac_finish<RB>(reinterpret_cast<const f32x2*>(Hs + (XH + 1) * W) + tid, Hs + tid, l.two, true, row,
+                                   Y + (size_t)i0 * cs, cs, nb - i0);
+                }
             }
             __syncthreads();
         }
-        if (live)
-            finish_run(MacCol<false>{Hg + tid, Xg + tid, cs, R * cs, sl * cs}, l, ys, Y + (size_t)i0 * cs, nb - i0,
-                       bf + i0 == 0);
         sl += RB;
         if (sl >= R) sl -= R;
     }
@@ -455,7 +527,7 @@ __global__ void __launch_bounds__(kMacAnyNT, 3) wide_mac_any_kernel(const int4* 
     if (i0 >= nb) return;
     int sl = wmod(bf, R) + i0;   // ring row of the run's first block
     if (sl >= R) sl -= R;
-    MacCol<false> c{l.H + (size_t)l.p_lo * cs + k, l.X + k, cs, R * cs, 0};
+    MacCol c{l.H + (size_t)l.p_lo * cs + k, l.X + k, cs, R * cs, 0};
     f32x2 ys[RB];   // partial-sum rows of the parts >= p_lo
 #pragma unroll
     for (int j = 0; j < RB; ++j) ys[j] = 0;
@@ -465,7 +537,7 @@ __global__ void __launch_bounds__(kMacAnyNT, 3) wide_mac_any_kernel(const int4* 
         c.ox = (o < 0 ? o + R : o) * cs;
         for (int q = 0; q < l.nrows; ++q) {
             f32x2 row[RB];
-            sum_parts<RB, false>(c, min(l.tp, P - l.p_lo - q * l.tp), l.tpg, l.multi ? 2 : 4, row);
+            sum_parts<RB>(c, min(l.tp, P - l.p_lo - q * l.tp), l.tpg, l.multi ? 2 : 4, row);
 #pragma unroll
             for (int j = 0; j < RB; ++j) ys[j] = q == 0 ? row[j] : add2(ys[j], row[j]);
         }
@@ -774,8 +846,9 @@ cudaError_t launch_wide_out(int N0, int grid, const int2* map, const WArgs& a, c
     return grid > 0 ? by_log(N0, WideOut{grid, map, a, st}) : cudaSuccess;
 }
 
-// filter rows and ring of a tile (the staged form needs less)
-constexpr size_t kMacSmem = sizeof(float2) * kMacTile * (size_t)(kMacRes + kMacRes - 1 + 2 * kWideRun);
+constexpr size_t kMacSmem = sizeof(float2) * kMacTile * (size_t)kMacRows;
+static_assert(kMacSeg == 4 * kWideRun, "four groups of copies");
+static_assert(kMacRows >= 2 * kMacRes - 1 + kWideRun, "a run of the longest resident level");
 
 cudaError_t launch_wide_mac(bool any, int grid, const int4* map, const WArgs& a, cudaStream_t st) {
     if (grid <= 0) return cudaSuccess;

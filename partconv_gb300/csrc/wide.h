@@ -52,7 +52,8 @@ __host__ __device__ __forceinline__ T* wide_at(T* p, long long rel) {
 constexpr int kWideRun = 8;       // consecutive blocks a thread of the sum over parts takes together
 constexpr int kMacTile = 96;      // bins per CTA of the sum over parts (three warps: 258 bins are three tiles of 86)
 constexpr int kMacSeg = 32;       // ... and blocks
-constexpr int kMacRes = 18;       // most parts whose filter rows stay in shared memory (the default 16 per row and 2)
+constexpr int kMacRes = 18;       // most parts whose filter rows stay in shared memory (16 of a partial-sum row and 2)
+constexpr int kMacRows = 59;      // shared rows of a tile (45 KB; registers admit four CTAs per SM)
 constexpr int kMacAnyNT = 128;    // threads of the general form
 
 // CTA maps: (level, first block of the chunk) for the transforms; for the sum
