@@ -43,6 +43,14 @@ constexpr int kWideMinSteps = 4;
 // the summed spectra, as many again, are still in the 129 MB L2 when the next
 // kernel reads them.
 constexpr size_t kWideBytes = (size_t)256 << 20;
+// Interleaved input is brought to rows of one channel each from this many
+// inputs on and for this many samples of a chunk: the pass costs 3 to 8 us and
+// saves the transforms' strided reads (blocks of 256 | 2048, 2^18 frames,
+// without and with it: 2 inputs 63.6 and 64.4, 3 inputs 66.6 and 68.0, 4 inputs
+// 81.2 and 77.5, 8 inputs 128 and 118, 32 inputs 478 and 376 us; 10240 frames:
+// 4 inputs 42.1 and 43.5, 8 inputs 46.6 and 45.4 us).
+constexpr int kPlanarInputs = 4;
+constexpr long long kPlanarSamples = 1 << 16;
 constexpr int kWideMinChunk = 32, kWideMaxChunk = 4096;
 constexpr int kMinN0 = 16;
 constexpr int kClasses = kNumClasses;
@@ -208,6 +216,8 @@ struct pc_handle {
     const WLevel* d_wlv = nullptr;
     const float2* d_wtab = nullptr;
     const int* d_lv0 = nullptr;    // level-0 index of every PC
+    float* d_planar = nullptr;     // from kPlanarInputs on: a chunk's interleaved samples by channel
+    long long planar_pitch = 0;
     int n_zero = 0, max_ring = 0;
     bool wide_ok = true;           // every ring's element offsets fit 32 bits
     bool mixed = false;
@@ -975,6 +985,11 @@ int do_setup(pc_handle* h, int fs, int buffer_size, int n_in, int n_out, std::ve
         off_Yw[li] = cv.take(sizeof(float2) * (size_t)((h->C + h->h_lv[li].T - 1) / h->h_lv[li].T) * h->h_lv[li].cs);
     for (int i = 0; i < npc; ++i)
         if (h->h_pcs[i].mix_mode == 2) off_pcw[i] = cv.take(sizeof(float) * (size_t)h->C * N0);
+    // a chunk's interleaved input by channel, with the samples that its windows reach back to
+    h->planar_pitch = (long long)h->C * N0;
+    for (int li = 0; li < nlv; ++li)
+        h->planar_pitch = std::max(h->planar_pitch, (long long)h->C * N0 + 2LL * h->h_lv[li].N);
+    const size_t off_planar = h->n_in >= kPlanarInputs ? cv.take(sizeof(float) * h->n_in * (size_t)h->planar_pitch) : 0;
     WideMaps wm;
     build_wide_maps(h, wm);
     const size_t off_wmap = cv.take(wm.bytes());
@@ -1085,6 +1100,7 @@ int do_setup(pc_handle* h, int fs, int buffer_size, int n_in, int n_out, std::ve
            "upload levels");
         h->d_wlv = reinterpret_cast<const WLevel*>(A + off_wlv);
         h->d_lv0 = reinterpret_cast<const int*>(A + off_lv0);
+        h->d_planar = h->n_in >= kPlanarInputs ? reinterpret_cast<float*>(A + off_planar) : nullptr;
         h->d_wtab = reinterpret_cast<const float2*>(A + off_wtab);
         CK(wm.place(h, A + off_wmap), "upload maps");
         CK(launch_wide_reset(h->d_wlv, nlv, A + h->state_off, h->state_bytes, h->stream), "clear state");
@@ -1244,10 +1260,25 @@ IOView make_view(const pc_handle* h, const float* in, float* out, long long fram
 int run_chunk(pc_handle* h, const IOView& view, int n, cudaStream_t st) {
     WArgs a = wide_args(h, view, n);
     auto grid = [n](const pc_handle::WMap& m) { return m.upto[n - 1]; };
-    CK(launch_wide_cluster(false, grid(h->w_cl), h->w_cl.map, a, st), "window transforms");
+    WArgs ai = a;   // the window transforms' view of the input
+    if (h->d_planar && view.in_ch == 1 && view.in_sample > 1 && (long long)n * h->N0 * h->n_in >= kPlanarSamples) {
+        // rows from the call's first sample, or as far back as the chunk's windows reach
+        const long long t0 = h->frame_num * (long long)h->N0, t_in0 = view.step0 * (long long)h->N0;
+        const long long len = (long long)n * h->N0, back = std::min(t0 - t_in0, h->planar_pitch - (long long)h->C * h->N0);
+        const long long first = t0 - back - t_in0;
+        CK(launch_wide_planar(view.in + first * view.in_sample, h->d_planar, h->n_in, h->planar_pitch, back + len, st),
+           "input by channel");
+        h->launches += 1;
+        IOView v = view;
+        v.in = reinterpret_cast<const float*>(reinterpret_cast<uintptr_t>(h->d_planar) - sizeof(float) * (uintptr_t)first);
+        v.in_sample = 1;
+        v.in_ch = h->planar_pitch;
+        ai = wide_args(h, v, n);
+    }
+    CK(launch_wide_cluster(false, grid(h->w_cl), h->w_cl.map, ai, st), "window transforms");
     const int g0 = n >= h->w_split ? 1 : 0, g1 = g0 ? 3 : 1;
     for (int g = g0; g < g1; ++g) {
-        CK(launch_wide_fft(false, h->w_nt[g], grid(h->w_fwd[g]), h->w_fwd[g].map, a, st), "window transforms");
+        CK(launch_wide_fft(false, h->w_nt[g], grid(h->w_fwd[g]), h->w_fwd[g].map, ai, st), "window transforms");
         h->launches += (grid(h->w_fwd[g]) > 0) + (grid(h->w_inv[g]) > 0);
     }
     for (int x = 0; x < 2; ++x) {

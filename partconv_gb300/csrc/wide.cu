@@ -684,6 +684,43 @@ __global__ void __launch_bounds__(out_threads(LOGN)) wide_out_kernel(const int2*
     ifft_body<LOGN, out_threads(LOGN), true, FULL>(l, e.y, a, reinterpret_cast<float2*>(dyn_smem));
 }
 
+// 0. interleaved input, frames of C samples, to rows of one channel each
+// (pitch apart).  Each channel is read by every level of every PC on it, twice
+// per window; from the interleaved frames those reads touch C times the memory
+// they use.  A tile of up to 32 channels, 1024 samples at most, goes through
+// shared memory.  Bound: the latency of one load and one store (6 inputs,
+// 128128 frames: 3 us; the transforms of 12 paths after it 24 us instead of
+// 37).
+__host__ __device__ constexpr int planar_frames(int cw) { return 1024 / cw & ~31; }
+__global__ void __launch_bounds__(256) wide_planar_kernel(const float* __restrict__ in, float* __restrict__ out, int C,
+                                                          long long pitch, long long frames) {
+    __shared__ float tile[1024 + 1024 / 2];   // frames cw | 1 apart
+    cudaTriggerProgrammaticLaunchCompletion();
+    cudaGridDependencySynchronize();
+    const int c0 = blockIdx.y * 32, cw = min(32, C - c0), F = planar_frames(min(32, C)), ld = cw | 1;
+    const long long f0 = (long long)blockIdx.x * F;
+    const int nf = (int)min((long long)F, frames - f0);
+    const float* src = in + f0 * C + c0;
+    float* dst = out + c0 * pitch + f0;
+    float v[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        const int i = threadIdx.x + u * 256, f = i / cw, c = i - f * cw;
+        if (f < nf) v[u] = __ldg(src + (long long)f * C + c);
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        const int i = threadIdx.x + u * 256, f = i / cw, c = i - f * cw;
+        if (f < nf) tile[f * ld + c] = v[u];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        const int i = threadIdx.x + u * 256, c = i / F, f = i - c * F;
+        if (c < cw && f < nf) dst[c * pitch + f] = tile[f * ld + c];
+    }
+}
+
 // 4. outputs fed by several PCs (summed in PC order) and outputs without any
 __global__ void wide_mix_kernel(Bank bank, int n_zero, int mixed, WArgs a) {
     cudaTriggerProgrammaticLaunchCompletion();
@@ -731,7 +768,7 @@ __global__ void wide_reset_kernel(const WLevel* __restrict__ lv, int nlv, float4
 
 // launch that may overlap the previous kernel's tail (see above)
 template <class... KA, class... A>
-cudaError_t launch_dep(void (*k)(KA...), int grid, int nt, size_t smem, cudaStream_t st, A&&... args) {
+cudaError_t launch_dep(void (*k)(KA...), dim3 grid, int nt, size_t smem, cudaStream_t st, A&&... args) {
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
@@ -859,6 +896,13 @@ cudaError_t launch_wide_mac(bool any, int grid, const int4* map, const WArgs& a,
 cudaError_t launch_wide_mix(const Bank& bank, int n_zero, bool mixed, const WArgs& a, cudaStream_t st) {
     const int len = a.nsteps * a.N0;
     return launch_dep(wide_mix_kernel, (len + 255) / 256, 256, 0, st, bank, n_zero, mixed ? 1 : 0, a);
+}
+
+cudaError_t launch_wide_planar(const float* in, float* out, int channels, long long pitch, long long frames,
+                               cudaStream_t st) {
+    const int F = planar_frames(std::min(32, channels));
+    return launch_dep(wide_planar_kernel, dim3((unsigned)((frames + F - 1) / F), (unsigned)((channels + 31) / 32)), 256, 0,
+                      st, in, out, channels, pitch, frames);
 }
 
 cudaError_t launch_wide_reset(const WLevel* lv, int nlv, void* state, size_t bytes, cudaStream_t st) {

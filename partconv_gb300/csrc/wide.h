@@ -60,6 +60,9 @@ constexpr int kMacAnyNT = 128;    // threads of the general form
 // over parts (level, first bin, first block, end block) of a tile and segment,
 // or (level, first of kMacAnyNT (run, bin) items) in the general form.
 cudaError_t prepare_wide_kernels();
+// frames of interleaved samples (at least two channels) to rows pitch apart
+cudaError_t launch_wide_planar(const float* in, float* out, int channels, long long pitch, long long frames,
+                               cudaStream_t st);
 // threads per CTA of the transform kernels for blocks up to max_n (a CTA runs
 // 16 threads / N transforms), and blocks per CTA of wide_out
 int wide_threads(int max_n);
