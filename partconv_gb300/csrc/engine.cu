@@ -1113,9 +1113,9 @@ int do_setup(pc_handle* h, int fs, int buffer_size, int n_in, int n_out, std::ve
         const std::vector<float2>& W = host_twiddles(kWlog);
         CK(cudaMemcpyAsync(A + off_W, W.data(), sizeof(float2) * W.size(), cudaMemcpyHostToDevice, h->stream),
            "upload twiddles");
-        const std::vector<float2>& tab = host_fft_tables();
-        CK(cudaMemcpyAsync(A + off_wtab, tab.data(), sizeof(float2) * tab.size(), cudaMemcpyHostToDevice, h->stream),
-           "upload twiddles");
+        CK(launch_fft_tables(reinterpret_cast<float2*>(A + off_wtab), reinterpret_cast<const float2*>(A + off_W), kWlog,
+                             h->stream),
+           "transform factors");
         CK(cudaStreamSynchronize(h->stream), "sync");
     }
     CK(cudaMemcpyAsync(A + off_pcs, h->h_pcs.data(), sizeof(DevPC) * npc, cudaMemcpyHostToDevice, h->stream),

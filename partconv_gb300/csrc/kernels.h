@@ -23,6 +23,8 @@ struct SpectraJob {
 // transform tables of fft_reg.cuh; computed once per process
 const std::vector<float2>& host_twiddles(int wlog);
 const std::vector<float2>& host_fft_tables();
+// the same tables from the twiddles on the device (about 5 us; their upload takes 60)
+cudaError_t launch_fft_tables(float2* tab, const float2* W, int wlog, cudaStream_t st);
 
 // kernel class by block size: 0 (N <= 1024), 1 (N <= 4096), 2 (N <= 16384),
 // 3 (N <= 65536: a cluster of kClusterCtas CTAs per fire, cluster_fire.cu)

@@ -888,12 +888,11 @@ int setup_wide(pcm_handle* h) {
         }
         return put(flat.data(), sizeof(E) * flat.size());
     };
-    size_t at[7];
+    size_t at[6];
     for (int m = 0; m < 3; ++m) at[m] = put_map(e[m], h->w_upto[m]);
     at[3] = put_map(mac, h->w_upto[3]);
     at[4] = put(wl.data(), sizeof(WLevel) * wl.size());
     at[5] = put(lv0.data(), sizeof(int) * lv0.size());
-    at[6] = put(host_fft_tables().data(), sizeof(float2) * host_fft_tables().size());
     char* d = nullptr;
     MCK(cudaMalloc(&d, blob.size()), "alloc tables");
     h->allocs.push_back(d);
@@ -904,7 +903,6 @@ int setup_wide(pcm_handle* h) {
     h->w_mac = reinterpret_cast<const int4*>(d + at[3]);
     h->d_wlv = reinterpret_cast<const WLevel*>(d + at[4]);
     h->d_lv0 = reinterpret_cast<const int*>(d + at[5]);
-    h->d_tab = reinterpret_cast<const float2*>(d + at[6]);
     MCK(launch_wide_reset(h->d_wlv, h->n_wlv, nullptr, 0, h->stream), "clear rings");
     return PC_OK;
 }
@@ -1030,6 +1028,10 @@ int pcm_setup(pcm_handle* h, int fs, int buffer_size, int n_in, int n_out, int M
         MCK(malloc_zero(h, &W, Wh.size(), false), "alloc");
         MCK(cudaMemcpyAsync(W, Wh.data(), sizeof(float2) * Wh.size(), cudaMemcpyHostToDevice, h->stream), "upload");
         MCK(cudaStreamSynchronize(h->stream), "sync");
+        float2* tab = nullptr;
+        MCK(malloc_raw(h, &tab, kFftTabEntries), "alloc");
+        MCK(launch_fft_tables(tab, W, kWlog, h->stream), "transform factors");
+        h->d_tab = tab;
         MCK(prepare_wide_kernels(), "kernel attributes");
         MCK(cudaFuncSetAttribute(mimo_wide_mac_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)sizeof(WideMacSmem)),

@@ -835,6 +835,14 @@ const std::vector<float2>& host_fft_tables() {
     return t;
 }
 
+static __global__ void fft_tables_kernel(float2* tab, const float2* W, int wlog) {
+    fill_fft_tables(tab, W, wlog, kRegMaxLog, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
+}
+cudaError_t launch_fft_tables(float2* tab, const float2* W, int wlog, cudaStream_t st) {
+    fft_tables_kernel<<<32, 256, 0, st>>>(tab, W, wlog);
+    return cudaGetLastError();
+}
+
 cudaError_t prepare_wide_kernels() {
     cudaError_t e = allow_smem(wide_fft_kernel<1024, false>, 1024);
     if (e == cudaSuccess) e = allow_smem(wide_fft_kernel<1024, true>, 1024);
