@@ -60,16 +60,16 @@ struct Geo {
 };
 
 // Forward column pass over this CTA's share of columns: 8-point DFTs over
-// the CTAs, twiddle w_n^(j2 k1), results back in place.  Ends with a
-// cluster barrier.
-__device__ void column_pass_fwd(const Geo& g, float2* const* rem, cg::cluster_group& cl) {
+// the CTAs, twiddle w_n^(j2 k1), results in place in every CTA; load(j2, v): the
+// column's points.  Ends with a cluster barrier.
+template <class Load>
+__device__ __forceinline__ void column_pass_fwd_from(const Geo& g, float2* const* rem, cg::cluster_group& cl, Load&& load) {
     const int cols = g.m / kC;
     for (int c = threadIdx.x; c < cols; c += kNT) {
         const int j2 = g.rank * cols + c;
         const int p = sidx<true>(j2);
         float2 v[8];
-#pragma unroll
-        for (int r = 0; r < 8; ++r) v[r] = rem[r][p];
+        load(j2, v);
         dft8(v, false);
 #pragma unroll
         for (int k1 = 1; k1 < 8; ++k1) v[k1] = cmul(v[k1], g.wn((long long)j2 * k1));
@@ -79,9 +79,18 @@ __device__ void column_pass_fwd(const Geo& g, float2* const* rem, cg::cluster_gr
     cl.sync();
 }
 
+__device__ void column_pass_fwd(const Geo& g, float2* const* rem, cg::cluster_group& cl) {
+    column_pass_fwd_from(g, rem, cl, [&](int j2, float2 (&v)[8]) {
+        const int p = sidx<true>(j2);
+#pragma unroll
+        for (int r = 0; r < 8; ++r) v[r] = rem[r][p];
+    });
+}
+
 // Inverse column pass: conj(w_n^(k1 j2)) then the inverse 8-point DFT over
-// k1; output index j2 + m j1 goes to CTA j1.  Ends with a cluster barrier.
-__device__ void column_pass_inv(const Geo& g, float2* const* rem, cg::cluster_group& cl) {
+// k1; store(j2, v): v[j1] is output j2 + m j1.
+template <class Store>
+__device__ __forceinline__ void column_pass_inv_to(const Geo& g, float2* const* rem, Store&& store) {
     const int cols = g.m / kC;
     for (int c = threadIdx.x; c < cols; c += kNT) {
         const int j2 = g.rank * cols + c;
@@ -92,9 +101,16 @@ __device__ void column_pass_inv(const Geo& g, float2* const* rem, cg::cluster_gr
 #pragma unroll
         for (int k1 = 1; k1 < 8; ++k1) v[k1] = cmul(v[k1], cconj(g.wn((long long)j2 * k1)));
         dft8(v, true);
+        store(j2, v);
+    }
+}
+// every output to its CTA j1; ends with a cluster barrier
+__device__ void column_pass_inv(const Geo& g, float2* const* rem, cg::cluster_group& cl) {
+    column_pass_inv_to(g, rem, [&](int j2, const float2 (&v)[8]) {
+        const int p = sidx<true>(j2);
 #pragma unroll
         for (int j1 = 0; j1 < 8; ++j1) rem[j1][p] = v[j1];
-    }
+    });
     cl.sync();
 }
 
@@ -289,7 +305,12 @@ __global__ void __cluster_dims__(kC, 1, 1) __launch_bounds__(kNT)
 // Block-parallel processing (wide.cu): the forward half of a fire -- window,
 // transform, spectrum row -- or its inverse half -- summed spectrum, inverse
 // transform, output ring -- of one block per cluster, with the operations of
-// cluster_fire_kernel in the same order.
+// cluster_fire_kernel in the same order.  The columns come straight from the
+// input and go straight to the output ring; only the passes between them go
+// through the cluster's shared memory.  Bound: the latency of the cluster
+// barriers and of the loads between them, one CTA per SM (two channels of
+// 200000 frames, blocks up to 65536, the call: 227 us with the window staged in
+// shared memory first and the block collected there last, 219 us so).
 template <bool INV>
 __global__ void __cluster_dims__(kC, 1, 1) __launch_bounds__(kNT)
     wide_cluster_kernel(const int2* __restrict__ map, WArgs a) {
@@ -319,19 +340,23 @@ __global__ void __cluster_dims__(kC, 1, 1) __launch_bounds__(kNT)
         const long long w0 = t_end - 2LL * N, t_in0 = a.io.step0 * (long long)a.N0;
         const float* in = a.io.in + (long long)l.in_ch * a.io.in_ch;
         const long long isamp = a.io.in_sample;
-        for (int j2 = tid; j2 < g.m; j2 += kNT) {
-            const long long ta = w0 + 2LL * (g.rank * (long long)g.m + j2);
-            float2 v;
-            if (ta >= t_in0) {
-                const float* p = in + (ta - t_in0) * isamp;
-                v = make_float2(p[0] * l.scale, p[isamp] * l.scale);
-            } else {
-                v = __ldcg(reinterpret_cast<const float2*>(l.xring + (ta & l.rin_mask)));
+        const bool vec = w0 >= t_in0 && a.vec_in;
+        cl.sync();   // every CTA of the cluster runs before its shared memory is written
+        column_pass_fwd_from(g, rem, cl, [&](int j2, float2 (&v)[8]) {
+#pragma unroll
+            for (int r = 0; r < 8; ++r) {
+                const long long ta = w0 + 2LL * (r * (long long)g.m + j2);
+                if (vec) {
+                    v[r] = __ldg(reinterpret_cast<const float2*>(in + (ta - t_in0)));
+                    v[r] = make_float2(v[r].x * l.scale, v[r].y * l.scale);
+                } else if (ta >= t_in0) {
+                    const float* p = in + (ta - t_in0) * isamp;
+                    v[r] = make_float2(p[0] * l.scale, p[isamp] * l.scale);
+                } else {
+                    v[r] = __ldcg(reinterpret_cast<const float2*>(l.xring + (ta & l.rin_mask)));
+                }
             }
-            S[sidx<true>(j2)] = v;
-        }
-        cl.sync();
-        column_pass_fwd(g, rem, cl);
+        });
         fft_smem<kNT, kMaxB, true>(S, g.m, g.logm, tw, false);
         cl.sync();
         float2* Xs = l.X + (size_t)(((b % l.slots) + l.slots) % l.slots) * l.cs;
@@ -359,12 +384,12 @@ __global__ void __cluster_dims__(kC, 1, 1) __launch_bounds__(kNT)
         cl.sync();
         fft_smem<kNT, kMaxB, true>(S, g.m, g.logm, tw, true);
         cl.sync();
-        column_pass_inv(g, rem, cl);
-        if (g.rank < kC / 2) {
-            const long long t0 = b * (long long)N + 2LL * g.rank * g.m;
-            for (int j2 = tid; j2 < g.m; j2 += kNT)
-                *reinterpret_cast<float2*>(l.yring + ((t0 + 2 * j2) & l.rmask)) = S[sidx<true>(j2)];
-        }
+        column_pass_inv_to(g, rem, [&](int j2, const float2 (&v)[8]) {
+#pragma unroll
+            for (int j1 = 0; j1 < kC / 2; ++j1)   // the block's samples are the first half
+                *reinterpret_cast<float2*>(l.yring + ((b * (long long)N + 2LL * (j1 * (long long)g.m + j2)) & l.rmask)) = v[j1];
+        });
+        cl.sync();   // no CTA leaves while others may still read its shared memory
     }
 }
 
