@@ -174,7 +174,8 @@ int pc_process(pc_handle* h, float* output, const float* input, long long frames
 int pc_process_device(pc_handle* h, float* d_output, const float* d_input, long long frames,
                       int layout, void* stream);
 
-/* PartConvMulti::reset() -- src/partconvMulti.cpp:806-813: clears all state. */
+/* PartConvMulti::reset() -- src/partconvMulti.cpp:806-813: clears all state,
+ * after the calls enqueued so far. */
 int pc_reset(pc_handle* h);
 
 /* PartConvMulti::cleanup() -- src/partconvMulti.cpp:720-804: frees device

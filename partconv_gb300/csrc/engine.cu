@@ -152,6 +152,7 @@ struct pc_handle {
     bool ready = false;
     int device = -1;
     cudaStream_t stream = nullptr;
+    cudaEvent_t used = nullptr;   // after the last call on a caller's stream
     cudaStream_t cin = nullptr, cout = nullptr;   // pc_process copy pipeline
 
     int fs = 0, N0 = 0, n_in = 0, n_out = 0;
@@ -272,6 +273,8 @@ void free_device(pc_handle* h) {
     if (h->cin) cudaStreamDestroy(h->cin);
     if (h->cout) cudaStreamDestroy(h->cout);
     h->cin = h->cout = nullptr;
+    if (h->used) cudaEventDestroy(h->used);
+    h->used = nullptr;
     if (h->stream) cudaStreamDestroy(h->stream);
     h->stream = nullptr;
     h->ready = false;
@@ -485,6 +488,7 @@ int do_setup(pc_handle* h, int fs, int buffer_size, int n_in, int n_out, std::ve
     int prio_least = 0, prio_greatest = 0;
     CK(cudaDeviceGetStreamPriorityRange(&prio_least, &prio_greatest), "priority range");
     CK(cudaStreamCreateWithPriority(&h->stream, cudaStreamNonBlocking, prio_greatest), "stream create");
+    CK(cudaEventCreateWithFlags(&h->used, cudaEventDisableTiming), "event create");
     CK(prepare_kernels(), "kernel attributes");
     CK(prepare_wide_kernels(), "kernel attributes");
 
@@ -1623,7 +1627,9 @@ int pc_process(pc_handle* h, float* output, const float* input, long long frames
 int pc_process_device(pc_handle* h, float* d_output, const float* d_input, long long frames, int layout,
                       void* stream) {
     if (!h) return PC_ERR_ARG;
-    return process_device_impl(h, d_output, d_input, frames, layout, (cudaStream_t)stream);
+    int r = process_device_impl(h, d_output, d_input, frames, layout, (cudaStream_t)stream);
+    if (r == PC_OK) CK(record_use(h->used, (cudaStream_t)stream), "event record");
+    return r;
 }
 
 int pc_reset(pc_handle* h) {
@@ -1631,6 +1637,7 @@ int pc_reset(pc_handle* h) {
     h->frame_num = 0;
     if (!h->ready) return PC_OK;
     CK(cudaSetDevice(h->device), "cudaSetDevice");
+    CK(cudaStreamWaitEvent(h->stream, h->used, 0), "reset");   // calls still running on a caller's stream
     CK(launch_wide_reset(h->d_wlv, (int)h->h_lv.size(), h->arena + h->state_off, h->state_bytes, h->stream), "reset");
     CK(cudaStreamSynchronize(h->stream), "reset sync");
     return PC_OK;

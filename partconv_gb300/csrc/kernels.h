@@ -23,6 +23,14 @@ struct SpectraJob {
 // transform tables of fft_reg.cuh; computed once per process
 const std::vector<float2>& host_twiddles(int wlog);
 const std::vector<float2>& host_fft_tables();
+// ev after the work enqueued on st so far, for a later reset on another stream
+// (not while st is being captured: the graph's work is the caller's to order)
+inline cudaError_t record_use(cudaEvent_t ev, cudaStream_t st) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    cudaError_t e = cudaStreamIsCapturing(st, &cs);
+    if (e == cudaSuccess && cs == cudaStreamCaptureStatusNone) e = cudaEventRecord(ev, st);
+    return e;
+}
 // the same tables from the twiddles on the device (about 5 us; their upload takes 60)
 cudaError_t launch_fft_tables(float2* tab, const float2* W, int wlog, cudaStream_t st);
 

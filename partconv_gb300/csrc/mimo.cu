@@ -704,6 +704,7 @@ struct pcm_handle {
     bool ready = false;
     int device = -1;
     cudaStream_t stream = nullptr;
+    cudaEvent_t used = nullptr;   // after the last call on a caller's stream
     int fs = 0, N0 = 0, nI = 0, nO = 0, M = 0, H = 1, maxN = 0, fft_cls = 0;
     std::vector<int> N, P;
     std::vector<void*> allocs;
@@ -775,6 +776,8 @@ void mfree(pcm_handle* h) {
     for (void* p : h->allocs) cudaFree(p);
     h->allocs.clear();
     h->state.clear();
+    if (h->used) cudaEventDestroy(h->used);
+    h->used = nullptr;
     if (h->stream) cudaStreamDestroy(h->stream);
     h->stream = nullptr;
     h->ready = false;
@@ -999,6 +1002,7 @@ int pcm_setup(pcm_handle* h, int fs, int buffer_size, int n_in, int n_out, int M
     for (int i = 0; i < M; ++i) P[i] = Pv[i];
     MCK(cudaGetDevice(&h->device), "cudaGetDevice");
     MCK(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking), "stream");
+    MCK(cudaEventCreateWithFlags(&h->used, cudaEventDisableTiming), "event");
     h->fs = fs;
     h->N0 = buffer_size;
     h->nI = n_in;
@@ -1286,13 +1290,18 @@ int pcm_process_device(pcm_handle* h, float* d_out, const float* d_in, long long
         rs.io.out_ch = 1;
     }
     const long long nsteps = frames / h->N0;
-    if (nsteps >= kWideMinSteps && h->wide_ok) return mimo_wide(h, rs.io, nsteps, st);
-    for (long long s = 0; s < nsteps; ++s) {
-        rs.step_base = h->frame_num + s;
-        int r = mimo_step(h, rs, st, s == 0, nullptr);
+    if (nsteps >= kWideMinSteps && h->wide_ok) {
+        int r = mimo_wide(h, rs.io, nsteps, st);
         if (r) return r;
+    } else {
+        for (long long s = 0; s < nsteps; ++s) {
+            rs.step_base = h->frame_num + s;
+            int r = mimo_step(h, rs, st, s == 0, nullptr);
+            if (r) return r;
+        }
+        h->frame_num += nsteps;
     }
-    h->frame_num += nsteps;
+    MCK(record_use(h->used, st), "event record");
     return PC_OK;
 }
 
@@ -1301,6 +1310,7 @@ int pcm_reset(pcm_handle* h) {
     h->frame_num = 0;
     if (!h->ready) return PC_OK;
     cudaSetDevice(h->device);
+    MCK(cudaStreamWaitEvent(h->stream, h->used, 0), "reset");   // calls still running on a caller's stream
     for (auto& z : h->state) MCK(cudaMemsetAsync(z.first, 0, z.second, h->stream), "reset");
     MCK(launch_wide_reset(h->d_wlv, h->n_wlv, nullptr, 0, h->stream), "reset");
     MCK(cudaStreamSynchronize(h->stream), "reset sync");
