@@ -36,8 +36,11 @@ using namespace pcg;
 namespace {
 
 constexpr int kWlog = 17;          // twiddle table 2^17 entries: real FFTs up to 2 * 65536
-// Calls of at least this many base steps run block-parallel (wide.cu).
-constexpr int kWideMinSteps = 4;
+// Calls of at least this many steps run block-parallel (wide.cu): its eight
+// launches cost as much as about ten steps (block-parallel and one-block steps,
+// 256x14 | 2048x50, 4, 8 and 16 steps: one stream 37.5, 37.5, 38.4 and 29.3,
+// 40.3, 69.3 us; 32 streams 53.5, 56.5, 60.2 and 32.3, 45.2, 79.1 us).
+constexpr int kWideMinSteps = 10;
 // Base steps per block-parallel chunk: as many as keep the chunk's spectra
 // (one ring row per block of every level) within kWideBytes, so that they and
 // the summed spectra, as many again, are still in the 129 MB L2 when the next
@@ -1320,7 +1323,7 @@ int finish_wide(pc_handle* h, const IOView& view, cudaStream_t st) {
 // for all but the last and again = true for all but the first.
 int run_steps(pc_handle* h, const IOView& view, long long nsteps, cudaStream_t st, bool again = false,
               bool more = false) {
-    if (!h->wide_ok || (nsteps < kWideMinSteps && !again && !more)) {
+    if (!h->wide_ok || (nsteps < kWideMinSteps * h->KB && !again && !more)) {
         RunState rs;
         rs.io = view;
         for (long long done = 0; done < nsteps; done += h->KB) {

@@ -68,7 +68,10 @@ constexpr int kMaxMimoLevels = 8;
 constexpr int kMaxMacTerms = 2048;  // (input, part) terms one MAC task sums
 // block-parallel calls: from this many base steps on; base steps per chunk, as
 // many as keep the chunk's spectra within kWideBytes
-constexpr int kWideMinSteps = 8;
+// (block-parallel and one-block steps, 128x16 | 2048xP, 4, 8 and 16 steps: 4 x 4
+// paths of 6001 taps 36, 41, 45 and 39, 70, 124 us; 32 x 32 of 2^15 taps 101,
+// 133, 141 and 64, 125, 231 us; at 12 steps 160 and 179)
+constexpr int kWideMinSteps = 10;
 constexpr size_t kWideBytes = (size_t)64 << 20;
 constexpr int kWideMinChunk = 32, kWideMaxChunk = 4096;
 constexpr int kOB = 4;             // outputs a warp sums together

@@ -47,7 +47,9 @@ constexpr size_t kScratchBytes = (size_t)32 << 20;   // PC_NOALLOC_SCRATCH_BYTES
 static_assert(kScratchBytes == (size_t)PC_NOALLOC_SCRATCH_BYTES, "header and implementation disagree");
 constexpr int kWlog = 15;
 constexpr int kMaxDevices = 64;
-constexpr int kWideMinBlocks = 4;   // calls of at least this many blocks run block-parallel ...
+// calls of at least this many blocks run block-parallel (four launches; 4, 6, 8 and 16 blocks, block-parallel and one at
+// a time: N = 64, 3000 taps 34 at any and 30, 35, 39, 58 us; N = 512, 48000 taps 40 at any and 35, 42, 48, 73 us) ...
+constexpr int kWideMinBlocks = 6;
 constexpr int kWideMinChunk = 8;    // ... if the array holds a chunk of this many
 constexpr int kWideMaxChunk = 4096;
 constexpr int kSeg = kWideRun;      // blocks per CTA of the sum over parts: one response has few tiles
