@@ -545,8 +545,11 @@ int pcs_step(pcs_handle* h, const float* in, float* out, int n_channels) {
     const size_t nb = sizeof(float) * (size_t)n_channels * h->N0;
     // Pinned buffers of exactly the pool's channels are read and written by the
     // kernels themselves (no copy engine start-up per block on either side);
-    // others, which the caller may change once this returns, go through copies.
-    bool direct = n_channels == h->channels && n_channels > 0;
+    // others, which the caller may change once this returns, go through copies,
+    // and so do buffers that overlap: a larger level's fire still reads an input
+    // block after level 0 has written that channel's output.
+    const char *bi = reinterpret_cast<const char*>(in), *bo = reinterpret_cast<const char*>(out);
+    bool direct = n_channels == h->channels && nb > 0 && (bi + nb <= bo || bo + nb <= bi);
     const float* src = h->d_in;
     float* dst = h->d_out;
     if (direct) {

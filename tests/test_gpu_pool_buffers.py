@@ -1,0 +1,55 @@
+"""Host buffers of a serving pool's step that the kernels must not use in place:
+one buffer for input and output and overlapping ones.  They give the samples of
+separate buffers, over steps in which larger levels fire."""
+import numpy as np
+import pytest
+
+from partconv_gb300 import workloads as wl
+from partconv_gb300.serving import ServingPool, serving_layout
+
+pytestmark = pytest.mark.gpu
+
+
+def _pool(irs, N0):
+    pool = ServingPool(N0, 64 << 20, len(irs))
+    for c, h in enumerate(irs):
+        assert pool.admit(h, *serving_layout(len(h), N0)) == c
+    return pool
+
+
+def _steps(pool, bi, bo, x):
+    """every block of x [steps][channels][N0] through the buffers (tensors [channels][N0])"""
+    y = np.zeros_like(x)
+    for t in range(len(x)):
+        bi.copy_(_t(x[t]))
+        pool.step(bi.data_ptr(), bo.data_ptr(), x.shape[1])
+        pool.sync()
+        y[t] = bo.numpy()
+    return y
+
+
+def _t(a):
+    import torch
+
+    return torch.from_numpy(a)
+
+
+@pytest.mark.parametrize("N0,L", [(64, 9000), (256, 30000), (1024, 20000)])
+def test_shared_and_split_buffers(gpu, N0, L):
+    import torch
+
+    rng = np.random.default_rng(N0)
+    n = 3
+    irs = [wl.decaying_ir(rng, L - 500 * c, 0.4) for c in range(n)]
+    x = (0.1 * rng.standard_normal((3 * L // N0 // 2 + 8, n, N0))).astype(np.float32)
+    sep = _steps(_pool(irs, N0), torch.zeros(n, N0).pin_memory(), torch.zeros(n, N0).pin_memory(), x)
+    for c in range(n):
+        assert wl.rel_l2(sep[:, c].ravel(), wl.conv_fp64(x[:, c].ravel(), irs[c], x[:, c].size)) <= 1e-5
+    one = torch.zeros(2 * n, N0).pin_memory()
+    assert np.array_equal(_steps(_pool(irs, N0), one[:n], one[:n], x), sep)              # in place
+    assert np.array_equal(_steps(_pool(irs, N0), one[1:n + 1], one[:n], x), sep)         # a row apart
+    assert np.array_equal(_steps(_pool(irs, N0), one[:n], one[n - 1:2 * n - 1], x), sep)
+    assert np.array_equal(_steps(_pool(irs, N0), one[:n], one[n:], x), sep)              # touching, not overlapping
+    flat = torch.zeros(2 * n * N0 + 2).pin_memory()                                      # rows at odd addresses
+    bi, bo = flat[1:1 + n * N0].view(n, N0), flat[2 + n * N0:].view(n, N0)
+    assert np.array_equal(_steps(_pool(irs, N0), bi, bo, x), sep)
