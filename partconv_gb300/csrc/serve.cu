@@ -11,6 +11,7 @@
 // Release marks the descriptors inactive and returns the arena space.  All
 // of this is ordered on the pool's stream, so it never races a step.
 // Every step batches all active PCs: one launch per block-size class.
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -190,6 +191,36 @@ size_t pc_bytes(int N0, const std::vector<int>& N, const std::vector<int>& P, si
         s += (long)N[L] * P[L];
     }
     return b;
+}
+
+// Device address of the n bytes at p when all of them lie in one page-locked
+// allocation or registration that the GPU can access; null otherwise.  (The
+// runtime's cudaPointerGetAttributes says nothing of a range's end.)
+const void* mapped_host(const void* p, size_t n) {
+    using Fn = CUresult (*)(unsigned, CUpointer_attribute*, void**, CUdeviceptr);
+    static const Fn get = [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult found = cudaDriverEntryPointSymbolNotFound;
+        if (cudaGetDriverEntryPointByVersion("cuPointerGetAttributes", &f, 7000, cudaEnableDefault, &found) != cudaSuccess ||
+            found != cudaDriverEntryPointSuccess) {
+            cudaGetLastError();
+            f = nullptr;
+        }
+        return reinterpret_cast<Fn>(f);
+    }();
+    if (!get) return nullptr;
+    CUpointer_attribute what[] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_IS_MANAGED,
+                                  CU_POINTER_ATTRIBUTE_DEVICE_POINTER, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR,
+                                  CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+    unsigned type = 0, managed = 0;
+    CUdeviceptr dev = 0, start = 0;
+    size_t size = 0;
+    void* data[] = {&type, &managed, &dev, &start, &size};
+    const CUdeviceptr q = reinterpret_cast<CUdeviceptr>(p);
+    if (get(5, what, data, q) != CUDA_SUCCESS || type != CU_MEMORYTYPE_HOST || managed || !dev || q < start ||
+        size < n || q - start > size - n)
+        return nullptr;
+    return reinterpret_cast<const void*>(dev);
 }
 
 int rebuild_map(pcs_handle* h) {
@@ -548,20 +579,16 @@ int pcs_step(pcs_handle* h, const float* in, float* out, int n_channels) {
     // others, which the caller may change once this returns, go through copies,
     // and so do buffers that overlap: a larger level's fire still reads an input
     // block after level 0 has written that channel's output.
-    const char *bi = reinterpret_cast<const char*>(in), *bo = reinterpret_cast<const char*>(out);
-    bool direct = n_channels == h->channels && nb > 0 && (bi + nb <= bo || bo + nb <= bi);
     const float* src = h->d_in;
     float* dst = h->d_out;
+    const char *bi = reinterpret_cast<const char*>(in), *bo = reinterpret_cast<const char*>(out);
+    bool direct = n_channels == h->channels && nb > 0 && (bi + nb <= bo || bo + nb <= bi);
     if (direct) {
-        cudaPointerAttributes ai, ao;
-        direct = cudaPointerGetAttributes(&ai, in) == cudaSuccess && ai.type == cudaMemoryTypeHost &&
-                 cudaPointerGetAttributes(&ao, out) == cudaSuccess && ao.type == cudaMemoryTypeHost &&
-                 ai.devicePointer && ao.devicePointer;
+        const void *mi = mapped_host(in, nb), *mo = mi ? mapped_host(out, nb) : nullptr;
+        direct = mo != nullptr;
         if (direct) {
-            src = static_cast<const float*>(ai.devicePointer);
-            dst = static_cast<float*>(ao.devicePointer);
-        } else {
-            cudaGetLastError();
+            src = static_cast<const float*>(mi);
+            dst = static_cast<float*>(const_cast<void*>(mo));
         }
     }
     if (nb && !direct) SCK(cudaMemcpyAsync(h->d_in, in, nb, cudaMemcpyHostToDevice, h->stream), "input copy");

@@ -1,9 +1,11 @@
 """Host buffers of a serving pool's step that the kernels must not use in place:
-one buffer for input and output and overlapping ones.  They give the samples of
-separate buffers, over steps in which larger levels fire."""
+one buffer for input and output, overlapping ones, and a buffer that runs from one
+registration of host memory into another.  The former give the samples of separate
+buffers, over steps in which larger levels fire; the latter is refused."""
 import numpy as np
 import pytest
 
+from partconv_gb300 import PartConvError
 from partconv_gb300 import workloads as wl
 from partconv_gb300.serving import ServingPool, serving_layout
 
@@ -53,3 +55,25 @@ def test_shared_and_split_buffers(gpu, N0, L):
     flat = torch.zeros(2 * n * N0 + 2).pin_memory()                                      # rows at odd addresses
     bi, bo = flat[1:1 + n * N0].view(n, N0), flat[2 + n * N0:].view(n, N0)
     assert np.array_equal(_steps(_pool(irs, N0), bi, bo, x), sep)
+
+
+def test_buffer_across_two_registrations_is_refused(gpu):
+    """A copy refuses such a buffer; the kernels must not be given it instead."""
+    import torch
+
+    n, N0, page = 4, 1024, 1 << 16
+    pool = _pool([wl.decaying_ir(np.random.default_rng(2), 9000, 0.4)] * n, N0)
+    raw = np.zeros(5 * page // 4, np.float32)
+    base = (raw.ctypes.data + page - 1) // page * page
+    rt = torch.cuda.cudart()
+    regs = [base, base + page]   # two registrations side by side
+    for r in regs:
+        assert int(rt.cudaHostRegister(r, page, 0)) == 0
+    try:
+        at = base + page - 2 * N0 * 4   # two rows in each
+        with pytest.raises(PartConvError):
+            pool.step(at, torch.zeros(n, N0).pin_memory().data_ptr(), n)
+    finally:
+        torch.cuda.synchronize()
+        for r in regs:
+            rt.cudaHostUnregister(r)
