@@ -225,7 +225,7 @@ const void* mapped_host(const void* p, size_t n) {
 
 int rebuild_map(pcs_handle* h) {
     std::vector<PoolCta> m[3];
-    const int c0 = fire_class_of(h->N0);
+    const int c0 = fire_class_of(h->N0), had = h->channels;
     h->channels = 0;
     int tmax = 1;
     for (int id = 0; id < (int)h->pcs.size(); ++id)
@@ -233,6 +233,11 @@ int rebuild_map(pcs_handle* h) {
             h->channels = id + 1;
             tmax = std::max(tmax, h->pcs[id].N.back() / h->N0);
         }
+    // rows of the staged output that no CTA writes any more: silence
+    if (h->channels < had)
+        SCK(cudaMemsetAsync(h->d_out + (size_t)h->channels * h->N0, 0,
+                            sizeof(float) * (size_t)(had - h->channels) * h->N0, h->stream),
+            "output clear");
     for (auto& d : h->due) d.assign(tmax, 0);
     for (int id = 0; id < h->channels; ++id) {
         const PoolPC& p = h->pcs[id];

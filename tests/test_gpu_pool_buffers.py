@@ -1,7 +1,8 @@
 """Host buffers of a serving pool's step that the kernels must not use in place:
 one buffer for input and output, overlapping ones, and a buffer that runs from one
 registration of host memory into another.  The former give the samples of separate
-buffers, over steps in which larger levels fire; the latter is refused."""
+buffers, over steps in which larger levels fire; the latter is refused.  And
+channels that were released, through staged and pinned buffers."""
 import numpy as np
 import pytest
 
@@ -77,3 +78,36 @@ def test_buffer_across_two_registrations_is_refused(gpu):
         torch.cuda.synchronize()
         for r in regs:
             rt.cudaHostUnregister(r)
+
+
+@pytest.mark.parametrize("pinned", [True, False])
+def test_released_channels_are_silent(gpu, pinned):
+    """The highest channel, then every channel released while the host goes on
+    stepping all of them: zeros, not the last block again; a channel admitted in
+    their place sounds at once."""
+    import torch
+
+    rng = np.random.default_rng(9)
+    n, N0 = 3, 64
+    irs = [wl.decaying_ir(rng, 700, 0.4) for _ in range(n)]
+    pool = _pool(irs, N0)
+    bi, bo = torch.zeros(n, N0), torch.ones(n, N0)
+    if pinned:
+        bi, bo = bi.pin_memory(), bo.pin_memory()
+
+    def step():
+        bi.copy_(_t((0.1 * rng.standard_normal((n, N0))).astype(np.float32)))
+        pool.step(bi.data_ptr(), bo.data_ptr(), n)
+        pool.sync()
+        return [bool(bo[c].any()) for c in range(n)]
+
+    for _ in range(12):
+        assert step() == [True, True, True]
+    pool.release(2)
+    assert [step() for _ in range(3)] == [[True, True, False]] * 3
+    pool.release(0)
+    assert [step() for _ in range(3)] == [[False, True, False]] * 3
+    pool.release(1)
+    assert [step() for _ in range(3)] == [[False, False, False]] * 3
+    assert pool.admit(irs[0], *serving_layout(700, N0)) == 0
+    assert [step() for _ in range(3)] == [[True, False, False]] * 3
