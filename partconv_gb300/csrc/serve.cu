@@ -108,9 +108,9 @@ struct pcs_handle {
     size_t map_cap = 0;
     int map_n[3] = {0, 0, 0};
     int channels = 0;                        // 1 + the largest live id: the channels the map writes
-    // levels of a class that fire within steps congruent to i modulo the table's
-    // length (a power of two): a class whose levels have nothing due is not launched
-    std::vector<int> due[3];
+    // whether a class has a level that fires at steps congruent to i modulo the
+    // table's length (a power of two): a class with nothing due is not launched
+    std::vector<char> due[3];
     bool map_dirty = false;
     float* d_in = nullptr;                   // [max_pcs][N0] staging
     float* d_out = nullptr;
@@ -239,6 +239,8 @@ int rebuild_map(pcs_handle* h) {
                             sizeof(float) * (size_t)(had - h->channels) * h->N0, h->stream),
             "output clear");
     for (auto& d : h->due) d.assign(tmax, 0);
+    std::vector<char> fires[3];
+    for (auto& f : fires) f.assign(2 * (size_t)tmax, 0);
     for (int id = 0; id < h->channels; ++id) {
         const PoolPC& p = h->pcs[id];
         if (!p.live) {
@@ -250,12 +252,18 @@ int rebuild_map(pcs_handle* h) {
             const int cls = fire_class_of(p.N[L]);
             m[cls].push_back({slot, 0});
             for (int t = 1; t <= p.spread_tiles[L]; ++t) m[c0].push_back({slot, t});
-            // the level fires at steps c with (c - origin + 1 + s) % T == 0
+            // the level fires at steps c with (c - origin + 1 + s) % T == 0 (T a
+            // power of two): entry T + the step's residue, for the classes that
+            // are not launched at every step anyway
             const Task& t = h->h_slots[slot];
-            long long r = (t.origin - 1 - t.s_blocks) % t.T;
-            for (int i = (int)(r < 0 ? r + t.T : r); i < tmax; i += t.T) h->due[cls][i]++;
+            if (cls != c0) fires[cls][t.T + (int)((t.origin - 1 - t.s_blocks) & (t.T - 1))] = 1;
         }
     }
+    for (int cls = 0; cls < 3; ++cls)
+        for (int T = 1; T <= tmax; T <<= 1)
+            for (int r = 0; r < T; ++r)
+                if (fires[cls][T + r])
+                    for (int i = r; i < tmax; i += T) h->due[cls][i] = 1;
     size_t need = std::max({m[0].size(), m[1].size(), m[2].size(), (size_t)1});
     if (need > h->map_cap) {
         // steps already enqueued may still read the old maps

@@ -111,3 +111,34 @@ def test_released_channels_are_silent(gpu, pinned):
     assert [step() for _ in range(3)] == [[False, False, False]] * 3
     assert pool.admit(irs[0], *serving_layout(700, N0)) == 0
     assert [step() for _ in range(3)] == [[True, False, False]] * 3
+
+
+def test_channels_admitted_at_any_step(gpu):
+    """The larger levels of channels admitted at different steps fire at different
+    steps; a class's launch is left out only where none of them does."""
+    import torch
+
+    rng = np.random.default_rng(11)
+    N0, L, steps = 64, 30000, 700
+    at = [0, 3, 17, 130, 131]   # admission steps; one channel leaves before the last comes
+    irs = [wl.decaying_ir(rng, L - 100 * c, 0.4) for c in range(len(at))]
+    pool = ServingPool(N0, 64 << 20, len(at))
+    n = len(at)
+    x = (0.1 * rng.standard_normal((steps, n, N0))).astype(np.float32)
+    bi, bo = torch.zeros(n, N0).pin_memory(), torch.zeros(n, N0).pin_memory()
+    y = np.zeros_like(x)
+    for t in range(steps):
+        for c in range(n):
+            if at[c] == t:
+                assert pool.admit(irs[c], *serving_layout(L - 100 * c, N0)) == c
+        if t == 400:
+            pool.release(1)
+        width = sum(a <= t for a in at)
+        bi.copy_(_t(x[t]))
+        pool.step(bi.data_ptr(), bo.data_ptr(), width)
+        pool.sync()
+        y[t, :width] = bo[:width].numpy()
+    for c in range(n):
+        end = 400 if c == 1 else steps
+        ref = wl.conv_fp64(x[at[c]:end, c].ravel(), irs[c], (end - at[c]) * N0)
+        assert wl.rel_l2(y[at[c]:end, c].ravel(), ref) <= 1e-5
