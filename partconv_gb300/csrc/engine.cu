@@ -55,6 +55,16 @@ constexpr size_t kWideBytes = (size_t)256 << 20;
 constexpr int kPlanarInputs = 4;
 constexpr long long kPlanarSamples = 1 << 16;
 constexpr int kWideMinChunk = 32, kWideMaxChunk = 4096;
+// A callback's kernels read and write the pinned host block themselves, which
+// saves the start of two copies (about 10 us), up to this many samples over PCs
+// (each reads its input channel) and outputs, or with at most kDirectRows PCs and
+// outputs; beyond that the strided accesses to host memory cost more than the
+// copies (us per callback, direct and copied; inputs-outputs-PCs): 64 samples
+// 64-64-64 22 and 32, 512 32-32-32 33 and 37, 1024 16-16-16 39 and 39, 1024
+// 32-32-32 50 and 47, 2048 8-8-8 35 and 39, 2048 32-32-32 74 and 60, 8192 8-8-8
+// 87 and 84, 16384 4-4-4 99 and 105, 16384 32-32-32 539 and 369.
+constexpr long long kDirectSamples = 40000;
+constexpr int kDirectRows = 8;
 constexpr int kMinN0 = 16;
 constexpr int kClasses = kNumClasses;
 
@@ -1534,12 +1544,14 @@ int pc_run(pc_handle* h, float* output, const float* input, int frame_count) {
                                          " blocks per step (use process)");
     CK(cudaSetDevice(h->device), "cudaSetDevice");
     const size_t in_b = sizeof(float) * (size_t)h->N0 * h->n_in, out_b = sizeof(float) * (size_t)h->N0 * h->n_out;
-    // the step's kernels read and write the pinned staging block themselves: one
-    // block is a few KB, and a copy engine takes longer to start than they do to
-    // fetch it (29.6 us per callback with two copies, N0 = 64)
+    const long long rows = (long long)h->h_pcs.size() + h->n_out;
+    const bool direct = rows <= kDirectRows || h->N0 * rows <= kDirectSamples;
     std::memcpy(h->h_in1, input, in_b);
-    int r = process_device_impl(h, h->h_out1, h->h_in1, h->N0, PC_INTERLEAVED, h->stream);
+    if (!direct) CK(cudaMemcpyAsync(h->d_in1, h->h_in1, in_b, cudaMemcpyHostToDevice, h->stream), "input copy");
+    int r = process_device_impl(h, direct ? h->h_out1 : h->d_out1, direct ? h->h_in1 : h->d_in1, h->N0, PC_INTERLEAVED,
+                                h->stream);
     if (r) return r;
+    if (!direct) CK(cudaMemcpyAsync(h->h_out1, h->d_out1, out_b, cudaMemcpyDeviceToHost, h->stream), "output copy");
     CK(cudaStreamSynchronize(h->stream), "run sync");
     std::memcpy(output, h->h_out1, out_b);
     return PC_OK;
