@@ -183,7 +183,8 @@ struct pc_handle {
     std::vector<int> lv_cls;   // kernel class of each level's fires (spectra layout follows it)
     Bank bank{};
     int H = 1;        // hyperperiod (base steps)
-    int C = 32;       // base steps per block-parallel chunk (a multiple of KB)
+    int C_max = 32;   // most base steps per block-parallel chunk (a multiple of KB)
+    int C = 0;        // ... that the workspace in hand holds (0: none yet)
     int req_kb = 1;   // base blocks per step requested (pc_set_step_blocks)
     int req_tile_bins = 0, req_tile_parts = 0;   // spread tile shape requested (pc_set_tiles; 0: default)
     int TB = 0, TP = 0;                          // spread tile shape in use: bins and parts per task
@@ -235,6 +236,16 @@ struct pc_handle {
     int n_zero = 0, max_ring = 0;
     bool wide_ok = true;           // every ring's element offsets fit 32 bits
     bool mixed = false;
+    // The rings of the block-parallel form, its summed spectra and its mixed and
+    // by-channel samples: allocated by the first call that runs block-parallel,
+    // for as many steps as it has (ensure_wide).  Until then the rings in the
+    // arena hold what one-block steps need.
+    char* work = nullptr;
+    size_t work_bytes = 0;
+    bool work_failed = false;      // no room for the smallest one: one-block steps until reset
+    std::vector<WLevel> h_wlv;
+    WLevel* d_wlv_of[2] = {};      // d_wlv and the other buffer of it
+    int n_tasks = 0;
 
     // run() staging and Relaxed carry (planar [n_out][N0])
     float* d_in1 = nullptr;
@@ -278,6 +289,12 @@ void free_device(pc_handle* h) {
     if (h->h_out1) cudaFreeHost(h->h_out1);
     h->h_in1 = h->h_out1 = nullptr;
     h->arena = nullptr;
+    if (h->work) cudaFree(h->work);
+    h->work = nullptr;
+    h->work_bytes = 0;
+    h->work_failed = false;
+    h->C = 0;
+    h->d_planar = nullptr;
     if (h->d_big_in) cudaFree(h->d_big_in);
     if (h->d_big_out) cudaFree(h->d_big_out);
     if (h->d_rtmp) cudaFree(h->d_rtmp);
@@ -407,7 +424,7 @@ struct WideMaps {
         };
         auto put_map = [&](Entries& e, pc_handle::WMap& m) {
             m.map = entries(e);
-            m.upto = prefix(e, h->C);
+            m.upto = prefix(e, h->C_max);
         };
         for (int g = 0; g < 3; ++g) {
             put_map(fwd[g], h->w_fwd[g]);
@@ -417,13 +434,22 @@ struct WideMaps {
         put_map(cl, h->w_cl);
         for (int x = 0; x < 2; ++x) {
             h->wmac_map[x] = entries(mac[x]);
-            h->wmac_upto[x] = prefix(mac[x], h->C);
+            h->wmac_upto[x] = prefix(mac[x], h->C_max);
         }
         h->w_part_map = reinterpret_cast<const int4*>(put(part.data(), sizeof(int4) * part.size()));
         h->w_part_n = (int)part.size();
         return err;
     }
 };
+
+// samples of a level's output ring: those due later (up to s + `ahead`)
+long out_ring(long N, long s, long ahead) {
+    long r = N;
+    while (r < s + ahead) r <<= 1;
+    return r;
+}
+// rows of a level's spectrum ring for chunks of C steps
+int wide_slots(const DevLevel& l, int C) { return l.P + std::max((C + l.T - 1) / l.T, kWideRun); }
 
 void build_wide_maps(pc_handle* h, WideMaps& m) {
     const int nt = spread_threads(h), lanes = spread_lane_count(h);
@@ -445,11 +471,11 @@ void build_wide_maps(pc_handle* h, WideMaps& m) {
     // six-level stereo ladder, half a wave: 285 and 238).
     h->w_nt[0] = h->w_nt[1] = wide_threads(big);
     h->w_nt[2] = wide_threads(1);
-    h->w_split = h->w_nt[0] == h->w_nt[2] ? h->C + 1 : (int)std::min(4.0 * 152 * 16384 / ((double)one * h->N0) + 1, 1e9);
+    h->w_split = h->w_nt[0] == h->w_nt[2] ? h->C_max + 1 : (int)std::min(4.0 * 152 * 16384 / ((double)one * h->N0) + 1, 1e9);
     for (int li = 0; li < nlv; ++li) {
         const DevLevel& l = h->h_lv[li];
         const bool l0 = l.T == 1, cluster = h->lv_cls[li] == 3;
-        const int nb = (h->C + l.T - 1) / l.T;   // most blocks of the level in a chunk
+        const int nb = (h->C_max + l.T - 1) / l.T;   // most blocks of the level in a chunk
         for (int g = 0; g < 3 && !cluster; ++g) {
             if (g > 0 && (l.N <= 16 * h->w_nt[2]) != (g == 2)) continue;
             for (int i = 0; i < nb; i += 16 * h->w_nt[g] / l.N) {
@@ -539,18 +565,21 @@ int do_setup(pc_handle* h, int fs, int buffer_size, int n_in, int n_out, std::ve
     // parts a K-block level-0 fire sums itself; spread rows take the rest
     const int QC = KB > 1 ? multi_fire_parts(N0, KB) : 2;
     {
-        // a block of N samples adds a row of N + 2 bins per N / N0 steps
-        const double row = sizeof(float2) * (double)N0 * nlv;   // bytes of spectra per base step
+        // a block of N samples adds a row of N + 2 bins per N / N0 steps; the
+        // input by channel takes its samples
+        const double row = sizeof(float2) * (double)N0 * nlv +   // bytes per base step
+                           (n_in >= kPlanarInputs ? sizeof(float) * (double)N0 * n_in : 0.0);
         int C = kWideMaxChunk;
         while (C > kWideMinChunk && C * row > (double)kWideBytes) C >>= 1;
-        h->C = C;
+        h->C_max = C;
+        h->C = 0;
     }
 
     // ---- arena layout --------------------------------------------------------------
     Carve cv;
     const size_t off_W = cv.take(sizeof(float2) << kWlog);
     const size_t off_wtab = cv.take(sizeof(float2) * kFftTabEntries);
-    const size_t off_wlv = cv.take(sizeof(WLevel) * nlv);
+    const size_t off_wlv = cv.take(sizeof(WLevel) * nlv), off_wlv2 = cv.take(sizeof(WLevel) * nlv);
     const size_t off_lv0 = cv.take(sizeof(int) * npc);
     const size_t off_pcs = cv.take(sizeof(DevPC) * npc);
     const size_t off_lv = cv.take(sizeof(DevLevel) * nlv);
@@ -636,10 +665,7 @@ int do_setup(pc_handle* h, int fs, int buffer_size, int n_in, int n_out, std::ve
         for (auto& p : h->specs) {
             long s = 0;
             for (size_t L = 0; L < p.N.size(); ++L, ++li) {
-                long r = p.N[L];
-                // samples in flight: due later (up to s + KB N0), or a whole chunk's
-                while (r < s + (long)std::max(KB, h->C) * N0) r <<= 1;
-                rl[li] = (int)r;
+                rl[li] = (int)out_ring(p.N[L], s, (long)KB * N0);
                 s += (long)p.N[L] * p.P[L];
             }
         }
@@ -694,8 +720,8 @@ int do_setup(pc_handle* h, int fs, int buffer_size, int n_in, int n_out, std::ve
                 l.cs = p.N[L] + 2;
                 l.rmask = rl[li] - 1;
                 l.pc = i;
-                l.slots = l.P + std::max((h->C + l.T - 1) / l.T, kWideRun);
-                if ((long long)l.slots * l.cs >= (1LL << 31)) h->wide_ok = false;
+                l.slots = l.P;
+                if ((long long)wide_slots(l, h->C_max) * l.cs >= (1LL << 31)) h->wide_ok = false;
                 {   // spread tasks sum parts >= 2 KB (level 0), >= 2 (deferred levels) or >= 1
                     const int p_lo = L == 0 ? (KB > 1 ? std::min(p.P[L], QC) : 2) : (dfl[li] ? 2 : 1);
                     const int np = p.P[L] - p_lo;
@@ -995,18 +1021,6 @@ int do_setup(pc_handle* h, int fs, int buffer_size, int n_in, int n_out, std::ve
         so.yr[li] = cv.take(sizeof(float) * (size_t)(l.rmask + 1));
     }
 
-    // block-parallel workspace: summed spectra of a chunk's blocks, mixed
-    // outputs' samples, and the CTA maps
-    std::vector<size_t> off_Yw(nlv), off_pcw(npc, 0);
-    for (int li = 0; li < nlv; ++li)
-        off_Yw[li] = cv.take(sizeof(float2) * (size_t)((h->C + h->h_lv[li].T - 1) / h->h_lv[li].T) * h->h_lv[li].cs);
-    for (int i = 0; i < npc; ++i)
-        if (h->h_pcs[i].mix_mode == 2) off_pcw[i] = cv.take(sizeof(float) * (size_t)h->C * N0);
-    // a chunk's interleaved input by channel, with the samples that its windows reach back to
-    h->planar_pitch = (long long)h->C * N0;
-    for (int li = 0; li < nlv; ++li)
-        h->planar_pitch = std::max(h->planar_pitch, (long long)h->C * N0 + 2LL * h->h_lv[li].N);
-    const size_t off_planar = h->n_in >= kPlanarInputs ? cv.take(sizeof(float) * h->n_in * (size_t)h->planar_pitch) : 0;
     WideMaps wm;
     build_wide_maps(h, wm);
     const size_t off_wmap = cv.take(wm.bytes());
@@ -1059,6 +1073,7 @@ int do_setup(pc_handle* h, int fs, int buffer_size, int n_in, int n_out, std::ve
                 all_tasks.push_back(t);
             }
     h->d_tasks = reinterpret_cast<Task*>(A + off_tasks);
+    h->n_tasks = (int)ntasks;
     if (!all_tasks.empty())
         CK(cudaMemcpyAsync(h->d_tasks, all_tasks.data(), sizeof(Task) * all_tasks.size(), cudaMemcpyHostToDevice,
                            h->stream),
@@ -1069,7 +1084,8 @@ int do_setup(pc_handle* h, int fs, int buffer_size, int n_in, int n_out, std::ve
         h->class_maxN[cls] = std::max(h->class_maxN[cls], h->h_lv[li].N);
     }
     {
-        std::vector<WLevel> wl(nlv);
+        std::vector<WLevel>& wl = h->h_wlv;
+        wl.assign(nlv, WLevel{});
         std::vector<int> lv0(npc);
         for (int i = 0; i < npc; ++i) {
             const DevPC& d = h->h_pcs[i];
@@ -1078,7 +1094,6 @@ int do_setup(pc_handle* h, int fs, int buffer_size, int n_in, int n_out, std::ve
                 const int li = d.lv0 + L;
                 const DevLevel& l = h->h_lv[li];
                 WLevel& w = wl[li];
-                w = WLevel{};
                 w.N = l.N;
                 w.logN = l.logN;
                 w.P = l.P;
@@ -1103,11 +1118,9 @@ int do_setup(pc_handle* h, int fs, int buffer_size, int n_in, int n_out, std::ve
                 w.scale = d.scale;
                 w.H = l.H;
                 w.X = l.X;
-                w.Yw = reinterpret_cast<float2*>(A + off_Yw[li]);
                 w.Yp = l.Yp;
                 w.yring = l.yring;
                 w.xring = d.xring;
-                w.pcw = d.mix_mode == 2 ? reinterpret_cast<float*>(A + off_pcw[i]) : nullptr;
                 h->max_ring = std::max(h->max_ring, d.rin_mask + 1);
             }
         }
@@ -1115,9 +1128,10 @@ int do_setup(pc_handle* h, int fs, int buffer_size, int n_in, int n_out, std::ve
            "upload levels");
         CK(cudaMemcpyAsync(A + off_lv0, lv0.data(), sizeof(int) * npc, cudaMemcpyHostToDevice, h->stream),
            "upload levels");
-        h->d_wlv = reinterpret_cast<const WLevel*>(A + off_wlv);
+        h->d_wlv_of[0] = reinterpret_cast<WLevel*>(A + off_wlv);
+        h->d_wlv_of[1] = reinterpret_cast<WLevel*>(A + off_wlv2);
+        h->d_wlv = h->d_wlv_of[0];
         h->d_lv0 = reinterpret_cast<const int*>(A + off_lv0);
-        h->d_planar = h->n_in >= kPlanarInputs ? reinterpret_cast<float*>(A + off_planar) : nullptr;
         h->d_wtab = reinterpret_cast<const float2*>(A + off_wtab);
         CK(wm.place(h, A + off_wmap), "upload maps");
         CK(launch_wide_reset(h->d_wlv, nlv, A + h->state_off, h->state_bytes, h->stream), "clear state");
@@ -1273,6 +1287,124 @@ IOView make_view(const pc_handle* h, const float* in, float* out, long long fram
     return v;
 }
 
+// Task descriptors after their levels' rings have moved.
+__global__ void retarget_kernel(Task* tasks, int n, const DevLevel* __restrict__ lv) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    Task& t = tasks[i];
+    const DevLevel& l = lv[t.lv_index];
+    t.X = l.X;
+    t.slots = l.slots;
+    t.yring = l.yring;
+    if (t.kind != 0) return;   // (a spread task keeps its parts per thread group in rmask)
+    t.rmask = l.rmask;
+    if (t.T == 1)
+        for (int L = 1; L <= kEmitLevels && L < t.M; ++L) {
+            t.eyring[L - 1] = lv[t.lv_index + L].yring;
+            t.emask[L - 1] = lv[t.lv_index + L].rmask;
+        }
+}
+
+// A workspace for chunks of up to C steps in place of the present one, its
+// rings holding what the present ones do.  PC_ERR_NOMEM if there is no room
+// for it: the present one stays in use.
+int move_to_work(pc_handle* h, int C, cudaStream_t st) {
+    const int nlv = (int)h->h_lv.size(), npc = (int)h->h_pcs.size(), N0 = h->N0;
+    Carve cv;
+    std::vector<size_t> off_X(nlv), off_yr(nlv), off_Yw(nlv), off_pcw(npc, 0);
+    std::vector<DevLevel> lv = h->h_lv;
+    std::vector<WLevel> wl = h->h_wlv;
+    long long pitch = (long long)C * N0;   // of the input by channel: a chunk and what its windows reach back to
+    for (int li = 0; li < nlv; ++li) {
+        DevLevel& l = lv[li];
+        l.slots = wide_slots(l, C);
+        l.rmask = (int)out_ring(l.N, (long)l.s_blocks * N0, (long)std::max(h->KB, C) * N0) - 1;
+        off_X[li] = cv.take(sizeof(float2) * (size_t)l.slots * l.cs);
+        off_yr[li] = cv.take(sizeof(float) * (size_t)(l.rmask + 1));
+        off_Yw[li] = cv.take(sizeof(float2) * (size_t)((C + l.T - 1) / l.T) * l.cs);
+        pitch = std::max(pitch, (long long)C * N0 + 2LL * l.N);
+    }
+    for (int i = 0; i < npc; ++i)
+        if (h->h_pcs[i].mix_mode == 2) off_pcw[i] = cv.take(sizeof(float) * (size_t)C * N0);
+    const bool planar = h->n_in >= kPlanarInputs;
+    const size_t off_planar = planar ? cv.take(sizeof(float) * h->n_in * (size_t)pitch) : 0;
+
+    // (another thread may be capturing a graph meanwhile)
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    char* W = nullptr;
+    cudaError_t e = cudaMalloc(&W, cv.off);
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        return PC_ERR_NOMEM;
+    }
+    for (int li = 0; li < nlv; ++li) {
+        DevLevel& l = lv[li];
+        l.X = reinterpret_cast<float2*>(W + off_X[li]);
+        l.yring = reinterpret_cast<float*>(W + off_yr[li]);
+        WLevel& w = wl[li];
+        w.slots = l.slots;
+        w.rmask = l.rmask;
+        w.X = l.X;
+        w.yring = l.yring;
+        w.Yw = reinterpret_cast<float2*>(W + off_Yw[li]);
+        w.pcw = w.mix_mode == 2 ? reinterpret_cast<float*>(W + off_pcw[l.pc]) : nullptr;
+    }
+    WLevel* next = h->d_wlv == h->d_wlv_of[0] ? h->d_wlv_of[1] : h->d_wlv_of[0];
+    e = cudaMemcpyAsync(next, wl.data(), sizeof(WLevel) * nlv, cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(const_cast<DevLevel*>(h->bank.lv), lv.data(), sizeof(DevLevel) * nlv, cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess) e = launch_wide_move(h->d_wlv, next, nlv, h->frame_num, N0, st);
+    if (e == cudaSuccess) {
+        retarget_kernel<<<(h->n_tasks + 127) / 128, 128, 0, st>>>(h->d_tasks, h->n_tasks, h->bank.lv);
+        e = cudaGetLastError();
+    }
+    if (h->work || e != cudaSuccess) {   // nothing may still read what is freed
+        const cudaError_t se = cudaStreamSynchronize(st);
+        if (e == cudaSuccess) e = se;
+        cudaFree(e == cudaSuccess ? h->work : W);
+    }
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    if (e != cudaSuccess) return cuda_fail(h, e, "block-parallel workspace");
+    h->work = W;
+    h->work_bytes = cv.off;
+    h->C = C;
+    h->planar_pitch = pitch;
+    h->d_planar = planar ? reinterpret_cast<float*>(W + off_planar) : nullptr;
+    h->h_lv.swap(lv);
+    h->h_wlv.swap(wl);
+    h->d_wlv = next;
+    h->launches += 2;
+    return PC_OK;
+}
+
+// Whether a call of nsteps base steps on st can run block-parallel.  The
+// workspace is made for it, in chunks as short as the call, and grows with
+// longer calls up to h->C_max steps; where there is no room for the longest
+// chunk a shorter one serves, and for none one-block steps do.  A stream that is
+// being captured takes the workspace as it is.  Results are the same either way.
+int ensure_wide(pc_handle* h, long long nsteps, cudaStream_t st, bool* wide) {
+    int want = kWideMinChunk;
+    while (want < nsteps && want < h->C_max) want <<= 1;
+    want = std::min(want, h->C_max);
+    *wide = h->C > 0;
+    if (h->C >= want || h->work_failed) return PC_OK;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    CK(cudaStreamIsCapturing(st, &cs), "capture status");
+    if (cs != cudaStreamCaptureStatusNone) return PC_OK;
+    for (; want > h->C && want >= kWideMinChunk; want >>= 1) {
+        const int r = move_to_work(h, want, st);
+        if (r == PC_OK) {
+            *wide = true;
+            return PC_OK;
+        }
+        if (r != PC_ERR_NOMEM) return r;
+        h->work_failed = true;   // (of the size asked for: not tried again until reset)
+    }
+    return PC_OK;
+}
+
 // One chunk of n <= h->C base steps from h->frame_num, block-parallel.
 int run_chunk(pc_handle* h, const IOView& view, int n, cudaStream_t st) {
     WArgs a = wide_args(h, view, n);
@@ -1330,10 +1462,16 @@ int finish_wide(pc_handle* h, const IOView& view, cudaStream_t st) {
 // Run nsteps base steps starting at h->frame_num through the view: direct
 // launches for a few steps, block-parallel chunks for more.  A call in several
 // pieces (pc_process's pipeline, one view for all of them) passes more = true
-// for all but the last and again = true for all but the first.
+// for all but the last and again = true for all but the first; pieces that find
+// no workspace run one-block steps, later ones may run block-parallel.
 int run_steps(pc_handle* h, const IOView& view, long long nsteps, cudaStream_t st, bool again = false,
               bool more = false) {
-    if (!h->wide_ok || (nsteps < kWideMinSteps * h->KB && !again && !more)) {
+    bool wide = h->wide_ok && (nsteps >= kWideMinSteps * h->KB || again || more);
+    if (wide) {
+        const int r = ensure_wide(h, nsteps, st, &wide);
+        if (r) return r;
+    }
+    if (!wide) {
         RunState rs;
         rs.io = view;
         for (long long done = 0; done < nsteps; done += h->KB) {
@@ -1581,7 +1719,7 @@ int pc_process(pc_handle* h, float* output, const float* input, long long frames
     // Long calls run as a pipeline of chunks: the input copy of chunk i + 1
     // and the output copy of chunk i - 1 (own streams) overlap the steps of
     // chunk i (the handle's stream); the steps of one call stay in order.
-    const long long chunk = (long long)std::max(h->C, 128) * h->N0;   // a multiple of KB N0
+    const long long chunk = (long long)std::max(h->C_max, 128) * h->N0;   // a multiple of KB N0
     if (!h->relaxed && frames >= 2 * chunk) {
         if (!h->cin) CK(cudaStreamCreateWithFlags(&h->cin, cudaStreamNonBlocking), "stream create");
         if (!h->cout) CK(cudaStreamCreateWithFlags(&h->cout, cudaStreamNonBlocking), "stream create");
@@ -1651,6 +1789,7 @@ int pc_reset(pc_handle* h) {
     if (!h) return PC_ERR_ARG;
     h->frame_num = 0;
     if (!h->ready) return PC_OK;
+    h->work_failed = false;
     CK(cudaSetDevice(h->device), "cudaSetDevice");
     CK(cudaStreamWaitEvent(h->stream, h->used, 0), "reset");   // calls still running on a caller's stream
     CK(launch_wide_reset(h->d_wlv, (int)h->h_lv.size(), h->arena + h->state_off, h->state_bytes, h->stream), "reset");
@@ -1689,7 +1828,7 @@ int pc_get_info(const pc_handle* h, pc_info* info) {
     info->spread_parts = h->TP;
     info->frame_num = h->frame_num;
     info->device_bytes =
-        (long long)h->arena_bytes + (long long)sizeof(float) * (h->big_in_cap + h->big_out_cap + h->rtmp_cap);
+        (long long)(h->arena_bytes + h->work_bytes) + (long long)sizeof(float) * (h->big_in_cap + h->big_out_cap + h->rtmp_cap);
     return PC_OK;
 }
 

@@ -772,6 +772,27 @@ __global__ void wide_reset_kernel(const WLevel* __restrict__ lv, int nlv, float4
     for (int i = t; i < ny; i += nt) reinterpret_cast<float4*>(l.yring)[i] = z;
 }
 
+// What a step c from which the rings go on reads of them: the spectrum rows of
+// the P - 1 blocks before its first one and the output ring from its first sample
+// to the last block's end, from the rings of lv to those of to.
+__global__ void wide_move_kernel(const WLevel* __restrict__ lv, const WLevel* __restrict__ to, long long c, int N0) {
+    const int nt = gridDim.y * blockDim.x, t = blockIdx.y * blockDim.x + threadIdx.x;
+    const WLevel &l = lv[blockIdx.x], &m = to[blockIdx.x];
+    const long long b0 = blocks_before(l, c);
+    const int n4 = l.cs >> 1;
+    int sl = wmod(b0, l.slots), sm = wmod(b0, m.slots);
+    for (int p = 1; p < l.P; ++p) {
+        sl = sl == 0 ? l.slots - 1 : sl - 1;
+        sm = sm == 0 ? m.slots - 1 : sm - 1;
+        const float4* src = reinterpret_cast<const float4*>(l.X + (size_t)sl * l.cs);
+        float4* dst = reinterpret_cast<float4*>(m.X + (size_t)sm * l.cs);
+        for (int i = t; i < n4; i += nt) dst[i] = __ldcg(src + i);
+    }
+    const long long end = b0 << l.logN;
+    for (long long x = c * N0 + 4LL * t; x < end; x += 4LL * nt)
+        *reinterpret_cast<float4*>(m.yring + (x & m.rmask)) = __ldcg(reinterpret_cast<const float4*>(l.yring + (x & l.rmask)));
+}
+
 // launch that may overlap the previous kernel's tail (see above)
 template <class... KA, class... A>
 cudaError_t launch_dep(void (*k)(KA...), dim3 grid, int nt, size_t smem, cudaStream_t st, A&&... args) {
@@ -917,6 +938,11 @@ cudaError_t launch_wide_planar(const float* in, float* out, int channels, long l
     const int F = planar_frames(std::min(32, channels));
     return launch_dep(wide_planar_kernel, dim3((unsigned)((frames + F - 1) / F), (unsigned)((channels + 31) / 32)), 256, 0,
                       st, in, out, channels, pitch, frames);
+}
+
+cudaError_t launch_wide_move(const WLevel* lv, const WLevel* to, int nlv, long long step, int N0, cudaStream_t st) {
+    wide_move_kernel<<<dim3(nlv, nlv > 512 ? 4 : 64), 256, 0, st>>>(lv, to, step, N0);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_wide_reset(const WLevel* lv, int nlv, void* state, size_t bytes, cudaStream_t st) {

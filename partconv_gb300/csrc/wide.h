@@ -79,6 +79,8 @@ cudaError_t launch_wide_mix(const Bank& bank, int n_zero, bool mixed, const WArg
 // clears what a run from the start reads before it writes it: spectrum rows,
 // output rings, and the state region (16-byte aligned)
 cudaError_t launch_wide_reset(const WLevel* lv, int nlv, void* state, size_t bytes, cudaStream_t st);
+// what the rings of lv hold for the steps from `step` on, to the rings of to
+cudaError_t launch_wide_move(const WLevel* lv, const WLevel* to, int nlv, long long step, int N0, cudaStream_t st);
 // class-3 levels (cluster_fire.cu)
 cudaError_t launch_wide_cluster(bool inverse, int grid, const int2* map, const WArgs& a, cudaStream_t st);
 // the state one-block steps would have left after step a.c0 - 1

@@ -50,7 +50,8 @@ def test_pieces_of_a_long_host_call(gpu, layout, N0, n_in, N, L, blocks):
         return m.kernel_launches() - n
 
     # a chunk's launches and the one that ends the call: as many chunks as the
-    # call's pieces, of 4096 blocks each
+    # call's pieces, of 4096 blocks each (the first call also makes the workspace)
+    launches(CHUNK)
     full, rest = launches(CHUNK) - 1, launches(blocks % CHUNK) - 1 if blocks % CHUNK > 64 else 0
     n = launches(blocks) - 1
     assert n >= blocks // CHUNK * full + rest and n > full
