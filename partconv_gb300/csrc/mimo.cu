@@ -36,7 +36,9 @@
 // blocks instead of once per block (mimo_wide_mac_kernel).  It reads a second
 // copy of H laid out for it, Hw: [output pair][tile of kTile bins][input][part]
 // [bins of the tile] of (re0, re1, im0, im1), operands of packed (f32x2)
-// multiply-adds as they lie (an odd last output is paired with zeros).  One
+// multiply-adds as they lie (an odd last output is paired with zeros).  The first
+// such call makes that copy and the rings and sums of its chunks (ensure_wide); a
+// handle of short calls holds neither.  One
 // layout for both was slower for one of them: the one-block kernel on the
 // pairs ran 29.7 instead of 25.5 us per launch, the block-parallel one on the
 // tiles of single outputs 727 instead of 640 us per 128 blocks.
@@ -85,7 +87,7 @@ struct MLevel {
     int slots;      // rows of an input's spectrum ring (block b in row b mod slots)
     int nbw;        // most blocks of a block-parallel chunk
     float2* H;      // [nO][tile][nI][P][tile width]
-    float4* Hw;     // [output pair][tile of kTile][nI][P][tile width] (null: one-block steps only)
+    float4* Hw;     // [output pair][tile of kTile][nI][P][tile width] (null before the first block-parallel call)
     float2* X;      // [nI][slots][cs]
     float2* Yp;     // [nO][npart][2][cs]
     float2* Yf;     // [nO][cs]
@@ -627,10 +629,39 @@ __global__ void __launch_bounds__(NT) mimo_yifft_kernel(const MBank* __restrict_
     }
 }
 
+// where bin k of row ip (input, part) of rows lies in an output's tiles of H
+__device__ __forceinline__ size_t tile_elem(const int* __restrict__ tstart, int ntile, int k, int rows, int ip) {
+    int lo = 0, hi = ntile;   // tile t with tstart[t] <= k < tstart[t + 1]
+    while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (tstart[mid] <= k) lo = mid;
+        else hi = mid;
+    }
+    const int k0 = tstart[lo], w = tstart[lo + 1] - k0;
+    return (size_t)k0 * rows + (size_t)ip * w + (k - k0);
+}
+
+// Hw from H, one row (output pair, input, part) per CTA; an odd last output is
+// paired with zeros
+__global__ void __launch_bounds__(256) mimo_pair_kernel(const MBank* __restrict__ bank_p, int level) {
+    const MBank& bank = *bank_p;
+    const MLevel& l = bank.lv[level];
+    const int rows = bank.nI * l.P, cs = l.cs, op = blockIdx.x / rows, ip = blockIdx.x - op * rows;
+    const bool two = 2 * op + 1 < bank.nO;
+    const float2* h = l.H + (size_t)(2 * op) * rows * cs;
+    float4* d = l.Hw + (size_t)op * rows * cs;
+    for (int k = threadIdx.x; k < cs; k += blockDim.x) {
+        const size_t e = tile_elem(l.tstart, l.ntile, k, rows, ip);
+        const float2 a = h[e], b = two ? h[(size_t)rows * cs + e] : make_float2(0.f, 0.f);
+        const int t0 = tile_start(cs, k);
+        d[(size_t)t0 * rows + (size_t)ip * tile_width(cs, t0) + (k - t0)] = make_float4(a.x, b.x, a.y, b.y);
+    }
+}
+
 // filter spectra of one path row: H[o][i][p] = rfft([0_N, h_{i,o}[start + pN ...]]) / 2N
 template <int NT, int MAXB>
 __global__ void __launch_bounds__(NT) mimo_spectra_kernel(const float* __restrict__ irs, int ir_len, int nI, int nO,
-                                                          int N, int logN, int P, int cs, long long start, float2* H, float4* Hw,
+                                                          int N, int logN, int P, int cs, long long start, float2* H,
                                                           const int* __restrict__ tstart, int ntile,
                                                           const float2* W, int wlog) {
     extern __shared__ float4 dyn_smem[];
@@ -655,26 +686,9 @@ __global__ void __launch_bounds__(NT) mimo_spectra_kernel(const float* __restric
     fft_smem<NT, MAXB>(s, N, logN, tw, false);
     const float inv = 1.0f / (float)(2 * N);
     // bin k of path (i, o), part p goes to its tile: H[o][tile][i][p][k - tile start]
-    // and to Hw[o / 2][tile][i][p][k - tile start], (re, im) of output o mod 2
     float2* Ho = H + (size_t)o * nI * P * cs;
-    float* Hwo = reinterpret_cast<float*>(Hw + (size_t)(o >> 1) * nI * P * cs) + (o & 1);
     const int ip = i * P + p;
-    auto put = [&](int kb, float2 v) {
-        int lo = 0, hi = ntile;   // tile t with tstart[t] <= kb < tstart[t + 1]
-        while (hi - lo > 1) {
-            const int mid = (lo + hi) >> 1;
-            if (tstart[mid] <= kb) lo = mid;
-            else hi = mid;
-        }
-        const int k0 = tstart[lo], w = tstart[lo + 1] - k0;
-        Ho[(size_t)k0 * nI * P + (size_t)ip * w + (kb - k0)] = v;
-        if (Hw) {
-            const int t0 = tile_start(cs, kb);
-            float* d = Hwo + 4 * ((size_t)t0 * nI * P + (size_t)ip * tile_width(cs, t0) + (kb - t0));
-            d[0] = v.x;
-            d[2] = v.y;
-        }
-    };
+    auto put = [&](int kb, float2 v) { Ho[tile_elem(tstart, ntile, kb, nI * P, ip)] = v; };
     for (int k = threadIdx.x; k <= N / 2; k += NT) {
         const int nk = (k == 0) ? 0 : N - k;
         float2 xk, xnk;
@@ -723,8 +737,14 @@ struct pcm_handle {
     // block-parallel calls (wide.cu): descriptors of every (level, input) and
     // (output, level), CTA maps in order of their first block's step and the
     // prefix of each that a chunk of n + 1 steps needs
-    int C = 32;       // base steps per chunk
-    bool wide_ok = true;
+    int C_max = 32;   // most base steps per chunk
+    int C = 0;        // ... that the workspace in hand holds (0: none yet)
+    char* work = nullptr;    // rings and sums of chunks of C steps (before: the rings among `allocs`)
+    float4* hw = nullptr;    // the levels' Hw
+    size_t work_bytes = 0, hw_bytes = 0;
+    bool work_failed = false;   // no room for the smallest: one-block steps until reset
+    std::vector<WLevel> h_wlv;
+    WLevel* d_wlv_of[2] = {};   // d_wlv and the other buffer of it
     const float2* d_tab = nullptr;
     const WLevel* d_wlv = nullptr;
     const int* d_lv0 = nullptr;   // level-0 descriptor of every input
@@ -779,6 +799,12 @@ void mfree(pcm_handle* h) {
     for (void* p : h->allocs) cudaFree(p);
     h->allocs.clear();
     h->state.clear();
+    if (h->work) cudaFree(h->work);
+    if (h->hw) cudaFree(h->hw);
+    h->work = nullptr;
+    h->hw = nullptr;
+    h->work_bytes = h->hw_bytes = 0;
+    h->C = 0;
     if (h->used) cudaEventDestroy(h->used);
     h->used = nullptr;
     if (h->stream) cudaStreamDestroy(h->stream);
@@ -816,7 +842,8 @@ cudaError_t launch_mac(pcm_handle* h, int grid, const MTask* tasks, const RunSta
 int setup_wide(pcm_handle* h) {
     const MBank& B = h->hbank;
     const int M = h->M, nI = h->nI, nO = h->nO;
-    std::vector<WLevel> wl;
+    std::vector<WLevel>& wl = h->h_wlv;
+    wl.clear();
     std::vector<int> lv0(nI);
     auto common = [&](int L) {
         const MLevel& l = B.lv[L];
@@ -853,7 +880,6 @@ int setup_wide(pcm_handle* h) {
             w.mix_mode = 1;
             w.lv0 = out0 + o * M;
             w.rmask = l.rmask;
-            w.Yw = l.Yw + (size_t)o * l.nbw * l.cs;
             w.yring = l.yring + (size_t)o * (l.rmask + 1);
             wl.push_back(w);
         }
@@ -863,13 +889,14 @@ int setup_wide(pcm_handle* h) {
     std::vector<std::pair<int, int4>> mac;
     for (int L = 0; L < M; ++L) {
         const MLevel& l = B.lv[L];
-        for (int b = 0; b < l.nbw; b += 16 * h->w_nt / l.N) {
+        const int nbw = (h->C_max + l.T - 1) / l.T;   // most blocks of a chunk
+        for (int b = 0; b < nbw; b += 16 * h->w_nt / l.N) {
             for (int i = 0; i < nI; ++i) e[0].push_back({b * l.T, make_int2(i * M + L, b)});
             for (int o = 0; o < nO && L > 0; ++o) e[1].push_back({b * l.T, make_int2(out0 + o * M + L, b)});
         }
-        for (int b = 0; b < l.nbw && L == 0; b += wide_out_blocks(l.N))
+        for (int b = 0; b < nbw && L == 0; b += wide_out_blocks(l.N))
             for (int o = 0; o < nO; ++o) e[2].push_back({b, make_int2(out0 + o * M, b)});
-        for (int b = 0; b < l.nbw; b += kSegBlocks)
+        for (int b = 0; b < nbw; b += kSegBlocks)
             for (int k = 0; k < l.cs; k += kTile)   // (the last two bins by themselves)
                 for (int o = 0; o < nO; o += kOB) mac.push_back({b * l.T, make_int4(L, k, o, b)});
     }
@@ -886,19 +913,20 @@ int setup_wide(pcm_handle* h) {
         std::stable_sort(v.begin(), v.end(), [](auto& a, auto& b) { return a.first < b.first; });
         std::vector<E> flat;
         for (auto& x : v) flat.push_back(x.second);
-        upto.assign(h->C, 0);
+        upto.assign(h->C_max, 0);
         size_t j = 0;
-        for (int n = 0; n < h->C; ++n) {
+        for (int n = 0; n < h->C_max; ++n) {
             while (j < v.size() && v[j].first <= n) ++j;
             upto[n] = (int)j;
         }
         return put(flat.data(), sizeof(E) * flat.size());
     };
-    size_t at[6];
+    size_t at[7];
     for (int m = 0; m < 3; ++m) at[m] = put_map(e[m], h->w_upto[m]);
     at[3] = put_map(mac, h->w_upto[3]);
     at[4] = put(wl.data(), sizeof(WLevel) * wl.size());
     at[5] = put(lv0.data(), sizeof(int) * lv0.size());
+    at[6] = put(wl.data(), sizeof(WLevel) * wl.size());
     char* d = nullptr;
     MCK(cudaMalloc(&d, blob.size()), "alloc tables");
     h->allocs.push_back(d);
@@ -907,9 +935,133 @@ int setup_wide(pcm_handle* h) {
     MCK(cudaStreamSynchronize(h->stream), "sync");
     for (int m = 0; m < 3; ++m) h->w_map[m] = reinterpret_cast<const int2*>(d + at[m]);
     h->w_mac = reinterpret_cast<const int4*>(d + at[3]);
-    h->d_wlv = reinterpret_cast<const WLevel*>(d + at[4]);
+    h->d_wlv_of[0] = reinterpret_cast<WLevel*>(d + at[4]);
+    h->d_wlv_of[1] = reinterpret_cast<WLevel*>(d + at[6]);
+    h->d_wlv = h->d_wlv_of[0];
     h->d_lv0 = reinterpret_cast<const int*>(d + at[5]);
     MCK(launch_wide_reset(h->d_wlv, h->n_wlv, nullptr, 0, h->stream), "clear rings");
+    return PC_OK;
+}
+
+// rings of a level for chunks of C steps (0: one-block steps)
+int ring_rows(const MLevel& l, int C) { return l.P + (C > 0 ? std::max((C + l.T - 1) / l.T, kBB) : 0); }
+long ring_samples(const MLevel& l, int N0, int C) {
+    long R = l.N;
+    while (R < ((long)l.s_blocks + std::max(C, 1)) * N0) R <<= 1;   // samples in flight
+    return R;
+}
+
+// A workspace for chunks of up to C steps in place of the present one, its rings
+// holding what the present ones do, and Hw if there is none yet.  PC_ERR_NOMEM if
+// there is no room: everything stays as it is.
+int move_to_work(pcm_handle* h, int C, cudaStream_t st) {
+    MBank B = h->hbank;
+    const int nI = h->nI, nO = h->nO;
+    size_t bytes = 0, hw_elems = 0;
+    auto take = [&](size_t n) {
+        const size_t o = bytes;
+        bytes += (n + 255) & ~(size_t)255;
+        return o;
+    };
+    std::vector<size_t> oX(h->M), oY(h->M), oR(h->M), oH(h->M);
+    for (int L = 0; L < h->M; ++L) {
+        MLevel& l = B.lv[L];
+        l.nbw = (C + l.T - 1) / l.T;
+        l.slots = ring_rows(l, C);
+        const long R = ring_samples(l, h->N0, C);
+        l.rmask = (int)R - 1;
+        if ((long long)nI * l.slots * l.cs >= (1LL << 31)) return PC_ERR_NOMEM;   // 32-bit offsets
+        oX[L] = take(sizeof(float2) * (size_t)nI * l.slots * l.cs);
+        oY[L] = take(sizeof(float2) * (size_t)nO * l.nbw * l.cs);
+        oR[L] = take(sizeof(float) * (size_t)nO * R);
+        oH[L] = hw_elems;
+        hw_elems += (size_t)((nO + 1) / 2) * nI * l.P * l.cs;
+    }
+    // (another thread may be capturing a graph meanwhile)
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    char* W = nullptr;
+    float4* hw = h->hw;
+    cudaError_t e = cudaMalloc(&W, bytes);
+    if (e == cudaSuccess && !hw) e = cudaMalloc(&hw, sizeof(float4) * hw_elems);
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        if (W) cudaFree(W);
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        return PC_ERR_NOMEM;
+    }
+    for (int L = 0; L < h->M; ++L) {
+        MLevel& l = B.lv[L];
+        l.X = reinterpret_cast<float2*>(W + oX[L]);
+        l.Yw = reinterpret_cast<float2*>(W + oY[L]);
+        l.yring = reinterpret_cast<float*>(W + oR[L]);
+        l.Hw = hw + oH[L];
+    }
+    std::vector<WLevel> wl = h->h_wlv;
+    for (int j = 0; j < h->n_wlv; ++j) {   // the inputs' levels, then the outputs'
+        const int L = j % h->M, ch = j / h->M;
+        const MLevel& l = B.lv[L];
+        WLevel& w = wl[j];
+        w.slots = l.slots;
+        if (ch < nI) {
+            w.X = l.X + (size_t)ch * l.slots * l.cs;
+        } else {
+            w.rmask = l.rmask;
+            w.Yw = l.Yw + (size_t)(ch - nI) * l.nbw * l.cs;
+            w.yring = l.yring + (size_t)(ch - nI) * (l.rmask + 1);
+        }
+    }
+    WLevel* next = h->d_wlv == h->d_wlv_of[0] ? h->d_wlv_of[1] : h->d_wlv_of[0];
+    e = cudaMemcpyAsync(next, wl.data(), sizeof(WLevel) * wl.size(), cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(h->d_bank, &B, sizeof(MBank), cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess) e = launch_wide_move(h->d_wlv, next, h->n_wlv, h->frame_num, h->N0, st);
+    for (int L = 0; L < h->M && !h->hw && e == cudaSuccess; ++L) {
+        mimo_pair_kernel<<<(nO + 1) / 2 * nI * B.lv[L].P, 256, 0, st>>>(h->d_bank, L);
+        e = cudaGetLastError();
+    }
+    if (h->work || e != cudaSuccess) {   // nothing may still read what is freed
+        const cudaError_t se = cudaStreamSynchronize(st);
+        if (e == cudaSuccess) e = se;
+        cudaFree(e == cudaSuccess ? h->work : W);
+        if (e != cudaSuccess && !h->hw) cudaFree(hw);
+    }
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    MCK(e, "block-parallel workspace");
+    h->launches += 1 + (h->hw ? 0 : h->M);
+    h->work = W;
+    h->work_bytes = bytes;
+    if (!h->hw) {
+        h->hw = hw;
+        h->hw_bytes = sizeof(float4) * hw_elems;
+    }
+    h->C = C;
+    h->hbank = B;
+    h->h_wlv.swap(wl);
+    h->d_wlv = next;
+    return PC_OK;
+}
+
+// Whether a call of nsteps base steps on st can run block-parallel: the workspace
+// is made for it, in chunks as short as the call, and grows with longer calls up
+// to h->C_max steps; where there is no room, a shorter chunk or one-block steps
+// serve.  A stream that is being captured takes the workspace as it is.
+int ensure_wide(pcm_handle* h, long long nsteps, cudaStream_t st, bool* wide) {
+    int want = kWideMinChunk;
+    while (want < nsteps && want < h->C_max) want <<= 1;
+    *wide = h->C > 0;
+    if (h->C >= want || h->work_failed) return PC_OK;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    MCK(cudaStreamIsCapturing(st, &cs), "capture status");
+    if (cs != cudaStreamCaptureStatusNone) return PC_OK;
+    for (; want > h->C && want >= kWideMinChunk; want >>= 1) {
+        const int r = move_to_work(h, want, st);
+        if (r == PC_OK) {
+            *wide = true;
+            return PC_OK;
+        }
+        if (r != PC_ERR_NOMEM) return r;
+        h->work_failed = true;   // (of the size asked for: not tried again until reset)
+    }
     return PC_OK;
 }
 
@@ -1023,10 +1175,11 @@ int pcm_setup(pcm_handle* h, int fs, int buffer_size, int n_in, int n_out, int M
     }
     {
         const double row = sizeof(float2) * (double)buffer_size * M * std::max(n_in, n_out);   // per base step
-        h->wide_ok = true;
         h->tiles.clear();
-        h->C = kWideMaxChunk;
-        while (h->C > kWideMinChunk && h->C * row > (double)kWideBytes) h->C >>= 1;
+        h->work_failed = false;
+        h->C = 0;
+        h->C_max = kWideMaxChunk;
+        while (h->C_max > kWideMinChunk && h->C_max * row > (double)kWideBytes) h->C_max >>= 1;
     }
     // twiddles
     float2* W = nullptr;
@@ -1068,8 +1221,7 @@ int pcm_setup(pcm_handle* h, int fs, int buffer_size, int n_in, int n_out, int M
         l.T = Nv[L] / buffer_size;
         l.s_blocks = (int)(s / buffer_size);
         l.cs = Nv[L] + 2;
-        long R = Nv[L];
-        while (R < s + (long)h->C * buffer_size) R <<= 1;   // a chunk's samples in flight
+        const long R = ring_samples(l, buffer_size, 0);
         l.rmask = (int)R - 1;
         // input ranges per spread task (about 8 inputs each, more ranges when
         // a range times the older parts exceeds what one MAC task sums)
@@ -1131,22 +1283,12 @@ int pcm_setup(pcm_handle* h, int fs, int buffer_size, int n_in, int n_out, int M
             h->tiles.push_back(ts);
         }
         MCK(malloc_zero(h, &l.H, (size_t)n_out * n_in * l.P * l.cs, false), "alloc H");
-        // the copy for block-parallel calls; without room for it every call runs one-block steps
-        if (h->wide_ok &&
-            malloc_zero(h, &l.Hw, (size_t)((n_out + 1) / 2) * n_in * l.P * l.cs, false) != cudaSuccess) {
-            cudaGetLastError();
-            l.Hw = nullptr;
-            h->wide_ok = false;
-        }
-        l.nbw = (h->C + l.T - 1) / l.T;
-        l.slots = l.P + std::max(l.nbw, kBB);
-        if ((long long)n_in * l.slots * l.cs >= (1LL << 31)) {   // 32-bit offsets: one-block steps only
-            l.slots = l.P;
-            h->wide_ok = false;
-        }
+        l.Hw = nullptr;
+        l.Yw = nullptr;
+        l.nbw = 0;
+        l.slots = ring_rows(l, 0);
         // (cleared in part by setup_wide)
         MCK(malloc_raw(h, &l.X, (size_t)n_in * l.slots * l.cs), "alloc");
-        MCK(malloc_raw(h, &l.Yw, (size_t)n_out * l.nbw * l.cs), "alloc");
         MCK(malloc_zero(h, &l.Yp, (size_t)n_out * l.npart * 2 * l.cs, true), "alloc");
         MCK(malloc_zero(h, &l.Yf, (size_t)n_out * l.cs, true), "alloc");
         MCK(malloc_raw(h, &l.yring, (size_t)n_out * R), "alloc");
@@ -1155,15 +1297,15 @@ int pcm_setup(pcm_handle* h, int fs, int buffer_size, int n_in, int n_out, int M
         switch (cls_of(l.N)) {
             case 0:
                 mimo_spectra_kernel<256, 1><<<rows, 256, smem, h->stream>>>(d_irs, ir_len, n_in, n_out, l.N, l.logN, l.P,
-                                                                            l.cs, s, l.H, l.Hw, l.tstart, l.ntile, W, kWlog);
+                                                                            l.cs, s, l.H, l.tstart, l.ntile, W, kWlog);
                 break;
             case 1:
                 mimo_spectra_kernel<512, 2><<<rows, 512, smem, h->stream>>>(d_irs, ir_len, n_in, n_out, l.N, l.logN, l.P,
-                                                                            l.cs, s, l.H, l.Hw, l.tstart, l.ntile, W, kWlog);
+                                                                            l.cs, s, l.H, l.tstart, l.ntile, W, kWlog);
                 break;
             default:
                 mimo_spectra_kernel<512, 8><<<rows, 512, smem, h->stream>>>(d_irs, ir_len, n_in, n_out, l.N, l.logN, l.P,
-                                                                            l.cs, s, l.H, l.Hw, l.tstart, l.ntile, W, kWlog);
+                                                                            l.cs, s, l.H, l.tstart, l.ntile, W, kWlog);
                 break;
         }
         MCK(cudaGetLastError(), "MIMO spectra");
@@ -1293,7 +1435,12 @@ int pcm_process_device(pcm_handle* h, float* d_out, const float* d_in, long long
         rs.io.out_ch = 1;
     }
     const long long nsteps = frames / h->N0;
-    if (nsteps >= kWideMinSteps && h->wide_ok) {
+    bool wide = nsteps >= kWideMinSteps;
+    if (wide) {
+        const int r = ensure_wide(h, nsteps, st, &wide);
+        if (r) return r;
+    }
+    if (wide) {
         int r = mimo_wide(h, rs.io, nsteps, st);
         if (r) return r;
     } else {
@@ -1312,6 +1459,7 @@ int pcm_reset(pcm_handle* h) {
     if (!h) return PC_ERR_ARG;
     h->frame_num = 0;
     if (!h->ready) return PC_OK;
+    h->work_failed = false;
     cudaSetDevice(h->device);
     MCK(cudaStreamWaitEvent(h->stream, h->used, 0), "reset");   // calls still running on a caller's stream
     for (auto& z : h->state) MCK(cudaMemsetAsync(z.first, 0, z.second, h->stream), "reset");
@@ -1379,7 +1527,9 @@ int pcm_profile_kernels(pcm_handle* h, long long nsteps, pc_kernel_stats* out, i
     return PC_OK;
 }
 
-long long pcm_device_bytes(const pcm_handle* h) { return h ? h->device_bytes : 0; }
+long long pcm_device_bytes(const pcm_handle* h) {
+    return h ? h->device_bytes + (long long)(h->work_bytes + h->hw_bytes) : 0;
+}
 long long pcm_kernel_launches(const pcm_handle* h) { return h ? h->launches : 0; }
 const char* pcm_last_error(const pcm_handle* h) { return h ? h->err.c_str() : ""; }
 

@@ -788,7 +788,7 @@ __global__ void wide_move_kernel(const WLevel* __restrict__ lv, const WLevel* __
         float4* dst = reinterpret_cast<float4*>(m.X + (size_t)sm * l.cs);
         for (int i = t; i < n4; i += nt) dst[i] = __ldcg(src + i);
     }
-    const long long end = b0 << l.logN;
+    const long long end = l.yring ? b0 << l.logN : 0;
     for (long long x = c * N0 + 4LL * t; x < end; x += 4LL * nt)
         *reinterpret_cast<float4*>(m.yring + (x & m.rmask)) = __ldcg(reinterpret_cast<const float4*>(l.yring + (x & l.rmask)));
 }
