@@ -258,8 +258,8 @@ __global__ void __cluster_dims__(kC, 1, 1) __launch_bounds__(kNT)
             a = __ldcg(&Ypb[pos]);
             for (int qr = 1; qr < npart; ++qr) a = cadd(a, __ldcg(&Ypb[qr * rstride + pos]));
         }
-        if (use_x1) a = cadd(a, cmul(__ldg(&tk.H[cs + pos]), __ldcg(&X1[pos])));
-        return cadd(cmul(__ldg(&tk.H[pos]), x), a);
+        if (use_x1) a = cadd(a, cmul(__ldcg(&X1[pos]), __ldg(&tk.H[cs + pos])));
+        return cadd(cmul(x, __ldg(&tk.H[pos])), a);
     };
     const int np = pair_count(g);
     float2 zo[kMaxPairs][2];

@@ -28,9 +28,14 @@ namespace pcg {
 
 // Rounding is spelled out (one product, one fused multiply-add per component),
 // so every kernel that inlines it gives the same bits: the one-block steps and
-// the block-parallel path must agree exactly.
+// the block-parallel path must agree exactly.  Both components round a's product
+// with b.x (cmac's order, from zero).  Of the four choices the two that round
+// a.x b.x have the least error: callbacks of 2^17 taps at 256 samples 2.485e-7
+// (relative, against float64, mean of four seeds) so, 2.522e-7 with -a.y b.y
+// rounded, 2.508e-7 as the compiler contracts the plain expression; 64 pool
+// channels 2.310e-7, 2.325e-7 and 2.318e-7.
 __device__ __forceinline__ float2 cmul(float2 a, float2 b) {
-    return make_float2(__fmaf_rn(a.x, b.x, -__fmul_rn(a.y, b.y)), __fmaf_rn(a.x, b.y, __fmul_rn(a.y, b.x)));
+    return make_float2(__fmaf_rn(-a.y, b.y, __fmul_rn(a.x, b.x)), __fmaf_rn(a.x, b.y, __fmul_rn(a.y, b.x)));
 }
 // acc + x h, two fused multiply-adds per component: first with h.x, then with
 // h.y, the order in which pairs of components fill packed instructions
@@ -503,16 +508,15 @@ __device__ __forceinline__ float2 mul_pi(float2 a) { return make_float2(-a.y, a.
 // 8-point DFT in registers, decimation in frequency (unnormalised; inverse =
 // conjugate rotations).  Output in natural order.
 __device__ __forceinline__ void dft8(float2 v[8], bool inv) {
-    // stage 1: pairs (i, i + 4), rotation w8^i of the differences
+    // stage 1: pairs (i, i + 4), rotation w8^i of the differences; those of i = 1
+    // and 3 without their factor sqrt(1/2), which stage 2 takes in (one rounding less)
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         const float2 a = cadd(v[i], v[i + 4]);
         float2 d = csub(v[i], v[i + 4]);
-        if (i == 1) d = inv ? make_float2(__fmul_rn(kSqrtHalf8, d.x - d.y), __fmul_rn(kSqrtHalf8, d.x + d.y))
-                            : make_float2(__fmul_rn(kSqrtHalf8, d.x + d.y), __fmul_rn(kSqrtHalf8, d.y - d.x));
+        if (i == 1) d = inv ? make_float2(d.x - d.y, d.x + d.y) : make_float2(d.x + d.y, d.y - d.x);
         if (i == 2) d = inv ? mul_pi(d) : mul_mi(d);
-        if (i == 3) d = inv ? make_float2(__fmul_rn(-kSqrtHalf8, d.x + d.y), __fmul_rn(kSqrtHalf8, d.x - d.y))
-                            : make_float2(__fmul_rn(kSqrtHalf8, d.y - d.x), __fmul_rn(-kSqrtHalf8, d.x + d.y));
+        if (i == 3) d = inv ? make_float2(-(d.x + d.y), d.x - d.y) : make_float2(d.y - d.x, -(d.x + d.y));
         v[i] = a;
         v[i + 4] = d;
     }
@@ -521,8 +525,15 @@ __device__ __forceinline__ void dft8(float2 v[8], bool inv) {
     for (int h = 0; h < 8; h += 4) {
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
-            const float2 a = cadd(v[h + i], v[h + i + 2]);
-            float2 d = csub(v[h + i], v[h + i + 2]);
+            float2 a, d;
+            if (h == 4 && i == 1) {
+                const float2 p = v[5], q = make_float2(__fmul_rn(kSqrtHalf8, v[7].x), __fmul_rn(kSqrtHalf8, v[7].y));
+                a = make_float2(__fmaf_rn(kSqrtHalf8, p.x, q.x), __fmaf_rn(kSqrtHalf8, p.y, q.y));
+                d = make_float2(__fmaf_rn(kSqrtHalf8, p.x, -q.x), __fmaf_rn(kSqrtHalf8, p.y, -q.y));
+            } else {
+                a = cadd(v[h + i], v[h + i + 2]);
+                d = csub(v[h + i], v[h + i + 2]);
+            }
             if (i == 1) d = inv ? mul_pi(d) : mul_mi(d);
             v[h + i] = a;
             v[h + i + 2] = d;

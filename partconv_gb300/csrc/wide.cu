@@ -193,26 +193,23 @@ struct MacCol {
     __device__ __forceinline__ float2 h() const { return __ldg(H); }
 };
 
-// Sums X_{b+j-p} H_p, j < RB, over n consecutive parts in groups of tg, a group
-// in running sums of `unit` parts (running sums added in order into the group,
-// groups in order into row); c stands at the first part on entry and after the
-// last one on return.  The run's RB spectra under part p stay in registers:
-// part p + 1 needs one new one.  The loads of four parts go together.
+// Sums X_{b+j-p} H_p, j < RB, over n consecutive parts, last to first, in groups
+// of tg, a group in running sums of `unit` parts (running sums added in order
+// into the group, groups in order into row); c stands at the last part on entry.
+// The run's RB spectra under part p stay in registers: part p - 1 needs one new
+// one.  The loads of four parts go together.
 template <int RB>
-__device__ __forceinline__ void sum_parts(MacCol& c, int n, int tg, int unit, f32x2 (&row)[RB]) {
+__device__ __forceinline__ void sum_parts(MacCol c, int n, int tg, int unit, f32x2 (&row)[RB]) {
     constexpr int U = 4;
     static_assert(RB % U == 0, "constant window rotation");
-    f32x2 acc[RB], w[RB], ws[RB];   // window: block (run's first) + d - first part at w[d mod RB], and its swapped pairs
+    f32x2 acc[RB], w[RB], ws[RB];   // window: block (run's first) + d - last part at w[d mod RB], and its swapped pairs
     f32x2 grp[RB];
-    {
-        int o = c.ox;
 #pragma unroll
-        for (int j = 0; j < RB; ++j) {
-            row[j] = acc[j] = grp[j] = 0;
-            w[j] = c.x(o);
-            ws[j] = swap2(w[j]);
-            o = c.fwd(o);
-        }
+    for (int j = 0; j < RB; ++j) {
+        row[j] = acc[j] = grp[j] = 0;
+        w[j] = c.x(c.ox);
+        ws[j] = swap2(w[j]);
+        c.ox = c.fwd(c.ox);
     }
     int left = tg, run = unit;   // parts until the group and the running sum end
     for (int i0 = 0; i0 < n; i0 += RB) {
@@ -225,23 +222,22 @@ __device__ __forceinline__ void sum_parts(MacCol& c, int n, int tg, int unit, f3
             for (int u = 0; u < U; ++u)
                 if (i0 + s * U + u < n) {
                     h[u] = c.h();
-                    c.H += c.cs;
-                    c.ox = c.back(c.ox);
-                    nx[u] = c.x(c.ox);
+                    c.H -= c.cs;
+                    nx[u] = c.x(c.ox);   // (not used after the last one)
+                    c.ox = c.fwd(c.ox);
                 }
 #pragma unroll
             for (int u = 0; u < U; ++u) {
                 if (i0 + s * U + u >= n) break;
-                const int r = s * U + u;   // part index mod RB
+                const int r = s * U + u;   // r-th part from the last, mod RB
                 const f32x2 hr = pack2(h[u].x, h[u].x), hi = pack2(-h[u].y, h[u].y);
 #pragma unroll
                 for (int j = 0; j < RB; ++j) {
-                    const int q = (j - r + RB) % RB;
+                    const int q = (j + r) % RB;
                     acc[j] = cmac2(acc[j], w[q], ws[q], hr, hi);
                 }
-                const int q = (RB - 1 - r + RB) % RB;
-                w[q] = nx[u];
-                ws[q] = swap2(nx[u]);
+                w[r % RB] = nx[u];
+                ws[r % RB] = swap2(nx[u]);
                 --left;
                 if (--run == 0 || left == 0 || i0 + r + 1 == n) {
                     run = unit;
@@ -297,8 +293,8 @@ __device__ __forceinline__ void finish_run(const MacCol& c, const WLevel& l, con
     for (int j = 0; j < RB; ++j) {
         const float2 x = unpack2(c.x(o));
         float2 s = unpack2(ys[j]);
-        if (x1) s = rows ? cadd(cmul(h1, xm), s) : cmul(h1, xm);
-        const float2 y = cadd(cmul(h0, x), s);
+        if (x1) s = rows ? cadd(cmul(xm, h1), s) : cmul(xm, h1);
+        const float2 y = cadd(cmul(x, h0), s);
         if (j < live) Y[(size_t)j * l.cs] = y;
         xm = x;
         o = c.fwd(o);
@@ -317,24 +313,24 @@ __device__ __forceinline__ void cp_async_wait() {
     asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
 }
 
-// row[j] = sum of X_{b+j-p} H_p over n consecutive parts in groups of four, from
-// shared memory; x: the spectrum of the run's first block under the first of
-// them, h: that part's row.  The window of a run under one part (RB spectra and
-// their swapped pairs) stays in registers: the next part needs one new one.
+// row[j] = sum of X_{b+j-p} H_p over n consecutive parts, last to first, in groups
+// of four, from shared memory; x: the spectrum of the run's first block under the
+// last of them, h: that part's row.  The window of a run under one part (RB spectra
+// and their swapped pairs) stays in registers: the part before needs one new one.
 // Shared rows are kMacTile apart, so every row is at a constant offset.  The
-// loads of four parts go together (the one after the last part is not used: it
-// is the shared row before the oldest spectrum).
+// loads of four parts go together (the spectrum after the first part is not used:
+// it may be the shared row after the newest one).
 template <int RB>
 __device__ __forceinline__ void sum_groups(const f32x2* x, const float2* h, int n, f32x2 (&row)[RB]) {
     constexpr int U = 4, W = kMacTile;
     static_assert(RB % U == 0, "constant window rotation");
-    f32x2 w[RB], ws[RB];   // the block of run index j under part r at w[(j - r) mod RB]
+    f32x2 w[RB], ws[RB];   // the block of run index j under the r-th part from the last at w[(j + r) mod RB]
 #pragma unroll
     for (int j = 0; j < RB; ++j) {
         w[j] = x[j * W];
         ws[j] = swap2(w[j]);
     }
-    for (int i0 = 0; i0 < n; i0 += RB, x -= RB * W, h += RB * W) {
+    for (int i0 = 0; i0 < n; i0 += RB, x += RB * W, h -= RB * W) {
 #pragma unroll
         for (int s = 0; s < RB; s += U) {
             if (i0 + s >= n) break;
@@ -343,8 +339,8 @@ __device__ __forceinline__ void sum_groups(const f32x2* x, const float2* h, int 
 #pragma unroll
             for (int u = 0; u < U; ++u)
                 if (i0 + s + u < n) {
-                    hv[u] = h[(s + u) * W];
-                    nx[u] = x[-(s + u + 1) * W];
+                    hv[u] = h[-(s + u) * W];
+                    nx[u] = x[(RB + s + u) * W];
                 }
 #pragma unroll
             for (int u = 0; u < U; ++u) {
@@ -352,12 +348,11 @@ __device__ __forceinline__ void sum_groups(const f32x2* x, const float2* h, int 
                 const f32x2 hr = pack2(hv[u].x, hv[u].x), hi = pack2(-hv[u].y, hv[u].y);
 #pragma unroll
                 for (int j = 0; j < RB; ++j) {
-                    const int q = (j + RB - s - u) % RB;
+                    const int q = (j + s + u) % RB;
                     acc[j] = u == 0 ? fma2(ws[q], hi, mul2(w[q], hr)) : cmac2(acc[j], w[q], ws[q], hr, hi);
                 }
-                const int q = RB - 1 - s - u;
-                w[q] = nx[u];
-                ws[q] = swap2(nx[u]);
+                w[s + u] = nx[u];
+                ws[s + u] = swap2(nx[u]);
             }
 #pragma unroll
             for (int j = 0; j < RB; ++j) row[j] = i0 + s == 0 ? acc[j] : add2(row[j], acc[j]);
@@ -367,7 +362,7 @@ __device__ __forceinline__ void sum_groups(const f32x2* x, const float2* h, int 
 
 // Y = X_b H_0 + (X_{b-1} H_1 + row) for the run, X_{b-1} H_1 with x1 and the row
 // with rows; x, h: the shared rows of the run's first block and of part 0.
-// Products as cmul(H, X).
+// Products as cmul(X, H).
 template <int RB>
 __device__ __forceinline__ void mac_finish(const f32x2* x, const float2* h, bool x1, bool rows, const f32x2 (&row)[RB],
                                            float2* Y, int cs, int live) {
@@ -381,10 +376,10 @@ __device__ __forceinline__ void mac_finish(const f32x2* x, const float2* h, bool
         const f32x2 xj = x[j * W], xs = swap2(xj);
         f32x2 s = row[j];
         if (x1) {
-            const f32x2 m1 = fma2(xm, hr1, mul2(xms, hi1));
+            const f32x2 m1 = fma2(xms, hi1, mul2(xm, hr1));
             s = rows ? add2(m1, s) : m1;
         }
-        if (j < live) y[(size_t)j * cs] = add2(fma2(xj, hr0, mul2(xs, hi0)), s);
+        if (j < live) y[(size_t)j * cs] = add2(fma2(xs, hi0, mul2(xj, hr0)), s);
         xm = xj;
         xms = xs;
     }
@@ -464,7 +459,19 @@ __global__ void __launch_bounds__(kMacTile, 4) wide_mac_kernel(const int4* __res
                 f32x2 row[RB];
 #pragma unroll
                 for (int j = 0; j < RB; ++j) row[j] = 0;
-                if (P > l.p_lo) sum_groups<RB>(x - l.p_lo * W, Hs + tid + l.p_lo * W, P - l.p_lo, row);
+                if (P > l.p_lo) {
+                    const int n1 = min(P, l.p_lo + kMacRes - 2);   // end of the first partial-sum row
+                    sum_groups<RB>(x - (n1 - 1) * W, Hs + tid + (n1 - 1) * W, n1 - l.p_lo, row);
+                    if (n1 < P) {   // (p_lo = 1: a part is left)
+                        const float2 h = Hs[tid + n1 * W];
+                        const f32x2 hr = pack2(h.x, h.x), hi = pack2(-h.y, h.y);
+#pragma unroll
+                        for (int j = 0; j < RB; ++j) {
+                            const f32x2 xj = x[(j - n1) * W];
+                            row[j] = add2(row[j], fma2(swap2(xj), hi, mul2(xj, hr)));
+                        }
+                    }
+                }
                 mac_finish<RB>(x, Hs + tid, l.two && P > 1, P > l.p_lo, row, y, cs, n - i);
             }
             sl += S;
@@ -475,7 +482,7 @@ __global__ void __launch_bounds__(kMacTile, 4) wide_mac_kernel(const int4* __res
     // shared rows: filter rows 0 and 1, the run's spectra and the one before them,
     // its partial sums so far, then the row of parts at hand
     constexpr int XH = 2, YS = XH + 1 + RB, HS = YS + RB;
-    static_assert(HS + 2 * (kMacRes - 2) - 1 + RB <= kMacRows, "a partial-sum row's parts");
+    static_assert(HS + 2 * (kMacRes - 2) + RB <= kMacRows, "a partial-sum row's parts, and the row after them");
     f32x2* ys = reinterpret_cast<f32x2*>(Hs + YS * W) + tid;
     for (int i0 = e.z; i0 < nb; i0 += RB) {
         for (int q = 0; q < l.nrows; ++q) {
@@ -494,7 +501,7 @@ __global__ void __launch_bounds__(kMacTile, 4) wide_mac_kernel(const int4* __res
             __syncthreads();
             if (live) {
                 f32x2 row[RB];
-                sum_groups<RB>(reinterpret_cast<const f32x2*>(Xs + (n - 1) * W) + tid, Hs + HS * W + tid, n, row);
+                sum_groups<RB>(reinterpret_cast<const f32x2*>(Xs) + tid, Hs + (HS + n - 1) * W + tid, n, row);
                 if (q > 0) {
 #pragma unroll
                     for (int j = 0; j < RB; ++j) row[j] = add2(ys[j * W], row[j]);
@@ -531,17 +538,18 @@ __global__ void __launch_bounds__(kMacAnyNT, 3) wide_mac_any_kernel(const int4* 
     if (i0 >= nb) return;
     int sl = wmod(bf, R) + i0;   // ring row of the run's first block
     if (sl >= R) sl -= R;
-    MacCol c{l.H + (size_t)l.p_lo * cs + k, l.X + k, cs, R * cs, 0};
+    MacCol c{l.H + k, l.X + k, cs, R * cs, 0};
     f32x2 ys[RB];   // partial-sum rows of the parts >= p_lo
 #pragma unroll
     for (int j = 0; j < RB; ++j) ys[j] = 0;
     const bool rows = P > l.p_lo;
     if (rows) {
-        const int o = sl - l.p_lo;
-        c.ox = (o < 0 ? o + R : o) * cs;
         for (int q = 0; q < l.nrows; ++q) {
             f32x2 row[RB];
-            sum_parts<RB>(c, min(l.tp, P - l.p_lo - q * l.tp), l.tpg, l.multi ? 2 : 4, row);
+            const int n = min(l.tp, P - l.p_lo - q * l.tp), p = l.p_lo + q * l.tp + n - 1;   // the row's last part
+            c.H = l.H + (size_t)p * cs + k;
+            c.ox = (sl < p ? sl - p + R : sl - p) * cs;
+            sum_parts<RB>(c, n, l.tpg, l.multi ? 2 : 4, row);
 #pragma unroll
             for (int j = 0; j < RB; ++j) ys[j] = q == 0 ? row[j] : add2(ys[j], row[j]);
         }
