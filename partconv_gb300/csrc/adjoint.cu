@@ -511,8 +511,8 @@ pcd_plan* pcd_create(int M, const int* N, int* P, int ir_len, int batch, long lo
     p->o_Dp = take(off, row * p->P * p->nrun * batch);
     p->o_D = take(off, row * p->P);
     p->total = off;
-    if ((long long)p->slots * p->cs >= (1LL << 31) || build_tables(p) != PC_OK) {
-        put(p->err.empty() ? "signal too long for one plan" : p->err.c_str());
+    if (build_tables(p) != PC_OK) {
+        put(p->err.c_str());
         delete p;
         return nullptr;
     }
