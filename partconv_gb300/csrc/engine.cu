@@ -1463,10 +1463,14 @@ int finish_wide(pc_handle* h, const IOView& view, cudaStream_t st) {
 // launches for a few steps, block-parallel chunks for more.  A call in several
 // pieces (pc_process's pipeline, one view for all of them) passes more = true
 // for all but the last and again = true for all but the first; pieces that find
-// no workspace run one-block steps, later ones may run block-parallel.
+// no workspace run one-block steps, later ones may run block-parallel.  in_place:
+// the output overlaps the input, of which a chunk reads blocks before its own, and
+// the end of the call the newest samples: one-block steps, whose level-0 fires
+// read a block before they write it (so a handle of one-level PCs, each the only
+// one of its input and its output, can run in place; larger levels read later).
 int run_steps(pc_handle* h, const IOView& view, long long nsteps, cudaStream_t st, bool again = false,
-              bool more = false) {
-    bool wide = h->wide_ok && (nsteps >= kWideMinSteps * h->KB || again || more);
+              bool more = false, bool in_place = false) {
+    bool wide = h->wide_ok && !in_place && (nsteps >= kWideMinSteps * h->KB || again || more);
     if (wide) {
         const int r = ensure_wide(h, nsteps, st, &wide);
         if (r) return r;
@@ -1476,6 +1480,11 @@ int run_steps(pc_handle* h, const IOView& view, long long nsteps, cudaStream_t s
         rs.io = view;
         for (long long done = 0; done < nsteps; done += h->KB) {
             rs.step_base = h->frame_num;
+            if (in_place) {   // (a step whose call begins with it does not look back into the call's input)
+                rs.io.step0 = h->frame_num;
+                rs.io.in = view.in + done * view.in_step;
+                rs.io.out = view.out + done * view.out_step;
+            }
             // the stream's work before the first step is not a step kernel
             int r = launch_step_direct(h, rs, st, done == 0);
             if (r) return r;
@@ -1537,7 +1546,7 @@ int process_device_impl(pc_handle* h, float* d_out, const float* d_in, long long
         target = h->d_rtmp;
     }
     IOView v = make_view(h, d_in, target, frames, layout, h->frame_num);
-    int r = run_steps(h, v, nsteps, st);
+    int r = run_steps(h, v, nsteps, st, false, false, overlap(d_in, frames * h->n_in, target, frames * h->n_out));
     if (r) return r;
     if (h->relaxed) {
         const long long os = v.out_sample, oc = v.out_ch;

@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 
 #include <cstddef>
+#include <cstdint>
 #include <string>
 #include <vector>
 
@@ -30,6 +31,11 @@ inline cudaError_t record_use(cudaEvent_t ev, cudaStream_t st) {
     cudaError_t e = cudaStreamIsCapturing(st, &cs);
     if (e == cudaSuccess && cs == cudaStreamCaptureStatusNone) e = cudaEventRecord(ev, st);
     return e;
+}
+// whether the na floats at a and the nb at b share any
+inline bool overlap(const float* a, long long na, const float* b, long long nb) {
+    const uintptr_t p = reinterpret_cast<uintptr_t>(a), q = reinterpret_cast<uintptr_t>(b);
+    return p < q + sizeof(float) * (uintptr_t)nb && q < p + sizeof(float) * (uintptr_t)na;
 }
 // the same tables from the twiddles on the device (about 5 us; their upload takes 60)
 cudaError_t launch_fft_tables(float2* tab, const float2* W, int wlog, cudaStream_t st);

@@ -1435,7 +1435,10 @@ int pcm_process_device(pcm_handle* h, float* d_out, const float* d_in, long long
         rs.io.out_ch = 1;
     }
     const long long nsteps = frames / h->N0;
-    bool wide = nsteps >= kWideMinSteps;
+    // in place: one-block steps read a block before they write it, each as a call
+    // of its own, which does not look back into its input as chunks do
+    const bool in_place = overlap(d_in, frames * h->nI, d_out, frames * h->nO);
+    bool wide = nsteps >= kWideMinSteps && !in_place;
     if (wide) {
         const int r = ensure_wide(h, nsteps, st, &wide);
         if (r) return r;
@@ -1446,6 +1449,11 @@ int pcm_process_device(pcm_handle* h, float* d_out, const float* d_in, long long
     } else {
         for (long long s = 0; s < nsteps; ++s) {
             rs.step_base = h->frame_num + s;
+            if (in_place) {
+                rs.io.step0 = rs.step_base;
+                rs.io.in = d_in + s * rs.io.in_step;
+                rs.io.out = d_out + s * rs.io.out_step;
+            }
             int r = mimo_step(h, rs, st, s == 0, nullptr);
             if (r) return r;
         }
