@@ -1103,10 +1103,13 @@ int mimo_wide(pcm_handle* h, const IOView& io, long long nsteps, cudaStream_t st
     for (int L = 0; L < h->M; ++L) {
         const MLevel& l = h->hbank.lv[L];
         const auto& cnt = h->state_cnt[L];
-        const int phi = (int)((h->frame_num + l.s_blocks) % l.T);   // slices built since the level's last block
-        const int n = cnt.size() < 2 ? 0 : cnt[l.T == 1 ? 1 : phi];
+        if (cnt.size() < 2) continue;
+        // slices since the level's last block, and those of them built before the call
+        const long long q = h->frame_num + l.s_blocks, q0 = io.step0 + l.s_blocks;
+        const int have = l.T > 1 && q / l.T == q0 / l.T ? cnt[q0 % l.T] : 0;
+        const int n = cnt[l.T == 1 ? 1 : q % l.T] - have;
         if (n <= 0) continue;
-        MCK(launch_mac(h, n, h->d_tasks + h->state_off[L], rs, st, true), "MIMO partial sums");
+        MCK(launch_mac(h, n, h->d_tasks + h->state_off[L] + have, rs, st, true), "MIMO partial sums");
         h->launches += 1;
     }
     return PC_OK;

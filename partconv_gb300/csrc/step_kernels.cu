@@ -1219,7 +1219,10 @@ cudaError_t launch_side_spreads(int grid, const Task* tasks, long long step, cud
 // End of a block-parallel call (wide.cu): the partial sums that the spread
 // tasks of the steps up to c1 - 1 would have built for the blocks in
 // progress, by the same code (one CTA per tile of bins and row; a tile whose
-// slices all come later has nothing to do), and, by ring_ctas CTAs per PC,
+// slices all come later has nothing to do, nor one whose slices the steps before
+// the call have built for the same block: a call of a few steps costs a few
+// slices: 128 streams of 64 | 256 | .. | 16384 in calls of ten steps 161 us with
+// all of them, 127 so), and, by ring_ctas CTAs per PC,
 // the call's newest samples (at most a ring's worth) in the input rings.
 // NT, LANES: as the handle's spread tasks.
 template <int NT, int LANES, bool MULTI>
@@ -1247,21 +1250,26 @@ __global__ void __launch_bounds__(NT) wide_state_kernel(const int4* __restrict__
     if (T > 1) {
         // bins of slice j of n start at (j cs / n) & ~1
         auto start = [&](long long j, int n) { return j >= n ? cs : (int)((j * cs / n) & ~1LL); };
-        const long long q = c1 + l.s_blocks;
-        const int phi = (int)(q & (T - 1));
-        bool need;
+        const long long q = c1 + l.s_blocks, q0 = a.io.step0 + l.s_blocks;   // after the call, before it
+        const bool same = q >> l.logT == q0 >> l.logT;   // the level's block in progress is still the one before the call
+        const int phi = (int)(q & (T - 1)), phi0 = (int)(q0 & (T - 1));
+        int lo = 0, hi;   // bins to build
         if (kb > 1) {   // slices since the step in which the level's previous block completed
             const long long bt = q >> l.logT, x = bt * T - l.s_blocks - 1;
             const long long sprev = x >= 0 ? x / kb : -((-x + kb - 1) / kb);
             const int n = T / kb;
-            const long long j = c1 / kb - 1 - sprev;
-            need = j > 0 && e.y < start(j, n);
+            const long long j = c1 / kb - 1 - sprev, j0 = a.io.step0 / kb - 1 - sprev;
+            if (same && j0 > 0) lo = start(j0, n);
+            hi = j > 0 ? start(j, n) : 0;
         } else if (l.dfer) {   // slice T - 1 at the previous fire's step, then 0, 1, ...
-            need = e.y < start(phi, T) || e.w > start(T - 1, T);
+            if (same) lo = start(phi0, T);
+            hi = start(phi, T);
         } else {
-            need = phi > 0 && e.y < start(phi, T - 1);
+            if (same && phi0 > 0) lo = start(phi0, T - 1);
+            hi = phi > 0 ? start(phi, T - 1) : 0;
         }
-        if (!need) return;
+        const bool last = kb == 1 && l.dfer && !same && e.w > start(T - 1, T);
+        if (!last && (e.y >= hi || e.w <= lo)) return;
     }
     if (threadIdx.x == 0) {
         Task t{};
