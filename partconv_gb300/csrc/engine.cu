@@ -39,8 +39,15 @@ constexpr int kWlog = 17;          // twiddle table 2^17 entries: real FFTs up t
 // Calls of at least this many steps run block-parallel (wide.cu): its eight
 // launches cost as much as about ten steps (block-parallel and one-block steps,
 // 256x14 | 2048x50, 4, 8 and 16 steps: one stream 37.5, 37.5, 38.4 and 29.3,
-// 40.3, 69.3 us; 32 streams 53.5, 56.5, 60.2 and 32.3, 45.2, 79.1 us).
+// 40.3, 69.3 us; 32 streams 53.5, 56.5, 60.2 and 32.3, 45.2, 79.1 us).  Levels
+// with about as many steps to a block or more cost a CTA per tile of bins in every
+// call, most of them idle, and are summed again as a whole when a block completes,
+// so handles with many of them begin later, a step per kWideStepTiles such tiles
+// (128 streams of 64 | 256 | 1024 | 4096 | 16384, 29 thousand tiles, 10, 16, 24 and
+// 32 steps: 127, 142, 158, 172 and 57, 92, 138, 183 us; 128 of 256 | 2048, 2800
+// tiles, 10 and 11 steps: 126, 127 and 116, 128 us).
 constexpr int kWideMinSteps = 10;
+constexpr int kWideStepTiles = 1500;
 // Base steps per block-parallel chunk: as many as keep the chunk's spectra
 // (one ring row per block of every level) within kWideBytes, so that they and
 // the summed spectra, as many again, are still in the 129 MB L2 when the next
@@ -223,6 +230,7 @@ struct pc_handle {
     // those up to 2048 by themselves)
     WMap w_fwd[3], w_inv[3], w_out, w_cl;
     int w_nt[3] = {};            // threads per CTA of w_fwd and w_inv
+    int w_min = 0;               // base steps from which a call runs block-parallel
     int w_split = 0;             // chunks of at least this many steps launch the block sizes apart
     const int4* wmac_map[2] = {};     // the sum over parts: default tiles, any
     std::vector<int> wmac_upto[2];
@@ -436,6 +444,10 @@ struct WideMaps {
             h->wmac_map[x] = entries(mac[x]);
             h->wmac_upto[x] = prefix(mac[x], h->C_max);
         }
+        int tiles = 0;   // of levels whose blocks take half as many steps as a short call has, or more
+        for (auto& l : h->h_lv)
+            if (2 * l.T > kWideMinSteps * h->KB) tiles += (l.cs + kMacTile - 1) / kMacTile;
+        h->w_min = h->KB * (kWideMinSteps + tiles / kWideStepTiles);
         h->w_part_map = reinterpret_cast<const int4*>(put(part.data(), sizeof(int4) * part.size()));
         h->w_part_n = (int)part.size();
         return err;
@@ -1470,7 +1482,7 @@ int finish_wide(pc_handle* h, const IOView& view, cudaStream_t st) {
 // one of its input and its output, can run in place; larger levels read later).
 int run_steps(pc_handle* h, const IOView& view, long long nsteps, cudaStream_t st, bool again = false,
               bool more = false, bool in_place = false) {
-    bool wide = h->wide_ok && !in_place && (nsteps >= kWideMinSteps * h->KB || again || more);
+    bool wide = h->wide_ok && !in_place && (nsteps >= h->w_min || again || more);
     if (wide) {
         const int r = ensure_wide(h, nsteps, st, &wide);
         if (r) return r;

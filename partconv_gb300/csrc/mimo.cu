@@ -68,12 +68,18 @@ constexpr int kTile = 32;          // bins per tile of Hw (a warp's lanes); a ro
                                    // and its padding, belong to the tile before them
 constexpr int kMaxMimoLevels = 8;
 constexpr int kMaxMacTerms = 2048;  // (input, part) terms one MAC task sums
-// block-parallel calls: from this many base steps on; base steps per chunk, as
-// many as keep the chunk's spectra within kWideBytes
-// (block-parallel and one-block steps, 128x16 | 2048xP, 4, 8 and 16 steps: 4 x 4
-// paths of 6001 taps 36, 41, 45 and 39, 70, 124 us; 32 x 32 of 2^15 taps 101,
-// 133, 141 and 64, 125, 231 us; at 12 steps 160 and 179)
+// block-parallel calls: from this many base steps on (small matrices would gain
+// from four: block-parallel and one-block steps, 128x16 | 2048xP, 4, 8 and 16
+// steps: 4 x 4 paths of 6001 taps 36, 41, 45 and 39, 70, 124 us; 32 x 32 of 2^15
+// taps 101, 133, 141 and 64, 125, 231 us).  A level whose blocks take more steps
+// than that is read twice in calls so short, once for the partial sums of the block
+// in progress and as a whole when it completes: a step later per kWideStepBytes of
+// its spectra (64 x 64 paths, 128x16 | 2048x15, 1 GB: 10, 14, 15 and 16 steps 389,
+// 446, 460, 434 and 292, 407, 434, 464 us; 32 x 32, 0.25 GB: 10, 11 and 12 steps
+// 152, 157, 155 and 139, 152, 165 us)
 constexpr int kWideMinSteps = 10;
+constexpr double kWideStepBytes = 165e6;
+// base steps per chunk: as many as keep the chunk's spectra within kWideBytes
 constexpr size_t kWideBytes = (size_t)64 << 20;
 constexpr int kWideMinChunk = 32, kWideMaxChunk = 4096;
 constexpr int kOB = 4;             // outputs a warp sums together
@@ -738,6 +744,7 @@ struct pcm_handle {
     // (output, level), CTA maps in order of their first block's step and the
     // prefix of each that a chunk of n + 1 steps needs
     int C_max = 32;   // most base steps per chunk
+    int w_min = kWideMinSteps;   // base steps from which a call runs block-parallel
     int C = 0;        // ... that the workspace in hand holds (0: none yet)
     char* work = nullptr;    // rings and sums of chunks of C steps (before: the rings among `allocs`)
     float4* hw = nullptr;    // the levels' Hw
@@ -1178,6 +1185,11 @@ int pcm_setup(pcm_handle* h, int fs, int buffer_size, int n_in, int n_out, int M
     }
     {
         const double row = sizeof(float2) * (double)buffer_size * M * std::max(n_in, n_out);   // per base step
+        double spectra = 0.0;
+        for (int L = 0; L < M; ++L)
+            if (Nv[L] / buffer_size > kWideMinSteps)
+                spectra += sizeof(float2) * (double)n_in * n_out * Pv[L] * (Nv[L] + 2);
+        h->w_min = kWideMinSteps + (int)(spectra / kWideStepBytes + 0.5);
         h->tiles.clear();
         h->work_failed = false;
         h->C = 0;
@@ -1441,7 +1453,7 @@ int pcm_process_device(pcm_handle* h, float* d_out, const float* d_in, long long
     // in place: one-block steps read a block before they write it, each as a call
     // of its own, which does not look back into its input as chunks do
     const bool in_place = overlap(d_in, frames * h->nI, d_out, frames * h->nO);
-    bool wide = nsteps >= kWideMinSteps && !in_place;
+    bool wide = nsteps >= h->w_min && !in_place;
     if (wide) {
         const int r = ensure_wide(h, nsteps, st, &wide);
         if (r) return r;
