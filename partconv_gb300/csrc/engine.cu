@@ -172,7 +172,8 @@ struct pc_handle {
     bool ready = false;
     int device = -1;
     cudaStream_t stream = nullptr;
-    cudaEvent_t used = nullptr;   // after the last call on a caller's stream
+    cudaEvent_t used = nullptr;   // after the last call on a caller's stream,
+    bool in_use = false;          // ... if there was one since the last reset
     cudaStream_t cin = nullptr, cout = nullptr;   // pc_process copy pipeline
 
     int fs = 0, N0 = 0, n_in = 0, n_out = 0;
@@ -183,6 +184,7 @@ struct pc_handle {
     char* arena = nullptr;
     size_t arena_bytes = 0;
     size_t state_off = 0, state_bytes = 0;   // zeroed by reset
+    size_t reset_bytes = 0;                  // ... and at most this much of each level's rings
 
     std::vector<DevPC> h_pcs;
     std::vector<DevLevel> h_lv;
@@ -1146,7 +1148,9 @@ int do_setup(pc_handle* h, int fs, int buffer_size, int n_in, int n_out, std::ve
         h->d_lv0 = reinterpret_cast<const int*>(A + off_lv0);
         h->d_wtab = reinterpret_cast<const float2*>(A + off_wtab);
         CK(wm.place(h, A + off_wmap), "upload maps");
-        CK(launch_wide_reset(h->d_wlv, nlv, A + h->state_off, h->state_bytes, h->stream), "clear state");
+        h->reset_bytes = 0;
+        for (auto& w : wl) h->reset_bytes = std::max(h->reset_bytes, wide_reset_bytes(w, N0));
+        CK(launch_wide_reset(h->d_wlv, nlv, h->reset_bytes, A + h->state_off, h->state_bytes, h->stream), "clear state");
     }
     // the level-0 class also runs spread tasks; its smem must fit its fires
     if (h->class_maxN[h->l0_class] == 0) h->class_maxN[h->l0_class] = N0;
@@ -1802,7 +1806,10 @@ int pc_process_device(pc_handle* h, float* d_output, const float* d_input, long 
                       void* stream) {
     if (!h) return PC_ERR_ARG;
     int r = process_device_impl(h, d_output, d_input, frames, layout, (cudaStream_t)stream);
-    if (r == PC_OK) CK(record_use(h->used, (cudaStream_t)stream), "event record");
+    if (r == PC_OK) {
+        CK(record_use(h->used, (cudaStream_t)stream), "event record");
+        h->in_use = true;
+    }
     return r;
 }
 
@@ -1812,8 +1819,10 @@ int pc_reset(pc_handle* h) {
     if (!h->ready) return PC_OK;
     h->work_failed = false;
     CK(cudaSetDevice(h->device), "cudaSetDevice");
-    CK(cudaStreamWaitEvent(h->stream, h->used, 0), "reset");   // calls still running on a caller's stream
-    CK(launch_wide_reset(h->d_wlv, (int)h->h_lv.size(), h->arena + h->state_off, h->state_bytes, h->stream), "reset");
+    if (h->in_use) CK(cudaStreamWaitEvent(h->stream, h->used, 0), "reset");   // calls still running on a caller's stream
+    h->in_use = false;
+    CK(launch_wide_reset(h->d_wlv, (int)h->h_lv.size(), h->reset_bytes, h->arena + h->state_off, h->state_bytes, h->stream),
+       "reset");
     CK(cudaStreamSynchronize(h->stream), "reset sync");
     return PC_OK;
 }

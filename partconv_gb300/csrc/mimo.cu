@@ -763,7 +763,7 @@ struct pcm_handle {
     // first task and tasks of the first j slices
     std::vector<int> state_off;
     std::vector<std::vector<int>> state_cnt;
-    size_t state_bytes_total = 0;
+    size_t reset_bytes = 0;   // most of a descriptor's rings that reset clears
     std::vector<std::pair<void*, size_t>> state;   // zeroed by reset
     long long frame_num = 0;
     long long launches = 0;
@@ -946,7 +946,9 @@ int setup_wide(pcm_handle* h) {
     h->d_wlv_of[1] = reinterpret_cast<WLevel*>(d + at[6]);
     h->d_wlv = h->d_wlv_of[0];
     h->d_lv0 = reinterpret_cast<const int*>(d + at[5]);
-    MCK(launch_wide_reset(h->d_wlv, h->n_wlv, nullptr, 0, h->stream), "clear rings");
+    h->reset_bytes = 0;
+    for (auto& w : wl) h->reset_bytes = std::max(h->reset_bytes, wide_reset_bytes(w, h->N0));
+    MCK(launch_wide_reset(h->d_wlv, h->n_wlv, h->reset_bytes, nullptr, 0, h->stream), "clear rings");
     return PC_OK;
 }
 
@@ -1486,7 +1488,7 @@ int pcm_reset(pcm_handle* h) {
     cudaSetDevice(h->device);
     MCK(cudaStreamWaitEvent(h->stream, h->used, 0), "reset");   // calls still running on a caller's stream
     for (auto& z : h->state) MCK(cudaMemsetAsync(z.first, 0, z.second, h->stream), "reset");
-    MCK(launch_wide_reset(h->d_wlv, h->n_wlv, nullptr, 0, h->stream), "reset");
+    MCK(launch_wide_reset(h->d_wlv, h->n_wlv, h->reset_bytes, nullptr, 0, h->stream), "reset");
     MCK(cudaStreamSynchronize(h->stream), "reset sync");
     return PC_OK;
 }

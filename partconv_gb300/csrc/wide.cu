@@ -769,13 +769,10 @@ __global__ void wide_reset_kernel(const WLevel* __restrict__ lv, int nlv, float4
     }
     const WLevel& l = lv[blockIdx.x];
     const long long b0 = blocks_before(l, 0);
-    const int n4 = l.cs >> 1;   // float4 per row (rows are 16-byte aligned)
-    int sl = wmod(b0, l.slots);
-    for (int p = 1; p < l.P; ++p) {
-        sl = sl == 0 ? l.slots - 1 : sl - 1;
-        float4* row = reinterpret_cast<float4*>(l.X + (size_t)sl * l.cs);
-        for (int i = t; i < n4; i += nt) row[i] = z;
-    }
+    const long long n4 = l.cs >> 1, ring = l.slots * n4;   // float4 per row (rows are 16-byte aligned) and ring
+    const long long first = wmod(b0 - (l.P - 1), l.slots) * n4;
+    float4* X = reinterpret_cast<float4*>(l.X);
+    for (long long i = t; i < (l.P - 1) * n4; i += nt) X[first + i < ring ? first + i : first + i - ring] = z;
     const int ny = (int)min((long long)l.rmask + 1, b0 << l.logN) >> 2;
     for (int i = t; i < ny; i += nt) reinterpret_cast<float4*>(l.yring)[i] = z;
 }
@@ -953,9 +950,10 @@ cudaError_t launch_wide_move(const WLevel* lv, const WLevel* to, int nlv, long l
     return cudaGetLastError();
 }
 
-cudaError_t launch_wide_reset(const WLevel* lv, int nlv, void* state, size_t bytes, cudaStream_t st) {
-    // about 16 KB per CTA for the region
-    const int gy = nlv > 512 ? 4 : 64;
+cudaError_t launch_wide_reset(const WLevel* lv, int nlv, size_t level_bytes, void* state, size_t bytes, cudaStream_t st) {
+    // gy CTAs for each level, 64 KB of the largest one for each (64 for each level:
+    // 32 us per reset of 64 streams of 64 | 512; so 15 us, an empty kernel being 10)
+    const int gy = (int)std::min<size_t>(std::max<size_t>(1, (level_bytes + 65535) >> 16), nlv > 512 ? 4 : 64);
     const int extra = (int)std::min<size_t>(64, bytes / ((size_t)gy << 14) + 1);
     wide_reset_kernel<<<dim3(nlv + extra, gy), 256, 0, st>>>(lv, nlv, static_cast<float4*>(state), bytes >> 4);
     return cudaGetLastError();

@@ -77,8 +77,12 @@ cudaError_t launch_wide_mac(bool any, int grid, const int4* map, const WArgs& a,
 // outputs fed by several PCs, and outputs without any
 cudaError_t launch_wide_mix(const Bank& bank, int n_zero, bool mixed, const WArgs& a, cudaStream_t st);
 // clears what a run from the start reads before it writes it: spectrum rows,
-// output rings, and the state region (16-byte aligned)
-cudaError_t launch_wide_reset(const WLevel* lv, int nlv, void* state, size_t bytes, cudaStream_t st);
+// output rings (at most level_bytes of each level), and the state region (16-byte
+// aligned)
+cudaError_t launch_wide_reset(const WLevel* lv, int nlv, size_t level_bytes, void* state, size_t bytes, cudaStream_t st);
+inline size_t wide_reset_bytes(const WLevel& l, int N0) {
+    return sizeof(float2) * (size_t)(l.P - 1) * l.cs + sizeof(float) * (size_t)l.s_blocks * N0;
+}
 // what the rings of lv hold for the steps from `step` on, to the rings of to
 cudaError_t launch_wide_move(const WLevel* lv, const WLevel* to, int nlv, long long step, int N0, cudaStream_t st);
 // class-3 levels (cluster_fire.cu)
