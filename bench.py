@@ -404,6 +404,8 @@ def run_ours(args):
     per_launch_b = dom["alg_bytes"] / dom["launches"]
     peak, peak_kind = measured_peak_gbs()
     achieved = per_launch_b / per_launch_s / 1e9
+    # what a pass cannot do without: input, output, and 8 bytes of spectra per tap
+    pass_bytes = 4.0 * 2 * S * frames1 + 8.0 * sum(len(h) for h in c["irs"])
     # captured per kernel kind and blocks per step (the K-block kernel is another instance)
     traffic = ncu_traffic().get(dom["name"] if K == 1 else f"{dom['name']}@K{K}")
     kernels = {r["name"]: {"launches": r["launches"], "avg_us": r["total_ms"] * 1e3 / r["launches"],
@@ -486,23 +488,32 @@ def run_ours(args):
                        "streams": S, "frames_per_stream": frames, "N0": N0,
                        "hyperperiod_steps": info.hyperperiod,
                        "l2": "256 MB buffer written between timed steps (outside the events); "
-                             "FDL state (%.0f MB) stays L2-resident within a step" % (info.device_bytes / 1e6),
+                             "a pass's input and output (264 MB at full size) exceed L2, and so do a chunk's spectra "
+                             "(device memory of the handle %.0f MB)" % (info.device_bytes / 1e6),
                        "parallelism": f"replicas x{ws}"},
             "e2e": {"value": e2e_v, "unit": "audio-s/s", "h2d_bytes_per_step": nbytes, "d2h_bytes_per_step": nbytes,
                     "how": "pc_process on pinned host buffers (planar), copies inside the timed region"},
             "gpu_launches": int(launches),
-            "roofline": {"bound": "hbm", "kernel": dom["name"], "achieved": achieved, "peak": peak, "unit": "GB/s",
-                         "limited_by": "latency: the level-0 kernel of one-block calls; the FDL state is L2-resident and "
-                                       "DRAM moves a few % of the algorithmic bytes (traffic below). The timed pass "
-                                       "runs block-parallel kernels, bound by issue slots and latency",
-                         "frac": achieved / peak, "peak_kind": peak_kind, "traffic": traffic,
-                         "alg_bytes_per_launch": per_launch_b, "avg_launch_us": per_launch_s * 1e6,
-                         "how": "CUDA events around single launches of one-block steps"},
+            "roofline": {"bound": "hbm", "kernel": "the timed pass (block-parallel: wide_fft, wide_mac, wide_ifft, "
+                                                   "wide_out, wide_state)",
+                         "achieved": pass_bytes / (ms / 1e3) / 1e9, "peak": peak, "unit": "GB/s",
+                         "frac": pass_bytes / (ms / 1e3) / 1e9 / peak, "peak_kind": peak_kind,
+                         "alg_bytes_per_pass": pass_bytes,
+                         "limited_by": "latency and issue: spectra of every block, in and out of three kernels, with "
+                                       "twelve to thirty-two warps per SM",
+                         "how": "input read, output written and every response's spectra read once, over the pass time"},
+            # the level-0 kernel of one-block calls (pc_run); the timed pass does not launch it
+            "one_block_kernel": {"kernel": dom["name"], "achieved_gbs": achieved, "frac_of_copy_rate": achieved / peak,
+                                 "limited_by": "latency: its state is L2-resident and DRAM moves a few % of the "
+                                               "algorithmic bytes (traffic)",
+                                 "traffic": traffic, "alg_bytes_per_launch": per_launch_b,
+                                 "avg_launch_us": per_launch_s * 1e6,
+                                 "how": "CUDA events around single launches of one-block steps"},
             "kernels": kernels,
             "path_alg_bytes_per_sample": bps,
-            # every block's own reads of filter and spectra, which a block-parallel pass shares between
-            # blocks: above 1 where that saves more than the pass is from the copy rate
-            "path_roofline_frac": (bps * S * frames1 / (ms / 1e3)) / 1e9 / peak,
+            # the rate a chain of one-block steps would need for this pass time (every block's own reads of
+            # filter and spectra, which the block-parallel kernels share between blocks) over the copy rate
+            "one_block_reads_over_copy_rate": (bps * S * frames1 / (ms / 1e3)) / 1e9 / peak,
             "block_latency_us": {"p50": float(np.percentile(lat_us, 50)), "p99": float(np.percentile(lat_us, 99)),
                                  "max": float(np.max(lat_us)), "deadline_us": B / FS * 1e6,
                                  "how": f"device time of one step ({K} base block{'s' if K > 1 else ''}, all "
@@ -591,20 +602,26 @@ def run_mimo(args):
     mac = [r for r in prof if r["name"] == "mimo_mac"][0]
     peak, peak_kind = measured_peak_gbs()
     ach = mac["alg_bytes"] / (mac["total_ms"] / 1e3) / 1e9
+    pass_bytes = 4.0 * frames * (n_in + n_out) + 8.0 * n_in * n_out * sum(p * (n + 2) for n, p in zip(m.N, m.P))
     line = {
         "metric": "audio-s/s (MIMO 64x64 per-bin channel sum)", "value": value, "unit": "audio-s/s",
         "n_gpus": 1, "steps": args.steps, "warmup": args.warmup, "ms_per_step": ms, "higher_is_better": True,
         "dtype": "f32", "data": "synthetic (seeded numpy PCG64, cfg seed 1003)",
         "config": {"workload": f"cfg3: {n_in}x{n_out} paths of {L} taps, {frames} frames, layout 128x16|2048x15",
                    "device_bytes": m.device_bytes(),
-                   "l2": "256 MB buffer written between timed steps (outside the events); the level-0 filter "
-                         "spectra (68 MB, read every base step) are loaded with an L2 evict-last policy, the "
-                         "level-1 spectra evict-first (the spectra, 1.07 GB, exceed L2)"},
+                   "l2": "256 MB buffer written between timed steps (outside the events); the spectra (1.07 GB) "
+                         "exceed L2"},
         "gpu_launches": int(launches),
-        "roofline": {"bound": "hbm", "kernel": "mimo_mac", "achieved": ach, "peak": peak, "unit": "GB/s",
-                     "frac": ach / peak, "peak_kind": peak_kind,
-                     "alg_bytes_per_launch": mac["alg_bytes"] / mac["launches"],
-                     "avg_launch_us": mac["total_ms"] * 1e3 / mac["launches"]},
+        # the filter spectra, input and output once, over the pass: the timed pass reads the spectra once
+        # per chunk and is bound by its float32 multiply-adds
+        "roofline": {"bound": "hbm", "kernel": "the timed pass (block-parallel: mimo_wide_mac and the wide transforms)",
+                     "achieved": pass_bytes / (ms / 1e3) / 1e9, "peak": peak, "unit": "GB/s",
+                     "frac": pass_bytes / (ms / 1e3) / 1e9 / peak, "peak_kind": peak_kind,
+                     "alg_bytes_per_pass": pass_bytes},
+        # one-block calls, which the timed pass does not make
+        "one_block_kernel": {"kernel": "mimo_mac", "achieved_gbs": ach, "frac_of_copy_rate": ach / peak,
+                             "alg_bytes_per_launch": mac["alg_bytes"] / mac["launches"],
+                             "avg_launch_us": mac["total_ms"] * 1e3 / mac["launches"]},
         "kernels": {r["name"]: {"launches": r["launches"], "avg_us": r["total_ms"] * 1e3 / r["launches"],
                                 "share": r["total_ms"] / sum(q["total_ms"] for q in prof)} for r in prof},
     }
@@ -689,7 +706,8 @@ def run_adjoint(args):
                       "unit": "audio-s/s", "n_gpus": 1, "steps": args.steps, "warmup": args.warmup,
                       "ms_per_step": ms, "higher_is_better": True, "dtype": "f32",
                       "data": "synthetic (seeded numpy PCG64, cfg seed 1004)",
-                      "config": {"workload": "cfg4: batch 8 x 2^18, IR 2^16 taps, layout 512x8|4096x15, MSE"},
+                      "config": {"workload": "cfg4: batch 8 x 2^18, IR 2^16 taps, layout 512x8|4096x15, MSE",
+                                 "execution": "one level of 4096-sample blocks, 16 parts, all blocks at once"},
                       "gpu_launches": launches,
                       "parity": {"dL_dh_rel_l2_vs_dense_fp64": rel(gh_ours, gh64),
                                  "dL_dx_rel_l2_vs_dense_fp64": rel(gx_ours, gx64),

@@ -125,7 +125,9 @@ int pc_set_relaxed(pc_handle* h, int relaxed);
  * Throughput option for calls of a few blocks, no reference counterpart:
  * compute k base blocks per step (k a power of two, 1..8; call before setup;
  * up to 4 are used).  Each step's level-0 work for all PCs is one launch that
- * transforms and convolves k consecutive blocks at once.
+ * transforms and convolves k consecutive blocks at once.  Calls of ten steps
+ * or more run block-parallel with or without it, and about a fifth slower with
+ * it (level 0 takes the general sum over parts).
  * The output equals that of k times as many one-block steps to float32
  * rounding (the same partitions and products, summed in another order).
  * Setup lowers k to the largest value the layouts allow (k buffer_size <=
@@ -143,15 +145,18 @@ int pc_set_step_blocks(pc_handle* h, int k);
  * bins (64, 128, 256 or 512) and spread_parts parts (1..64; a level
  * keeps one partial-sum row per group of spread_parts parts).  0 keeps the
  * default (128 bins, 16 parts).  Call before setup; results differ between
- * tile shapes only by float32 rounding (sums grouped differently).
+ * tile shapes only by float32 rounding (sums grouped differently).  The shape
+ * is chosen for callbacks and calls of a few blocks; long calls of a handle with
+ * another than the default shape take the general sum over parts, which is slower.
  */
 int pc_set_tiles(pc_handle* h, int spread_bins, int spread_parts);
 
 /*
  * PartConvMulti::run(output, input, frameCount) -- src/partconvMulti.h:60,
  * src/partconvMulti.cpp:815-928.  Host interleaved buffers of frame_count ==
- * buffer_size frames.  Copies the block to the device, runs one base step and
- * copies the mixed output back before returning.
+ * buffer_size frames.  Runs one base step and returns with its mixed output;
+ * the kernels read and write a pinned copy of the block, or copies on the device
+ * where the block has many channels or samples.
  */
 int pc_run(pc_handle* h, float* output, const float* input, int frame_count);
 
@@ -161,7 +166,10 @@ int pc_run(pc_handle* h, float* output, const float* input, int frame_count);
  * many pc_run calls.  Host buffers in the given layout (PC_INTERLEAVED or
  * PC_PLANAR with row length frames).  Calls of more than a few blocks run
  * block-parallel: whole chunks of callbacks per launch, bit for bit the
- * results of pc_run.
+ * results of pc_run.  The first such call allocates the handle's workspace for
+ * chunks of its length (up to some hundred MB for long chunks of many levels;
+ * pc_get_info counts it), a longer one replaces it; where the device has no room,
+ * shorter chunks or one-block steps serve.
  * No reference counterpart (the reference has only run()).
  */
 int pc_process(pc_handle* h, float* output, const float* input, long long frames, int layout);
@@ -169,7 +177,11 @@ int pc_process(pc_handle* h, float* output, const float* input, long long frames
 /*
  * Same as pc_process with device-resident buffers, enqueued on the caller's
  * stream (void* = cudaStream_t; NULL is the CUDA default stream, as in every
- * CUDA API).  Returns after enqueueing; the caller synchronises the stream.
+ * CUDA API).  Returns after enqueueing; the caller synchronises the stream.  A
+ * stream that is being captured takes the workspace as it is (one-block steps
+ * without one).  The buffers may be the same only if every PC has one level and
+ * is the only one of its input and its output, of the same index; such calls run
+ * one-block steps.
  */
 int pc_process_device(pc_handle* h, float* d_output, const float* d_input, long long frames,
                       int layout, void* stream);
@@ -315,7 +327,11 @@ int pcm_setup(pcm_handle* h, int fs, int buffer_size, int n_in, int n_out, int M
               const float* irs, int ir_len);
 
 /* frames (a multiple of buffer_size) of device input -> device output,
- * PC_INTERLEAVED or PC_PLANAR, enqueued on stream (NULL = default). */
+ * PC_INTERLEAVED or PC_PLANAR, enqueued on stream (NULL = default).  Calls of ten
+ * blocks or more (later for large matrices) run block-parallel; the first one
+ * makes a second copy of the filter spectra and a workspace as pc_process does.
+ * Their sums run in another order than those of one-block steps, so a result
+ * depends on how a signal is cut into calls to float32 rounding. */
 int pcm_process_device(pcm_handle* h, float* d_out, const float* d_in, long long frames, int layout,
                        void* stream);
 int pcm_reset(pcm_handle* h);
@@ -329,9 +345,12 @@ void pcm_destroy(pcm_handle* h);
 /* ---------------------------------------------------------------------------
  * Differentiable partitioned convolution (no reference counterpart: the
  * reference has no gradients).  y_s = (x_s * h)[0:T] for a batch of signals,
- * all blocks of a level computed in parallel, and hand-written adjoints:
- * dL/dx with conjugated filter spectra (anti-causal), dL/dh as a partitioned
- * cross-correlation of the input with dL/dy in the same layout.
+ * all blocks computed in parallel, and hand-written adjoints: dL/dx as the same
+ * convolution of dL/dy backwards in time, dL/dh as a partitioned
+ * cross-correlation of the input with dL/dy.  Nothing is gained here by a
+ * layout's small first blocks, so the layout is checked and its part counts
+ * reported, and the computation takes one level of blocks (256 .. 16384) with at
+ * most 16 parts where the response allows it.
  * ------------------------------------------------------------------------- */
 typedef struct pcd_plan pcd_plan;
 
@@ -381,7 +400,10 @@ int pcs_poll(pcs_handle* h, int* n_published);
 int pcs_is_live(const pcs_handle* h, int pc_id);
 int pcs_release(pcs_handle* h, int pc_id);
 /* One step: host in/out [n_channels][buffer_size] (pinned for asynchrony);
- * returns after enqueueing; pcs_query / pcs_sync observe completion. */
+ * returns after enqueueing; pcs_query / pcs_sync observe completion.  Pinned
+ * buffers that do not overlap and hold exactly the pool's channels (up to the
+ * largest live id) are used by the kernels in place, others are copied; channels
+ * without a live PC give zeros. */
 int pcs_step(pcs_handle* h, const float* in, float* out, int n_channels);
 int pcs_query(pcs_handle* h);
 int pcs_sync(pcs_handle* h);

@@ -2,9 +2,10 @@
 
 ``PartitionedConvFunction`` is a ``torch.autograd.Function`` whose forward
 and backward are the hand-written CUDA kernels of the pcd_* C ABI: the
-forward pass is the FDL over all blocks of every level, dL/dx uses the
-conjugated filter spectra anti-causally, and dL/dh is a partitioned
-cross-correlation of the input with dL/dy in the same level layout.
+forward pass is the FDL over all blocks at once, dL/dx the same convolution of
+dL/dy backwards in time, and dL/dh a partitioned cross-correlation of the input
+with dL/dy.  The layout is checked and its part counts reported; the computation
+takes one level of larger blocks, for which small first ones gain nothing.
 ``PartitionedConv`` is a module holding a learnable impulse response.
 """
 from __future__ import annotations

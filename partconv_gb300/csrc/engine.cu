@@ -49,9 +49,10 @@ constexpr int kWlog = 17;          // twiddle table 2^17 entries: real FFTs up t
 constexpr int kWideMinSteps = 10;
 constexpr int kWideStepTiles = 1500;
 // Base steps per block-parallel chunk: as many as keep the chunk's spectra
-// (one ring row per block of every level) within kWideBytes, so that they and
-// the summed spectra, as many again, are still in the 129 MB L2 when the next
-// kernel reads them.
+// (one ring row per block of every level) within kWideBytes.  Beyond about 64 MB
+// they and the summed spectra, as many again, leave the 129 MB L2 before the next
+// kernel reads them, but the launches' fixed costs and last waves count for more
+// (32 streams of 2^18 samples, chunks of 128, 256 and 512 MB: 518, 456 and 460 us).
 constexpr size_t kWideBytes = (size_t)256 << 20;
 // Interleaved input is brought to rows of one channel each from this many
 // inputs on and for this many samples of a chunk: the pass costs 3 to 8 us and

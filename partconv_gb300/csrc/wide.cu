@@ -391,12 +391,14 @@ __device__ __forceinline__ void mac_finish(const f32x2* x, const float2* h, bool
 // segment's spectra with the P - 1 before them (up to 14 parts all 32, then 24)
 // are all on their way before the first run is waited for; with more, every run
 // takes the parts a partial-sum row at a time.
-// Bound: issue slots; half of the instructions are the packed products.  32
-// streams of 2^18 samples (14 | 14 | 1 .. 31 parts, 300 M products, 201 MB of
-// spectra in and out): 154 us with rows in a ring of shared memory walked with
-// wrapped offsets and the first two parts one float at a time, 136 us with
-// constant offsets and packed ends.  Four CTAs per SM with 152 registers a
-// thread beat five with 128 (424 against 432 us for the call).
+// Bound: latency, with twelve warps per SM: instructions are issued in 53 % of the
+// cycles (stalls per issue: wait 1.6, long scoreboard 0.9), 41 % of them for the
+// packed products (their pipe 45 % busy).  32 streams of 2^18 samples (14 | 14 |
+// 1 .. 31 parts, 300 M products, 201 MB of spectra in and out): 154 us with rows
+// in a ring of shared memory walked with wrapped offsets and the first two parts
+// one float at a time, 136 us with constant offsets and packed ends; serialised
+// 148 us first part to last, 142 us last to first.  Four CTAs per SM with 152
+// registers a thread beat five with 128 (424 against 432 us for the call).
 __global__ void __launch_bounds__(kMacTile, 4) wide_mac_kernel(const int4* __restrict__ map, WArgs a) {
     constexpr int RB = kWideRun, W = kMacTile;
     extern __shared__ float4 dyn_smem[];

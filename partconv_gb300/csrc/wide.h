@@ -50,7 +50,7 @@ __host__ __device__ __forceinline__ T* wide_at(T* p, long long rel) {
 }
 
 constexpr int kWideRun = 8;       // consecutive blocks a thread of the sum over parts takes together
-constexpr int kMacTile = 96;      // bins per CTA of the sum over parts (three warps: 258 bins are three tiles of 86)
+constexpr int kMacTile = 96;      // bins per CTA of the sum over parts (three warps: 258 bins are tiles of 96, 96 and 66)
 constexpr int kMacSeg = 32;       // ... and blocks
 constexpr int kMacRes = 18;       // most parts whose filter rows stay in shared memory (16 of a partial-sum row and 2)
 constexpr int kMacRows = 59;      // shared rows of a tile (45 KB; registers admit four CTAs per SM)
