@@ -253,7 +253,8 @@ struct pc_handle {
     // arena hold what one-block steps need.
     char* work = nullptr;
     size_t work_bytes = 0;
-    bool work_failed = false;      // no room for the smallest one: one-block steps until reset
+    bool work_failed = false;      // no room for the size last asked for: not tried again until reset
+    bool work_kept = false;        // a graph uses it: no larger one replaces it
     std::vector<WLevel> h_wlv;
     WLevel* d_wlv_of[2] = {};      // d_wlv and the other buffer of it
     int n_tasks = 0;
@@ -303,7 +304,7 @@ void free_device(pc_handle* h) {
     if (h->work) cudaFree(h->work);
     h->work = nullptr;
     h->work_bytes = 0;
-    h->work_failed = false;
+    h->work_failed = h->work_kept = false;
     h->C = 0;
     h->d_planar = nullptr;
     if (h->d_big_in) cudaFree(h->d_big_in);
@@ -1400,16 +1401,18 @@ int move_to_work(pc_handle* h, int C, cudaStream_t st) {
 // workspace is made for it, in chunks as short as the call, and grows with
 // longer calls up to h->C_max steps; where there is no room for the longest
 // chunk a shorter one serves, and for none one-block steps do.  A stream that is
-// being captured takes the workspace as it is.  Results are the same either way.
+// being captured takes the workspace as it is, and that one then stays, for the
+// graph's launches hold its addresses (those of one-block steps read the task
+// table).  Results are the same either way.
 int ensure_wide(pc_handle* h, long long nsteps, cudaStream_t st, bool* wide) {
     int want = kWideMinChunk;
     while (want < nsteps && want < h->C_max) want <<= 1;
     want = std::min(want, h->C_max);
     *wide = h->C > 0;
-    if (h->C >= want || h->work_failed) return PC_OK;
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     CK(cudaStreamIsCapturing(st, &cs), "capture status");
-    if (cs != cudaStreamCaptureStatusNone) return PC_OK;
+    if (cs != cudaStreamCaptureStatusNone) h->work_kept = *wide;
+    if (h->C >= want || h->work_failed || h->work_kept || cs != cudaStreamCaptureStatusNone) return PC_OK;
     for (; want > h->C && want >= kWideMinChunk; want >>= 1) {
         const int r = move_to_work(h, want, st);
         if (r == PC_OK) {

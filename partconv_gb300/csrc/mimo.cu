@@ -749,7 +749,8 @@ struct pcm_handle {
     char* work = nullptr;    // rings and sums of chunks of C steps (before: the rings among `allocs`)
     float4* hw = nullptr;    // the levels' Hw
     size_t work_bytes = 0, hw_bytes = 0;
-    bool work_failed = false;   // no room for the smallest: one-block steps until reset
+    bool work_failed = false;   // no room for the size last asked for: not tried again until reset
+    bool work_kept = false;     // a graph uses it: no larger one replaces it
     std::vector<WLevel> h_wlv;
     WLevel* d_wlv_of[2] = {};   // d_wlv and the other buffer of it
     const float2* d_tab = nullptr;
@@ -811,6 +812,7 @@ void mfree(pcm_handle* h) {
     h->work = nullptr;
     h->hw = nullptr;
     h->work_bytes = h->hw_bytes = 0;
+    h->work_kept = false;
     h->C = 0;
     if (h->used) cudaEventDestroy(h->used);
     h->used = nullptr;
@@ -964,7 +966,8 @@ long ring_samples(const MLevel& l, int N0, int C) {
 // holding what the present ones do, and Hw if there is none yet.  PC_ERR_NOMEM if
 // there is no room: everything stays as it is.
 int move_to_work(pcm_handle* h, int C, cudaStream_t st) {
-    MBank B = h->hbank;
+    const MBank old = h->hbank;
+    MBank& B = h->hbank;   // (what is uploaded outlives the call; old again on failure)
     const int nI = h->nI, nO = h->nO;
     size_t bytes = 0, hw_elems = 0;
     auto take = [&](size_t n) {
@@ -979,7 +982,10 @@ int move_to_work(pcm_handle* h, int C, cudaStream_t st) {
         l.slots = ring_rows(l, C);
         const long R = ring_samples(l, h->N0, C);
         l.rmask = (int)R - 1;
-        if ((long long)nI * l.slots * l.cs >= (1LL << 31)) return PC_ERR_NOMEM;   // 32-bit offsets
+        if ((long long)nI * l.slots * l.cs >= (1LL << 31)) {   // 32-bit offsets
+            h->hbank = old;
+            return PC_ERR_NOMEM;
+        }
         oX[L] = take(sizeof(float2) * (size_t)nI * l.slots * l.cs);
         oY[L] = take(sizeof(float2) * (size_t)nO * l.nbw * l.cs);
         oR[L] = take(sizeof(float) * (size_t)nO * R);
@@ -997,6 +1003,7 @@ int move_to_work(pcm_handle* h, int C, cudaStream_t st) {
         cudaGetLastError();
         if (W) cudaFree(W);
         cudaThreadExchangeStreamCaptureMode(&mode);
+        h->hbank = old;
         return PC_ERR_NOMEM;
     }
     for (int L = 0; L < h->M; ++L) {
@@ -1035,6 +1042,7 @@ int move_to_work(pcm_handle* h, int C, cudaStream_t st) {
         if (e != cudaSuccess && !h->hw) cudaFree(hw);
     }
     cudaThreadExchangeStreamCaptureMode(&mode);
+    if (e != cudaSuccess) h->hbank = old;
     MCK(e, "block-parallel workspace");
     h->launches += 1 + (h->hw ? 0 : h->M);
     h->work = W;
@@ -1044,7 +1052,6 @@ int move_to_work(pcm_handle* h, int C, cudaStream_t st) {
         h->hw_bytes = sizeof(float4) * hw_elems;
     }
     h->C = C;
-    h->hbank = B;
     h->h_wlv.swap(wl);
     h->d_wlv = next;
     return PC_OK;
@@ -1053,15 +1060,16 @@ int move_to_work(pcm_handle* h, int C, cudaStream_t st) {
 // Whether a call of nsteps base steps on st can run block-parallel: the workspace
 // is made for it, in chunks as short as the call, and grows with longer calls up
 // to h->C_max steps; where there is no room, a shorter chunk or one-block steps
-// serve.  A stream that is being captured takes the workspace as it is.
+// serve.  A stream that is being captured takes the workspace as it is, and that
+// one then stays, for the graph's launches hold its addresses.
 int ensure_wide(pcm_handle* h, long long nsteps, cudaStream_t st, bool* wide) {
     int want = kWideMinChunk;
     while (want < nsteps && want < h->C_max) want <<= 1;
     *wide = h->C > 0;
-    if (h->C >= want || h->work_failed) return PC_OK;
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     MCK(cudaStreamIsCapturing(st, &cs), "capture status");
-    if (cs != cudaStreamCaptureStatusNone) return PC_OK;
+    if (cs != cudaStreamCaptureStatusNone) h->work_kept = *wide;
+    if (h->C >= want || h->work_failed || h->work_kept || cs != cudaStreamCaptureStatusNone) return PC_OK;
     for (; want > h->C && want >= kWideMinChunk; want >>= 1) {
         const int r = move_to_work(h, want, st);
         if (r == PC_OK) {

@@ -96,6 +96,35 @@ def test_first_long_call_while_its_stream_is_captured(gpu):
         assert wl.rel_l2(yd[o].cpu().numpy(), ref[o]) <= 1e-5
 
 
+def test_a_captured_workspace_stays(gpu):
+    import torch
+
+    rng = np.random.default_rng(14)
+    irs = _irs(rng, 3, 3, 3000)
+    blocks = 40
+    x = torch.from_numpy((0.1 * rng.standard_normal((3, blocks * 64))).astype(np.float32)).cuda()
+    long = x.repeat(1, 10)
+    m = _handle(irs, [64, 256], [6, 0])
+    y, z = torch.zeros_like(x), torch.zeros_like(long)
+    m.process_device(y, x, blocks * 64, PC_PLANAR)
+    torch.cuda.synchronize()
+    want, held = y.clone(), m.device_bytes()
+    m.reset()
+    y.zero_()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        m.process_device(y, x, blocks * 64, PC_PLANAR)
+    m.reset()
+    m.process_device(z, long, 10 * blocks * 64, PC_PLANAR)
+    m.reset()
+    g.replay()
+    torch.cuda.synchronize()
+    assert m.device_bytes() == held and torch.equal(y, want)
+    ref = _ref(irs, long.cpu().numpy())
+    for o in range(3):
+        assert wl.rel_l2(z[o].cpu().numpy(), ref[o]) <= 1e-5
+
+
 @pytest.mark.parametrize("left_mb", [700, 200])
 def test_no_room_for_the_workspace(gpu, left_mb):
     """16 x 16 paths of 2^17 taps at 1024-sample blocks: 269 MB of spectra, twice.

@@ -121,6 +121,40 @@ def test_first_long_call_while_its_stream_is_captured(gpu):
     assert _bytes(m) > before and np.array_equal(y.cpu().numpy(), want)
 
 
+def test_a_captured_workspace_stays(gpu):
+    """A graph of a block-parallel call holds the workspace's addresses: longer
+    calls afterwards run in its chunks, and the graph still gives the call."""
+    import torch
+
+    rng = np.random.default_rng(14)
+    N0, blocks = 128, 40
+    pcs = [dict(ir=wl.decaying_ir(rng, 9000, 0.3), N=[128, 1024], P=[14, 0])]
+    x = torch.from_numpy((0.1 * rng.standard_normal((20 * blocks * N0, 1))).astype(np.float32)).cuda()
+    m = _setup(pcs, N0)
+    y, z = torch.zeros(blocks * N0, 1, device="cuda"), torch.zeros_like(x)
+    m.process_device(y, x, blocks * N0)
+    torch.cuda.synchronize()
+    want, held = y.clone(), _bytes(m)
+    m.reset()
+    y.zero_()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        m.process_device(y, x, blocks * N0)
+    m.reset()
+    m.process_device(z, x, len(x))          # twenty times as long
+    torch.cuda.synchronize()
+    assert _bytes(m) == held and torch.equal(z[:blocks * N0], want)
+    m.reset()
+    g.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(y, want)
+    n = _setup(pcs, N0)
+    w = torch.zeros_like(x)
+    n.process_device(w, x, len(x))
+    torch.cuda.synchronize()
+    assert _bytes(n) > held and torch.equal(w, z)
+
+
 @pytest.mark.parametrize("left_mb", [330, 160])
 def test_no_room_for_the_workspace(gpu, left_mb):
     """32 streams of 8192-sample blocks: a chunk of 64 steps takes about 420 MB, of
